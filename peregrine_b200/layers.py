@@ -64,6 +64,8 @@ class Device:
         t = self._buffers.get(key)
         if t is None or t.shape[0] < rows:
             t = self._buffers[key] = self.torch.zeros(rows, cols, dtype=dtype, device=self.dev)
+            # torch clears the memory on a stream of its own; the kernels and copies that use it next are on the context's
+            self.torch.cuda.current_stream(self.dev).synchronize()
         return t
 
     def rotation(self, base: float, dims: int, positions: int):

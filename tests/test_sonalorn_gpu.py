@@ -215,6 +215,19 @@ DELTAS = [t.delta(4, 2, 24, 40, 4), t.delta(2, 2, 128, 128, 2), t.delta(4, 1, 17
           t.delta(3, 1, 256, 16, 2), t.delta(2, 1, 96, 100, 3)]
 
 
+def test_first_batch_of_a_device_outlives_the_clearing_of_its_buffer(lm):
+    """The batch's arrays are made by torch on its stream and filled on the context's: torch's clearing, held up by other work,
+    must not come behind the first upload."""
+    from peregrine_b200.layers import Batch
+
+    d = device(lm, "bfloat16")
+    d.torch.cuda._sleep(200_000_000)       # keeps torch's stream busy for a tenth of a second
+    b = Batch(d, [(2, 5, [7, 8, 9])])
+    lm.sync()
+    d.torch.cuda.synchronize()
+    assert b.mem.flatten().cpu().tolist()[:12] == [7, 8, 9, 5, 6, 7, 0, 0, 0, 0, 3, 2]
+
+
 def run_mixer(lm, d, mixer, width, x, cuts, slot=1, between=None):
     """x [T, width] in portions -> [T, width] outputs; `between` is called before every portion."""
     from peregrine_b200.layers import Batch, up
