@@ -15,9 +15,11 @@ PG_API int32_t pg_linear_wrap(pg_ctx *ctx, const void *d_w_bf16, int64_t n, int6
     PG_REQUIRE(k % 64 == 0 && ((uintptr_t)d_w_bf16 & 15) == 0, "linear_wrap: K must be a multiple of 64 (K = %lld) and the weights 16-byte aligned",
                (long long)k);
     PG_REQUIRE(n < (1 << 30) && k < (1 << 30), "linear_wrap: shape too large");
-    // now, since the workspace cannot grow while a step is being recorded
+    // now, since the workspaces cannot grow while a step is being recorded
     const int32_t rc = pg_splitk_reserve(ctx, std::max(pgk_linear_gemv_workspace(n, k), PG_LM_TICKET_BYTES + (size_t)ctx->sm_count * 128 * 128 * sizeof(float)));
     if (rc != PG_OK) return rc;
+    const int32_t rs = pg_scratch_reserve(ctx, pgk_linear_f32_workspace(k));
+    if (rs != PG_OK) return rs;
     pg_linear *l = new (std::nothrow) pg_linear();
     if (!l) PG_FAIL(PG_ERR_NOMEM, "out of host memory");
     l->w = (const bf16 *)d_w_bf16;
@@ -75,17 +77,17 @@ PG_API int32_t pg_linear_run_routed(pg_ctx *ctx, pg_linear *lin, pg_route *route
     const int64_t pairs = route->m * route->top;
     const int64_t rows = pg_up(pairs + (pairs < route->experts ? pairs : route->experts) * (PG_ROUTE_BLOCK - 1), PG_ROUTE_BLOCK);
     PG_REQUIRE(rows <= route->max_rows, "linear: the route is larger than it was created for");
+    if (dtype == PG_F32) return pgk_linear_f32(ctx, lin, (const float *)d_a, lin->k, rows, act, limit, d_y, y_dtype, ldy, &rt);
     const void *a = d_a;
     if (by_token) {
         // the tokens' rows in the order of the route
-        const size_t row_bytes = (size_t)lin->k * (dtype == PG_F32 ? 4 : 2);
+        const size_t row_bytes = (size_t)lin->k * 2;
         const int32_t rr = pg_scratch_reserve(ctx, (size_t)rows * row_bytes);
         if (rr != PG_OK) return rr;
         const int32_t rc = pgk_route_gather(ctx, route, d_a, row_bytes, ctx->scratch);
         if (rc != PG_OK) return rc;
         a = ctx->scratch;
     }
-    if (dtype == PG_F32) return pgk_linear_f32(ctx, lin, (const float *)a, lin->k, rows, act, limit, d_y, y_dtype, ldy, &rt);
     return pgk_linear_tc(ctx, lin, (const bf16 *)a, lin->k, rows, act, limit, d_y, y_dtype, ldy, &rt);
 }
 

@@ -1,87 +1,397 @@
-// y = a W^T in true f32: bf16 weights widened exactly, FFMA sums.  64 x 64 tiles, 4 x 4 outputs per thread; the tile
-// edges are masked on load and store.  Also the routed form (a row block of 128 has one expert).
+// y = a W^T in f32 accuracy on the 5th-generation tensor cores: bf16 weights as they are, f32 activations as three bf16 pieces.
+//
+//   * a = a1 + a2 + a3 with each piece the next eight significant bits (cut off, not rounded): exact, and so is every product
+//     with a bf16 weight.  `linear_split_kernel` writes the pieces as three planes (routed rows in the order of the route).
+//   * D[n][m] = W (128 rows) x A^T (MT rows of a, all three planes): weights are the M side of the instruction, so that a lane of
+//     the epilogue owns a column of y and 32 lanes store 128 contiguous bytes of a row.
+//   * the sums: tcgen05's f32 accumulator cuts off what falls below its last bit, always towards zero, and a chain over a whole K
+//     would add that up.  An accumulator therefore only lives for one block of 64 k (smallest pieces first); four warps add the
+//     blocks in registers, rounded, while the next block's products run in the other accumulator.  MT = 128: twelve products of 64
+//     cycles a block, against about 300 cycles for the 128 additions per lane.
+//   * few tiles: K is divided over CTAs with slabs and tickets, as in linear_tc_kernel.
+//
+// What bounds it: the tensor cores at three products for each of the bf16 form's, from about 64 rows; the stream of W below.
+// Every mbarrier wait is bounded (pg_async.cuh).
+#include <algorithm>
+
+#include "pg_async.cuh"
 #include "pg_lm.cuh"
+#include "pg_tcgen05.cuh"
 
 namespace {
 
-constexpr int FM = 64, FN = 64, FK = 16;
+constexpr int FN = 128;                // columns of y (rows of W) per tile
+constexpr int FK = 64;                 // elements of K per stage = one 128-byte swizzle span
+constexpr int F_THREADS = 192;
+constexpr int F_ROWS = 128;            // rows for which the planes always find room (pg_linear_wrap)
 
-template <int ACT, typename TY>
+template <int MT>
+struct FCfg {
+    static constexpr int STAGE_W = FN * FK * 2;
+    static constexpr int PLANE = MT * FK * 2;
+    static constexpr int STAGE = STAGE_W + 3 * PLANE;
+    static constexpr int ROOM = 232448 - (1024 + 256);
+    static constexpr int STAGES = ROOM / STAGE > 10 ? 10 : ROOM / STAGE;
+    static constexpr int ACC = MT < 32 ? 32 : MT;          // TMEM columns of an accumulator
+    static constexpr size_t SMEM = (size_t)STAGES * STAGE + 1024 + 256;
+};
+
+struct FParts {
+    int parts, blocks;       // K in `parts` parts of `blocks` 64-element blocks
+    float *slabs;            // [unit][MT][128]
+    unsigned int *tickets;   // one per (tile, quarter), zero between calls
+};
+
+// ---- the three planes of rows row0 .. of a: planes [3][rows][K] --------------------------------------------------------
+// rt.row_pair (by token): row r takes token row_pair[r] / top, zeros where it is -1; rows behind the route's blocks are left out
 __global__ void __launch_bounds__(256)
-    linear_f32_kernel(const float *__restrict__ a, int64_t lda, const bf16 *__restrict__ w, int M, int N, int K, float limit, TY *__restrict__ y, int64_t ldy,
-                      const PgRouted rt)
+    linear_split_kernel(const float *__restrict__ a, int64_t lda, int row0, int rows, int K, const PgRouted rt, uint2 *__restrict__ planes)
 {
-    __shared__ float sa[FK][FM + 4];
-    __shared__ float sw[FK][FN + 4];
     pg_pdl_begin();
-    const int m0 = blockIdx.x * FM, n0 = blockIdx.y * FN;
-    if (rt.blocks) {
-        if (m0 >= __ldcg(rt.blocks) * PG_ROUTE_BLOCK) return;
-        w += (int64_t)__ldcg(rt.block_expert + m0 / PG_ROUTE_BLOCK) * N * K;
-    }
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int lr = threadIdx.x >> 2, lk = (threadIdx.x & 3) * 4;   // one row, four k per thread and tile
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += FK) {
-        float4 va = make_float4(0.f, 0.f, 0.f, 0.f);
-        uint2 vw = make_uint2(0u, 0u);
-        if (m0 + lr < M) va = __ldcg(reinterpret_cast<const float4 *>(a + (m0 + lr) * lda + k0 + lk));
-        if (n0 + lr < N) vw = __ldg(reinterpret_cast<const uint2 *>(w + (int64_t)(n0 + lr) * K + k0 + lk));
-        __syncthreads();
-        sa[lk][lr] = va.x, sa[lk + 1][lr] = va.y, sa[lk + 2][lr] = va.z, sa[lk + 3][lr] = va.w;
-        sw[lk][lr] = pg_bf16_lo(vw.x), sw[lk + 1][lr] = pg_bf16_hi(vw.x), sw[lk + 2][lr] = pg_bf16_lo(vw.y), sw[lk + 3][lr] = pg_bf16_hi(vw.y);
-        __syncthreads();
-        float sub[4][4] = {};                              // sums of 16 terms meet in acc: shorter chains, smaller error
-#pragma unroll
-        for (int k = 0; k < FK; k++) {
-            float x[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) x[i] = sa[k][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = sw[k][ACT == PG_ACT_NONE ? tx * 4 + j : (tx >> 2) * 16 + (tx & 3) * 2 + (j & 1) + (j >> 1) * 8];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) sub[i][j] = fmaf(x[i], b[j], sub[i][j]);
+    const int quads = K / 4;
+    const int limit = rt.blocks ? min(rows, __ldcg(rt.blocks) * PG_ROUTE_BLOCK - row0) : rows;
+    const int64_t plane = (int64_t)rows * quads;
+    for (int r = blockIdx.y; r < limit; r += gridDim.y) {
+        int64_t src = row0 + r;
+        if (rt.blocks && rt.by_token) {
+            const int pair = __ldcg(rt.row_pair + row0 + r);
+            src = pair < 0 ? -1 : pair / rt.top;
         }
+        for (int c = blockIdx.x * 256 + threadIdx.x; c < quads; c += gridDim.x * 256) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (src >= 0) v = __ldcg(reinterpret_cast<const float4 *>(a + src * lda) + c);
+            const float x[4] = {v.x, v.y, v.z, v.w};
+            uint32_t p[3][4];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) acc[i][j] += sub[i][j];
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= M) continue;
-        if (ACT == PG_ACT_NONE) {
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-                if (n0 + tx * 4 + j < N) pg_put(y + m * ldy + n0 + tx * 4 + j, acc[i][j]);
-        } else {
-            // this thread's columns: two gates and, eight rows of W further, their ups
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-                const int n = n0 / 2 + (tx >> 2) * 8 + (tx & 3) * 2 + j;
-                if (n < N / 2) pg_put(y + m * ldy + n, pg_glu<ACT>(acc[i][j], acc[i][j + 2], limit));
+            for (int i = 0; i < 4; i++) {
+                const uint32_t bits = __float_as_uint(x[i]);
+                const bool finite = (bits & 0x7f800000u) != 0x7f800000u;
+                p[0][i] = finite || (bits & 0x007fffffu) == 0 ? bits & 0xffff0000u : bits | 0x00400000u;   // (a NaN stays one)
+                const float r1 = finite ? x[i] - __uint_as_float(p[0][i]) : 0.0f;
+                p[1][i] = __float_as_uint(r1) & 0xffff0000u;
+                p[2][i] = __float_as_uint(r1 - __uint_as_float(p[1][i]));
             }
+#pragma unroll
+            for (int l = 0; l < 3; l++)
+                planes[l * plane + (int64_t)r * quads + c] = make_uint2(__byte_perm(p[l][0], p[l][1], 0x7632), __byte_perm(p[l][2], p[l][3], 0x7632));
         }
     }
 }
 
+template <int MT, int ACT>
+__global__ void __launch_bounds__(F_THREADS, 1)
+    linear_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, int M, int N, int K, float limit,
+                      float *__restrict__ y, int64_t ldy, const PgRouted rt, int block0, const FParts kp, int32_t *status, unsigned long long limit_ns)
+{
+    using C = FCfg<MT>;
+    constexpr int STAGES = C::STAGES;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw_addr = pg_smem(smem_raw);
+    const uint32_t base = (raw_addr + 1023u) & ~1023u;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw + (base - raw_addr) + (size_t)STAGES * C::STAGE);
+    const uint32_t bar_full = pg_smem(bars);
+    const uint32_t bar_empty = bar_full + 8 * STAGES;
+    const uint32_t bar_tfull = bar_empty + 8 * STAGES;
+    const uint32_t bar_tempty = bar_tfull + 16;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; s++) {
+            pg_mbar_init(bar_full + 8 * s, 1);
+            pg_mbar_init(bar_empty + 8 * s, 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            pg_mbar_init(bar_tfull + 8 * i, 1);
+            pg_mbar_init(bar_tempty + 8 * i, 4);   // one arrival per epilogue warp
+        }
+        *abort_flag = 0;
+        pg_mbar_fence();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pg_smem(tmem_slot)), "r"(2 * C::ACC) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const bool routed = rt.blocks != nullptr;
+    if (routed) asm volatile("griddepcontrol.wait;" ::: "memory");   // the list of tiles comes from the preceding kernels
+    constexpr int PER_BLOCK = PG_ROUTE_BLOCK / MT < 1 ? 1 : PG_ROUTE_BLOCK / MT;
+    const int tiles_m = routed ? max(0, min(__ldcg(rt.blocks) - block0, M / PG_ROUTE_BLOCK)) * PER_BLOCK : (M + MT - 1) / MT;
+    const int tiles_n = (N + FN - 1) / FN;
+    const int sp = kp.parts, total = tiles_m * tiles_n * sp;   // unit u: part u % sp of tile u / sp
+    const int kblocks = K / FK;
+    auto k_first = [&](int u) { return (u % sp) * kp.blocks; };
+    auto k_end = [&](int u) { return min(kblocks, (u % sp + 1) * kp.blocks); };
+
+    if (warp == 0) {
+        // ---------------------------------------------------------------- producer
+        if (lane == 0) {
+            uint32_t stage = 0, phase = 0;
+            bool ok = true;
+            // without a route the weight tiles of the first stages are requested before the predecessor has finished
+            int early = 0;
+            if (!routed) {
+                if ((int)blockIdx.x < total) {
+                    const int n0 = ((int)blockIdx.x / sp / tiles_m) * FN, first = k_first(blockIdx.x);
+                    early = min(k_end(blockIdx.x) - first, STAGES);
+                    for (int i = 0; i < early; i++) {
+                        pg_mbar_expect(bar_full + 8 * i, C::STAGE);
+                        tma_load_2d(base + i * C::STAGE, &tmap_w, bar_full + 8 * i, (first + i) * FK, n0);
+                    }
+                }
+                asm volatile("griddepcontrol.wait;" ::: "memory");
+            }
+            for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+                const int tile = u / sp;
+                const int m0 = (tile % tiles_m) * MT, n0 = (tile / tiles_m) * FN;
+                const int w0 = routed ? __ldcg(rt.block_expert + block0 + m0 / PG_ROUTE_BLOCK) * N + n0 : n0;
+                for (int kb = k_first(u), end = k_end(u); kb < end; kb++) {
+                    if (!(ok = pg_mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, status, limit_ns))) break;
+                    const uint32_t at = base + stage * C::STAGE;
+                    if (early > 0) {
+                        early--;                            // announced and half filled above
+                    } else {
+                        pg_mbar_expect(bar_full + 8 * stage, C::STAGE);
+                        tma_load_2d(at, &tmap_w, bar_full + 8 * stage, kb * FK, w0);
+                    }
+#pragma unroll
+                    for (int l = 0; l < 3; l++) tma_load_3d(at + C::STAGE_W + l * C::PLANE, &tmap_a, bar_full + 8 * stage, kb * FK, m0, l);
+                    if (++stage == STAGES) {
+                        stage = 0;
+                        phase ^= 1;
+                    }
+                }
+            }
+            if (!ok) {
+                // give copies that are still in flight a bounded time to land before the CTA exits
+                const unsigned long long t0 = pg_globaltimer_ns();
+                while (pg_globaltimer_ns() - t0 < 2000000ull) {
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------------------------------------------------------- MMA issuer (the whole warp; one lane's products count)
+        const uint32_t on = pg_elect();
+        constexpr uint32_t idesc = make_idesc(FN, MT);
+        uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+            for (int kb = k_first(u), end = k_end(u); kb < end; kb++) {
+                ok = pg_mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, status, limit_ns);
+                ok = ok && pg_mbar_wait(bar_full + 8 * stage, phase, abort_flag, status, limit_ns);
+                if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                tc_fence_after();
+                const uint32_t at = base + stage * C::STAGE, d_tmem = tmem_base + acc * C::ACC;
+                const uint64_t dw = make_smem_desc(at), da = make_smem_desc(at + C::STAGE_W);
+#pragma unroll
+                for (int l = 2; l >= 0; l--)
+#pragma unroll
+                    for (int j = 0; j < FK / 16; j++)
+                        umma_f16(d_tmem, dw + (uint64_t)(j * 2), da + (uint64_t)(l * (C::PLANE >> 4) + j * 2), idesc, l != 2 || j != 0 ? 1u : 0u, on);
+                umma_commit(bar_empty + 8 * stage, on);     // stage reusable once these products have read it
+                umma_commit(bar_tfull + 8 * acc, on);
+                if (++stage == STAGES) {
+                    stage = 0;
+                    phase ^= 1;
+                }
+                if (++acc == 2) {
+                    acc = 0;
+                    acc_phase ^= 1;
+                }
+            }
+        }
+    } else {
+        // ---------------------------------------------------------------- sums and outputs: lane = column of y
+        const int q = warp & 3;                             // TMEM lane quarter this warp may read
+        if (!routed) asm volatile("griddepcontrol.wait;" ::: "memory");   // y may still be read by the predecessor
+        const int rows = routed ? tiles_m * MT : M;
+        uint32_t acc = 0, acc_phase = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+            const int tile = u / sp;
+            const int m0 = (tile % tiles_m) * MT, n0 = (tile / tiles_m) * FN;
+            float sum[MT] = {};
+            for (int kb = k_first(u), end = k_end(u); kb < end; kb++) {
+                ok = pg_mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, status, limit_ns);
+                if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                tc_fence_after();
+                const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * C::ACC;
+#pragma unroll
+                for (int c = 0; c < C::ACC; c += 32) {
+                    uint32_t v[32];
+                    tmem_ld32(taddr + c, v);
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        if (c + j < MT) sum[c + j] += __uint_as_float(v[j]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) pg_mbar_arrive(bar_tempty + 8 * acc);
+                if (++acc == 2) {
+                    acc = 0;
+                    acc_phase ^= 1;
+                }
+            }
+            if (!ok) break;
+            const int n = n0 + q * 32 + lane;
+            bool mine = true;
+            if (sp > 1) {
+                float *slab = kp.slabs + (int64_t)u * MT * FN + q * 32 + lane;
+#pragma unroll
+                for (int j = 0; j < MT; j++) __stcg(slab + j * FN, sum[j]);
+                unsigned int *ticket = kp.tickets + tile * 4 + q;
+                __threadfence();
+                __syncwarp();
+                const unsigned int before = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(ticket, 1u) : 0u, 0);
+                mine = before == (unsigned)(sp - 1);
+                if (mine) {
+                    // the last part of these columns to finish adds all parts up, in their order
+                    __threadfence();
+                    if (lane == 0) *ticket = 0;
+                    slab = kp.slabs + (int64_t)tile * sp * MT * FN + q * 32 + lane;
+#pragma unroll
+                    for (int j = 0; j < MT; j++) sum[j] = __ldcg(slab + j * FN);
+                    for (int p = 1; p < sp; p++) {
+                        slab += MT * FN;
+#pragma unroll
+                        for (int j = 0; j < MT; j++) sum[j] += __ldcg(slab + j * FN);
+                    }
+                }
+            }
+            if (!mine) continue;
+            if (ACT == PG_ACT_NONE) {
+                if (n < N) {
+                    float *dst = y + (int64_t)m0 * ldy + n;
+#pragma unroll
+                    for (int j = 0; j < MT; j++)
+                        if (m0 + j < rows) dst[j * ldy] = sum[j];
+                }
+            } else {
+                // columns [8 gates | 8 ups] twice per warp; N is a multiple of 16
+                float *dst = y + (int64_t)m0 * ldy + (n0 + q * 32) / 2 + (lane >> 4) * 8 + (lane & 7);
+#pragma unroll
+                for (int j = 0; j < MT; j++) {
+                    const float u2 = __shfl_down_sync(0xffffffffu, sum[j], 8);
+                    if (!(lane & 8) && n < N && m0 + j < rows) dst[j * ldy] = pg_glu<ACT>(sum[j], u2, limit);
+                }
+            }
+        }
+    }
+
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * C::ACC) : "memory");
+    }
+}
+
+// ---------------------------------------------------------------- host side ----
+template <int MT, int ACT>
+int32_t launch(pg_ctx *ctx, const pg_linear *lin, const bf16 *planes, int64_t m, float limit, float *y, int64_t ldy, const PgRouted &rt, int block0, FParts kp)
+{
+    using C = FCfg<MT>;
+    CUtensorMap tw, ta;
+    const cuuint64_t wd[2] = {(cuuint64_t)lin->k, (cuuint64_t)(lin->experts * lin->n)}, ws[1] = {(cuuint64_t)lin->k * 2};
+    const cuuint32_t wb[2] = {FK, FN};
+    int32_t rc = pg_encode_bf16(&tw, lin->w, 2, wd, ws, wb);
+    if (rc != PG_OK) return rc;
+    const cuuint64_t ad[3] = {(cuuint64_t)lin->k, (cuuint64_t)m, 3}, as[2] = {(cuuint64_t)lin->k * 2, (cuuint64_t)(lin->k * m) * 2};
+    const cuuint32_t ab[3] = {FK, MT, 1};
+    rc = pg_encode_bf16(&ta, planes, 3, ad, as, ab);
+    if (rc != PG_OK) return rc;
+    auto kern = linear_f32_kernel<MT, ACT>;
+    static std::atomic<uint64_t> smem_set{0};
+    PG_CUDA(pg_max_smem_once(kern, (int)C::SMEM, ctx->device, smem_set));
+    const int64_t units = ((m + MT - 1) / MT) * ((lin->n + FN - 1) / FN) * kp.parts;
+    kp.tickets = reinterpret_cast<unsigned int *>(ctx->splitk);
+    kp.slabs = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(ctx->splitk) + PG_LM_TICKET_BYTES);
+    return launch_pdl(ctx, kern, dim3((unsigned)std::min<int64_t>(units, ctx->sm_count)), dim3(F_THREADS), C::SMEM, tw, ta, (int)m, (int)lin->n, (int)lin->k,
+                      limit, y, ldy, rt, block0, kp, ctx->d_status, ctx->wait_limit_ns);
+}
+
+template <int ACT>
+int32_t dispatch(pg_ctx *ctx, const pg_linear *lin, const bf16 *planes, int64_t m, float limit, float *y, int64_t ldy, const PgRouted &rt, int block0)
+{
+    const int64_t kblocks = lin->k / FK, tiles_n = (lin->n + FN - 1) / FN;
+    const bool routed = rt.blocks != nullptr;
+    int mt = routed ? 128 : 16;
+    while (mt < 128 && mt < m) mt *= 2;
+    FParts kp = {1, (int)kblocks, nullptr, nullptr};
+    if (!routed) {
+        // rows per tile and parts of K: the fewest cycles by count -- blocks of the busiest CTA, each the products' time or its copies'
+        // (about 40 bytes per cycle and SM), and what a tile costs at its end, more where slabs meet; slabs within what
+        // pg_linear_wrap has reserved
+        const int64_t room = (int64_t)(ctx->splitk_bytes > PG_LM_TICKET_BYTES ? ctx->splitk_bytes - PG_LM_TICKET_BYTES : 0) / (FN * (int64_t)sizeof(float));
+        const int full = mt;
+        double best = 0;
+        for (int cand = full; cand >= std::min(full, 64); cand /= 2) {
+            const int64_t tiles = tiles_n * ((m + cand - 1) / cand);
+            for (int64_t parts = 1; parts <= std::max<int64_t>(1, std::min<int64_t>(16, kblocks / 4)); parts++) {
+                const int64_t blocks = (kblocks + parts - 1) / parts;
+                if ((kblocks + blocks - 1) / blocks != parts) continue;
+                if (parts > 1 && (tiles * parts * cand > room || tiles * 4 * (int64_t)sizeof(int) > (int64_t)PG_LM_TICKET_BYTES)) break;
+                const int64_t rounds = (tiles * parts + ctx->sm_count - 1) / ctx->sm_count;
+                const double block = std::max(std::max(480.0, cand * 6.0), (FN * FK * 2 + 3.0 * cand * FK * 2) / 40.0);
+                const double cost = rounds * (blocks * block + 2500.0 + cand * 8.0 + (parts > 1 ? 3000.0 + cand * parts * 6.0 : 0.0));
+                if (best == 0 || cost < best) {
+                    best = cost;
+                    mt = cand;
+                    kp.parts = (int)parts;
+                    kp.blocks = (int)blocks;
+                }
+            }
+        }
+    }
+    if (mt == 128) return launch<128, ACT>(ctx, lin, planes, m, limit, y, ldy, rt, block0, kp);
+    if (mt == 64) return launch<64, ACT>(ctx, lin, planes, m, limit, y, ldy, rt, block0, kp);
+    if (mt == 32) return launch<32, ACT>(ctx, lin, planes, m, limit, y, ldy, rt, block0, kp);
+    return launch<16, ACT>(ctx, lin, planes, m, limit, y, ldy, rt, block0, kp);
+}
+
 }  // namespace
+
+size_t pgk_linear_f32_workspace(int64_t k) { return (size_t)F_ROWS * k * 3 * sizeof(bf16); }
 
 int32_t pgk_linear_f32(pg_ctx *ctx, const pg_linear *lin, const float *a, int64_t lda, int64_t m, int act, float limit, void *y, int y_dtype, int64_t ldy,
                        const PgRouted *routed)
 {
     PG_REQUIRE(y_dtype == PG_F32, "linear: an f32 step has f32 outputs");
+    PG_REQUIRE((lin->n + 63) / 64 <= 65535, "linear: too many output columns for the f32 form");
+    PG_REQUIRE(m < (1ll << 31) - 256 && lin->experts * lin->n < (1ll << 31) - 256, "linear: too many rows");
     const PgRouted none = {};
-    const PgRouted rt = routed ? *routed : none;
-    const dim3 grid((unsigned)((m + FM - 1) / FM), (unsigned)((lin->n + FN - 1) / FN));
-    PG_REQUIRE(grid.y <= 65535, "linear: too many output columns for the f32 form");
-#define PG_F32_CASE(A) \
-    return launch_pdl(ctx, linear_f32_kernel<A, float>, grid, dim3(256), 0, a, lda, lin->w, (int)m, (int)lin->n, (int)lin->k, limit, (float *)y, ldy, rt)
-    if (act == PG_ACT_NONE) PG_F32_CASE(PG_ACT_NONE);
-    if (act == PG_ACT_GELU_TANH_GLU) PG_F32_CASE(PG_ACT_GELU_TANH_GLU);
-    PG_F32_CASE(PG_ACT_CLAMPED_SWISH_GLU);
-#undef PG_F32_CASE
+    const PgRouted &rt = routed ? *routed : none;
+    // all rows at once if there is room for their planes; while a graph is recorded the workspace cannot grow, and what
+    // pg_linear_wrap has reserved then takes them in portions
+    const int64_t row_bytes = lin->k * 3 * (int64_t)sizeof(bf16);
+    int64_t portion = m;
+    if ((size_t)(m * row_bytes) > ctx->scratch_bytes) {
+        if (ctx->capturing) {
+            portion = (int64_t)(ctx->scratch_bytes / (size_t)row_bytes) / F_ROWS * F_ROWS;
+            PG_REQUIRE(portion > 0, "linear: the context has no workspace for the f32 form");
+        } else {
+            const int32_t rc = pg_scratch_reserve(ctx, (size_t)(m * row_bytes));
+            if (rc != PG_OK) return rc;
+        }
+    }
+    bf16 *planes = reinterpret_cast<bf16 *>(ctx->scratch);
+    for (int64_t r0 = 0; r0 < m; r0 += portion) {
+        const int64_t rows = std::min(portion, m - r0);
+        const dim3 grid((unsigned)((lin->k / 4 + 255) / 256), (unsigned)std::min<int64_t>(rows, 8192));
+        int32_t rc = launch_pdl(ctx, linear_split_kernel, grid, dim3(256), 0, a, lda, (int)r0, (int)rows, (int)lin->k, rt, reinterpret_cast<uint2 *>(planes));
+        if (rc != PG_OK) return rc;
+        float *out = (float *)y + r0 * ldy;
+        const int block0 = (int)(r0 / PG_ROUTE_BLOCK);
+        rc = act == PG_ACT_NONE             ? dispatch<PG_ACT_NONE>(ctx, lin, planes, rows, limit, out, ldy, rt, block0)
+             : act == PG_ACT_GELU_TANH_GLU ? dispatch<PG_ACT_GELU_TANH_GLU>(ctx, lin, planes, rows, limit, out, ldy, rt, block0)
+                                            : dispatch<PG_ACT_CLAMPED_SWISH_GLU>(ctx, lin, planes, rows, limit, out, ldy, rt, block0);
+        if (rc != PG_OK) return rc;
+    }
+    return PG_OK;
 }

@@ -82,6 +82,67 @@ def test_product(lm, dtype, n, k):
     lin.free()
 
 
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 65, 128, 129, 300])
+@pytest.mark.parametrize("n,k", [(127, 64), (128, 320), (1300, 1024), (260, 5184)])
+def test_f32_product_is_f32(lm, m, n, k):
+    """Tiles and parts of K at their edges, element by element: three exact pieces and sums that are rounded once per 64 k.  A block's
+    twelve instructions cut off below 2^-23 of its largest sum each, a sum of blocks is rounded to 2^-24."""
+    from peregrine_b200.layers import Linear, up
+
+    d = device(lm, "float32", 320)
+    g = rng(n + k + m)
+    w = t.bf16_values(g.standard_normal((n, k)))
+    a = (g.standard_normal((m, k)) * 2.0 ** g.integers(-20, 20, (m, k))).astype(np.float32)
+    a[0, 0] = 1e-30
+    lin = Linear(d, d.bf16(w))
+    y = d.torch.full((m, up(n, 8)), 7.0, device=d.dev)
+    x = act(d, a)
+    lin.run(x, m, y)
+    lm.sync()
+    got, want = y.cpu().numpy(), a.astype(np.float64) @ w.T.astype(np.float64)
+    bound = np.abs(a).astype(np.float64) @ np.abs(w).T.astype(np.float64) * (12 * 2.0 ** -23 + (k // 64 + 16) * 2.0 ** -24)
+    assert (np.abs(got[:, :n] - want) <= bound).all() and (got[:, n:] == 7.0).all() and lm.device_status() == 0
+    # what is not finite stays in its row
+    a[m - 1, 5], a[m // 2, 7] = np.inf, np.nan
+    x.copy_(act(d, a))
+    d.torch.cuda.synchronize()
+    lin.run(x, m, y)
+    lm.sync()
+    again = y.cpu().numpy()[:, :n]
+    for r in range(m):
+        if r == m // 2:
+            assert np.isnan(again[r]).all()
+        elif r == m - 1:
+            assert (again[r] == np.inf * w[:, 5]).all()
+        else:
+            assert (again[r] == got[r, :n]).all()
+    lin.free()
+
+
+def test_f32_product_is_recorded_without_a_run_before(lm):
+    """The workspace cannot grow in a recording: the rows then go through what there is in portions, with the same results."""
+    from peregrine_b200.layers import Linear
+    from peregrine_b200.runtime import GpuContext
+
+    gpu = GpuContext(component="lm")
+    d = device(gpu, "float32", 700)
+    g = rng(3)
+    lin = Linear(d, d.bf16(t.bf16_values(g.standard_normal((200, 192)))))
+    x, y, z = act(d, g.standard_normal((700, 192)).astype(np.float32)), d.torch.zeros(700, 200, device=d.dev), d.torch.zeros(700, 200, device=d.dev)
+    d.torch.cuda.synchronize()
+    with gpu.record() as graph:
+        lin.run(x, 700, y)
+    graph.launch()
+    gpu.sync()
+    assert graph.kernels > 2               # in portions
+    lin.run(x, 700, z)
+    gpu.sync()
+    assert (y == z).all() and gpu.device_status() == 0
+    graph.free()
+    lin.free()
+    gpu.close()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("f,k", [(5, 64), (72, 130), (300, 384), (24, 4500)])
 def test_gated_products(lm, dtype, f, k):
