@@ -9,7 +9,7 @@ from typing import List, Sequence
 
 import numpy as np
 
-from .layers import BATCH_WORDS, Batch, Device, Linear, up
+from .layers import Batch, Device, Linear, up
 from .safetensors_file import SafetensorsFile
 from .state import SlotPool
 
@@ -97,7 +97,6 @@ class ResidualModel(SlotModel):
         self.max_wanted = max(int(max_wanted), slots)
         self.picked = torch.zeros(self.max_wanted, self.ldh, dtype=d.act, device=d.dev)
         self.logits = torch.zeros(self.max_wanted, cfg.vocab, dtype=f32, device=d.dev)
-        d.buffer("batch", 1, BATCH_WORDS(d.rows), torch.int32)
         self.weights = None
         torch.cuda.synchronize()   # torch filled the buffers on its own stream; the kernels use the context's
 
