@@ -1,0 +1,555 @@
+// Dequantising product y = x . dequant(W)^T for GGUF Q4_0 / Q8_0 weights and several rows of x on the 5th-generation tensor cores
+// (up to eight rows: csrc/pg_gguf_stream.cu, which also describes the layout of the weights).
+//
+// Arithmetic, per 32-element block:
+//   * x * 2^s (s per row: the largest element lies in [2^14, 2^15)) = h1 + h2, two f16 numbers: 22 significant bits, and more than
+//     that of the row's largest element for all of them.  `gguf_planes_kernel` writes the two planes once per call.
+//   * the quants become f16 exactly.  Each product (at most 11 + 8 bits) is exact in f32; the block's sum in the tensor core is the
+//     sum of 64 of them, smaller plane first.
+//   * the block's f16 scale is applied in f32 by the warps that take the sum out of TMEM: sum += d * block, rounded once per block.
+//   * a row that holds a NaN or an infinity gives NaN, as in the streaming form (2^-s is then a NaN).
+//
+// Weights are the M side of the instruction (128 rows of W), rows of x the N side (MT): a lane of the epilogue owns a row of W, so
+// that a block's scale is one register, and 32 lanes store 128 contiguous bytes of a row of y.  A CTA (15 or 19 warps, one per SM):
+//   warps 0, 10   copies: blocks of 64 k of both planes by TMA; slices of W as they lie in memory (eight fills of 16 rows x 256 k)
+//   warp 1        products: two planes x two steps of 16 k per block of W into an accumulator of its own; up to 64 rows the planes lie
+//                 side by side in one product, whose issue (not its time in the tensor core) is what counts there
+//   warps 2-9     two per TMEM quarter, half of the columns each: sum += d * accumulator
+//   warps 11-     quants -> f16 in the 128-byte-swizzled tiles that the products read, 128 k at a time, two such buffers
+// With few tiles K is divided over CTAs; the last part of a tile to finish adds all parts in their order.
+//
+// What bounds it: shared memory, then the epilogue's way through TMEM.  At MT = 128 a block of 32 k takes 256 cycles of products, which
+// read 32 KB of it, while 16 KB of planes come in, 8 KB of f16 weights are written and 2 KB of quants read: 470 cycles at 128 bytes
+// each, about 460 of the warp that issues the products (800 with its waits).  N 14336, K 4096, 9 / 16 / 33 / 64 / 300 rows: Q4_0 25 / 26 /
+// 39 / 43 / 126 us, where eight rows at a time through the streaming form took 31 / 42 / 92 / 167 / 787; error against 64 bits 2e-7 ...
+// 3e-7 with 1 % of the channels x 20 (1.2e-6).  Up to eight rows the streaming form is the faster one (21 against 25 us).
+// Every mbarrier wait is bounded (pg_async.cuh).
+#include <algorithm>
+
+#include "pg_async.cuh"
+#include "pg_gguf_f16.cuh"
+#include "pg_internal.cuh"
+#include "pg_launch.cuh"
+#include "pg_tcgen05.cuh"
+
+namespace {
+
+constexpr int GT_N = 128;                         // rows of W per tile
+constexpr int GT_ROWS = 64;                       // rows for which the planes always find room (pgk_gguf_tc_reserve)
+constexpr size_t GT_TICKET_BYTES = 64 * 1024;     // as in the int8 kernel: tickets, zero between calls, then slabs
+
+template <int TYPE, int MT>
+struct GtCfg {
+    static constexpr int SEG = TYPE == PG_GGUF_Q4_0 ? 128 : 256;   // quant bytes per row and slice
+    static constexpr int FILL = 16 * SEG + 256;
+    static constexpr int RAW = 8 * FILL;                           // a slice (256 k) of 128 rows
+    static constexpr int A_TILE = GT_N * 64 * 2;                   // 64 k of 128 rows in f16
+    static constexpr int A_BYTES = 4 * A_TILE;                     // two buffers of 128 k
+    static constexpr bool STACK = MT <= 64;                        // both planes as columns of one product, added up in the epilogue
+    static constexpr int COLS = STACK ? 2 * MT : MT;               // accumulator columns of a block
+    static constexpr int PLANE = MT * 64 * 2;
+    static constexpr int BK64 = MT <= 64 ? 2 : 1;                  // 64-k blocks of the planes per stage
+    static constexpr int B_STAGE = BK64 * 2 * PLANE;
+    static constexpr int ROOM = 232448 - 1024 - 512;
+    static constexpr int BST = MT >= 160 ? 2 : MT >= 64 ? (TYPE == PG_GGUF_Q4_0 ? 3 : 2) : MT == 32 ? 4 : 6;
+    static constexpr int FIT = (ROOM - A_BYTES - BST * B_STAGE) / RAW;
+    static constexpr int RST = FIT > 7 ? 7 : FIT;
+    static constexpr int GB = MT <= 32 ? 4 : MT <= 128 ? 2 : 1;    // blocks per group of accumulators
+    static constexpr int NBUF = 512 / (GB * COLS) > 4 ? 4 : 512 / (GB * COLS);
+    static constexpr int HALF = MT / 2;                            // rows of x per warp of the epilogue
+    static constexpr int DW = MT <= 64 ? 8 : 4;                    // warps that turn quants into f16 (the wide tiles' registers leave room for four)
+    static constexpr int THREADS = (11 + DW) * 32;
+    static constexpr size_t SMEM = (size_t)A_BYTES + BST * B_STAGE + RST * RAW + 1024 + 512;
+    static_assert(RST >= 2 && NBUF >= 2, "shared memory or TMEM too small");
+};
+
+struct GtParts {
+    int parts, slices;       // K in `parts` parts of `slices` 256-element slices
+    float *slabs;            // [unit][MT][128]
+    unsigned int *tickets;   // one per (tile, TMEM quarter, half of the columns), zero between calls
+};
+
+// ---- planes of rows row0 .. row0 + rows - 1 of x: [2][rows][K] f16, and 2^-s per row.  grid (rows, parts of K) -----------------
+template <bool Q4>
+__global__ void __launch_bounds__(256)
+    gguf_planes_kernel(const float *__restrict__ x, int row0, int rows, int K, uint4 *__restrict__ planes, float *__restrict__ us)
+{
+    __shared__ float red[16];
+    pg_pdl_begin();
+    const int r = blockIdx.x, tid = threadIdx.x, eights = K / 8;
+    const float4 *src = reinterpret_cast<const float4 *>(x + (int64_t)(row0 + r) * K);
+    float top = 0.0f, poison = 0.0f;              // every part looks at the whole row: it comes from L2
+    for (int c = tid; c < K / 4; c += 256) {
+        const float4 v = __ldcg(src + c);
+        top = fmaxf(top, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+        poison += (v.x - v.x) + (v.y - v.y) + (v.z - v.z) + (v.w - v.w);   // 0, or NaN
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        poison += __shfl_xor_sync(0xffffffffu, poison, o);
+    }
+    if ((tid & 31) == 0) {
+        red[tid >> 5] = top;
+        red[8 + (tid >> 5)] = poison;
+    }
+    __syncthreads();
+    for (int i = 0; i < 8; i++) {
+        top = fmaxf(top, red[i]);
+        poison += red[8 + i];
+    }
+    // (a row that is not finite has NaN for 2^-s, and zeros)
+    const bool fine = poison == 0.0f;
+    const int e = fine ? gguf_exponent(top) : 0;
+    const float sc = scalbnf(1.0f, 14 - e);
+    if (tid == 0 && blockIdx.y == 0) us[r] = fine ? scalbnf(1.0f, e - 14) : NAN;
+    const int per = (eights + gridDim.y - 1) / gridDim.y, hi = min(eights, (int)(blockIdx.y + 1) * per);
+    for (int c = blockIdx.y * per + tid; c < hi; c += 256) {
+        const float4 a = __ldcg(src + 2 * c), b = __ldcg(src + 2 * c + 1);
+        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        uint4 h1, h2;
+        gguf_split8<Q4>(v, sc, h1, h2);
+        if (!fine) h1 = h2 = make_uint4(0u, 0u, 0u, 0u);
+        planes[(int64_t)r * eights + c] = h1;
+        planes[((int64_t)rows + r) * eights + c] = h2;
+    }
+}
+
+// ---- pieces of the product ------------------------------------------------------------------------------------------------
+// kind::f16 with f16 operands (0 at bits 7 and 10), f32 sums, both K-major
+__host__ __device__ constexpr uint32_t gt_idesc(int m, int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24); }
+
+// sum[0 .. NC) += d * the next NC columns of this lane's TMEM row
+template <int NC>
+__device__ __forceinline__ void gt_add(uint32_t taddr, float d, float *sum)
+{
+    constexpr int P = NC >= 32 ? 32 : NC;
+    static_assert(P == 8 || P == 16 || P == 32, "pieces of 32, 16 or 8 columns");
+    uint32_t t[P];
+    if constexpr (P == 32) {
+        tmem_ld32_async(taddr, t);
+    } else if constexpr (P == 16) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7]), "=r"(t[8]), "=r"(t[9]), "=r"(t[10]),
+              "=r"(t[11]), "=r"(t[12]), "=r"(t[13]), "=r"(t[14]), "=r"(t[15])
+            : "r"(taddr)
+            : "memory");
+    } else {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7])
+                     : "r"(taddr)
+                     : "memory");
+    }
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < P; i++) sum[i] = fmaf(d, __uint_as_float(t[i]), sum[i]);
+    if constexpr (NC > P) gt_add<NC - P>(taddr + P, d, sum + P);
+}
+__device__ __forceinline__ void gt_sts128(uint32_t addr, const uint32_t (&v)[4])
+{
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+// gives copies that are still in flight a bounded time to land before a CTA that gives up exits
+__device__ __forceinline__ void gt_settle()
+{
+    const unsigned long long t0 = pg_globaltimer_ns();
+    while (pg_globaltimer_ns() - t0 < 2000000ull) {
+    }
+}
+
+template <int TYPE, int MT>
+__global__ void __launch_bounds__(GtCfg<TYPE, MT>::THREADS, 1)
+    gguf_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const uint8_t *__restrict__ qs, int64_t N, int nslices, int M, const float *__restrict__ us,
+                   float *__restrict__ y, const GtParts kp, int32_t *status, unsigned long long limit_ns)
+{
+    using C = GtCfg<TYPE, MT>;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw_addr = pg_smem(smem_raw);
+    const uint32_t base = (raw_addr + 1023u) & ~1023u;
+    const uint32_t a_at = base, b_at = a_at + C::A_BYTES, r_at = b_at + C::BST * C::B_STAGE;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw + (r_at - raw_addr) + C::RST * C::RAW);
+    const uint32_t bar = pg_smem(bars);
+    // full and empty of: slices, blocks of the planes, f16 buffers, groups of accumulators
+    const uint32_t r_full = bar, r_empty = r_full + 8 * C::RST, b_full = r_empty + 8 * C::RST, b_empty = b_full + 8 * C::BST;
+    const uint32_t a_full = b_empty + 8 * C::BST, a_empty = a_full + 16, t_full = a_empty + 16, t_empty = t_full + 8 * C::NBUF;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * C::RST + 2 * C::BST + 4 + 2 * C::NBUF);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < C::RST; i++) {
+            pg_mbar_init(r_full + 8 * i, 1);
+            pg_mbar_init(r_empty + 8 * i, 8 + C::DW);   // the scales, the quants
+        }
+        for (int i = 0; i < C::BST; i++) {
+            pg_mbar_init(b_full + 8 * i, 1);
+            pg_mbar_init(b_empty + 8 * i, 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            pg_mbar_init(a_full + 8 * i, C::DW);
+            pg_mbar_init(a_empty + 8 * i, 1);
+        }
+        for (int i = 0; i < C::NBUF; i++) {
+            pg_mbar_init(t_full + 8 * i, 1);
+            pg_mbar_init(t_empty + 8 * i, 8);
+        }
+        *abort_flag = 0;
+        pg_mbar_fence();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pg_smem(tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    const int tiles_m = (M + MT - 1) / MT, tiles_n = (int)((N + GT_N - 1) / GT_N);
+    const int sp = kp.parts, total = tiles_m * tiles_n * sp;   // unit u: part u % sp of tile u / sp; the tiles of a row of W follow each other
+    auto s_first = [&](int u) { return (u % sp) * kp.slices; };
+    auto s_end = [&](int u) { return min(nslices, (u % sp + 1) * kp.slices); };
+    bool ok = true;
+
+    if (warp == 0) {
+        // ---------------------------------------------------------------- planes of x
+        if (lane == 0) {
+            uint32_t bs = 0, bp = 0;
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+                const int m0 = (u / sp % tiles_m) * MT;
+                for (int kb = 4 * s_first(u), end = 4 * s_end(u); kb < end; kb += C::BK64) {
+                    if (!(ok = pg_mbar_wait(b_empty + 8 * bs, bp ^ 1, abort_flag, status, limit_ns))) break;
+                    pg_mbar_expect(b_full + 8 * bs, C::B_STAGE);
+#pragma unroll
+                    for (int i = 0; i < C::BK64; i++)
+                        tma_load_3d(b_at + bs * C::B_STAGE + i * 2 * C::PLANE, &tmap_x, b_full + 8 * bs, (kb + i) * 64, m0, 0);
+                    if (++bs == C::BST) {
+                        bs = 0;
+                        bp ^= 1;
+                    }
+                }
+            }
+            if (!ok) gt_settle();
+        }
+    } else if (warp == 10) {
+        // ---------------------------------------------------------------- slices of W, which no kernel writes: no wait for the preceding one
+        if (lane == 0) {
+            const int64_t fills = (N + 15) >> 4;               // (fills behind the last one do not exist)
+            uint32_t rs = 0, rp = 0;
+            for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+                const int64_t f0 = (int64_t)(u / sp / tiles_m) * (GT_N / 16);
+                const int n = (int)min((int64_t)8, fills - f0);
+                for (int s = s_first(u), end = s_end(u); s < end; s++) {
+                    if (!(ok = pg_mbar_wait(r_empty + 8 * rs, rp ^ 1, abort_flag, status, limit_ns))) break;
+                    pg_mbar_expect(r_full + 8 * rs, (uint32_t)n * C::FILL);
+                    for (int i = 0; i < n; i++)
+                        pg_bulk_load(r_at + rs * C::RAW + i * C::FILL, qs + ((f0 + i) * nslices + s) * (int64_t)C::FILL, C::FILL, r_full + 8 * rs);
+                    if (++rs == C::RST) {
+                        rs = 0;
+                        rp ^= 1;
+                    }
+                }
+            }
+            if (!ok) gt_settle();
+        }
+    } else if (warp == 1) {
+        // ---------------------------------------------------------------- products (the whole warp; one lane's count)
+        const uint32_t on = pg_elect();
+        constexpr uint32_t idesc = gt_idesc(GT_N, C::COLS);
+        const uint64_t desc_a = make_smem_desc(a_at), desc_b = make_smem_desc(b_at);
+        uint32_t bs = 0, bp = 0, as = 0, ap = 0, ts = 0, tp = 0;
+        auto wait = [&](uint32_t b, uint32_t parity) { return (bool)__all_sync(0xffffffffu, pg_mbar_wait(b, parity, abort_flag, status, limit_ns)); };
+        for (int u = blockIdx.x; ok && u < total; u += gridDim.x)
+            for (int h = 2 * s_first(u), end = 2 * s_end(u); ok && h < end; h++) {
+                if (!(ok = wait(a_full + 8 * as, ap))) break;
+#pragma unroll
+                for (int blk = 0; blk < 4; blk++) {             // blocks of the 128 k
+                    constexpr int PER_B = 2 * C::BK64;          // blocks per stage of the planes
+                    if (blk % PER_B == 0 && !(ok = wait(b_full + 8 * bs, bp))) break;
+                    if (blk % C::GB == 0 && !(ok = wait(t_empty + 8 * ts, tp ^ 1))) break;
+                    tc_fence_after();
+                    const uint32_t d = tmem + (ts * C::GB + blk % C::GB) * C::COLS;
+                    const uint64_t da = desc_a + (uint64_t)((as * 2 + (blk >> 1)) * (C::A_TILE >> 4) + (blk & 1) * 4);
+                    const uint64_t db = desc_b + (uint64_t)(bs * (C::B_STAGE >> 4) + (blk % PER_B >> 1) * (2 * C::PLANE >> 4) + (blk & 1) * 4);
+                    if constexpr (C::STACK) {
+#pragma unroll
+                        for (int j = 0; j < 2; j++) umma_f16(d, da + (uint64_t)(j * 2), db + (uint64_t)(j * 2), idesc, j != 0 ? 1u : 0u, on);
+                    } else {
+#pragma unroll
+                        for (int l = 1; l >= 0; l--)
+#pragma unroll
+                            for (int j = 0; j < 2; j++)
+                                umma_f16(d, da + (uint64_t)(j * 2), db + (uint64_t)(l * (C::PLANE >> 4) + j * 2), idesc, l != 1 || j != 0 ? 1u : 0u, on);
+                    }
+                    if ((blk + 1) % C::GB == 0) {
+                        umma_commit(t_full + 8 * ts, on);
+                        if (++ts == C::NBUF) {
+                            ts = 0;
+                            tp ^= 1;
+                        }
+                    }
+                    if ((blk + 1) % PER_B == 0) {
+                        umma_commit(b_empty + 8 * bs, on);
+                        if (++bs == C::BST) {
+                            bs = 0;
+                            bp ^= 1;
+                        }
+                    }
+                }
+                if (!ok) break;
+                umma_commit(a_empty + 8 * as, on);
+                as ^= 1;
+                if (as == 0) ap ^= 1;
+            }
+    } else if (warp > 10) {
+        // ---------------------------------------------------------------- quants -> f16: 128 / DW rows of W per warp, eight at a time
+        constexpr int ROUNDS = GT_N / C::DW / 8, LOADS = TYPE == PG_GGUF_Q4_0 ? 1 : 2;
+        const int row0 = (warp - 11) * (GT_N / C::DW) + (lane >> 2), t = lane & 3;
+        // lane: row r, quarter t of the blocks; rows of odd number take their blocks in the other order, so that two rows never write
+        // to the same banks (and the layout has them read from different ones)
+        const int odd = row0 & 1;
+        uint32_t rs = 0, rp = 0, as = 0, ap = 0;
+        for (int u = blockIdx.x; ok && u < total; u += gridDim.x)
+            for (int s = s_first(u), end = s_end(u); ok && s < end; s++) {
+                ok = __all_sync(0xffffffffu, pg_mbar_wait(r_full + 8 * rs, rp, abort_flag, status, limit_ns));
+                for (int h = 0; ok && h < 2; h++) {
+                    // Q4_0: word t of four blocks; Q8_0: eight bytes of two blocks, twice
+                    uint4 q[ROUNDS][LOADS];
+#pragma unroll
+                    for (int i = 0; i < ROUNDS; i++) {
+                        const int r = row0 + i * 8;
+                        const uint32_t src = r_at + rs * C::RAW + (uint32_t)(r >> 4) * C::FILL + (uint32_t)(r & 15) * C::SEG;
+#pragma unroll
+                        for (int p = 0; p < LOADS; p++) q[i][p] = pg_lds128(src + (uint32_t)((((h * LOADS + p) * 4 + t) ^ (odd << 2)) * 16));
+                    }
+                    ok = __all_sync(0xffffffffu, pg_mbar_wait(a_empty + 8 * as, ap ^ 1, abort_flag, status, limit_ns));
+                    if (!ok) break;
+#pragma unroll
+                    for (int i = 0; i < ROUNDS; i++) {
+                        const int r = row0 + i * 8;
+                        const uint32_t dst = a_at + as * (2 * C::A_TILE) + (uint32_t)r * 128;
+                        auto put = [&](int blk, const uint32_t (&v)[4]) {   // block blk of the 128 k
+                            gt_sts128(dst + (blk >> 1) * C::A_TILE + (uint32_t)((((blk & 1) * 4 + t) ^ (r & 7)) * 16), v);
+                        };
+                        uint32_t v[4];
+#pragma unroll
+                        for (int p = 0; p < 2; p++) {           // blocks 2 p and 2 p + 1
+                            if constexpr (TYPE == PG_GGUF_Q4_0) {
+                                const uint32_t w0 = p ? q[i][0].z : q[i][0].x, w1 = p ? q[i][0].w : q[i][0].y;
+                                gguf_nibbles_f16(odd ? w1 : w0, v);
+                                put(2 * p + odd, v);
+                                gguf_nibbles_f16(odd ? w0 : w1, v);
+                                put(2 * p + (odd ^ 1), v);
+                            } else {
+                                const uint4 w = q[i][p < LOADS ? p : 0];
+                                gguf_bytes_f16(odd ? w.z : w.x, odd ? w.w : w.y, v);
+                                put(2 * p + odd, v);
+                                gguf_bytes_f16(odd ? w.x : w.z, odd ? w.y : w.w, v);
+                                put(2 * p + (odd ^ 1), v);
+                            }
+                        }
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) {
+                        pg_mbar_arrive(a_full + 8 * as);
+                        if (h == 1) pg_mbar_arrive(r_empty + 8 * rs);
+                    }
+                    as ^= 1;
+                    if (as == 0) ap ^= 1;
+                }
+                if (++rs == C::RST) {
+                    rs = 0;
+                    rp ^= 1;
+                }
+            }
+    } else {
+        // ---------------------------------------------------------------- sums and outputs: lane = row of W
+        const int q = warp & 3, half = (warp - 2) >> 2, row = q * 32 + lane;
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + half * C::HALF;
+        asm volatile("griddepcontrol.wait;" ::: "memory");     // y may still be read by the predecessor
+        uint32_t rs = 0, rp = 0, ts = 0, tp = 0;
+        for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+            const int tile = u / sp;
+            float sum[C::HALF];
+#pragma unroll
+            for (int j = 0; j < C::HALF; j++) sum[j] = 0.0f;
+            for (int s = s_first(u), end = s_end(u); ok && s < end; s++) {
+                ok = __all_sync(0xffffffffu, pg_mbar_wait(r_full + 8 * rs, rp, abort_flag, status, limit_ns));
+                if (!ok) break;
+                const uint4 sc = pg_lds128(r_at + rs * C::RAW + (uint32_t)(row >> 4) * C::FILL + 16 * C::SEG + (uint32_t)(row & 15) * 16);
+                const uint32_t scw[4] = {sc.x, sc.y, sc.z, sc.w};
+                __syncwarp();
+                if (lane == 0) pg_mbar_arrive(r_empty + 8 * rs);
+                if (++rs == C::RST) {
+                    rs = 0;
+                    rp ^= 1;
+                }
+#pragma unroll
+                for (int b = 0; b < 8; b++) {
+                    if (b % C::GB == 0) {
+                        ok = ok && pg_mbar_wait(t_full + 8 * ts, tp, abort_flag, status, limit_ns);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
+                    const __half2 hh = *reinterpret_cast<const __half2 *>(&scw[b >> 1]);
+                    const float d = (b & 1) ? __high2float(hh) : __low2float(hh);
+                    const uint32_t at = taddr + (ts * C::GB + b % C::GB) * C::COLS;
+                    if constexpr (C::STACK) gt_add<C::HALF>(at + MT, d, sum);
+                    gt_add<C::HALF>(at, d, sum);
+                    if ((b + 1) % C::GB == 0) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) pg_mbar_arrive(t_empty + 8 * ts);
+                        if (++ts == C::NBUF) {
+                            ts = 0;
+                            tp ^= 1;
+                        }
+                    }
+                }
+            }
+            if (!ok) break;
+            if (sp > 1) {
+                float *slab = kp.slabs + ((int64_t)u * MT + half * C::HALF) * GT_N + row;
+#pragma unroll
+                for (int j = 0; j < C::HALF; j++) __stcg(slab + j * GT_N, sum[j]);
+                unsigned int *ticket = kp.tickets + tile * 8 + half * 4 + q;
+                __threadfence();
+                __syncwarp();
+                const unsigned int before = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(ticket, 1u) : 0u, 0);
+                if (before != (unsigned)(sp - 1)) continue;
+                __threadfence();
+                if (lane == 0) *ticket = 0;
+                slab = kp.slabs + ((int64_t)tile * sp * MT + half * C::HALF) * GT_N + row;
+#pragma unroll
+                for (int j = 0; j < C::HALF; j++) sum[j] = __ldcg(slab + j * GT_N);
+                for (int p = 1; p < sp; p++) {
+                    slab += MT * GT_N;
+#pragma unroll
+                    for (int j = 0; j < C::HALF; j++) sum[j] += __ldcg(slab + j * GT_N);
+                }
+            }
+            const int64_t n = (int64_t)(tile / tiles_m) * GT_N + row;
+            const int m0 = (tile % tiles_m) * MT + half * C::HALF;
+            if (n < N) {
+                float *dst = y + (int64_t)m0 * N + n;
+#pragma unroll
+                for (int j = 0; j < C::HALF; j++)
+                    if (m0 + j < M) dst[j * N] = sum[j] * __ldcg(us + m0 + j);
+            }
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+// ---------------------------------------------------------------- host side ----
+int64_t gt_row_bytes(int64_t k) { return 4 * k + 4; }    // two planes and 2^-s
+
+template <int TYPE, int MT>
+int32_t gt_launch(pg_ctx *ctx, const pg_gguf_weight *w, const void *planes, const float *us, int64_t m, float *y, GtParts kp)
+{
+    using C = GtCfg<TYPE, MT>;
+    CUtensorMap tx;
+    const cuuint64_t dims[3] = {(cuuint64_t)w->k, (cuuint64_t)m, 2}, strides[2] = {(cuuint64_t)w->k * 2, (cuuint64_t)(w->k * m) * 2};
+    const cuuint32_t box[3] = {64, MT, 2};
+    const int32_t rc = pg_encode_bf16(&tx, planes, 3, dims, strides, box);   // (f16: the copies only move it)
+    if (rc != PG_OK) return rc;
+    auto kern = gguf_tc_kernel<TYPE, MT>;
+    static std::atomic<uint64_t> smem_set{0};
+    PG_CUDA(pg_max_smem_once(kern, (int)C::SMEM, ctx->device, smem_set));
+    const int64_t units = ((m + MT - 1) / MT) * ((w->n + GT_N - 1) / GT_N) * kp.parts;
+    kp.tickets = reinterpret_cast<unsigned int *>(ctx->splitk);
+    kp.slabs = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(ctx->splitk) + GT_TICKET_BYTES);
+    return launch_pdl(ctx, kern, dim3((unsigned)std::min<int64_t>(units, ctx->sm_count)), dim3(C::THREADS), C::SMEM, tx, (const uint8_t *)w->d_qs, w->n,
+                      (int)(w->k / 256), (int)m, us, y, kp, ctx->d_status, ctx->wait_limit_ns);
+}
+
+template <int TYPE>
+int32_t gt_run(pg_ctx *ctx, const pg_gguf_weight *w, const void *planes, const float *us, int64_t m, float *y)
+{
+    // rows per tile and parts of K: the fewest cycles by count -- slices of the busiest CTA and what a tile costs at its end, more
+    // where slabs meet.  Measured at N 14336, K 4096, a block of 32 k takes 350 / 430 / 570 / 800 / 930 cycles with 16 / 32 / 64 / 128 /
+    // 160 rows.
+    const int64_t nslices = w->k / 256, tiles_n = (w->n + GT_N - 1) / GT_N;
+    const int64_t room = (int64_t)(ctx->splitk_bytes > GT_TICKET_BYTES ? ctx->splitk_bytes - GT_TICKET_BYTES : 0) / (GT_N * (int64_t)sizeof(float));
+    static const int sizes[] = {16, 32, 64, 128, 160};
+    double best = 0;
+    int mt = 16;
+    GtParts kp = {1, (int)nslices, nullptr, nullptr};
+    for (int cand : sizes) {
+        if (cand < 64 && cand < m) continue;
+        if (cand > 16 && cand / 2 >= m) break;
+        const int64_t tiles = tiles_n * ((m + cand - 1) / cand);
+        for (int64_t parts = 1; parts <= std::min<int64_t>(16, nslices); parts++) {
+            const int64_t slices = (nslices + parts - 1) / parts;
+            if ((nslices + slices - 1) / slices != parts) continue;
+            if (parts > 1 && (tiles * parts * cand > room || tiles * 8 * (int64_t)sizeof(int) > (int64_t)GT_TICKET_BYTES)) break;
+            const int64_t rounds = (tiles * parts + ctx->sm_count - 1) / ctx->sm_count;
+            const double cost = rounds * (slices * 8.0 * (280.0 + cand * 4.0) + 1500.0 + cand * 8.0 + (parts > 1 ? 2500.0 + cand * parts * 4.0 : 0.0));
+            if (best == 0 || cost < best) {
+                best = cost;
+                mt = cand;
+                kp.parts = (int)parts;
+                kp.slices = (int)slices;
+            }
+        }
+    }
+    if (mt == 160) return gt_launch<TYPE, 160>(ctx, w, planes, us, m, y, kp);
+    if (mt == 128) return gt_launch<TYPE, 128>(ctx, w, planes, us, m, y, kp);
+    if (mt == 64) return gt_launch<TYPE, 64>(ctx, w, planes, us, m, y, kp);
+    if (mt == 32) return gt_launch<TYPE, 32>(ctx, w, planes, us, m, y, kp);
+    return gt_launch<TYPE, 16>(ctx, w, planes, us, m, y, kp);
+}
+
+}  // namespace
+
+bool pgk_matmul_gguf_tc_supports(const pg_gguf_weight *w, int64_t m)
+{
+    return w->tiled && m > 8 && m < (1 << 24) && w->n >= 1 && w->n < (1ll << 30);
+}
+
+int32_t pgk_gguf_tc_reserve(pg_ctx *ctx, int64_t k)
+{
+    const int32_t rc = pg_scratch_reserve(ctx, (size_t)(GT_ROWS * gt_row_bytes(k)));
+    if (rc != PG_OK) return rc;
+    return pg_splitk_reserve(ctx, GT_TICKET_BYTES + (size_t)ctx->sm_count * 3 * 64 * GT_N * sizeof(float));
+}
+
+int32_t pgk_matmul_gguf_tc(pg_ctx *ctx, const float *d_x, int64_t m, const pg_gguf_weight *w, float *d_y)
+{
+    // all rows at once if there is room for their planes; while a graph is recorded the workspace cannot grow, and what the upload
+    // has reserved then takes them in portions
+    int64_t portion = m;
+    if ((size_t)(m * gt_row_bytes(w->k)) > ctx->scratch_bytes) {
+        if (ctx->capturing) {
+            portion = (int64_t)(ctx->scratch_bytes / (size_t)gt_row_bytes(w->k)) / 16 * 16;
+            PG_REQUIRE(portion > 0, "matmul_gguf: the context has no workspace for %lld rows", (long long)m);
+        } else {
+            const int32_t rc = pg_scratch_reserve(ctx, (size_t)(m * gt_row_bytes(w->k)));
+            if (rc != PG_OK) return rc;
+        }
+    }
+    for (int64_t r0 = 0; r0 < m; r0 += portion) {
+        const int64_t rows = std::min(portion, m - r0);
+        uint4 *planes = reinterpret_cast<uint4 *>(ctx->scratch);
+        float *us = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(ctx->scratch) + rows * w->k * 4);
+        // (few rows: several CTAs each, which all look for the largest element)
+        const dim3 grid((unsigned)rows, (unsigned)std::max<int64_t>(1, std::min<int64_t>(w->k / 2048, 2 * ctx->sm_count / rows)));
+        int32_t rc = w->type == PG_GGUF_Q4_0
+                         ? launch_pdl(ctx, gguf_planes_kernel<true>, grid, dim3(256), 0, d_x, (int)r0, (int)rows, (int)w->k, planes, us)
+                         : launch_pdl(ctx, gguf_planes_kernel<false>, grid, dim3(256), 0, d_x, (int)r0, (int)rows, (int)w->k, planes, us);
+        if (rc != PG_OK) return rc;
+        rc = w->type == PG_GGUF_Q4_0 ? gt_run<PG_GGUF_Q4_0>(ctx, w, planes, us, rows, d_y + r0 * w->n)
+                                     : gt_run<PG_GGUF_Q8_0>(ctx, w, planes, us, rows, d_y + r0 * w->n);
+        if (rc != PG_OK) return rc;
+    }
+    return PG_OK;
+}

@@ -162,6 +162,58 @@ def test_matmul_gguf_tensor_core_path_edges(pg, gpu, oracle_mt, kind, m, n, k):
     assert np.abs(y - ref).max() <= REL_TOL * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("kind", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("n,k", [(1, 256), (127, 512), (128, 1024), (129, 4352), (700, 2304)])
+def test_matmul_gguf_many_rows(pg, gpu, oracle_mt, kind, n, k):
+    """Row counts around the tiles' sizes, element by element: two f16 planes hold 2^-22 of an element (2^-39 of its row's largest), a
+    block's instructions cut off 2^-23 of their sum, and there is one rounding to 2^-24 per block and part of K."""
+    g = rng(n + k)
+    raw = oracle_mt.encode(kind, normal(g, (n, k), 0.02))
+    w64 = oracle_mt.dequant(kind, raw, n * k).reshape(n, k).astype(np.float64)
+    w = pg.gguf.GgufWeight(kind, raw, n, k, gpu)
+    for m in (9, 16, 17, 32, 33, 64, 65, 128, 129, 160, 161, 330):
+        x = normal(g, (m, k))
+        x[:, ::97] *= 50.0
+        x[m // 2] *= 1e-30
+        x[m // 3] *= 1e30
+        x[m - 2] = 0.0
+        got = w.matmul(x, m)
+        x64 = np.abs(x).astype(np.float64)
+        bound = x64 @ np.abs(w64).T * (2.0 ** -22 + 4 * 2.0 ** -23 + (k // 32 + 18) * 2.0 ** -24) + x64.max(1, keepdims=True) * 2.0 ** -39 * np.abs(w64).sum(1)
+        assert (np.abs(got - x.astype(np.float64) @ w64.T) <= bound).all(), m
+        assert (got[m - 2] == 0).all()
+        x[1, k - 1], x[m - 1, 0] = np.inf, np.nan          # stays in its row
+        again = w.matmul(x, m)
+        assert np.isnan(again[[1, m - 1]]).all()
+        keep = [r for r in range(m) if r not in (1, m - 1)]
+        assert np.array_equal(again[keep], got[keep]), m
+    assert gpu.device_status() == 0
+    w.free()
+
+
+def test_matmul_gguf_many_rows_recorded_without_a_run_before(pg, oracle_mt):
+    """The workspace cannot grow in a recording: the rows then go through what the upload has reserved, in portions."""
+    import torch
+
+    g = pg.GpuContext()
+    n, k, m = 200, 512, 1000
+    w = pg.gguf.GgufWeight("q8_0", oracle_mt.encode("q8_0", normal(rng(8), (n, k), 0.02)), n, k, g)
+    x = torch.randn(m, k, device="cuda")
+    y, z = torch.zeros(m, n, device="cuda"), torch.zeros(m, n, device="cuda")
+    torch.cuda.synchronize()
+    with g.record() as graph:
+        w.matmul_device(x, m, y)
+    graph.launch()
+    g.sync()
+    w.matmul_device(x, m, z)
+    g.sync()
+    # (portions may divide K otherwise)
+    assert graph.kernels > 2 and torch.allclose(y, z, rtol=0, atol=1e-5 * z.abs().max().item()) and g.device_status() == 0
+    graph.free()
+    w.free()
+    g.close()
+
+
 def test_matmul_gguf_row_shard_and_errors(pg, gpu, oracle_mt):
     g = rng(7)
     n, k, m = 96, 256, 4
