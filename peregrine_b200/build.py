@@ -28,6 +28,7 @@ SOURCES = CORE + [
     "pg_quantize.cu",
     "pg_gemm_naive.cu",
     "pg_gemv_w8a8.cu", "pg_gemv_wstream.cu",
+    "pg_gemm_i8_mid.cu",
     "pg_gemm_tcgen05.cu",
     "pg_gemm_tcgen05_2cta.cu",
     "pg_gguf.cu",

@@ -42,6 +42,17 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t desc_a, uint6
         ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(on)
         : "memory");
 }
+// signed bytes, s32 sums
+__device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t on)
+{
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(on)
+        : "memory");
+}
 // A (bf16, two per 32-bit column) from TMEM
 __device__ __forceinline__ void umma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t on)
 {
@@ -125,8 +136,9 @@ __host__ __device__ constexpr uint32_t make_idesc(int m, int n)
 typedef CUresult (*PgEncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                                     const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// bf16 tensor; the box's inner extent is 64 elements (one 128-byte swizzle span); reads past the edge give 0
-inline int32_t pg_encode_bf16(CUtensorMap *map, const void *ptr, int rank, const cuuint64_t *dims, const cuuint64_t *strides, const cuuint32_t *box)
+// the box's inner extent is one 128-byte swizzle span; reads past the edge give 0
+inline int32_t pg_encode_map(CUtensorMap *map, CUtensorMapDataType type, const void *ptr, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
+                             const cuuint32_t *box)
 {
     static PgEncodeTiledFn enc = nullptr;
     if (!enc) {
@@ -137,8 +149,13 @@ inline int32_t pg_encode_bf16(CUtensorMap *map, const void *ptr, int rank, const
     }
     if (!enc) PG_FAIL(PG_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void *>(ptr), dims, strides, box, estr,
+    const CUresult r = enc(map, type, (cuuint32_t)rank, const_cast<void *>(ptr), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) PG_FAIL(PG_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
     return PG_OK;
+}
+// bf16 tensor: 64 elements per span
+inline int32_t pg_encode_bf16(CUtensorMap *map, const void *ptr, int rank, const cuuint64_t *dims, const cuuint64_t *strides, const cuuint32_t *box)
+{
+    return pg_encode_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, ptr, rank, dims, strides, box);
 }
