@@ -1,9 +1,9 @@
 // Prefill-size W8A8 product on CTA pairs: the integer GEMM of src/quant.rs:154-166 /
 // simd_kernels::gemm_i8_sdot (src/simd_kernels.rs:1087-1214) with tcgen05.mma.cta_group::2.
 //
-// Two CTAs of a thread-block cluster (two SMs) compute one 256 x 256 tile together.  Each CTA
-// stages its own 128 rows of A and ITS HALF (128 rows) of the B tile, and one thread of the leader
-// CTA issues MMAs that read both CTAs' shared memory; each CTA's tensor memory receives its 128
+// Two CTAs of a thread-block cluster (two SMs) compute one 256 x 256 tile together (or 256 x 224 / 192
+// where that fills the last round of tiles better).  Each CTA stages its own 128 rows of A and ITS HALF
+// (128 rows) of the B tile, and one lane of the leader CTA's warp 1 issues MMAs that read both CTAs' shared memory; each CTA's tensor memory receives its 128
 // rows of the accumulator.  Compared with one CTA per 128 x 256 tile this moves a third fewer
 // operand bytes from L2 per multiply-accumulate, which is what bounds the one-CTA kernel (its
 // shared memory cannot hold more bytes in flight).  No multicast load is used: every CTA fetches
@@ -19,21 +19,26 @@
 // word, CTA-wide abort flag, normal teardown including the TMEM release).
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "pg_internal.cuh"
 #include "pg_tc_epilogue.cuh"
 
 namespace {
 
 constexpr int TM = 128;        // rows of A per CTA
-constexpr int TNH = 128;       // rows of B per CTA (half of the 256-wide tile)
-constexpr int TN = 256;
 constexpr int BK = 128;        // bytes of K per stage = one 128-byte swizzle span
 constexpr int UMMA_K = 32;
-constexpr int STAGES = 6;
-constexpr int STAGE_A = TM * BK, STAGE_B = TNH * BK, STAGE = STAGE_A + STAGE_B;   // 32 KiB
 constexpr int NUM_THREADS = 192;
 constexpr int TMEM_COLS = 512;  // two 256-column accumulators
-constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE + 1024 + 256 + 4 * PG_EPI_WARP_BYTES;
+// TNH: rows of B per CTA, half of the tile's width
+template <int TNH>
+struct Cfg {
+    static constexpr int TN = 2 * TNH;
+    static constexpr int STAGE_A = TM * BK, STAGE = STAGE_A + TNH * BK;   // 32 KiB at 256 columns
+    static constexpr int STAGES = (232448 - (1024 + 256 + 4 * PG_EPI_WARP_BYTES)) / STAGE;
+    static constexpr size_t SMEM = (size_t)STAGES * STAGE + 1024 + 256 + 4 * PG_EPI_WARP_BYTES;
+};
 constexpr unsigned long long WAIT_LIMIT_NS = 1000ull * 1000ull * 1000ull;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -112,22 +117,26 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void umma_i8_pair(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
+__device__ __forceinline__ void umma_i8_pair(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t on)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-        ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(on)
         : "memory");
 }
 // arrives on the barrier at this shared-memory offset in both CTAs of the pair
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar)
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint32_t on)
 {
     const uint16_t mask = 3;
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-                 "h"(mask)
-                 : "memory");
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar),
+        "h"(mask), "r"(on)
+        : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32])
 {
@@ -155,13 +164,15 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr)
     return d;
 }
 // kind::i8: D = s32, A/B = s8, K-major, N >> 3 at bit 17, M >> 4 at bit 24 (M = 256 over the pair)
-constexpr uint32_t IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+__host__ __device__ constexpr uint32_t make_idesc(int n) { return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24); }
 
+template <int TNH>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
     gemm_i8_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                                 const float *__restrict__ a_scales, const float *__restrict__ w_scales, int M, int N, int K,
                                 float *__restrict__ y, int32_t *__restrict__ acc_out, int32_t *status)
 {
+    constexpr int TN = Cfg<TNH>::TN, STAGE_A = Cfg<TNH>::STAGE_A, STAGE = Cfg<TNH>::STAGE, STAGES = Cfg<TNH>::STAGES;
     // programmatic dependent launch: see gemm_i8_tcgen05_kernel; the predecessor's output (activations, their scales) is
     // touched only behind griddepcontrol.wait
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -256,33 +267,37 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             }
         }
     } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issuer (leader only)
-        if (leader && lane == 0) {
+        // ---------------------------------------------------------------- MMA issuer (leader only; the whole warp, one lane's count:
+        // issued from a branch that one thread is in, an MMA costs 112 cycles of issue, so about 40; at 224 columns it runs for 112)
+        if (leader) {
+            uint32_t on;
+            asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(on));
+            constexpr uint32_t idesc = make_idesc(TN);
             uint32_t stage = 0, phase = 0;
             uint32_t acc = 0, acc_phase = 0;
             bool ok = true;
             for (int t = pair; ok && t < total_tiles; t += npairs) {
-                if (!(ok = mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, status))) break;
+                if (!(ok = __all_sync(0xffffffffu, mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, status)))) break;
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + acc * TN;
+                const uint32_t d_tmem = tmem_base + acc * 256;
                 for (int kb = 0; kb < kblocks; kb++) {
-                    if (!(ok = mbar_wait(bar_full + 8 * stage, phase, abort_flag, status))) break;
+                    if (!(ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * stage, phase, abort_flag, status)))) break;
                     tc_fence_after();
                     const uint32_t sa = base + stage * STAGE;
                     const uint64_t da = make_smem_desc(sa);
                     const uint64_t db = make_smem_desc(sa + STAGE_A);
 #pragma unroll
                     for (int j = 0; j < BK / UMMA_K; j++)
-                        umma_i8_pair(d_tmem, da + (uint64_t)(j * (UMMA_K >> 4)), db + (uint64_t)(j * (UMMA_K >> 4)), IDESC,
-                                     (kb | j) != 0 ? 1u : 0u);
-                    umma_commit_pair(bar_empty + 8 * stage);
+                        umma_i8_pair(d_tmem, da + (uint64_t)(j * (UMMA_K >> 4)), db + (uint64_t)(j * (UMMA_K >> 4)), idesc,
+                                     (kb | j) != 0 ? 1u : 0u, on);
+                    umma_commit_pair(bar_empty + 8 * stage, on);
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
                 if (!ok) break;
-                umma_commit_pair(bar_tfull + 8 * acc);
+                umma_commit_pair(bar_tfull + 8 * acc, on);
                 if (++acc == 2) {
                     acc = 0;
                     acc_phase ^= 1;
@@ -307,7 +322,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             const int row_base = m0 + q * 32;
             const int row = row_base + lane;
             const float as = (row < M && y) ? a_scales[row] : 0.0f;
-            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * TN;
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * 256;
             const uint32_t stage_buf = base + (uint32_t)((size_t)STAGES * STAGE) + 256u + (uint32_t)q * PG_EPI_WARP_BYTES;
 #pragma unroll 1
             for (int c = 0; c < TN; c += 32) {
@@ -388,12 +403,11 @@ int32_t encode_kmajor(CUtensorMap *map, const void *ptr, int64_t rows, int64_t k
     return PG_OK;
 }
 
-}  // namespace
-
-int32_t pgk_gemm_i8_tcgen05_2cta(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, pg_qtensor *w,
-                                 float *d_y, int32_t *d_acc)
+template <int TNH>
+int32_t launch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, pg_qtensor *w, float *d_y, int32_t *d_acc)
 {
-    const int M = (int)m, K = (int)k, N = (int)w->cols;
+    using C = Cfg<TNH>;
+    const int N = (int)w->cols;
     CUtensorMap ta;
     int32_t rc = encode_kmajor(&ta, d_a, M, K, TM);
     if (rc) return rc;
@@ -402,15 +416,15 @@ int32_t pgk_gemm_i8_tcgen05_2cta(pg_ctx *ctx, const int8_t *d_a, const float *d_
         if (rc) return rc;
         w->tmap_b_box_rows = TNH;
     }
+    auto kern = gemm_i8_tcgen05_2cta_kernel<TNH>;
     static std::atomic<uint64_t> smem_set{0};
-    PG_CUDA(pg_max_smem_once(gemm_i8_tcgen05_2cta_kernel, (int)SMEM_BYTES, ctx->device, smem_set));
-    const int tiles = ((M + 2 * TM - 1) / (2 * TM)) * ((N + TN - 1) / TN);
-    const int max_pairs = ctx->sm_count / 2;
-    const int pairs = tiles < max_pairs ? tiles : max_pairs;
+    PG_CUDA(pg_max_smem_once(kern, (int)C::SMEM, ctx->device, smem_set));
+    const int64_t tiles = (int64_t)((M + 2 * TM - 1) / (2 * TM)) * ((N + C::TN - 1) / C::TN);
+    const int pairs = (int)std::min<int64_t>(tiles, ctx->sm_count / 2);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
     cfg.blockDim = dim3(NUM_THREADS);
-    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -421,8 +435,33 @@ int32_t pgk_gemm_i8_tcgen05_2cta(pg_ctx *ctx, const int8_t *d_a, const float *d_
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    PG_CUDA(cudaLaunchKernelEx(&cfg, gemm_i8_tcgen05_2cta_kernel, ta, *reinterpret_cast<CUtensorMap *>(w->tmap_b), d_as,
-                               (const float *)w->d_scales, M, N, K, d_y, d_acc, ctx->d_status));
+    PG_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, *reinterpret_cast<CUtensorMap *>(w->tmap_b), d_as, (const float *)w->d_scales, M, N, K, d_y, d_acc,
+                               ctx->d_status));
     PG_LAUNCHED();
     return PG_OK;
+}
+
+}  // namespace
+
+int32_t pgk_gemm_i8_tcgen05_2cta(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, pg_qtensor *w,
+                                 float *d_y, int32_t *d_acc)
+{
+    // The width whose rounds of tiles take least: a pair runs ceil(tiles / pairs) tiles, each as long as it is wide (and some 16 columns'
+    // worth at its end).  M 2048, N 14336: 448 tiles of 256 columns are 6.05 rounds on 74 pairs, the seventh nearly empty; 512 of 224
+    // are 6.92.  Narrower tiles take more bytes per multiplication, so they have to win by 3 %.
+    auto cost = [&](int tn) {
+        const int64_t tiles = ((m + 2 * TM - 1) / (2 * TM)) * ((w->cols + tn - 1) / tn), pairs = ctx->sm_count / 2;
+        return (double)((tiles + pairs - 1) / pairs) * (tn + 16);
+    };
+    double best = cost(256);
+    int width = 256;
+    for (int tn = 224; tn >= 192; tn -= 32)
+        if (cost(tn) < 0.97 * best) {
+            best = cost(tn);
+            width = tn;
+        }
+    const int M = (int)m, K = (int)k;
+    if (width == 224) return launch<112>(ctx, d_a, d_as, M, K, w, d_y, d_acc);
+    if (width == 192) return launch<96>(ctx, d_a, d_as, M, K, w, d_y, d_acc);
+    return launch<128>(ctx, d_a, d_as, M, K, w, d_y, d_acc);
 }
