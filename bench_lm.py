@@ -302,8 +302,8 @@ def kernel_figures(torch, gpu, hbm: float, tflops: float) -> dict:
 
         def delta(state, b):
             mx.c.d_work = d.buffer("delta.work", 1, 1, torch.float32).data_ptr()
-            d.check(d.lib.pg_delta_run(gpu.handle, C.byref(mx.c), C.byref(b.c), proj.data_ptr(), proj.stride(0), state["ring"].data_ptr(),
-                                       state["state"].data_ptr(), mixed.data_ptr(), d.code, mixed.stride(0)))
+            d.check(mx.kernel(gpu.handle, C.byref(mx.c), C.byref(b.c), proj.data_ptr(), proj.stride(0), state["ring"].data_ptr(),
+                              state["state"].data_ptr(), mixed.data_ptr(), d.code, mixed.stride(0)))
         note(f"delta.step.b{B}", time_us([(lambda s=s: delta(s, batch)) for s in states]), nbytes=B * 2 * 32 * 128 * 128 * 4)
         if B == 16:
             long = Batch(d, [(0, 0, [1] * T)], fixed=True)

@@ -197,6 +197,8 @@ LM_SIGNATURES = {
     "pg_norm_rows": (_i32, [_vp, _vp, _vp, _i64, _i64, _vp, _f, _vp, _i32, _i64]),
     "pg_delta_work_floats": (_i64, [_pd, _i64]),
     "pg_delta_run": (_i32, [_vp, _pd, _pb, _vp, _i64, _vp, _vp, _vp, _i32, _i64]),
+    "pg_delta_chunks_work_floats": (_i64, [_pd, _i64]),
+    "pg_delta_run_chunks": (_i32, [_vp, _pd, _pb, _vp, _i64, _vp, _vp, _vp, _i32, _i64]),
     "pg_attention_part_floats": (_i64, [_vp, _pa, _i64]),
     "pg_attention_run": (_i32, [_vp, _pa, _pb, _vp, _i64, _vp, _vp, _vp, _i32, _i64]),
     "pg_latent_part_floats": (_i64, [_vp, _pl, _i32, _i64, _i64]),

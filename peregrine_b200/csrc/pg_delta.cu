@@ -17,37 +17,14 @@
 // Convolution inputs are kept per slot in a ring of `taps` entries, position p in entry p mod taps: a single token
 // writes an entry that nobody reads any more, so heads that share channels need no order among their CTAs.
 // A sequence starts at position 0: what its slot holds is then taken as zero.
+#include <algorithm>
+#include <climits>
+
 #include "pg_async.cuh"
+#include "pg_delta.cuh"
 #include "pg_lm.cuh"
 
 namespace {
-
-struct DeltaShape {
-    int H, G, D, V, taps, C;        // C: convolution channels 2 G D + H V
-    int vs;                         // state row stride
-    float eps, unit_eps, qscale;
-    const float *conv, *a_log, *dt_bias, *norm;
-};
-
-__device__ __forceinline__ float softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
-__device__ __forceinline__ float log_decay(float a, float a_log, float dt_bias) { return -expf(a_log) * softplus(a + dt_bias); }
-
-// one channel of the convolution at position pos; row: this token's input row, t: tokens of the same sequence and step
-// in front of it; older inputs come from the ring
-__device__ __forceinline__ float conv_at(const DeltaShape &s, const float *row, int64_t ldp, const float *ring, int c, int t, int pos)
-{
-    float acc = 0.0f;
-    for (int j = 0; j < s.taps; j++) {
-        const int back = s.taps - 1 - j;                  // tokens back
-        float x = 0.0f;
-        if (back <= t)
-            x = __ldcg(row - (int64_t)back * ldp + c);
-        else if (back <= pos)
-            x = __ldcg(ring + (int64_t)((pos - back) % s.taps) * s.C + c);
-        acc = fmaf(__ldg(s.conv + (int64_t)j * s.C + c), x, acc);
-    }
-    return pg_silu(acc);
-}
 
 // ---- one token per sequence: grid (H, rows) ----------------------------------------------------------------------
 constexpr int DS_T = 256;
@@ -229,15 +206,12 @@ __global__ void __launch_bounds__(DS_T)
 }
 
 // ---- longer portions ---------------------------------------------------------------------------------------------
-// work rows: q [G D] | k [G D] | v [H V] | o [H V] per token; coef: 32 floats per block of four tokens and head.  With the
-// decays g_a of a block's tokens, c_a = g_0 .. g_a and r_ab = g_{b+1} .. g_a:
+// coef: 32 floats per block of four tokens and head.  With the decays g_a of a block's tokens, c_a = g_0 .. g_a and
+// r_ab = g_{b+1} .. g_a:
 //   u_a = beta_a (v_a - c_a S^T k_a - sum_{b<a} r_ab (k_b . k_a) u_b)
 //   o_a = c_a S^T q_a + sum_{b<=a} r_ab (k_b . q_a) u_b
 //   S <- c_3 S + sum_b r_3b k_b u_b^T
-// coef: c [4] | beta [4] | r_3b [4] | r_ab (k_b . k_a) of the 6 pairs b < a | r_ab (k_b . q_a) of the 10 pairs b <= a
-struct DeltaWork {
-    float *q, *k, *v, *o, *coef;
-};
+// they hold c [4] | beta [4] | r_3b [4] | r_ab (k_b . k_a) of the 6 pairs b < a | r_ab (k_b . q_a) of the 10 pairs b <= a
 constexpr int BT = 4;            // tokens of a block
 // blocks of a sequence are numbered from here on
 __device__ __forceinline__ int64_t first_block(int row0, int seq) { return row0 / BT + seq; }
@@ -271,13 +245,14 @@ __device__ __forceinline__ void store_lanes(float *p, const Lanes<V> &r)
 // groups of channels start on 16-byte boundaries)
 template <int TAPS, int V>
 __global__ void __launch_bounds__(256)
-    delta_prep_kernel(const DeltaShape s, const pg_batch bt, const float *__restrict__ proj, int64_t ldp, const float *__restrict__ ring, const DeltaWork w)
+    delta_prep_kernel(const DeltaShape s, const pg_batch bt, const float *__restrict__ proj, int64_t ldp, const float *__restrict__ ring, const DeltaWork w,
+                      int most)
 {
     extern __shared__ __align__(16) float sm[];   // q and k channels [4][2 G D], then the pairs' products [G][16]
     pg_pdl_begin();
     const int seq = blockIdx.y, row0 = __ldcg(bt.d_seq_row0 + seq), T = __ldcg(bt.d_seq_row0 + seq + 1) - row0;
     const int t0 = blockIdx.x * BT, n = min(BT, T - t0), m0 = row0 + t0;
-    if (n <= 0) return;
+    if (n <= 0 || T > most) return;
     const int pos0 = __ldcg(bt.d_pos + row0);
     const float *row = proj + (int64_t)m0 * ldp;
     const float *rg = ring + (int64_t)__ldcg(bt.d_seq_slot + seq) * s.taps * s.C;
@@ -438,7 +413,7 @@ struct ScanTile {
 };
 
 template <int NI>
-__global__ void __launch_bounds__(128) delta_scan_kernel(const DeltaShape s, const pg_batch bt, const DeltaWork w, float *state)
+__global__ void __launch_bounds__(128) delta_scan_kernel(const DeltaShape s, const pg_batch bt, const DeltaWork w, float *state, int most)
 {
     using C = ScanTile<NI>;
     constexpr int DP = C::DP, TB = C::TB;
@@ -447,7 +422,7 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(const DeltaShape s, con
     // (launched whole, and the successor is not let in early either)
     const int h = blockIdx.y, seq = blockIdx.z, g = h / (s.H / s.G), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row0 = __ldcg(bt.d_seq_row0 + seq), T = __ldcg(bt.d_seq_row0 + seq + 1) - row0;
-    if (T <= 0) return;
+    if (T <= 0 || T > most) return;
     const int pos0 = __ldcg(bt.d_pos + row0);
     const int c0 = blockIdx.x * 32, col = warp * 8 + (lane >> 3) * 2, l = lane & 7, par = lane & 1;
     const int64_t block0 = first_block(row0, seq);
@@ -609,30 +584,33 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(const DeltaShape s, con
 }
 
 template <int NI>
-int32_t run_scan(pg_ctx *ctx, const DeltaShape &s, const pg_batch *bt, const DeltaWork &w, float *state)
+int32_t run_scan(pg_ctx *ctx, const DeltaShape &s, const pg_batch *bt, const DeltaWork &w, float *state, int most)
 {
     constexpr int smem = ScanTile<NI>::STAGES * (int)sizeof(typename ScanTile<NI>::Stage);
     static std::atomic<uint64_t> set{0};
     PG_CUDA(pg_max_smem_once(delta_scan_kernel<NI>, smem, ctx->device, set));
-    return launch_whole(ctx, delta_scan_kernel<NI>, dim3((unsigned)((s.V + 31) / 32), (unsigned)s.H, (unsigned)bt->seqs), dim3(128), (size_t)smem, s, *bt, w, state);
+    return launch_whole(ctx, delta_scan_kernel<NI>, dim3((unsigned)((s.V + 31) / 32), (unsigned)s.H, (unsigned)bt->seqs), dim3(128), (size_t)smem, s, *bt, w, state, most);
 }
 
 template <int TAPS, int V>
-int32_t run_prep_v(pg_ctx *ctx, const DeltaShape &s, const pg_batch *bt, const float *proj, int64_t ldp, const float *ring, const DeltaWork &w)
+int32_t run_prep_v(pg_ctx *ctx, const DeltaShape &s, const pg_batch *bt, const float *proj, int64_t ldp, const float *ring, const DeltaWork &w,
+                   int most)
 {
     const size_t smem = ((size_t)BT * 2 * s.G * s.D + 16 * s.G) * 4;
     PG_REQUIRE(smem <= 220 * 1024, "delta: too many query / key channels");
     static std::atomic<uint64_t> set{0};
     PG_CUDA(pg_max_smem_once(delta_prep_kernel<TAPS, V>, 220 * 1024, ctx->device, set));
-    return launch_pdl(ctx, delta_prep_kernel<TAPS, V>, dim3((unsigned)((bt->max_len + BT - 1) / BT), (unsigned)bt->seqs), dim3(256), smem, s, *bt, proj, ldp, ring, w);
+    return launch_pdl(ctx, delta_prep_kernel<TAPS, V>, dim3((unsigned)((std::min(bt->max_len, most) + BT - 1) / BT), (unsigned)bt->seqs), dim3(256), smem, s, *bt, proj, ldp, ring, w,
+                      most);
 }
 
 template <int TAPS>
-int32_t run_prep(pg_ctx *ctx, const DeltaShape &s, const pg_batch *bt, const float *proj, int64_t ldp, const float *ring, const DeltaWork &w)
+int32_t run_prep(pg_ctx *ctx, const DeltaShape &s, const pg_batch *bt, const float *proj, int64_t ldp, const float *ring, const DeltaWork &w,
+                 int most)
 {
     const bool vec = ((2 * s.G * s.D) & 3) == 0 && ((s.H * s.V) & 3) == 0 && ldp % 4 == 0 &&
                      (((uintptr_t)proj | (uintptr_t)ring | (uintptr_t)s.conv | (uintptr_t)w.v) & 15) == 0;
-    return vec ? run_prep_v<TAPS, 4>(ctx, s, bt, proj, ldp, ring, w) : run_prep_v<TAPS, 1>(ctx, s, bt, proj, ldp, ring, w);
+    return vec ? run_prep_v<TAPS, 4>(ctx, s, bt, proj, ldp, ring, w, most) : run_prep_v<TAPS, 1>(ctx, s, bt, proj, ldp, ring, w, most);
 }
 
 // a CTA per token: o / rms(o) * norm * silu(gate) per head; the sequence's last taps - 1 tokens also store their
@@ -707,22 +685,9 @@ DeltaShape shape_of(const pg_delta *p)
     return s;
 }
 
-}  // namespace
-
-extern "C" {
-
-PG_API int64_t pg_delta_work_floats(const pg_delta *p, int64_t max_rows)
+int32_t run_delta(pg_ctx *ctx, const pg_delta *p, const pg_batch *batch, const float *d_proj, int64_t ldp, float *d_ring, float *d_state, void *d_out,
+                  int32_t dtype, int64_t ldo, bool by_chunks)
 {
-    if (!p || max_rows < 0) return 0;
-    const int64_t G = p->kv_heads, H = p->heads, D = p->dim, V = p->vdim;
-    // (a block of four tokens per sequence may be a single token)
-    return max_rows * (2 * G * D + 2 * H * V) + (max_rows + 8) * H * 32 + 64;
-}
-
-PG_API int32_t pg_delta_run(pg_ctx *ctx, const pg_delta *p, const pg_batch *batch, const float *d_proj, int64_t ldp, float *d_ring, float *d_state,
-                            void *d_out, int32_t dtype, int64_t ldo)
-{
-    PG_ENTER(ctx);
     PG_REQUIRE(p && batch && d_proj && d_ring && d_state && d_out && p->d_work, "delta: null pointer");
     PG_REQUIRE(p->heads > 0 && p->kv_heads > 0 && p->heads % p->kv_heads == 0 && p->dim > 0 && p->dim <= 256 && p->vdim > 0 && p->vdim <= 1024 && p->taps >= 1,
                "delta: bad shape (heads %d / %d, dim %d <= 256, vdim %d <= 1024, taps %d)", p->heads, p->kv_heads, p->dim, p->vdim, p->taps);
@@ -752,35 +717,75 @@ PG_API int32_t pg_delta_run(pg_ctx *ctx, const pg_delta *p, const pg_batch *batc
     w.k = at, at += pg_up((int64_t)M * s.G * s.D, 4);
     w.v = at, at += pg_up((int64_t)M * s.H * s.V, 4);
     w.o = at, at += pg_up((int64_t)M * s.H * s.V, 4);
-    w.coef = at;
-    int32_t rc;
-    if (s.taps == 2)
-        rc = run_prep<2>(ctx, s, batch, d_proj, ldp, d_ring, w);
-    else if (s.taps == 3)
-        rc = run_prep<3>(ctx, s, batch, d_proj, ldp, d_ring, w);
-    else if (s.taps == 4)
-        rc = run_prep<4>(ctx, s, batch, d_proj, ldp, d_ring, w);
-    else
-        rc = run_prep<0>(ctx, s, batch, d_proj, ldp, d_ring, w);
+    w.coef = at, at += (int64_t)(M + 8) * s.H * 32;
+    w.chunks = reinterpret_cast<unsigned char *>(((uintptr_t)at + 127) & ~(uintptr_t)127);
+    const bool chunks = by_chunks && batch->max_len >= DELTA_CHUNK && pgk_delta_chunk_supports(s, d_proj, ldp, d_ring, d_state);
+    int32_t rc = PG_OK;
+    if (chunks) rc = pgk_delta_chunk(ctx, s, batch, d_proj, ldp, d_ring, w, d_state);
     if (rc != PG_OK) return rc;
-    if (s.D <= 32)
-        rc = run_scan<1>(ctx, s, batch, w, d_state);
-    else if (s.D <= 64)
-        rc = run_scan<2>(ctx, s, batch, w, d_state);
-    else if (s.D <= 96)
-        rc = run_scan<3>(ctx, s, batch, w, d_state);
-    else if (s.D <= 128)
-        rc = run_scan<4>(ctx, s, batch, w, d_state);
-    else if (s.D <= 192)
-        rc = run_scan<6>(ctx, s, batch, w, d_state);
-    else
-        rc = run_scan<8>(ctx, s, batch, w, d_state);
+    // (sequences of equal length are all of one kind)
+    if (!chunks || (int64_t)batch->seqs * batch->max_len != M) {
+        const int most = chunks ? DELTA_CHUNK - 1 : INT_MAX;
+        if (s.taps == 2)
+            rc = run_prep<2>(ctx, s, batch, d_proj, ldp, d_ring, w, most);
+        else if (s.taps == 3)
+            rc = run_prep<3>(ctx, s, batch, d_proj, ldp, d_ring, w, most);
+        else if (s.taps == 4)
+            rc = run_prep<4>(ctx, s, batch, d_proj, ldp, d_ring, w, most);
+        else
+            rc = run_prep<0>(ctx, s, batch, d_proj, ldp, d_ring, w, most);
+        if (rc != PG_OK) return rc;
+        if (s.D <= 32)
+            rc = run_scan<1>(ctx, s, batch, w, d_state, most);
+        else if (s.D <= 64)
+            rc = run_scan<2>(ctx, s, batch, w, d_state, most);
+        else if (s.D <= 96)
+            rc = run_scan<3>(ctx, s, batch, w, d_state, most);
+        else if (s.D <= 128)
+            rc = run_scan<4>(ctx, s, batch, w, d_state, most);
+        else if (s.D <= 192)
+            rc = run_scan<6>(ctx, s, batch, w, d_state, most);
+        else
+            rc = run_scan<8>(ctx, s, batch, w, d_state, most);
+    }
     if (rc != PG_OK) return rc;
     const bool vec = s.V % 4 == 0 && s.V <= 128 && s.C % 4 == 0 && ldp % 4 == 0 && ldo % 4 == 0 &&
                      (((uintptr_t)d_proj | (uintptr_t)d_out | (uintptr_t)s.norm | (uintptr_t)w.o) & 15) == 0;
     if (dtype == PG_BF16)
         return launch_pdl(ctx, delta_out_kernel<bf16>, dim3((unsigned)M), dim3(256), 0, s, *batch, d_proj, ldp, w, d_ring, (bf16 *)d_out, ldo, vec);
     return launch_pdl(ctx, delta_out_kernel<float>, dim3((unsigned)M), dim3(256), 0, s, *batch, d_proj, ldp, w, d_ring, (float *)d_out, ldo, vec);
+}
+
+}  // namespace
+
+extern "C" {
+
+PG_API int64_t pg_delta_work_floats(const pg_delta *p, int64_t max_rows)
+{
+    if (!p || max_rows < 0) return 0;
+    const int64_t G = p->kv_heads, H = p->heads, D = p->dim, V = p->vdim;
+    // (a block of four tokens per sequence may be a single token)
+    return max_rows * (2 * G * D + 2 * H * V) + (max_rows + 8) * H * 32 + 64;
+}
+
+PG_API int32_t pg_delta_run(pg_ctx *ctx, const pg_delta *p, const pg_batch *batch, const float *d_proj, int64_t ldp, float *d_ring, float *d_state,
+                            void *d_out, int32_t dtype, int64_t ldo)
+{
+    PG_ENTER(ctx);
+    return run_delta(ctx, p, batch, d_proj, ldp, d_ring, d_state, d_out, dtype, ldo, false);
+}
+
+PG_API int64_t pg_delta_chunks_work_floats(const pg_delta *p, int64_t max_rows)
+{
+    if (!p || max_rows < 0) return 0;
+    return pg_delta_work_floats(p, max_rows) + pgk_delta_chunk_floats(p->kv_heads, p->heads, p->dim, p->vdim, max_rows);
+}
+
+PG_API int32_t pg_delta_run_chunks(pg_ctx *ctx, const pg_delta *p, const pg_batch *batch, const float *d_proj, int64_t ldp, float *d_ring, float *d_state,
+                                   void *d_out, int32_t dtype, int64_t ldo)
+{
+    PG_ENTER(ctx);
+    return run_delta(ctx, p, batch, d_proj, ldp, d_ring, d_state, d_out, dtype, ldo, true);
 }
 
 }  // extern "C"

@@ -150,12 +150,14 @@ def stack_rows(d: Device, parts, multiple: int = 4):
 
 # ---- mixers: weights are shared by layers that name another layer's; state is per layer ---------------------------
 class GatedDelta:
-    """p: heads, kv_heads, dim, vdim, conv (taps).  W: name -> host array, the tensors of one mixer."""
+    """p: heads, kv_heads, dim, vdim, conv (taps).  W: name -> host array, the tensors of one mixer.  chunks: long portions go by
+    chunks of 64 tokens where the kernels have that form; else by blocks of four."""
 
     UNIT_EPS = 1e-6
 
-    def __init__(self, d: Device, p: dict, W, width: int, eps: float):
+    def __init__(self, d: Device, p: dict, W, width: int, eps: float, chunks: bool = True):
         self.d, self.p, self.eps = d, p, float(eps)
+        self.kernel, work = (d.lib.pg_delta_run_chunks, d.lib.pg_delta_chunks_work_floats) if chunks else (d.lib.pg_delta_run, d.lib.pg_delta_work_floats)
         H, G, D, V, taps = (int(p[k]) for k in ("heads", "kv_heads", "dim", "vdim", "conv"))
         self.H, self.G, self.D, self.V, self.taps = H, G, D, V, taps
         self.channels = 2 * G * D + H * V
@@ -169,7 +171,7 @@ class GatedDelta:
         self.c = _lib.PgDelta(H, G, D, V, taps, self.eps, self.UNIT_EPS, self.conv.data_ptr(), self.a_log.data_ptr(), self.dt_bias.data_ptr(),
                               self.norm.data_ptr(), 0)
         # shared buffers exist before the first step: torch fills them on a stream of its own
-        d.buffer("delta.work", 1, d.lib.pg_delta_work_floats(C.byref(self.c), d.rows), d.torch.float32)
+        d.buffer("delta.work", 1, work(C.byref(self.c), d.rows), d.torch.float32)
         d.buffer("proj", self.proj.n, dtype=d.torch.float32)
         d.buffer("mixed", self.out.k)
 
@@ -185,8 +187,8 @@ class GatedDelta:
         mixed = d.buffer("mixed", self.out.k)
         self.proj.run(h, rows, proj)
         self.c.d_work = d.buffer("delta.work", 1, 1, d.torch.float32).data_ptr()
-        d.check(d.lib.pg_delta_run(d.gpu.handle, C.byref(self.c), C.byref(batch.c), proj.data_ptr(), proj.stride(0), state["ring"].data_ptr(),
-                                   state["state"].data_ptr(), mixed.data_ptr(), d.code, mixed.stride(0)))
+        d.check(self.kernel(d.gpu.handle, C.byref(self.c), C.byref(batch.c), proj.data_ptr(), proj.stride(0), state["ring"].data_ptr(),
+                            state["state"].data_ptr(), mixed.data_ptr(), d.code, mixed.stride(0)))
         self.out.run(mixed, rows, y)
 
     def bytes(self) -> int:

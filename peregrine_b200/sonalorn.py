@@ -59,13 +59,15 @@ class SonalornModel(ResidualModel):
 
     def build(self, weights) -> None:
         cfg, d = self.cfg, self.d
+        # A router turns the last bit of a near tie into another expert: models with experts keep the order of sums that they have had
+        routed = any(L.get("mlp") and L["mlp"]["kind"] != "dense" for L in cfg.layers)
         self.pos, self.embed_norm = self.matrix("pos", cfg.max_positions), self.vector("embed.norm")
 
         def tensors(i, L):
             mix = Below(weights, f"l{i}.mix.")
             out = {"norm1": self.vector(f"l{i}.norm1"), "ls1": self.vector(f"l{i}.ls1"), "ff": None}
             if L["type"] == "delta":
-                out["mixer"] = GatedDelta(d, L["mixer"], mix, cfg.width, cfg.eps)
+                out["mixer"] = GatedDelta(d, L["mixer"], mix, cfg.width, cfg.eps, chunks=not routed)
             else:
                 out["mixer"] = Attention(d, L["mixer"], mix, cfg.width, cfg.eps, self.capacity, self.slots)
             if L.get("mlp"):

@@ -350,6 +350,80 @@ def test_delta_state_is_f32_over_a_long_sequence(lm):
         mixer.free()
 
 
+# heads of 128 x 128: portions of 64 and more tokens go by chunks of 64, shorter ones by blocks of four
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,kv_heads,taps,slow", [(2, 2, 2, False), (4, 2, 4, True), (3, 1, 3, False), (1, 1, 4, True)])
+def test_delta_chunks(lm, dtype, heads, kv_heads, taps, slow):
+    from peregrine_b200.layers import GatedDelta
+
+    p, width, T = t.delta(heads, kv_heads, 128, 128, taps), 80, 333
+    d = device(lm, dtype, 400)
+    g = rng(heads)
+    W = {k: t.bf16_values(v) for k, v in t.mixer_weights(g, "delta", p, width).items()}
+    if slow:      # little is forgotten, and the keys of a chunk have much in common
+        W["A_log"], W["dt_bias"] = t.bf16_values(np.full(heads, -5.0)), t.bf16_values(np.full(heads, -2.0))
+    x = t.bf16_values(g.standard_normal((T, width)) + (g.standard_normal(width) if slow else 0.0))
+    mixer = GatedDelta(d, p, W, width, 1e-4)
+    want, carried = so.delta_mixer(x.astype(np.float64), {k: v.astype(np.float64) for k, v in W.items()}, p, 1e-4, so.delta_start(p))
+    # (f32: operands of 22 bits and more, sums of 32; errors of one chunk fade or stay in the next)
+    tol = 1e-5 if dtype == "float32" else 6e-2
+    for cuts in ([T], [64, 65, 1, 127, 10, 63, 3], [128, 192, 13], [1] * 20 + [64] * 4 + [57]):
+        got, state = run_mixer(lm, d, mixer, width, x, cuts)
+        close(got, want, tol, f"cuts {cuts[:4]}")
+        close(state["state"][1].cpu().numpy(), carried["S"], tol, "state")
+        assert (state["state"][0] == 0).all() and (state["state"][2] == 0).all()
+    mixer.free()
+
+
+def test_delta_chunks_beside_short_portions(lm):
+    """Sequences of one step that go by chunks and by blocks of four, in any order; each as if it were alone."""
+    from peregrine_b200.layers import Batch, GatedDelta, up
+    from peregrine_b200.state import SlotPool
+
+    p, width, lengths = t.delta(4, 2, 128, 128, 4), 80, [5, 64, 63, 200, 1, 65]
+    d = device(lm, "float32", 400)
+    g = rng(5)
+    W = {k: t.bf16_values(v) for k, v in t.mixer_weights(g, "delta", p, width).items()}
+    mixer = GatedDelta(d, p, W, width, 1e-4)
+    x = t.bf16_values(g.standard_normal((sum(lengths), width)))
+    state = mixer.new_state(SlotPool(len(lengths), 512, d.dev))
+    y = d.torch.zeros(d.rows, up(width, 4), device=d.dev)
+    h = act(d, x)
+    mixer.run(Batch(d, [(i, 0, [0] * n) for i, n in enumerate(lengths)]), h, state, y)
+    lm.sync()
+    at, W64 = 0, {k: v.astype(np.float64) for k, v in W.items()}
+    for i, n in enumerate(lengths):
+        want, carried = so.delta_mixer(x[at:at + n].astype(np.float64), W64, p, 1e-4, so.delta_start(p))
+        close(y[at:at + n, :width].cpu().numpy(), want, 1e-5, f"sequence {i}")
+        close(state["state"][i].cpu().numpy(), carried["S"], 1e-5, f"state {i}")
+        at += n
+    mixer.free()
+
+
+def test_delta_chunks_keep_infinities_to_later_tokens(lm):
+    """A value that is not finite reaches its own token and those behind it, also within a chunk of 64."""
+    from peregrine_b200.layers import Batch, GatedDelta, up
+    from peregrine_b200.state import SlotPool
+
+    p, width, T, at = t.delta(2, 1, 128, 128, 2), 80, 200, 100
+    d = device(lm, "float32", 400)
+    g = rng(6)
+    W = {k: t.bf16_values(v) for k, v in t.mixer_weights(g, "delta", p, width).items()}
+    mixer = GatedDelta(d, p, W, width, 1e-4)
+    x = t.bf16_values(g.standard_normal((T, width)))
+    want, _ = so.delta_mixer(x.astype(np.float64), {k: v.astype(np.float64) for k, v in W.items()}, p, 1e-4, so.delta_start(p))
+    x[at] = np.inf
+    state = mixer.new_state(SlotPool(1, 512, d.dev))
+    y = d.torch.zeros(d.rows, up(width, 4), device=d.dev)
+    h = act(d, x)
+    mixer.run(Batch(d, [(0, 0, [0] * T)]), h, state, y)
+    lm.sync()
+    got = y[:T, :width].cpu().numpy()
+    close(got[:at], want[:at], 1e-5, "before")
+    assert not np.isfinite(got[at:]).any()
+    mixer.free()
+
+
 # ---- attention ---------------------------------------------------------------------------------------------------------
 ATTENTIONS = [t.attention(6, 2, 40, 24, 0.3, (0.7, 16)), t.attention(8, 1, 64, 64, 0.2), t.attention(2, 2, 128, 128, 0.1, (1.5, 1)),
               t.attention(34, 2, 16, 80, 0.4, (0.2, 9)), t.attention(4, 4, 200, 256, 0.08), t.attention(3, 1, 5, 7, 1.0, (0.9, 33)),
