@@ -145,22 +145,28 @@ __global__ void __launch_bounds__(512, 1)
     const int64_t chunk = first_chunk(row0) + nth;
     const uint32_t k_at = pg_smem(sm.k), q_at = pg_smem(sm.q);
     if (tid == 0) sm.bad_k = CT;
-    if (tid < 2) sm.bad[tid] = CT, sm.top_v[tid] = sm.largest[tid] = 0;
-    __syncthreads();
 
-    // gates: warp x for head h0 + x, two tokens a lane; log decays are added up in 64 bits
+    // gates of a head: two tokens a lane; log decays are added up in 64 bits
+    float in_a[2], in_b[2];                                           // (asked for well before they are used)
+    auto load_gates = [&](int h) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int a = lane * 2 + i;
+            const float *tail = first + (int64_t)(t0 + a) * ldp + s.C + (int64_t)s.H * s.V;
+            in_a[i] = t0 + a < T ? __ldcg(tail + s.H + h) : 0.0f;
+            in_b[i] = t0 + a < T ? __ldcg(tail + h) : 0.0f;
+        }
+    };
     auto gates = [&](int x, int h) {
         const float al = __ldg(s.a_log + h), db = __ldg(s.dt_bias + h);
         double v[2];
         float be[2];
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-            const int a = lane * 2 + i;
-            const float *tail = first + (int64_t)(t0 + a) * ldp + s.C + (int64_t)s.H * s.V;
-            const bool in = t0 + a < T;
-            const float ld = in ? log_decay(__ldcg(tail + s.H + h), al, db) : 0.0f;
+            const bool in = t0 + lane * 2 + i < T;
+            const float ld = in ? log_decay(in_a[i], al, db) : 0.0f;
             v[i] = (double)(ld < -1e4f ? -1e4f : ld);              // (its exponential is 0 either way; differences stay numbers)
-            be[i] = in ? pg_sigmoid(__ldcg(tail + h)) : 0.0f;
+            be[i] = in ? pg_sigmoid(in_b[i]) : 0.0f;
         }
         double sum = v[0] + v[1];
 #pragma unroll
@@ -246,21 +252,11 @@ __global__ void __launch_bounds__(512, 1)
             if (lane == 0) atomicMax(&sm.top_v[i - 2], top);
         }
     };
-    if (warp < min(2, rep)) gates(warp, g * rep + warp);
-#pragma unroll 1
-    for (int i = warp >> 3; i < 2 + min(2, rep); i += 2) convolve(i, g * rep);
-    __syncthreads();
-    {
-        uint4 *dst = reinterpret_cast<uint4 *>(group_data(s, w, chunk, g));
-#pragma unroll
-        for (int i = 0; i < GROUP_BYTES / 16 / 512; i++) dst[i * 512 + tid] = reinterpret_cast<const uint4 *>(sm.q)[i * 512 + tid];
-    }
-
     // products of the pairs: warps 0 .. 7 k_a . k_b, 8 .. 15 q_a . k_b; sixteen rows and every other block of sixteen columns
     // up to the diagonal a warp
     const int slab = (warp >> 1) & 3, odd = warp & 1;
     float dots[2][2][4] = {};
-    {
+    auto products = [&]() {
         const uint32_t rows_at = warp < 8 ? k_at : q_at;
         const int ra = slab * 16 + (lane & 15), rb = odd * 16 + (lane & 7) + (lane >> 4) * 8;
 #pragma unroll 4
@@ -282,18 +278,27 @@ __global__ void __launch_bounds__(512, 1)
                 mma_pair(dots[j], ah, al, bh, bl);
             }
         }
-    }
+    };
 
 #pragma unroll 1
     for (int h0 = g * rep; h0 < (g + 1) * rep; h0 += 2) {
         const int heads = min(2, (g + 1) * rep - h0);
-        if (h0 > g * rep) {
-            if (tid < 2) sm.bad[tid] = CT, sm.top_v[tid] = sm.largest[tid] = 0;
-            __syncthreads();
-            if (warp < heads) gates(warp, h0 + warp);
-            if ((warp >> 3) < heads) convolve(2 + (warp >> 3), h0);
-            __syncthreads();
+        const bool keys = h0 == g * rep;                              // the first heads come with the queries and keys
+        if (tid < 2) sm.bad[tid] = CT, sm.top_v[tid] = sm.largest[tid] = 0;
+        __syncthreads();
+        const int gate = (warp & 7) == 1 ? warp >> 3 : 2;             // warps 1 and 9 have no products of pairs: gates meanwhile
+        if (gate < heads) load_gates(h0 + gate);
+#pragma unroll 1
+        for (int i = (keys ? 0 : 2) + (warp >> 3); i < 2 + heads; i += 2) convolve(i, h0);
+        __syncthreads();
+        if (keys) {
+            uint4 *dst = reinterpret_cast<uint4 *>(group_data(s, w, chunk, g));
+#pragma unroll
+            for (int i = 0; i < GROUP_BYTES / 16 / 512; i++) dst[i * 512 + tid] = reinterpret_cast<const uint4 *>(sm.q)[i * 512 + tid];
+            products();
         }
+        if (gate < heads) gates(gate, h0 + gate);
+        __syncthreads();
         // A (warps 0 .. 7; its diagonal blocks apart, in f32) and P
         for (int x = 0; x < heads; x++) {
             unsigned char *out = warp < 8 ? sm.a[x] : head_data(s, w, chunk, h0 + x) + P_AT;
@@ -388,85 +393,93 @@ __global__ void __launch_bounds__(512, 1)
             unsigned char *img = x == 0 ? sm.w0 : sm.w1;
             const uint32_t a_at = pg_smem(sm.a[x]), w_at = pg_smem(img);
             const int rn = (lane & 7) + (lane >> 4) * 8, cn = (lane >> 3) & 1;      // rows and chunks of ldmatrix: plain; transposed alike
-            uint32_t xh[2][4][4], xl[2][4][4];                                       // [16 columns][block of rows] left operands
             uint32_t top = 0;
             int worst = CT;
-#pragma unroll
-            for (int J = 0; J < 4; J++) {
-                float acc[2][2][4] = {};
-#pragma unroll
-                for (int I = 0; I < J; I++) {
-                    uint32_t bh[4], bl[4];
+            // (loops are not unrolled: code that runs once is waited for)
+#pragma unroll 1
+            for (int d = d0; d < d0 + 32; d += 16) {
+                uint32_t xh[3][4], xl[3][4];                                         // [block of rows] left operands
+#pragma unroll 1
+                for (int J = 0; J < 4; J++) {
                     const int r = J * 16 + rn;
-                    const uint32_t at = a_at + r * 128 + (((2 * I + cn) ^ (r & 7)) << 4);
-                    pg_ldsm4(bh, at);
-                    pg_ldsm4(bl, at + TILE);
+                    float acc[2][4] = {};
 #pragma unroll
-                    for (int m = 0; m < 2; m++) mma_pair(acc[m], xh[m][I], xl[m][I], bh, bl);
-                }
-                uint32_t th[4], tl[4];
-                pg_ldsm4(th, pg_smem(sm.t[x][J][0]) + rn * T_PITCH + cn * 16);
-                pg_ldsm4(tl, pg_smem(sm.t[x][J][1]) + rn * T_PITCH + cn * 16);
-#pragma unroll
-                for (int m = 0; m < 2; m++) {
-                    const int d = d0 + m * 16, r = J * 16 + rn;
+                    for (int I = 0; I < 3; I++) {
+                        if (I >= J) break;
+                        uint32_t bh[4], bl[4];
+                        const uint32_t at = a_at + r * 128 + (((2 * I + cn) ^ (r & 7)) << 4);
+                        pg_ldsm4(bh, at);
+                        pg_ldsm4(bl, at + TILE);
+                        mma_pair(acc, xh[I], xl[I], bh, bl);
+                    }
+                    uint32_t th[4], tl[4];
+                    pg_ldsm4(th, pg_smem(sm.t[x][J][0]) + rn * T_PITCH + cn * 16);
+                    pg_ldsm4(tl, pg_smem(sm.t[x][J][1]) + rn * T_PITCH + cn * 16);
                     const uint32_t tile_at = (d >> 6) * TILE + r * 128 + (((((d & 63) >> 3) + cn) ^ (r & 7)) << 4);
-                    uint32_t kh[4], kl[4], yh[4], yl[4];
-                    if (!of_v) {
+                    const int a0 = J * 16 + (lane & 3) * 2, col = d + (lane >> 2);  // of this lane: columns col and col + 8, rows a0, + 1, + 8, + 9
+                    float2 z[2][2];
+                    if (of_v) {
+#pragma unroll
+                        for (int n = 0; n < 2; n++)
+#pragma unroll
+                            for (int i = 0; i < 2; i++) z[n][i] = make_float2(sm.v[x][a0 + 8 * n][col + 8 * i], sm.v[x][a0 + 8 * n + 1][col + 8 * i]);
+                    } else {
+                        uint32_t kh[4], kl[4];
                         pg_ldsm4_t(kh, k_at + tile_at);
                         pg_ldsm4_t(kl, k_at + 2 * TILE + tile_at);
+#pragma unroll
+                        for (int n = 0; n < 2; n++)
+#pragma unroll
+                            for (int i = 0; i < 2; i++) z[n][i] = join2(kh[2 * n + i], kl[2 * n + i]);
                     }
-                    // right side minus the sums; lane: columns d + (lane >> 2) and + 8, rows a and a + 1
+                    // right side minus the sums
+                    uint32_t yh[4], yl[4];
 #pragma unroll
                     for (int n = 0; n < 2; n++) {
-                        const int a = J * 16 + n * 8 + (lane & 3) * 2;
-                        float2 f = *reinterpret_cast<const float2 *>(&sm.beta[x][a]);
-                        if (of_v) {
-                            f.x *= scale.x, f.y *= scale.x;
-                        } else {
-                            const float2 c = *reinterpret_cast<const float2 *>(&sm.c[x][a]);
-                            f.x *= c.x, f.y *= c.y;
-                        }
+                        const int a = a0 + 8 * n;
+                        const float2 be = *reinterpret_cast<const float2 *>(&sm.beta[x][a]);
+                        const float2 c = of_v ? make_float2(scale.x, scale.x) : *reinterpret_cast<const float2 *>(&sm.c[x][a]);
+                        const float f0 = be.x * c.x, f1 = be.y * c.y;
 #pragma unroll
                         for (int i = 0; i < 2; i++) {
-                            const int col = d + (lane >> 2) + 8 * i;
-                            const float2 z = of_v ? make_float2(sm.v[x][a][col], sm.v[x][a + 1][col]) : join2(kh[2 * n + i], kl[2 * n + i]);
-                            float y0 = fmaf(f.x, z.x, -OPERAND_INV * acc[m][n][2 * i]), y1 = fmaf(f.y, z.y, -OPERAND_INV * acc[m][n][2 * i + 1]);
-                            y0 = a < bad ? y0 : 0.0f;
-                            y1 = a + 1 < bad ? y1 : 0.0f;
-                            split2(y0, y1, yh[2 * n + i], yl[2 * n + i]);
+                            const float y0 = fmaf(f0, z[n][i].x, -OPERAND_INV * acc[n][2 * i]), y1 = fmaf(f1, z[n][i].y, -OPERAND_INV * acc[n][2 * i + 1]);
+                            split2(a < bad ? y0 : 0.0f, a + 1 < bad ? y1 : 0.0f, yh[2 * n + i], yl[2 * n + i]);
                         }
                     }
                     float o[2][4] = {};
                     mma_pair(o, yh, yl, th, tl);
+                    uint32_t nh[4], nl[4];
 #pragma unroll
                     for (int n = 0; n < 2; n++)
 #pragma unroll
                         for (int i = 0; i < 2; i++) {
-                            const float v0 = o[n][2 * i] * OPERAND_INV, v1 = o[n][2 * i + 1] * OPERAND_INV;
-                            split2(v0, v1, xh[m][J][2 * n + i], xl[m][J][2 * n + i]);
-                            if (of_v) {
-                                const int a = J * 16 + n * 8 + (lane & 3) * 2, col = d + (lane >> 2) + 8 * i;
-                                const float u0 = v0 * scale.y, u1 = v1 * scale.y;
-                                sm.v[x][a][col] = u0;
-                                sm.v[x][a + 1][col] = u1;
-                                if (a < bad) {
-                                    if (bits(u0) < NOT_FINITE)
-                                        top = max(top, bits(u0));
-                                    else
-                                        worst = min(worst, a);
-                                }
-                                if (a + 1 < bad) {
-                                    if (bits(u1) < NOT_FINITE)
-                                        top = max(top, bits(u1));
-                                    else
-                                        worst = min(worst, a + 1);
+                            z[n][i] = make_float2(o[n][2 * i] * OPERAND_INV, o[n][2 * i + 1] * OPERAND_INV);
+                            split2(z[n][i].x, z[n][i].y, nh[2 * n + i], nl[2 * n + i]);
+                        }
+#pragma unroll
+                    for (int I = 0; I < 3; I++)
+                        if (I == J) {
+#pragma unroll
+                            for (int e = 0; e < 4; e++) xh[I][e] = nh[e], xl[I][e] = nl[e];
+                        }
+                    if (of_v) {
+#pragma unroll
+                        for (int n = 0; n < 2; n++)
+#pragma unroll
+                            for (int i = 0; i < 2; i++) {
+                                const int a = a0 + 8 * n;
+                                const float u[2] = {z[n][i].x * scale.y, z[n][i].y * scale.y};
+#pragma unroll
+                                for (int e = 0; e < 2; e++) {
+                                    sm.v[x][a + e][col + 8 * i] = u[e];
+                                    const bool fine = bits(u[e]) < NOT_FINITE;
+                                    top = a + e < bad && fine ? max(top, bits(u[e])) : top;
+                                    worst = a + e < bad && !fine ? min(worst, a + e) : worst;
                                 }
                             }
-                        }
-                    if (!of_v) {
-                        stsm4_t(w_at + tile_at, xh[m][J]);
-                        stsm4_t(w_at + 2 * TILE + tile_at, xl[m][J]);
+                    } else {
+                        stsm4_t(w_at + tile_at, nh);
+                        stsm4_t(w_at + 2 * TILE + tile_at, nl);
                     }
                 }
             }
