@@ -374,6 +374,26 @@ int ws_cluster_for(int64_t m, int64_t k)
     return 0;
 }
 
+static int ws_part_bytes(int KH, int parts) { return (((KH + parts - 1) / parts) + 63) & ~63; }
+// more warps per tile while every (tile, K part) still finds a warp of its own: the whole matrix is then requested at once
+static int ws_parts(int KH, int64_t tiles, int64_t units)
+{
+    int kw = 1;
+    while (kw < WS_WARPS && KH / (kw * 2) >= 512 && tiles * (kw * 2) <= units * WS_WARPS) kw *= 2;
+    while (kw > 1 && (int64_t)(kw - 1) * ws_part_bytes(KH, kw) >= KH) kw /= 2;   // rounding to k-steps must leave no part of a full range empty
+    return kw;
+}
+
+// Where this kernel has an SM busy with every tile it can: deep rings beside the activations, eight rows (with more, a weight byte
+// costs twice the shared-memory traffic), and CTAs for two thirds of the SMs (1250 tiles of eight columns are 79 CTAs of sixteen
+// warps).
+bool pgk_gemm_i8_wstream_fills(const pg_ctx *ctx, int64_t m, int64_t k, int64_t n)
+{
+    if (m > 8 || ws_cluster_for<512>(m, k) != 1) return false;
+    const int64_t tiles = (n + 7) / 8, groups = WS_WARPS / ws_parts((int)k, tiles, ctx->sm_count);
+    return 3 * std::min<int64_t>(ctx->sm_count, (tiles + groups - 1) / groups) > 2 * ctx->sm_count;
+}
+
 bool pgk_gemm_i8_wstream_supports(int64_t m, int64_t k, int64_t n)
 {
     if (!(m >= 1 && m <= 16 && n >= 1 && k >= 64 && (k % 64 == 0) && k <= (1 << 20))) return false;
@@ -399,14 +419,10 @@ static int32_t ws_dispatch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, in
     const int KH = cs > 1 ? (int)ws_range(K, cs) : K;       // K range of one CTA
     PG_REQUIRE(cs == 1 || (int64_t)(cs - 1) * KH < K, "gemm_i8 warp-stream: K too short for a cluster of %d", cs);
     const int64_t units = sms / cs;                         // CTAs or clusters that take tiles
-    // more warps per tile while every (tile, K part) still finds a warp of its own: the whole matrix is then requested at once
-    int kw = 1;
-    while (kw < WS_WARPS && KH / (kw * 2) >= 512 && tiles * (kw * 2) <= units * WS_WARPS) kw *= 2;
-    auto part_bytes = [&](int parts) { return (((KH + parts - 1) / parts) + 63) & ~63; };
-    while (kw > 1 && (int64_t)(kw - 1) * part_bytes(kw) >= KH) kw /= 2;   // rounding to k-steps must leave no part of a full range empty
+    int kw = ws_parts(KH, tiles, units);
     if (g_force_kw) kw = g_force_kw;
     PG_REQUIRE(kw == 1 || kw == 2 || kw == 4 || kw == 8 || kw == 16, "gemm_i8 warp-stream: kw must be a power of two <= 16");
-    const int KW = part_bytes(kw);
+    const int KW = ws_part_bytes(KH, kw);
     PG_REQUIRE((int64_t)(kw - 1) * KW < KH, "gemm_i8 warp-stream: K too short for %d parts", kw);
     const int groups = WS_WARPS / kw;
     // CTAs with every warp busy, the rest of the SMs idle: spreading 1792 tiles as 12 or 13 per CTA over all 148 SMs instead of 16 over

@@ -427,6 +427,7 @@ int32_t pgk_gemm_i8_stream(pg_ctx *ctx, const int8_t *d_a, const float *d_as, in
                            const float *d_ws, int64_t n, float *d_y, int32_t *d_acc);
 // pg_gemv_wstream.cu
 bool pgk_gemm_i8_wstream_supports(int64_t m, int64_t k, int64_t n);
+bool pgk_gemm_i8_wstream_fills(const pg_ctx *ctx, int64_t m, int64_t k, int64_t n);
 int32_t pgk_gemm_i8_wstream(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, const int8_t *d_bt,
                             const float *d_ws, int64_t n, float *d_y, int32_t *d_acc);
 // the same product with its outputs stored into every rank's exchange buffer and the exchange published by the kernel

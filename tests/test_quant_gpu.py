@@ -298,6 +298,13 @@ def test_mid_batch_dispatch(pg, gpu, oracle_mt, m, k, n):
     _check_product(pg, gpu, oracle_mt, x, w, m, k, n, ["naive"])
 
 
+@pytest.mark.parametrize("m,k,n", [(1, 4096, 10000), (8, 12800, 1600), (9, 4096, 5003), (16, 14336, 4096), (16, 3136, 7001), (9, 4096, 4096), (8, 4096, 12999)])
+def test_few_rows_dispatch(pg, gpu, oracle_mt, m, k, n):
+    """Up to 16 rows with the automatic kernel choice, on both sides of its line: sums are whole numbers, the same from either kernel."""
+    x, w = linear_inputs(m, k, n, 70 + m)
+    _check_product(pg, gpu, oracle_mt, x, w, m, k, n, ["wstream"])
+
+
 @pytest.mark.parametrize("split", [0, 2, 4, 8])
 @pytest.mark.parametrize("m,k,n,bn", [(17, 14336, 4096, 0), (64, 4096, 4096, 0), (128, 4096, 520, 64), (33, 1040, 1000, 32), (100, 2048, 14336, 256),
                                       (20, 384, 96, 0)])
