@@ -1,5 +1,5 @@
 // Dequantising product y = x . dequant(W)^T for GGUF Q4_0 / Q8_0 weights and several rows of x on the 5th-generation tensor cores
-// (up to eight rows: csrc/pg_gguf_stream.cu, which also describes the layout of the weights).
+// (few rows: csrc/pg_gguf_stream.cu, which also describes the layout of the weights).
 //
 // Arithmetic, per 32-element block:
 //   * x * 2^s (s per row: the largest element lies in [2^14, 2^15)) = h1 + h2, two f16 numbers: 22 significant bits, and more than
@@ -22,7 +22,8 @@
 // read 32 KB of it, while 16 KB of planes come in, 8 KB of f16 weights are written and 2 KB of quants read: 470 cycles at 128 bytes
 // each, about 460 of the warp that issues the products (800 with its waits).  N 14336, K 4096, 9 / 16 / 33 / 64 / 300 rows: Q4_0 25 / 26 /
 // 39 / 43 / 126 us, where eight rows at a time through the streaming form took 31 / 42 / 92 / 167 / 787; error against 64 bits 2e-7 ...
-// 3e-7 with 1 % of the channels x 20 (1.2e-6).  Up to eight rows the streaming form is the faster one (21 against 25 us).
+// 3e-7 with 1 % of the channels x 20 (1.2e-6).  At eight rows
+// and K 4096 the streaming form is the faster one (21 against 25 us).
 // Every mbarrier wait is bounded (pg_async.cuh).
 #include <algorithm>
 
@@ -511,9 +512,18 @@ int32_t gt_run(pg_ctx *ctx, const pg_gguf_weight *w, const void *planes, const f
 
 }  // namespace
 
-bool pgk_matmul_gguf_tc_supports(const pg_gguf_weight *w, int64_t m)
+// From nine rows on, and for fewer where the streaming form walks K in several chunks (it has room for 16384 elements of x in all),
+// each with its own start: from four chunks on, from three on narrow layers, and from two with seven and eight rows there.  Q4_0, us,
+// streaming / this: K 14336, N 4096 at 2 / 3 / 5 / 8 rows 18.5 / 28.4 / 40.7 / 48.7 against 25.7 / 26.2 / 26.7 / 27.7; K 8192, N 8192 at 4 / 5 / 8
+// rows 23.3 / 29.4 / 34.2 against 28.2 / 28.3 / 28.9; K 6144, at 5 rows: N 4096 17.3 / 15.1, N 12000 29.7 / 32.9; K 4096, at 8 rows: N 4096
+// 13.9 / 12.4, N 14336 21.9 / 25.3.
+bool pgk_matmul_gguf_tc_supports(const pg_ctx *ctx, const pg_gguf_weight *w, int64_t m)
 {
-    return w->tiled && m > 8 && m < (1 << 24) && w->n >= 1 && w->n < (1ll << 30);
+    if (!(w->tiled && m >= 1 && m < (1 << 24) && w->n >= 1 && w->n < (1ll << 30))) return false;
+    if (m > 8) return true;
+    const int64_t rows = m > 4 ? 8 : m > 2 ? 4 : m, chunks = (w->k * rows + 16383) / 16384;
+    const bool narrow = w->n <= 32ll * ctx->sm_count;
+    return chunks >= 4 || (narrow && (chunks == 3 || (chunks == 2 && m > 6)));
 }
 
 int32_t pgk_gguf_tc_reserve(pg_ctx *ctx, int64_t k)

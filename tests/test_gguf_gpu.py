@@ -191,6 +191,23 @@ def test_matmul_gguf_many_rows(pg, gpu, oracle_mt, kind, n, k):
     w.free()
 
 
+@pytest.mark.parametrize("kind", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("m,n,k", [(3, 300, 12544), (4, 260, 8448), (5, 129, 4352), (7, 200, 2304), (8, 5000, 6400), (6, 131, 16640)])
+def test_matmul_gguf_few_rows_long_k(pg, gpu, oracle_mt, kind, m, n, k):
+    """Up to eight rows, on both sides of the line between the streaming form and the tensor cores: the bound of the latter's planes and
+    sums (above) holds for both but for the streaming form's three digits of 7 bits of the row's largest element."""
+    g = rng(n + k + m)
+    raw = oracle_mt.encode(kind, normal(g, (n, k), 0.02))
+    w64 = oracle_mt.dequant(kind, raw, n * k).reshape(n, k).astype(np.float64)
+    w = pg.gguf.GgufWeight(kind, raw, n, k, gpu)
+    x = normal(g, (m, k))
+    got = w.matmul(x, m)
+    x64 = np.abs(x).astype(np.float64)
+    bound = x64 @ np.abs(w64).T * (2.0 ** -22 + 4 * 2.0 ** -23 + (k // 32 + 18) * 2.0 ** -24) + x64.max(1, keepdims=True) * 2.0 ** -20 * np.abs(w64).sum(1)
+    assert (np.abs(got - x.astype(np.float64) @ w64.T) <= bound).all() and gpu.device_status() == 0
+    w.free()
+
+
 def test_matmul_gguf_many_rows_recorded_without_a_run_before(pg, oracle_mt):
     """The workspace cannot grow in a recording: the rows then go through what the upload has reserved, in portions."""
     import torch
