@@ -93,9 +93,11 @@ __device__ __forceinline__ float2 scale_of(float bound, int to)
 // ---- what does not depend on the state: grid (G, chunks of the longest sequence, seqs), 512 threads ---------------------
 // (I + A)^-1 goes by blocks of sixteen rows: X_J = T_J (rhs_J - sum over I < J of A_JI X_I), T_J the inverse of the diagonal
 // block.  The blocks are mma.sync products of transposed tiles, X^T [sixteen columns][64 rows]: the sums of one are the left operand
-// of the next without leaving the warp's registers.  (f32 multiply-adds over columns in registers took twice the time of the whole
-// kernel: 13000 instructions a warp, many of them fetched once.)  The last chunks come first, so that the chain finds the
-// first ones in L2.
+// of the next without leaving the warp's registers.  The last chunks come first, so that the chain finds the first ones in L2.
+//
+// Bound by instructions: 55000 cycles a CTA at 4096 tokens, 20000 of them the convolution, 15000 the substitution.  4096 tokens of 32
+// heads (430 MB in and out): 212 us; with f32 multiply-adds over columns in place of the tiles 290, with all 64 rows of two columns in
+// a thread's registers, unrolled, 448 (code that runs once is waited for).
 constexpr int V_PITCH = 132, DIAG_PITCH = 20, T_PITCH = 48;
 struct ChunkSmem {
     unsigned char k[4 * TILE];
@@ -517,6 +519,9 @@ __global__ void __launch_bounds__(512, 1)
 // A chunk is a chain of two products and what turns the sums of one into operands of the next; the third, and the writing of
 // O, run beside it.  Operands come through a ring of 16 KB slots, seven a chunk, as soon as a slot is free, and are asked for in L2
 // some chunks ahead (the four CTAs of a head share that).
+//
+// Bound by that chain: 4000 cycles a chunk, 1200 of them the first product, whose operands are 96 KB of shared memory.  4096 tokens of
+// 32 heads 145 us (192 with two fixed buffers and eight warps; delta_scan_kernel, four tokens at a time, 820).
 constexpr int CHAIN_WARPS = 16, CHAIN_THREADS = (CHAIN_WARPS + 2) * 32, COLS = 32, PART = 8;
 constexpr int SLOT = 2 * TILE, SLOTS = 12, PER_CHUNK = 7, AHEAD = 3;
 constexpr int S_SM = 0, U_SM = 2 * TILE, RING_SM = 3 * TILE, BARS_SM = RING_SM + SLOTS * SLOT;
