@@ -464,6 +464,31 @@ def planted(p, width, T, far, at):
     return t.bf16_values(x), W
 
 
+def test_attention_f32_tokens_of_several_sequences(lm):
+    """f32: up to four tokens of a sequence share a CTA; whatever the lengths, each sequence is as if it were alone (products of other row counts aside)."""
+    from peregrine_b200.layers import Attention, Batch, up
+    from peregrine_b200.state import SlotPool
+
+    p, width, lengths = t.attention(4, 2, 40, 24, 0.3, (0.7, 16)), 80, [1, 5, 4, 3, 130, 2, 1, 7]
+    d = device(lm, "float32", 160)
+    g = rng(9)
+    mixer = Attention(d, p, {k: t.bf16_values(v) for k, v in t.mixer_weights(g, "attention", p, width).items()}, width, 1e-4, 200, len(lengths))
+    x = t.bf16_values(g.standard_normal((sum(lengths), width)))
+    y = d.torch.zeros(d.rows, up(width, 4), device=d.dev)
+    entries, at = [], 0
+    for i, n in enumerate(lengths):
+        entries.append((i, at, n))
+        at += n
+    h = act(d, x)
+    mixer.run(Batch(d, [(i, 0, [0] * n) for i, _, n in entries]), h, mixer.new_state(SlotPool(len(lengths), 512, d.dev)), y)
+    lm.sync()
+    together = y[:at, :width].cpu().numpy()
+    for i, a, n in entries:
+        got, _state = run_mixer(lm, d, mixer, width, x[a:a + n], [n])
+        close(together[a:a + n], got, 1e-6, f"sequence {i}")
+    mixer.free()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads", [(4, 2, 32, 32, 0.5), (4, 2, 64, 64, 0.25), (8, 1, 128, 128, 0.13)])
 @pytest.mark.parametrize("far", [0, 1, 63, 64, 65, 127, 128, 300, 440, 447])
