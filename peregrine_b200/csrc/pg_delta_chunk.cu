@@ -9,9 +9,15 @@
 // lines above, is three tcgen05 products per chunk (delta_chain_kernel, a CTA per head and 32 columns of the state, which stays in
 // registers).
 //
-// Precision.  A product's operands are pairs of f16 numbers, h + l with 22 to 24 significant bits, added in f32.  W, Q, K~, P, A
-// and the inverses have rows of norm at most one (keys are unit vectors and every step is a contraction), so a fixed scale of
-// 2^14 keeps their bits; values, S and U are scaled by a power of two that follows from the largest element.
+// Precision: that of delta_scan_kernel's f32.  A product's operands are pairs of f16 numbers, h + l: 23 significant bits, and all 24 of
+// three in four f32 numbers.  All four products of the parts are taken.  W, Q, K~, P, A and the inverses have rows of norm at most one
+// (keys are unit vectors and every step is a contraction), so a fixed scale of 2^14 keeps their bits; values, S and U are scaled by a
+// power of two that follows from the largest element.  The tensor core cuts off what falls below an accumulator's last bit, so an
+// accumulator takes the small products first or alone, and of the large ones two steps of sixteen; sums of accumulators are rounded,
+// in registers.  What needs no product stays in f32: the diagonals of the inverses, and a token's own key in P.
+// Against 64 bits, from the same inputs, these kernels / delta_scan_kernel, 130 to 4000 tokens: outputs 1.59e-7 ... 1.61e-7 / 1.57e-7 ...
+// 1.65e-7, states 1.7e-7 / 2.0e-7 ... 2.2e-7; where little is forgotten 3.3e-7 / 4.3e-6 at 4000 tokens; where a few tokens are all that
+// is kept 1.45e-7 / 1.39e-7, states 1.5e-7 / 1.3e-7.
 //
 // What is not finite stays with its token and those behind it: from the first token of a chunk with such a value, key or gate on,
 // U is zero in the products, O is NaN, and so is the state behind the chunk.
@@ -32,8 +38,8 @@ constexpr float OPERAND = 16384.0f, OPERAND_INV = 1.0f / 16384.0f;
 // Per (chunk, head): W [part][half of d] | K~ [part][half of d] | P [part] | U0 [64][128] f32 | coefficients
 // Per (chunk, key head): Q [part][half of d]
 constexpr int TILE = 8192, W_AT = 0, KT_AT = 4 * TILE, P_AT = 8 * TILE, U0_AT = 10 * TILE, COEF_AT = U0_AT + CT * CD * 4;
-constexpr int HEAD_BYTES = COEF_AT + 512, GROUP_BYTES = 4 * TILE;
-constexpr int COEF_LAST = CT, COEF_MAX = CT + 1, COEF_BAD = CT + 2;   // c [64], c_63, largest |U0|, first token that is not finite
+constexpr int HEAD_BYTES = COEF_AT + 640, GROUP_BYTES = 4 * TILE;
+constexpr int COEF_OWN = CT, COEF_LAST = 2 * CT, COEF_MAX = COEF_LAST + 1, COEF_BAD = COEF_LAST + 2;   // c [64], q_a . k_a [64], c_63, largest |U0|, first token that is not finite
 
 // A sequence has at least 64 tokens: the chunks of the one at row0 are numbered from row0 / 32 on.
 __host__ __device__ __forceinline__ int64_t first_chunk(int64_t row0) { return row0 / 32; }
@@ -66,13 +72,15 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// (ah + al) times sixteen columns, without the product of the two low parts
-__device__ __forceinline__ void mma_pair(float (&d)[2][4], const uint32_t (&ah)[4], const uint32_t (&al)[4], const uint32_t (&bh)[4], const uint32_t (&bl)[4])
+// (ah + al) times sixteen columns: the products of the two high parts, and the others
+__device__ __forceinline__ void mma_pair(float (&d)[2][4], float (&e)[2][4], const uint32_t (&ah)[4], const uint32_t (&al)[4], const uint32_t (&bh)[4],
+                                         const uint32_t (&bl)[4])
 {
 #pragma unroll
     for (int n = 0; n < 2; n++) {
-        mma_f16(d[n], al, bh[2 * n], bh[2 * n + 1]);
-        mma_f16(d[n], ah, bl[2 * n], bl[2 * n + 1]);
+        mma_f16(e[n], al, bl[2 * n], bl[2 * n + 1]);
+        mma_f16(e[n], al, bh[2 * n], bh[2 * n + 1]);
+        mma_f16(e[n], ah, bl[2 * n], bl[2 * n + 1]);
         mma_f16(d[n], ah, bh[2 * n], bh[2 * n + 1]);
     }
 }
@@ -95,8 +103,8 @@ __device__ __forceinline__ float2 scale_of(float bound, int to)
 // block.  The blocks are mma.sync products of transposed tiles, X^T [sixteen columns][64 rows]: the sums of one are the left operand
 // of the next without leaving the warp's registers.  The last chunks come first, so that the chain finds the first ones in L2.
 //
-// Bound by instructions: 55000 cycles a CTA at 4096 tokens, 20000 of them the convolution, 15000 the substitution.  4096 tokens of 32
-// heads (430 MB in and out): 212 us; with f32 multiply-adds over columns in place of the tiles 290, with all 64 rows of two columns in
+// Bound by instructions: 55000 cycles a CTA at 4096 tokens, 20000 of them the convolution, 15000 the substitution (before the sums
+// went apart, which took the two kernels from 395 to 444 us).  4096 tokens of 32 heads (430 MB in and out): 212 us; with f32 multiply-adds over columns in place of the tiles 290, with all 64 rows of two columns in
 // a thread's registers, unrolled, 448 (code that runs once is waited for).
 constexpr int V_PITCH = 132, DIAG_PITCH = 20, T_PITCH = 48;
 struct ChunkSmem {
@@ -114,6 +122,12 @@ struct ChunkSmem {
     int bad[2], bad_k;                                // first token that is not finite: of a head, of the keys
 };
 
+// z / (1 + e^-z), the quotient with a step of Newton's behind it (the exponent ends where the denominator's inverse does)
+__device__ __forceinline__ float silu(float z)
+{
+    const float d = 1.0f + expf(fminf(-z, 87.0f)), r = __fdividef(1.0f, d), y = z * r;
+    return fmaf(fmaf(-d, y, z), r, y);
+}
 // inputs of the convolution of four channels and tokens t .. t + 7
 template <int TAPS>
 __device__ __forceinline__ void load_inputs(const DeltaShape &s, const float *row0, int64_t ldp, const float *ring, int pos0, int t, int T, int c, float4 (&x)[TAPS + 7])
@@ -168,7 +182,7 @@ __global__ void __launch_bounds__(512, 1)
             const bool in = t0 + lane * 2 + i < T;
             const float ld = in ? log_decay(in_a[i], al, db) : 0.0f;
             v[i] = (double)(ld < -1e4f ? -1e4f : ld);              // (its exponential is 0 either way; differences stay numbers)
-            be[i] = in ? pg_sigmoid(in_b[i]) : 0.0f;
+            be[i] = in ? __fdiv_rn(1.0f, 1.0f + expf(-in_b[i])) : 0.0f;
         }
         double sum = v[0] + v[1];
 #pragma unroll
@@ -213,7 +227,7 @@ __global__ void __launch_bounds__(512, 1)
                 acc.z = fmaf(wt[j].z, x[a + j].z, acc.z), acc.w = fmaf(wt[j].w, x[a + j].w, acc.w);
             }
             const bool in = t0 + a0 + a < T;
-            y[a] = in ? make_float4(pg_silu(acc.x), pg_silu(acc.y), pg_silu(acc.z), pg_silu(acc.w)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            y[a] = in ? make_float4(silu(acc.x), silu(acc.y), silu(acc.z), silu(acc.w)) : make_float4(0.f, 0.f, 0.f, 0.f);
             const uint32_t m = max(max(bits(y[a].x), bits(y[a].y)), max(bits(y[a].z), bits(y[a].w)));
             if (i > 0 && m >= NOT_FINITE)
                 atomicMin(i == 1 ? &sm.bad_k : &sm.bad[i - 2], a0 + a);
@@ -259,6 +273,7 @@ __global__ void __launch_bounds__(512, 1)
     const int slab = (warp >> 1) & 3, odd = warp & 1;
     float dots[2][2][4] = {};
     auto products = [&]() {
+        float low[2][2][4] = {}, two[2][2][4];
         const uint32_t rows_at = warp < 8 ? k_at : q_at;
         const int ra = slab * 16 + (lane & 15), rb = odd * 16 + (lane & 7) + (lane >> 4) * 8;
 #pragma unroll 4
@@ -277,9 +292,27 @@ __global__ void __launch_bounds__(512, 1)
                 const uint32_t bat = k_at + half + r * 128 + ((cb ^ (r & 7)) << 4);
                 pg_ldsm4(bh, bat);
                 pg_ldsm4(bl, bat + 2 * TILE);
-                mma_pair(dots[j], ah, al, bh, bl);
+                if (!(kk & 1)) {
+#pragma unroll
+                    for (int n = 0; n < 2; n++)
+#pragma unroll
+                        for (int i = 0; i < 4; i++) two[j][n][i] = 0.0f;
+                }
+                mma_pair(two[j], low[j], ah, al, bh, bl);
+                if (kk & 1) {
+#pragma unroll
+                    for (int n = 0; n < 2; n++)
+#pragma unroll
+                        for (int i = 0; i < 4; i++) dots[j][n][i] += two[j][n][i];
+                }
             }
         }
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int n = 0; n < 2; n++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) dots[j][n][i] += low[j][n][i];
     };
 
 #pragma unroll 1
@@ -304,6 +337,7 @@ __global__ void __launch_bounds__(512, 1)
         // A (warps 0 .. 7; its diagonal blocks apart, in f32) and P
         for (int x = 0; x < heads; x++) {
             unsigned char *out = warp < 8 ? sm.a[x] : head_data(s, w, chunk, h0 + x) + P_AT;
+            float *own = reinterpret_cast<float *>(head_data(s, w, chunk, h0 + x) + COEF_AT) + COEF_OWN;
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 const int a = slab * 16 + (lane >> 2) + i * 8;
@@ -325,8 +359,10 @@ __global__ void __launch_bounds__(512, 1)
                             *reinterpret_cast<float2 *>(&sm.diag[x][slab][a & 15][b & 15]) =
                                 make_float2(b < a ? e0 * OPERAND_INV : 0.0f, b + 1 < a ? e1 * OPERAND_INV : 0.0f);
                         } else {
+                            // (a token's own key is added in f32)
+                            if (warp >= 8 && (b == a || b + 1 == a)) own[a] = (b == a ? e0 : e1) * OPERAND_INV;
                             uint32_t h, l;
-                            split2(b <= a ? e0 : 0.0f, b + 1 <= a ? e1 : 0.0f, h, l);
+                            split2(b < a ? e0 : 0.0f, b + 1 < a ? e1 : 0.0f, h, l);
                             unsigned char *p = out + a * 128 + (((b >> 3) ^ (a & 7)) << 4) + (b & 7) * 2;
                             *reinterpret_cast<uint32_t *>(p) = h;
                             *reinterpret_cast<uint32_t *>(p + TILE) = l;
@@ -357,7 +393,8 @@ __global__ void __launch_bounds__(512, 1)
                 if (lane < 16) {
 #pragma unroll
                     for (int a = 0; a < 16; a++) {
-                        const __half h = __float2half_rn(v[a] * OPERAND), l = __float2half_rn(v[a] * OPERAND - __half2float(h));
+                        const float e = a == c ? 0.0f : v[a] * OPERAND;              // (the diagonal is added in f32)
+                        const __half h = __float2half_rn(e), l = __float2half_rn(e - __half2float(h));
                         *reinterpret_cast<__half *>(&sm.t[x][J][0][a * T_PITCH + c * 2]) = h;
                         *reinterpret_cast<__half *>(&sm.t[x][J][1][a * T_PITCH + c * 2]) = l;
                     }
@@ -404,7 +441,7 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll 1
                 for (int J = 0; J < 4; J++) {
                     const int r = J * 16 + rn;
-                    float acc[2][4] = {};
+                    float acc[2][4] = {}, low[2][4] = {};
 #pragma unroll
                     for (int I = 0; I < 3; I++) {
                         if (I >= J) break;
@@ -412,8 +449,17 @@ __global__ void __launch_bounds__(512, 1)
                         const uint32_t at = a_at + r * 128 + (((2 * I + cn) ^ (r & 7)) << 4);
                         pg_ldsm4(bh, at);
                         pg_ldsm4(bl, at + TILE);
-                        mma_pair(acc, xh[I], xl[I], bh, bl);
+                        float one[2][4] = {};
+                        mma_pair(one, low, xh[I], xl[I], bh, bl);
+#pragma unroll
+                        for (int n = 0; n < 2; n++)
+#pragma unroll
+                            for (int i = 0; i < 4; i++) acc[n][i] += one[n][i];
                     }
+#pragma unroll
+                    for (int n = 0; n < 2; n++)
+#pragma unroll
+                        for (int i = 0; i < 4; i++) acc[n][i] += low[n][i], low[n][i] = 0.0f;
                     uint32_t th[4], tl[4];
                     pg_ldsm4(th, pg_smem(sm.t[x][J][0]) + rn * T_PITCH + cn * 16);
                     pg_ldsm4(tl, pg_smem(sm.t[x][J][1]) + rn * T_PITCH + cn * 16);
@@ -445,17 +491,18 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll
                         for (int i = 0; i < 2; i++) {
                             const float y0 = fmaf(f0, z[n][i].x, -OPERAND_INV * acc[n][2 * i]), y1 = fmaf(f1, z[n][i].y, -OPERAND_INV * acc[n][2 * i + 1]);
-                            split2(a < bad ? y0 : 0.0f, a + 1 < bad ? y1 : 0.0f, yh[2 * n + i], yl[2 * n + i]);
+                            z[n][i] = make_float2(a < bad ? y0 : 0.0f, a + 1 < bad ? y1 : 0.0f);
+                            split2(z[n][i].x, z[n][i].y, yh[2 * n + i], yl[2 * n + i]);
                         }
                     }
                     float o[2][4] = {};
-                    mma_pair(o, yh, yl, th, tl);
+                    mma_pair(o, low, yh, yl, th, tl);
                     uint32_t nh[4], nl[4];
 #pragma unroll
                     for (int n = 0; n < 2; n++)
 #pragma unroll
                         for (int i = 0; i < 2; i++) {
-                            z[n][i] = make_float2(o[n][2 * i] * OPERAND_INV, o[n][2 * i + 1] * OPERAND_INV);
+                            z[n][i].x = fmaf(o[n][2 * i] + low[n][2 * i], OPERAND_INV, z[n][i].x), z[n][i].y = fmaf(o[n][2 * i + 1] + low[n][2 * i + 1], OPERAND_INV, z[n][i].y);
                             split2(z[n][i].x, z[n][i].y, nh[2 * n + i], nl[2 * n + i]);
                         }
 #pragma unroll
@@ -520,12 +567,14 @@ __global__ void __launch_bounds__(512, 1)
 // O, run beside it.  Operands come through a ring of 16 KB slots, seven a chunk, as soon as a slot is free, and are asked for in L2
 // some chunks ahead (the four CTAs of a head share that).
 //
-// Bound by that chain: 4000 cycles a chunk, 1200 of them the first product, whose operands are 96 KB of shared memory.  4096 tokens of
-// 32 heads 145 us (192 with two fixed buffers and eight warps; delta_scan_kernel, four tokens at a time, 820).
+// Bound by that chain: 4000 cycles a chunk and more, 1200 of them the first product, whose operands are 96 KB of shared memory.  4096 tokens of
+// 32 heads 145 us before its accumulators were divided (192 with two fixed buffers and eight warps; delta_scan_kernel, four tokens at a time, 820).
 constexpr int CHAIN_WARPS = 16, CHAIN_THREADS = (CHAIN_WARPS + 2) * 32, COLS = 32, PART = 8;
 constexpr int SLOT = 2 * TILE, SLOTS = 12, PER_CHUNK = 7, AHEAD = 3;
-constexpr int S_SM = 0, U_SM = 2 * TILE, RING_SM = 3 * TILE, BARS_SM = RING_SM + SLOTS * SLOT;
+constexpr int S_SM = 0, U_SM = 2 * TILE, RING_SM = 3 * TILE, OWN_SM = RING_SM + SLOTS * SLOT, BARS_SM = OWN_SM + CT * COLS * 4;
 constexpr int CHAIN_SMEM = BARS_SM + 256 + 1024;
+// TMEM columns: four accumulators of [W; Q] S, two of K~^T U, two of P U, each [32 with the high part | 32 with the low part]
+constexpr int ACC = 2 * COLS, WS_ACC = 0, KU_ACC = 4 * ACC, PU_ACC = 6 * ACC;
 
 __device__ __forceinline__ void tmem_ld8_async(uint32_t taddr, uint32_t (&v)[8])
 {
@@ -569,16 +618,15 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
             pg_mbar_init(empty + 8 * i, 1);
         }
         pg_mbar_init(bar_s, CHAIN_WARPS);
-        pg_mbar_init(bar_u, CHAIN_WARPS / 2);
+        pg_mbar_init(bar_u, CHAIN_WARPS);
         pg_mbar_init(bar_d1, 1);
         pg_mbar_init(bar_d2, 1);
         pg_mbar_init(bar_d3, 1);
-        pg_mbar_init(bar_d3 + 8, 1);
         abort_flag = 0;
         pg_mbar_fence();
     }
     if (warp == CHAIN_WARPS) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pg_smem(&tmem_slot)), "r"(256) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pg_smem(&tmem_slot)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
@@ -607,11 +655,12 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
                     const uint32_t bar = full + 8 * slot, at = base + RING_SM + slot * SLOT;
                     if (!(ok = pg_mbar_wait(empty + 8 * slot, phase ^ 1, &abort_flag, status, limit_ns))) break;
                     pg_mbar_expect(bar, SLOT);
+                    // (the low parts come first)
                     if (j < 4) {                          // 64 rows of W, 64 of Q
-                        pg_bulk_load(at, hd + W_AT + j * TILE, TILE, bar);
-                        pg_bulk_load(at + TILE, gd + j * TILE, TILE, bar);
+                        pg_bulk_load(at, hd + W_AT + (j ^ 2) * TILE, TILE, bar);
+                        pg_bulk_load(at + TILE, gd + (j ^ 2) * TILE, TILE, bar);
                     } else {                              // K~, its other part, P
-                        pg_bulk_load(at, hd + KT_AT + (j - 4) * SLOT, SLOT, bar);
+                        pg_bulk_load(at, hd + KT_AT + (j < 6 ? (j ^ 1) - 4 : 2) * SLOT, SLOT, bar);
                     }
                     if (++slot == SLOTS) {
                         slot = 0;
@@ -652,7 +701,9 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
                 if (!(ok = wait(full + 8 * slot, phase))) break;
                 const uint64_t desc = make_smem_desc(base + RING_SM + slot * SLOT);
 #pragma unroll
-                for (int j = 0; j < 4; j++) umma_f16(tmem, desc + (uint64_t)(j * 2), desc_s + (uint64_t)(((t & 1) * 4 + j) * (2048 >> 4)), idesc, (t | j) != 0 ? 1u : 0u, on);
+                for (int j = 0; j < 4; j++) 
+                    umma_f16(tmem + WS_ACC + (t < 2 ? 0 : ((t & 1) * 2 + (j >> 1)) * ACC), desc + (uint64_t)(j * 2), desc_s + (uint64_t)(((t & 1) * 4 + j) * (2048 >> 4)), idesc,
+                             (t | j) == 0 || (t == 3 && !(j & 1)) || (t == 2 && j == 2) ? 0u : 1u, on);
                 if (t == 3) umma_commit(bar_d1, on);
                 next();
             }
@@ -663,7 +714,8 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
                 const uint64_t desc = make_smem_desc_mn(base + RING_SM + slot * SLOT, TILE);
 #pragma unroll
                 for (int j = 0; j < 4; j++)
-                    umma_f16(tmem + 64, desc + (uint64_t)(j * (2048 >> 4)), desc_u + (uint64_t)(j * (2048 >> 4)), idesc | IDESC_A_MN_MAJOR, (t | j) != 0 ? 1u : 0u, on);
+                    umma_f16(tmem + KU_ACC + (t & (j >> 1)) * ACC, desc + (uint64_t)(j * (2048 >> 4)), desc_u + (uint64_t)(j * (2048 >> 4)), idesc | IDESC_A_MN_MAJOR,
+                             (t | j) == 0 || (t == 1 && j == 2) ? 0u : 1u, on);
                 if (t == 1) umma_commit(bar_d2, on);
                 next();
             }
@@ -671,11 +723,12 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
             // the products of P are rows 64 .. 127 of the instruction, where the read-outs lie; rows 0 .. 63 are what lies in front
             const uint64_t desc = make_smem_desc(base + RING_SM + slot * SLOT - TILE);
 #pragma unroll
-            for (int t = 0; t < 2; t++)
+            for (int t = 1; t >= 0; t--)
 #pragma unroll
                 for (int j = 0; j < 4; j++)
-                    umma_f16(tmem + 128 + 64 * (i & 1), desc + (uint64_t)(t * (TILE >> 4) + j * 2), desc_u + (uint64_t)(j * (2048 >> 4)), idesc, (t | j) != 0 ? 1u : 0u, on);
-            umma_commit(bar_d3 + 8 * (i & 1), on);
+                    umma_f16(tmem + PU_ACC + (t == 0 ? (j >> 1) * ACC : 0), desc + (uint64_t)(t * (TILE >> 4) + j * 2), desc_u + (uint64_t)(j * (2048 >> 4)), idesc,
+                             (t == 1 && j == 0) || (t == 0 && j == 2) ? 0u : 1u, on);
+            umma_commit(bar_d3, on);
             next();
         }
     } else {
@@ -684,13 +737,15 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
         const bool outputs = q >= 2;                                                    // rows of Q, else of W
         const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16) + part * PART;
         auto wait = [&](uint32_t bar, uint32_t parity) { return (bool)__all_sync(0xffffffffu, pg_mbar_wait(bar, parity, &abort_flag, status, limit_ns)); };
-        auto sums = [&](uint32_t at, float (&v)[PART]) {  // products with the two parts, added
-            uint32_t x[PART], y[PART];
+        auto sums = [&](uint32_t at, float (&v)[PART]) {  // two accumulators: products with the high parts, and with the low ones
+            uint32_t x[PART], y[PART], z[PART], t[PART];
             tmem_ld8_async(at, x);
+            tmem_ld8_async(at + ACC, z);
             tmem_ld8_async(at + COLS, y);
+            tmem_ld8_async(at + ACC + COLS, t);
             tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < PART; j++) v[j] = __uint_as_float(x[j]) + __uint_as_float(y[j]);
+            for (int j = 0; j < PART; j++) v[j] = (__uint_as_float(x[j]) + __uint_as_float(z[j])) + (__uint_as_float(y[j]) + __uint_as_float(t[j]));
         };
         auto largest_of = [&](const uint32_t (&v)[CHAIN_WARPS]) {
             const uint4 *p = reinterpret_cast<const uint4 *>(v);
@@ -717,12 +772,14 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
         __syncwarp();
         if (lane == 0) pg_mbar_arrive(bar_s);
         const unsigned char *next_chunk = mine;
-        float u0[PART], n_c = 0.0f, n_last = 0.0f, n_max = 0.0f;
+        float u0[PART], n_c = 0.0f, n_own = 0.0f, n_last = 0.0f, n_max = 0.0f;
+        float4 *mine_f32 = reinterpret_cast<float4 *>(chain_raw + (base - raw) + OWN_SM) + ((q & 1) * 4 + part) * 64 + lane;   // U of this lane's token
         int n_bad = CT;
         auto load_next = [&]() {                          // what the next chunk needs besides operands
             const float *coef = reinterpret_cast<const float *>(next_chunk + COEF_AT);
             if (outputs) {
                 n_c = __ldcg(coef + a);
+                n_own = __ldcg(coef + COEF_OWN + a);
             } else {
                 const float4 *src = reinterpret_cast<const float4 *>(next_chunk + U0_AT) + (a * CD + col) / 4;
 #pragma unroll
@@ -739,16 +796,26 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
         load_next();
         bool ok = true;
         for (int i = 0; i < chunks; i++) {
-            const float c = n_c, last = n_last, u0_max = n_max;
+            const float c = n_c, own = n_own, last = n_last, u0_max = n_max;
             const int bad = n_bad;
             if (!(ok = wait(bar_s, i & 1))) break;
             const float largest = largest_of(top_s[i & 1]);
             // |U| <= |U0| + |w| |S column|, and a column of S has 128 elements
             const float2 scale_u = scale_of(u0_max + 12.0f * largest, 14);
+            if (outputs) {                                // the sums of the read-outs in front may go
+                tc_fence_before();
+                if (lane == 0) pg_mbar_arrive(bar_u);
+            }
             if (!(ok = wait(bar_d1, i & 1))) break;
             tc_fence_after();
             float o[PART];
-            sums(lanes, o);
+            {
+                float more[PART];
+                sums(lanes + WS_ACC, o);
+                sums(lanes + WS_ACC + 2 * ACC, more);
+#pragma unroll
+                for (int j = 0; j < PART; j++) o[j] += more[j];
+            }
             if (!outputs) {
                 const float inv = scale_s.y * OPERAND_INV;
                 uint32_t most = 0;
@@ -758,6 +825,8 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
                     most = max(most, bits(o[j]));
                 }
                 put_row(base + U_SM, a, part, o, scale_u.x);
+#pragma unroll
+                for (int j = 0; j < PART / 4; j++) mine_f32[j * 32] = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
                 most = warp_max(most);
                 if (lane == 0) top_u[i & 1][q * 4 + part] = most;
                 tc_fence_before();
@@ -775,12 +844,20 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
                 const uint4 *p = reinterpret_cast<const uint4 *>(top_u[i & 1]);
                 scale_s = scale_of(fmaf(64.5f, __uint_as_float(max(max4(p[0]), max4(p[1]))), largest), 14);
             }
+            if (outputs) {
+#pragma unroll
+                for (int j = 0; j < PART / 4; j++) {
+                    const float4 u = mine_f32[j * 32];
+                    o[4 * j] = fmaf(own, u.x, o[4 * j]), o[4 * j + 1] = fmaf(own, u.y, o[4 * j + 1]);
+                    o[4 * j + 2] = fmaf(own, u.z, o[4 * j + 2]), o[4 * j + 3] = fmaf(own, u.w, o[4 * j + 3]);
+                }
+            }
             const float inv_u = scale_u.y * OPERAND_INV;
             if (!(ok = wait(bar_d2, i & 1))) break;
             tc_fence_after();
             {
                 float v[PART];
-                sums(lanes + 64, v);
+                sums(lanes + KU_ACC, v);
                 top = 0;
 #pragma unroll
                 for (int j = 0; j < PART; j++) {
@@ -799,10 +876,10 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
                 if (lane == 0) pg_mbar_arrive(bar_s);
             }
             if (outputs) {
-                if (!(ok = wait(bar_d3 + 8 * (i & 1), (i >> 1) & 1))) break;
+                if (!(ok = wait(bar_d3, i & 1))) break;
                 tc_fence_after();
                 float v[PART];
-                sums(lanes + 128 + 64 * (i & 1), v);
+                sums(lanes + PU_ACC, v);
                 if (i * CT + a < T) {
                     float4 *dst = reinterpret_cast<float4 *>(w.o + ((int64_t)(row0 + i * CT + a) * s.H + h) * CD + col);
 #pragma unroll
@@ -825,7 +902,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
     __syncthreads();
     if (warp == CHAIN_WARPS) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     }
 }
 

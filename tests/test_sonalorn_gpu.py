@@ -375,6 +375,31 @@ def test_delta_chunks(lm, dtype, heads, kv_heads, taps, slow):
     mixer.free()
 
 
+@pytest.mark.parametrize("slow", [False, True])
+def test_delta_chunks_are_as_exact_as_blocks_of_four(lm, slow):
+    """The error against 64 bits of the form with tensor cores is that of the f32 form, or less (a twentieth for what six draws differ
+    by), with rates of decay between 1 and 16 and steps between 0.001 and 0.1, and where little is forgotten."""
+    from peregrine_b200.layers import GatedDelta
+
+    p, width, T = t.delta(4, 2, 128, 128, 4), 64, 450
+    d = device(lm, "float32", 512)
+    off = {False: np.zeros(2), True: np.zeros(2)}
+    for seed in range(6):
+        g = rng(seed)
+        W = {k: t.bf16_values(v) for k, v in t.mixer_weights(g, "delta", p, width).items()}
+        W["A_log"], W["dt_bias"] = (t.bf16_values(v) for v in ((np.full(4, -5.0), np.full(4, -2.0)) if slow else
+                                    (np.log(g.uniform(1, 16, 4)), np.log(np.expm1(np.exp(g.uniform(np.log(1e-3), np.log(0.1), 4)))))))
+        x = t.bf16_values(g.standard_normal((T, width)))
+        want, carried = so.delta_mixer(x.astype(np.float64), {k: v.astype(np.float64) for k, v in W.items()}, p, 1e-4, so.delta_start(p))
+        for chunks in off:
+            mixer = GatedDelta(d, p, W, width, 1e-4, chunks)
+            got, state = run_mixer(lm, d, mixer, width, x, [T])
+            for i, (a, b) in enumerate(((got, want), (state["state"][1].cpu().numpy(), carried["S"]))):
+                off[chunks][i] += np.linalg.norm(a - b) / np.linalg.norm(b)
+            mixer.free()
+    assert (off[True] <= 1.05 * off[False]).all(), f"outputs and states: {off}"
+
+
 def test_delta_chunks_beside_short_portions(lm):
     """Sequences of one step that go by chunks and by blocks of four, in any order; each as if it were alone."""
     from peregrine_b200.layers import Batch, GatedDelta, up
