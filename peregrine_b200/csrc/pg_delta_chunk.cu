@@ -191,6 +191,8 @@ __global__ void __launch_bounds__(512, 1)
             if (lane >= o) sum += up;
         }
         const double all = __shfl_sync(0xffffffffu, sum, 31);
+        double l = __shfl_up_sync(0xffffffffu, sum, 1);              // of the tokens in front of this lane's two
+        if (lane == 0) l = 0.0;
         float *coef = reinterpret_cast<float *>(head_data(s, w, chunk, h) + COEF_AT);
         auto decay = [](double l) {                                   // e^l; the rest of l is below 2^-24 of it
             const float hi = (float)l;
@@ -199,7 +201,7 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll
         for (int i = 0; i < 2; i++) {
             const int a = lane * 2 + i;
-            const double l = i ? sum : sum - v[1];
+            l += v[i];
             sm.l_hi[x][a] = (float)l;
             sm.l_lo[x][a] = (float)(l - (double)(float)l);
             sm.beta[x][a] = be[i];

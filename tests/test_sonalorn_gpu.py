@@ -425,12 +425,13 @@ def test_delta_chunks_beside_short_portions(lm):
     mixer.free()
 
 
-def test_delta_chunks_keep_infinities_to_later_tokens(lm):
-    """A value that is not finite reaches its own token and those behind it, also within a chunk of 64."""
+@pytest.mark.parametrize("at", [1, 2, 63, 64, 65, 100, 101, 127, 128, 199])
+def test_delta_chunks_keep_infinities_to_later_tokens(lm, at):
+    """A value that is not finite reaches its own token and those behind it, also within a chunk of 64 and of a pair of tokens."""
     from peregrine_b200.layers import Batch, GatedDelta, up
     from peregrine_b200.state import SlotPool
 
-    p, width, T, at = t.delta(2, 1, 128, 128, 2), 80, 200, 100
+    p, width, T = t.delta(2, 1, 128, 128, 2), 80, 200
     d = device(lm, "float32", 400)
     g = rng(6)
     W = {k: t.bf16_values(v) for k, v in t.mixer_weights(g, "delta", p, width).items()}
