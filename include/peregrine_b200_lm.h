@@ -105,7 +105,7 @@ typedef struct pg_delta {
 PG_API int64_t pg_delta_work_floats(const pg_delta *p, int64_t max_rows);
 PG_API int32_t pg_delta_run(pg_ctx *ctx, const pg_delta *p, const pg_batch *batch, const float *d_proj, int64_t ldp, float *d_ring, float *d_state,
                             void *d_out, int32_t dtype, int64_t ldo);
-/* The same; portions of 64 and more tokens of heads of 128 x 128 (two to four taps) go by chunks of 64, with products on the
+/* The same; portions of 128 and more tokens of heads of 128 x 128 (two to four taps) go by chunks of 64, with products on the
  * tensor cores and sums in another order.  d_work: pg_delta_chunks_work_floats(...) */
 PG_API int64_t pg_delta_chunks_work_floats(const pg_delta *p, int64_t max_rows);
 PG_API int32_t pg_delta_run_chunks(pg_ctx *ctx, const pg_delta *p, const pg_batch *batch, const float *d_proj, int64_t ldp, float *d_ring, float *d_state,

@@ -720,13 +720,13 @@ int32_t run_delta(pg_ctx *ctx, const pg_delta *p, const pg_batch *batch, const f
     w.o = at, at += pg_up((int64_t)M * s.H * s.V, 4);
     w.coef = at, at += (int64_t)(M + 8) * s.H * 32;
     w.chunks = reinterpret_cast<unsigned char *>(((uintptr_t)at + 127) & ~(uintptr_t)127);
-    const bool chunks = by_chunks && batch->max_len >= DELTA_CHUNK && pgk_delta_chunk_supports(s, d_proj, ldp, d_ring, d_state);
+    const bool chunks = by_chunks && batch->max_len >= DELTA_LONG && pgk_delta_chunk_supports(s, d_proj, ldp, d_ring, d_state);
     int32_t rc = PG_OK;
     if (chunks) rc = pgk_delta_chunk(ctx, s, batch, d_proj, ldp, d_ring, w, d_state);
     if (rc != PG_OK) return rc;
     // (sequences of equal length are all of one kind)
     if (!chunks || (int64_t)batch->seqs * batch->max_len != M) {
-        const int most = chunks ? DELTA_CHUNK - 1 : INT_MAX;
+        const int most = chunks ? DELTA_LONG - 1 : INT_MAX;
         if (s.taps == 2)
             rc = run_prep<2>(ctx, s, batch, d_proj, ldp, d_ring, w, most);
         else if (s.taps == 3)
@@ -779,7 +779,7 @@ PG_API int32_t pg_delta_run(pg_ctx *ctx, const pg_delta *p, const pg_batch *batc
 PG_API int64_t pg_delta_chunks_work_floats(const pg_delta *p, int64_t max_rows)
 {
     if (!p || max_rows < 0) return 0;
-    return pg_delta_work_floats(p, max_rows) + pgk_delta_chunk_floats(p->kv_heads, p->heads, p->dim, p->vdim, max_rows);
+    return pg_delta_work_floats(p, max_rows) + pgk_delta_chunk_floats(p->kv_heads, p->heads, p->dim, p->vdim, p->taps, max_rows);
 }
 
 PG_API int32_t pg_delta_run_chunks(pg_ctx *ctx, const pg_delta *p, const pg_batch *batch, const float *d_proj, int64_t ldp, float *d_ring, float *d_state,

@@ -37,9 +37,12 @@ struct DeltaWork {
     unsigned char *chunks;
 };
 
-// pg_delta_chunk.cu: sequences of at least DELTA_CHUNK tokens of a step, o for their rows and their states
-constexpr int DELTA_CHUNK = 64;
+// pg_delta_chunk.cu: sequences of at least DELTA_LONG tokens of a step, o for their rows and their states.  From there on the chunks are
+// the faster form: 64 / 100 / 128 / 192 tokens of 32 heads 48 / 51 / 51 / 54 us against 48 / 56 / 64 / 78 by blocks of four, of 16 heads 43 / 44 / 45 / 48
+// against 35 / 42 / 50 / 62; sixty sequences of 65 tokens 843 against 724, eight of 64 tokens 98 against 116.  Below that a chunk that is
+// hardly filled takes as much workspace as a full one, and the outputs' error is 1 to 2 % above that of blocks of four.
+constexpr int DELTA_CHUNK = 64, DELTA_LONG = 128;
 bool pgk_delta_chunk_supports(const DeltaShape &s, const float *proj, int64_t ldp, const float *ring, const float *state);
-int64_t pgk_delta_chunk_floats(int64_t kv_heads, int64_t heads, int64_t dim, int64_t vdim, int64_t max_rows);
+int64_t pgk_delta_chunk_floats(int64_t kv_heads, int64_t heads, int64_t dim, int64_t vdim, int64_t taps, int64_t max_rows);
 int32_t pgk_delta_chunk(pg_ctx *ctx, const DeltaShape &s, const pg_batch *bt, const float *proj, int64_t ldp, const float *ring, const DeltaWork &w,
                         float *state);

@@ -41,8 +41,16 @@ constexpr int TILE = 8192, W_AT = 0, KT_AT = 4 * TILE, P_AT = 8 * TILE, U0_AT = 
 constexpr int HEAD_BYTES = COEF_AT + 640, GROUP_BYTES = 4 * TILE;
 constexpr int COEF_OWN = CT, COEF_LAST = 2 * CT, COEF_MAX = COEF_LAST + 1, COEF_BAD = COEF_LAST + 2;   // c [64], q_a . k_a [64], c_63, largest |U0|, first token that is not finite
 
-// A sequence has at least 64 tokens: the chunks of the one at row0 are numbered from row0 / 32 on.
-__host__ __device__ __forceinline__ int64_t first_chunk(int64_t row0) { return row0 / 32; }
+// The chunks of the sequence at row0 are numbered from here on; none has another's number, since a sequence has at least DELTA_LONG tokens.
+constexpr int ROWS_PER_CHUNK = 43;
+__host__ __device__ constexpr int64_t first_chunk(int64_t row0) { return row0 / ROWS_PER_CHUNK; }
+constexpr bool chunks_find_room()
+{
+    for (int T = DELTA_LONG; T < DELTA_LONG + 64 * ROWS_PER_CHUNK; T++)
+        if (T / ROWS_PER_CHUNK < (T + CT - 1) / CT) return false;
+    return true;
+}
+static_assert(chunks_find_room(), "two sequences would share a chunk");
 __device__ __forceinline__ unsigned char *head_data(const DeltaShape &s, const DeltaWork &w, int64_t chunk, int h)
 {
     return w.chunks + chunk * ((int64_t)s.H * HEAD_BYTES + (int64_t)s.G * GROUP_BYTES) + (int64_t)h * HEAD_BYTES;
@@ -153,7 +161,7 @@ __global__ void __launch_bounds__(512, 1)
     pg_pdl_begin();
     const int seq = blockIdx.z, g = blockIdx.x, nth = gridDim.y - 1 - blockIdx.y, row0 = __ldcg(bt.d_seq_row0 + seq), T = __ldcg(bt.d_seq_row0 + seq + 1) - row0;
     const int t0 = nth * CT;
-    if (T < CT || t0 >= T) return;
+    if (T < DELTA_LONG || t0 >= T) return;
     const int rep = s.H / s.G, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int pos0 = __ldcg(bt.d_pos + row0);
     const float *first = proj + (int64_t)row0 * ldp;                  // the sequence's rows
@@ -611,7 +619,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
     pg_pdl_begin();
     const int seq = gridDim.z - 1 - blockIdx.z, h = blockIdx.y, g = h / (s.H / s.G), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row0 = __ldcg(bt.d_seq_row0 + seq), T = __ldcg(bt.d_seq_row0 + seq + 1) - row0;
-    if (T < CT) return;
+    if (T < DELTA_LONG) return;
     const uint32_t raw = pg_smem(chain_raw), base = (raw + 1023u) & ~1023u, full = base + BARS_SM, empty = full + 8 * SLOTS, bar_s = empty + 8 * SLOTS,
                    bar_u = bar_s + 8, bar_d1 = bar_s + 16, bar_d2 = bar_s + 24, bar_d3 = bar_s + 32;
     if (threadIdx.x == 0) {
@@ -926,9 +934,9 @@ bool pgk_delta_chunk_supports(const DeltaShape &s, const float *proj, int64_t ld
            (((uintptr_t)proj | (uintptr_t)ring | (uintptr_t)state | (uintptr_t)s.conv) & 15) == 0;
 }
 
-int64_t pgk_delta_chunk_floats(int64_t kv_heads, int64_t heads, int64_t dim, int64_t vdim, int64_t max_rows)
+int64_t pgk_delta_chunk_floats(int64_t kv_heads, int64_t heads, int64_t dim, int64_t vdim, int64_t taps, int64_t max_rows)
 {
-    if (dim != CD || vdim != CD || max_rows < CT) return 0;
+    if (dim != CD || vdim != CD || taps < 2 || taps > 4 || max_rows < DELTA_LONG) return 0;
     return (first_chunk(max_rows) + 1) * ((heads * HEAD_BYTES + kv_heads * GROUP_BYTES) / 4) + 256;
 }
 

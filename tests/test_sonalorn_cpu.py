@@ -228,6 +228,22 @@ def test_lm_library_exports_its_header_and_the_shared_part():
     assert lib.pg_linear_wrap(None, None, 1, 64, 1, C.byref(h)) == _lib.PG_ERR_INVALID
 
 
+def test_delta_chunks_take_room_for_what_they_can_use():
+    """What chunks of 64 tokens add to the workspace: at most half as many again as a step of one sequence fills, nothing where the
+    layer has no such form."""
+    from peregrine_b200 import _lib
+    from peregrine_b200.build import ensure_built
+
+    ensure_built("lm")
+    lib = _lib.load("lm")
+    more = lambda rows, **k: (lambda p: lib.pg_delta_chunks_work_floats(p, rows) - lib.pg_delta_work_floats(p, rows))(
+        C.byref(_lib.PgDelta(**{**dict(heads=32, kv_heads=16, dim=128, vdim=128, taps=4), **k})))
+    image = (32 * 113 * 1024 + 16 * 32 * 1024) // 4        # floats of a chunk: operands, values and coefficients of each head, queries
+    for rows in (128, 1000, 4096, 65536):
+        assert image * (rows // 64) <= more(rows) <= image * (rows // 64) * 3 // 2 + 2 * image
+    assert more(127) == more(4096, taps=5) == more(4096, taps=1) == more(4096, dim=64) == more(4096, vdim=256) == 0
+
+
 def test_command_line_help_and_bad_model(tmp_path):
     run = lambda *a: subprocess.run([sys.executable, "-m", "peregrine_b200", *a], cwd=ROOT, capture_output=True, text=True)
     assert "generate" in run("--help").stdout

@@ -350,7 +350,7 @@ def test_delta_state_is_f32_over_a_long_sequence(lm):
         mixer.free()
 
 
-# heads of 128 x 128: portions of 64 and more tokens go by chunks of 64, shorter ones by blocks of four
+# heads of 128 x 128: portions of 128 and more tokens go by chunks of 64, shorter ones by blocks of four
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads,kv_heads,taps,slow", [(2, 2, 2, False), (4, 2, 4, True), (3, 1, 3, False), (1, 1, 4, True)])
 def test_delta_chunks(lm, dtype, heads, kv_heads, taps, slow):
@@ -367,7 +367,7 @@ def test_delta_chunks(lm, dtype, heads, kv_heads, taps, slow):
     want, carried = so.delta_mixer(x.astype(np.float64), {k: v.astype(np.float64) for k, v in W.items()}, p, 1e-4, so.delta_start(p))
     # (f32: operands of 22 bits and more, sums of 32; errors of one chunk fade or stay in the next)
     tol = 1e-5 if dtype == "float32" else 6e-2
-    for cuts in ([T], [64, 65, 1, 127, 10, 63, 3], [128, 192, 13], [1] * 20 + [64] * 4 + [57]):
+    for cuts in ([T], [64, 65, 1, 127, 10, 63, 3], [128, 192, 13], [1] * 20 + [64] * 4 + [57], [129, 1, 203]):
         got, state = run_mixer(lm, d, mixer, width, x, cuts)
         close(got, want, tol, f"cuts {cuts[:4]}")
         close(state["state"][1].cpu().numpy(), carried["S"], tol, "state")
@@ -405,8 +405,8 @@ def test_delta_chunks_beside_short_portions(lm):
     from peregrine_b200.layers import Batch, GatedDelta, up
     from peregrine_b200.state import SlotPool
 
-    p, width, lengths = t.delta(4, 2, 128, 128, 4), 80, [5, 64, 63, 200, 1, 65]
-    d = device(lm, "float32", 400)
+    p, width, lengths = t.delta(4, 2, 128, 128, 4), 80, [5, 129, 64, 128, 63, 200, 1, 127, 193, 65]
+    d = device(lm, "float32", sum(lengths))
     g = rng(5)
     W = {k: t.bf16_values(v) for k, v in t.mixer_weights(g, "delta", p, width).items()}
     mixer = GatedDelta(d, p, W, width, 1e-4)
