@@ -344,6 +344,7 @@ __global__ void __launch_bounds__(512, 1)
         }
         if (gate < heads) gates(gate, h0 + gate);
         __syncthreads();
+        const int bad = min(sm.bad[warp >> 3], sm.bad_k);             // (of the head whose substitution this warp does, which may lower it)
         // A (warps 0 .. 7; its diagonal blocks apart, in f32) and P
         for (int x = 0; x < heads; x++) {
             unsigned char *out = warp < 8 ? sm.a[x] : head_data(s, w, chunk, h0 + x) + P_AT;
@@ -436,7 +437,7 @@ __global__ void __launch_bounds__(512, 1)
         const int x = warp >> 3;
         if (x < heads) {
             const bool of_v = (warp & 4) != 0;
-            const int d0 = (warp & 3) * 32, bad = min(sm.bad[x], sm.bad_k);
+            const int d0 = (warp & 3) * 32;
             // (|u_a| <= 65 max |v|, and so are the sums in front of T: a state is at most the sum of the values behind it)
             const float2 scale = of_v ? scale_of(__uint_as_float(sm.top_v[x]), 7) : make_float2(1.0f, 1.0f);
             unsigned char *img = x == 0 ? sm.w0 : sm.w1;
