@@ -99,10 +99,11 @@ __device__ __forceinline__ void stsm4_t(uint32_t addr, const uint32_t (&r)[4])
 __device__ __forceinline__ uint32_t bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }   // |x|; NaN is the largest
 __device__ __forceinline__ uint32_t warp_max(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
 constexpr uint32_t NOT_FINITE = 0x7f800000u;
-// a power of two that brings a bound into [2^to, 2^(to + 1)), and its inverse
+// a power of two that brings a bound into [2^to, 2^(to + 1)), and its inverse (both normal numbers; no bound is so large that the
+// lower limit counts)
 __device__ __forceinline__ float2 scale_of(float bound, int to)
 {
-    const int e = min(100, max(-100, 127 + to - (int)(bits(bound) >> 23)));
+    const int e = min(100, max(-126, 127 + to - (int)(bits(bound) >> 23)));
     return make_float2(__uint_as_float((uint32_t)(127 + e) << 23), __uint_as_float((uint32_t)(127 - e) << 23));
 }
 

@@ -425,6 +425,25 @@ def test_delta_chunks_beside_short_portions(lm):
     mixer.free()
 
 
+@pytest.mark.parametrize("size", [1e-25, 1e10, 3e36])
+def test_delta_chunks_of_values_of_any_size(lm, size):
+    """Values and states are f32: their operands' scale follows them, to either end of the range."""
+    from peregrine_b200.layers import GatedDelta
+
+    p, width, T = t.delta(2, 1, 128, 128, 2), 80, 200
+    d = device(lm, "float32", 256)
+    g = rng(7)
+    W = {k: t.bf16_values(v) for k, v in t.mixer_weights(g, "delta", p, width).items()}
+    W["v"] = t.bf16_values(W["v"] * size)
+    x = t.bf16_values(g.standard_normal((T, width)))
+    mixer = GatedDelta(d, p, W, width, 1e-4)
+    _, carried = so.delta_mixer(x.astype(np.float64), {k: v.astype(np.float64) for k, v in W.items()}, p, 1e-4, so.delta_start(p))
+    _, state = run_mixer(lm, d, mixer, width, x, [T])
+    S = state["state"][1].cpu().numpy().astype(np.float64)
+    assert np.abs(carried["S"]).max() > 1e-3 * size and np.linalg.norm(S - carried["S"]) <= 1e-5 * np.linalg.norm(carried["S"])
+    mixer.free()
+
+
 @pytest.mark.parametrize("at", [1, 2, 63, 64, 65, 100, 101, 127, 128, 199])
 def test_delta_chunks_keep_infinities_to_later_tokens(lm, at):
     """A value that is not finite reaches its own token and those behind it, also within a chunk of 64 and of a pair of tokens."""
