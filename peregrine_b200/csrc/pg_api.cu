@@ -277,7 +277,7 @@ static int32_t gemm_dispatch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, 
         case PG_ALGO_STREAM:
             return pgk_gemm_i8_stream(ctx, d_a, d_as, m, k, w->d_data_i8_t, w->d_scales, n, d_y, d_acc);
         case PG_ALGO_TCGEN05:
-            return pgk_gemm_i8_tcgen05(ctx, d_a, d_as, m, k, const_cast<pg_qtensor *>(w), d_y, d_acc);
+            return pgk_gemm_i8_tcgen05(ctx, d_a, d_as, m, k, w, d_y, d_acc);
         case PG_ALGO_WSTREAM:
             return pgk_gemm_i8_wstream(ctx, d_a, d_as, m, k, w->d_data_i8_t, w->d_scales, n, d_y, d_acc);
         case PG_ALGO_AUTO:
@@ -295,7 +295,7 @@ static int32_t gemm_dispatch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, 
                 !(pgk_gemm_i8_tcgen05_supports(m, k, n) && m > 16 && (m > 32 || n >= 40ll * ctx->sm_count || k >= 8192)))
                 return pgk_gemm_i8_stream(ctx, d_a, d_as, m, k, w->d_data_i8_t, w->d_scales, n, d_y, d_acc);
             if (aligned && pgk_gemm_i8_tcgen05_supports(m, k, n))
-                return pgk_gemm_i8_tcgen05(ctx, d_a, d_as, m, k, const_cast<pg_qtensor *>(w), d_y, d_acc);
+                return pgk_gemm_i8_tcgen05(ctx, d_a, d_as, m, k, w, d_y, d_acc);
             // shapes neither fast kernel takes (K not a multiple of 16, odd alignment)
             return pgk_gemm_i8_naive(ctx, d_a, d_as, m, k, w->d_data_i8_t, w->d_scales, n, d_y, d_acc);
     }

@@ -515,18 +515,15 @@ constexpr size_t SPLIT_TICKET_BYTES = 64 * 1024;
 constexpr size_t SPLIT_MAX_BYTES = 64u << 20;
 
 template <int BN, int AR>
-int32_t launch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, pg_qtensor *w, float *d_y, int32_t *d_acc, int splits)
+int32_t launch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, const pg_qtensor *w, float *d_y, int32_t *d_acc, int splits)
 {
     using C = Cfg<BN, AR>;
     const int N = (int)w->cols;
-    CUtensorMap ta;
+    // (both of the call's own: a weight may be in use by other threads and contexts, with other tiles)
+    CUtensorMap ta, tb;
     int32_t rc = encode_kmajor(&ta, d_a, M, K, AR);
+    if (rc == PG_OK) rc = encode_kmajor(&tb, w->d_data_i8_t, N, K, BN);
     if (rc) return rc;
-    if (w->tmap_b_box_rows != BN) {
-        rc = encode_kmajor(reinterpret_cast<CUtensorMap *>(w->tmap_b), w->d_data_i8_t, N, K, BN);
-        if (rc) return rc;
-        w->tmap_b_box_rows = BN;
-    }
     auto kern = gemm_i8_tcgen05_kernel<BN, AR>;
     static std::atomic<uint64_t> smem_set{0};
     PG_CUDA(pg_max_smem_once(kern, (int)C::SMEM, ctx->device, smem_set));
@@ -548,7 +545,7 @@ int32_t launch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, 
     cfg.stream = ctx->stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    PG_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, *reinterpret_cast<CUtensorMap *>(w->tmap_b), d_as, (const float *)w->d_scales, M, N, K,
+    PG_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, d_as, (const float *)w->d_scales, M, N, K,
                                d_y, d_acc, ctx->d_status, splits, ws, tickets));
     PG_LAUNCHED();
     return PG_OK;
@@ -570,7 +567,7 @@ bool pgk_gemm_i8_tcgen05_supports(int64_t m, int64_t k, int64_t n)
            m * n < (1ll << 40);
 }
 
-int32_t pgk_gemm_i8_tcgen05(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, pg_qtensor *w, float *d_y,
+int32_t pgk_gemm_i8_tcgen05(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, const pg_qtensor *w, float *d_y,
                             int32_t *d_acc)
 {
     const int64_t n = w->cols;

@@ -404,18 +404,15 @@ int32_t encode_kmajor(CUtensorMap *map, const void *ptr, int64_t rows, int64_t k
 }
 
 template <int TNH>
-int32_t launch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, pg_qtensor *w, float *d_y, int32_t *d_acc)
+int32_t launch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, const pg_qtensor *w, float *d_y, int32_t *d_acc)
 {
     using C = Cfg<TNH>;
     const int N = (int)w->cols;
-    CUtensorMap ta;
+    // (both of the call's own: a weight may be in use by other threads and contexts, with tiles of another width)
+    CUtensorMap ta, tb;
     int32_t rc = encode_kmajor(&ta, d_a, M, K, TM);
+    if (rc == PG_OK) rc = encode_kmajor(&tb, w->d_data_i8_t, N, K, TNH);
     if (rc) return rc;
-    if (w->tmap_b_box_rows != TNH) {
-        rc = encode_kmajor(reinterpret_cast<CUtensorMap *>(w->tmap_b), w->d_data_i8_t, N, K, TNH);
-        if (rc) return rc;
-        w->tmap_b_box_rows = TNH;
-    }
     auto kern = gemm_i8_tcgen05_2cta_kernel<TNH>;
     static std::atomic<uint64_t> smem_set{0};
     PG_CUDA(pg_max_smem_once(kern, (int)C::SMEM, ctx->device, smem_set));
@@ -435,7 +432,7 @@ int32_t launch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    PG_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, *reinterpret_cast<CUtensorMap *>(w->tmap_b), d_as, (const float *)w->d_scales, M, N, K, d_y, d_acc,
+    PG_CUDA(cudaLaunchKernelEx(&cfg, kern, ta, tb, d_as, (const float *)w->d_scales, M, N, K, d_y, d_acc,
                                ctx->d_status));
     PG_LAUNCHED();
     return PG_OK;
@@ -443,7 +440,7 @@ int32_t launch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, 
 
 }  // namespace
 
-int32_t pgk_gemm_i8_tcgen05_2cta(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, pg_qtensor *w,
+int32_t pgk_gemm_i8_tcgen05_2cta(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, const pg_qtensor *w,
                                  float *d_y, int32_t *d_acc)
 {
     // The width whose rounds of tiles take least: a pair runs ceil(tiles / pairs) tiles, each as long as it is wide (and some 16 columns'

@@ -173,9 +173,6 @@ struct pg_qtensor {
     int64_t cols = 0;                     // N held on this GPU
     bool owned = false;
     void *block = nullptr;                // where the three arrays are parts of one allocation: that allocation
-    // TMA descriptor of data_i8_t for the tcgen05 path, built on first use (128 B, opaque)
-    alignas(64) unsigned char tmap_b[128];
-    int tmap_b_box_rows = 0;
 };
 
 struct pg_gguf_weight {
@@ -446,10 +443,10 @@ int32_t pgk_gqa_decode_stream(pg_ctx *ctx, const float *d_q, float *d_k, float *
 bool pgk_gemm_i8_mid_supports(pg_ctx *ctx, int64_t m, int64_t k, int64_t n);
 int32_t pgk_gemm_i8_mid(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, const pg_qtensor *w, float *d_y, int32_t *d_acc);
 bool pgk_gemm_i8_tcgen05_supports(int64_t m, int64_t k, int64_t n);
-int32_t pgk_gemm_i8_tcgen05(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, pg_qtensor *w,
+int32_t pgk_gemm_i8_tcgen05(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, const pg_qtensor *w,
                             float *d_y, int32_t *d_acc);
 // pg_gemm_tcgen05_2cta.cu
-int32_t pgk_gemm_i8_tcgen05_2cta(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, pg_qtensor *w,
+int32_t pgk_gemm_i8_tcgen05_2cta(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, const pg_qtensor *w,
                                  float *d_y, int32_t *d_acc);
 // pg_gguf.cu
 int32_t pgk_dequant_blocks(pg_ctx *ctx, int32_t type, const uint8_t *d_raw, int64_t num_blocks, float *d_out);

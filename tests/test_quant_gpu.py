@@ -353,6 +353,51 @@ def test_tcgen05_cta_pairs(pg, gpu, oracle_mt, m, k, n):
         gpu.lib.pg_tune_tcgen05_pair(0)
 
 
+def test_threads_share_a_weight(pg, gpu):
+    """Two contexts on two threads multiply with one weight, each with tiles of another width: calls share nothing that a call writes.
+    (1024, 300 and 40 rows of 4100 columns: 256 and 192 columns a tile, and the kernel of few rows)"""
+    import threading
+
+    import torch
+
+    from peregrine_b200.runtime import GpuContext
+
+    k, n, sizes = 272, 4100, (1024, 300, 40, 1400)
+    g = rng(12)
+    q, s = g.integers(-127, 128, (n, k)).astype(np.int8), g.random(n, np.float32) + 0.5
+    qt = pg.quant.QuantizedTensor(np.ascontiguousarray(q.T), q, s, k, n)
+    qt.to_gpu(gpu)
+    x = {m: torch.from_numpy(normal(g, (m, k))).cuda() for m in sizes}
+    want = {}
+    for m in sizes:
+        y = torch.zeros(m, n, device="cuda")
+        torch.cuda.synchronize()
+        pg._lib.check(gpu.lib.pg_matmul_quantized_ex(gpu.handle, x[m].data_ptr(), m, k, qt._gpu, y.data_ptr(), None, None, None, ALGOS["naive"]))
+        gpu.sync()
+        want[m] = y
+    wrong = []
+
+    def work(order):
+        ctx = GpuContext(0)
+        for _ in range(25):
+            for m in order:
+                y = torch.zeros(m, n, device="cuda")
+                torch.cuda.synchronize()
+                pg._lib.check(ctx.lib.pg_matmul_quantized(ctx.handle, x[m].data_ptr(), m, k, qt._gpu, y.data_ptr()))
+                ctx.sync()
+                if not torch.equal(y, want[m]) or ctx.device_status() != 0:
+                    wrong.append(m)
+        ctx.close()
+
+    threads = [threading.Thread(target=work, args=(o,)) for o in (sizes, sizes[::-1])]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    qt.free_gpu()
+
+
 @pytest.mark.parametrize("ng", [1, 2, 4])
 def test_stream_every_column_group(pg, gpu, oracle_mt, ng):
     gpu.lib.pg_tune_stream_ng(ng)
