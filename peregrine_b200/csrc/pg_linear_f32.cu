@@ -8,7 +8,10 @@
 //     would add that up.  An accumulator therefore only lives for one block of 64 k (smallest pieces first); four warps add the
 //     blocks in registers, rounded, while the next block's products run in the other accumulator.  MT = 128: twelve products of 64
 //     cycles a block, against about 300 cycles for the 128 additions per lane.
-//   * few tiles: K is divided over CTAs with slabs and tickets, as in linear_tc_kernel.
+//   * K has parts, whose number follows from the matrix alone (f32_parts): each part is summed up by itself, and the parts are added in
+//     their order.  With few tiles they are spread over CTAs and meet in slabs, with tickets, as in linear_tc_kernel; else a CTA goes
+//     through them one after the other and keeps the sum so far in TMEM.  So a row's outputs are the same whatever rows are beside it,
+//     however a call is divided, and whatever workspace there is.
 //
 // What bounds it: the tensor cores at three products for each of the bf16 form's, from about 64 rows; the stream of W below.
 // Every mbarrier wait is bounded (pg_async.cuh).
@@ -24,6 +27,7 @@ constexpr int FN = 128;                // columns of y (rows of W) per tile
 constexpr int FK = 64;                 // elements of K per stage = one 128-byte swizzle span
 constexpr int F_THREADS = 192;
 constexpr int F_ROWS = 128;            // rows for which the planes always find room (pg_linear_wrap)
+constexpr int64_t F_SLABS = 64 << 20;  // most bytes of slabs
 
 template <int MT>
 struct FCfg {
@@ -33,12 +37,14 @@ struct FCfg {
     static constexpr int ROOM = 232448 - (1024 + 256);
     static constexpr int STAGES = ROOM / STAGE > 10 ? 10 : ROOM / STAGE;
     static constexpr int ACC = MT < 32 ? 32 : MT;          // TMEM columns of an accumulator
+    static constexpr int COLS = 4 * ACC;                   // two accumulators, the sum so far, and up to a power of two
     static constexpr size_t SMEM = (size_t)STAGES * STAGE + 1024 + 256;
 };
 
 struct FParts {
     int parts, blocks;       // K in `parts` parts of `blocks` 64-element blocks
-    float *slabs;            // [unit][MT][128]
+    int runs, run;           // a unit takes `run` parts that follow each other; `runs` units make a tile
+    float *slabs;            // [tile][part][MT][128]
     unsigned int *tickets;   // one per (tile, quarter), zero between calls
 };
 
@@ -78,6 +84,19 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// 32 columns of this lane's TMEM row
+__device__ __forceinline__ void f32_keep(uint32_t taddr, const uint32_t (&v)[32])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, "
+        "%22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]),
+        "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]),
+        "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 template <int MT, int ACT>
 __global__ void __launch_bounds__(F_THREADS, 1)
     linear_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, int M, int N, int K, float limit,
@@ -111,7 +130,7 @@ __global__ void __launch_bounds__(F_THREADS, 1)
         pg_mbar_fence();
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pg_smem(tmem_slot)), "r"(2 * C::ACC) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pg_smem(tmem_slot)), "r"(C::COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
@@ -123,10 +142,10 @@ __global__ void __launch_bounds__(F_THREADS, 1)
     constexpr int PER_BLOCK = PG_ROUTE_BLOCK / MT < 1 ? 1 : PG_ROUTE_BLOCK / MT;
     const int tiles_m = routed ? max(0, min(__ldcg(rt.blocks) - block0, M / PG_ROUTE_BLOCK)) * PER_BLOCK : (M + MT - 1) / MT;
     const int tiles_n = (N + FN - 1) / FN;
-    const int sp = kp.parts, total = tiles_m * tiles_n * sp;   // unit u: part u % sp of tile u / sp
-    const int kblocks = K / FK;
-    auto k_first = [&](int u) { return (u % sp) * kp.blocks; };
-    auto k_end = [&](int u) { return min(kblocks, (u % sp + 1) * kp.blocks); };
+    const int sp = kp.runs, total = tiles_m * tiles_n * sp;    // unit u: run u % sp of tile u / sp
+    const int kblocks = K / FK, per = kp.run * kp.blocks;
+    auto k_first = [&](int u) { return (u % sp) * per; };
+    auto k_end = [&](int u) { return min(kblocks, (u % sp + 1) * per); };
 
     if (warp == 0) {
         // ---------------------------------------------------------------- producer
@@ -215,12 +234,14 @@ __global__ void __launch_bounds__(F_THREADS, 1)
         for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
             const int tile = u / sp;
             const int m0 = (tile % tiles_m) * MT, n0 = (tile / tiles_m) * FN;
+            const uint32_t lanes = tmem_base + ((uint32_t)(q * 32) << 16), so_far = lanes + 2 * C::ACC;
             float sum[MT] = {};
+            int part = (u % sp) * kp.run, next = k_first(u) + kp.blocks;   // the part under way, and the block behind it
             for (int kb = k_first(u), end = k_end(u); kb < end; kb++) {
                 ok = pg_mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, status, limit_ns);
                 if (!(ok = __all_sync(0xffffffffu, ok))) break;
                 tc_fence_after();
-                const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * C::ACC;
+                const uint32_t taddr = lanes + acc * C::ACC;
 #pragma unroll
                 for (int c = 0; c < C::ACC; c += 32) {
                     uint32_t v[32];
@@ -236,14 +257,45 @@ __global__ void __launch_bounds__(F_THREADS, 1)
                     acc = 0;
                     acc_phase ^= 1;
                 }
+                if (kp.parts > 1 && (kb + 1 == next || kb + 1 == end)) {
+                    // the end of a part: to its slab, or onto the sum of those in front of it
+                    if (sp > 1) {
+                        float *slab = kp.slabs + ((int64_t)tile * kp.parts + part) * MT * FN + q * 32 + lane;
+#pragma unroll
+                        for (int j = 0; j < MT; j++) __stcg(slab + j * FN, sum[j]);
+                    } else {
+                        if (part > 0) {
+#pragma unroll
+                            for (int c = 0; c < C::ACC; c += 32) {
+                                uint32_t v[32];
+                                tmem_ld32(so_far + c, v);
+#pragma unroll
+                                for (int j = 0; j < 32; j++)
+                                    if (c + j < MT) sum[c + j] = __uint_as_float(v[j]) + sum[c + j];
+                            }
+                        }
+                        if (kb + 1 < end) {
+#pragma unroll
+                            for (int c = 0; c < C::ACC; c += 32) {
+                                uint32_t v[32];
+#pragma unroll
+                                for (int j = 0; j < 32; j++) v[j] = c + j < MT ? __float_as_uint(sum[c + j]) : 0u;
+                                f32_keep(so_far + c, v);
+                            }
+                        }
+                    }
+                    if (kb + 1 < end) {
+#pragma unroll
+                        for (int j = 0; j < MT; j++) sum[j] = 0.0f;
+                    }
+                    part++;
+                    next += kp.blocks;
+                }
             }
             if (!ok) break;
             const int n = n0 + q * 32 + lane;
             bool mine = true;
             if (sp > 1) {
-                float *slab = kp.slabs + (int64_t)u * MT * FN + q * 32 + lane;
-#pragma unroll
-                for (int j = 0; j < MT; j++) __stcg(slab + j * FN, sum[j]);
                 unsigned int *ticket = kp.tickets + tile * 4 + q;
                 __threadfence();
                 __syncwarp();
@@ -253,10 +305,10 @@ __global__ void __launch_bounds__(F_THREADS, 1)
                     // the last part of these columns to finish adds all parts up, in their order
                     __threadfence();
                     if (lane == 0) *ticket = 0;
-                    slab = kp.slabs + (int64_t)tile * sp * MT * FN + q * 32 + lane;
+                    const float *slab = kp.slabs + (int64_t)tile * kp.parts * MT * FN + q * 32 + lane;
 #pragma unroll
                     for (int j = 0; j < MT; j++) sum[j] = __ldcg(slab + j * FN);
-                    for (int p = 1; p < sp; p++) {
+                    for (int p = 1; p < kp.parts; p++) {
                         slab += MT * FN;
 #pragma unroll
                         for (int j = 0; j < MT; j++) sum[j] += __ldcg(slab + j * FN);
@@ -288,7 +340,7 @@ __global__ void __launch_bounds__(F_THREADS, 1)
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * C::ACC) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::COLS) : "memory");
     }
 }
 
@@ -309,11 +361,38 @@ int32_t launch(pg_ctx *ctx, const pg_linear *lin, const bf16 *planes, int64_t m,
     auto kern = linear_f32_kernel<MT, ACT>;
     static std::atomic<uint64_t> smem_set{0};
     PG_CUDA(pg_max_smem_once(kern, (int)C::SMEM, ctx->device, smem_set));
-    const int64_t units = ((m + MT - 1) / MT) * ((lin->n + FN - 1) / FN) * kp.parts;
+    const int64_t units = ((m + MT - 1) / MT) * ((lin->n + FN - 1) / FN) * kp.runs;
     kp.tickets = reinterpret_cast<unsigned int *>(ctx->splitk);
     kp.slabs = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(ctx->splitk) + PG_LM_TICKET_BYTES);
     return launch_pdl(ctx, kern, dim3((unsigned)std::min<int64_t>(units, ctx->sm_count)), dim3(F_THREADS), C::SMEM, tw, ta, (int)m, (int)lin->n, (int)lin->k,
                       limit, y, ldy, rt, block0, kp, ctx->d_status, ctx->wait_limit_ns);
+}
+
+// Cycles by count: blocks of the busiest CTA, which its copies bound (695 / 1004 / 1413 cycles with 16 / 64 / 128 rows), and what a tile
+// costs at its end, much more where parts meet.  K = N = 4096, four parts one after the other / two by two / all apart: 128 rows 50 / 42 / 32 us,
+// 333 rows 54 / 73 / 77, 1000 rows 97 / 140 / 179.
+double f32_cost(int64_t rounds, int64_t blocks, int rows, int64_t parts, bool slabs)
+{
+    const double block = 320.0 + (FN + 3.0 * rows) * FK * 2 / 60.0;
+    return rounds * (blocks * block + 2500.0 + rows * 8.0 + (slabs ? 3000.0 + rows * (100.0 + parts * 12.0) : (parts - 1) * rows * 4.0));
+}
+
+// The parts of K: what is best for one tile of 16 rows, where dividing K counts most, but no more than eight (N 512, 333 / 1000 rows: 30 / 40 us,
+// with sixteen 34 / 46).  They do not follow the number of rows, so that the order of a row's sums does not either.
+void f32_parts(const pg_ctx *ctx, const pg_linear *lin, FParts *kp)
+{
+    const int64_t kblocks = lin->k / FK, tiles = (lin->n + FN - 1) / FN;
+    double best = 0;
+    for (int64_t parts = 1; parts <= std::max<int64_t>(1, std::min<int64_t>(8, kblocks / 4)); parts++) {
+        const int64_t blocks = (kblocks + parts - 1) / parts;
+        if ((kblocks + blocks - 1) / blocks != parts || tiles * 4 * (int64_t)sizeof(int) > (int64_t)PG_LM_TICKET_BYTES) continue;
+        const double cost = f32_cost((tiles * parts + ctx->sm_count - 1) / ctx->sm_count, blocks, 16, parts, parts > 1);
+        if (best == 0 || cost < best) {
+            best = cost;
+            kp->parts = (int)parts;
+            kp->blocks = (int)blocks;
+        }
+    }
 }
 
 template <int ACT>
@@ -323,30 +402,34 @@ int32_t dispatch(pg_ctx *ctx, const pg_linear *lin, const bf16 *planes, int64_t 
     const bool routed = rt.blocks != nullptr;
     int mt = routed ? 128 : 16;
     while (mt < 128 && mt < m) mt *= 2;
-    FParts kp = {1, (int)kblocks, nullptr, nullptr};
+    FParts kp = {1, (int)kblocks, 1, 1, nullptr, nullptr};
     if (!routed) {
-        // rows per tile and parts of K: the fewest cycles by count -- blocks of the busiest CTA, each the products' time or its copies'
-        // (about 40 bytes per cycle and SM), and what a tile costs at its end, more where slabs meet; slabs within what
-        // pg_linear_wrap has reserved
-        const int64_t room = (int64_t)(ctx->splitk_bytes > PG_LM_TICKET_BYTES ? ctx->splitk_bytes - PG_LM_TICKET_BYTES : 0) / (FN * (int64_t)sizeof(float));
+        // rows per tile, and how many parts a CTA takes; slabs for parts of their own as far as there is room, which may grow except
+        // while a graph is recorded
+        f32_parts(ctx, lin, &kp);
+        const int64_t slab = FN * (int64_t)sizeof(float);
+        const int64_t room = ctx->capturing ? (int64_t)ctx->splitk_bytes - (int64_t)PG_LM_TICKET_BYTES : F_SLABS;
         const int full = mt;
+        int64_t need = 0;
         double best = 0;
         for (int cand = full; cand >= std::min(full, 64); cand /= 2) {
             const int64_t tiles = tiles_n * ((m + cand - 1) / cand);
-            for (int64_t parts = 1; parts <= std::max<int64_t>(1, std::min<int64_t>(16, kblocks / 4)); parts++) {
-                const int64_t blocks = (kblocks + parts - 1) / parts;
-                if ((kblocks + blocks - 1) / blocks != parts) continue;
-                if (parts > 1 && (tiles * parts * cand > room || tiles * 4 * (int64_t)sizeof(int) > (int64_t)PG_LM_TICKET_BYTES)) break;
-                const int64_t rounds = (tiles * parts + ctx->sm_count - 1) / ctx->sm_count;
-                const double block = std::max(std::max(480.0, cand * 6.0), (FN * FK * 2 + 3.0 * cand * FK * 2) / 40.0);
-                const double cost = rounds * (blocks * block + 2500.0 + cand * 8.0 + (parts > 1 ? 3000.0 + cand * parts * 6.0 : 0.0));
+            for (int64_t run = kp.parts; run >= 1; run--) {
+                const int64_t runs = (kp.parts + run - 1) / run;
+                if (runs > 1 && (tiles * kp.parts * cand * slab > room || tiles * 4 * (int64_t)sizeof(int) > (int64_t)PG_LM_TICKET_BYTES)) break;
+                const double cost = f32_cost((tiles * runs + ctx->sm_count - 1) / ctx->sm_count, run * kp.blocks, cand, kp.parts, runs > 1);
                 if (best == 0 || cost < best) {
                     best = cost;
                     mt = cand;
-                    kp.parts = (int)parts;
-                    kp.blocks = (int)blocks;
+                    kp.run = (int)run;
+                    kp.runs = (int)runs;
+                    need = runs > 1 ? tiles * kp.parts * cand * slab : 0;
                 }
             }
+        }
+        if (need > 0 && !ctx->capturing) {
+            const int32_t rc = pg_splitk_reserve(ctx, PG_LM_TICKET_BYTES + (size_t)need);
+            if (rc != PG_OK) return rc;
         }
     }
     if (mt == 128) return launch<128, ACT>(ctx, lin, planes, m, limit, y, ldy, rt, block0, kp);

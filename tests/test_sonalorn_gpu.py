@@ -119,16 +119,36 @@ def test_f32_product_is_f32(lm, m, n, k):
     lin.free()
 
 
-def test_f32_product_is_recorded_without_a_run_before(lm):
-    """The workspace cannot grow in a recording: the rows then go through what there is in portions, with the same results."""
+@pytest.mark.parametrize("n,k", [(200, 4096), (4100, 1024), (136, 14336), (20000, 512)])
+def test_f32_product_rows_do_not_depend_on_each_other(lm, n, k):
+    """A row's outputs are the same bits whatever other rows there are, in tiles of any height and with K divided in any way."""
+    from peregrine_b200.layers import Linear
+
+    d = device(lm, "float32", 700)
+    g = rng(n)
+    lin = Linear(d, d.bf16(t.bf16_values(g.standard_normal((n, k)))))
+    x = act(d, g.standard_normal((700, k)).astype(np.float32))
+    y = {m: d.torch.zeros(m, (n + 7) // 8 * 8, device=d.dev) for m in (700, 300, 129, 128, 65, 64, 33, 17, 16, 1)}
+    d.torch.cuda.synchronize()
+    for m in y:
+        lin.run(x, m, y[m])
+    lm.sync()
+    assert [m for m in y if not d.torch.equal(y[m], y[700][:m])] == [] and lm.device_status() == 0
+    lin.free()
+
+
+@pytest.mark.parametrize("k", [192, 4096])
+def test_f32_product_is_recorded_without_a_run_before(lm, k):
+    """The workspace does not grow for all rows in a recording: they go through what there is in portions, with the same results, also
+    where K is divided."""
     from peregrine_b200.layers import Linear
     from peregrine_b200.runtime import GpuContext
 
     gpu = GpuContext(component="lm")
     d = device(gpu, "float32", 700)
     g = rng(3)
-    lin = Linear(d, d.bf16(t.bf16_values(g.standard_normal((200, 192)))))
-    x, y, z = act(d, g.standard_normal((700, 192)).astype(np.float32)), d.torch.zeros(700, 200, device=d.dev), d.torch.zeros(700, 200, device=d.dev)
+    lin = Linear(d, d.bf16(t.bf16_values(g.standard_normal((200, k)))))
+    x, y, z = act(d, g.standard_normal((700, k)).astype(np.float32)), d.torch.zeros(700, 200, device=d.dev), d.torch.zeros(700, 200, device=d.dev)
     d.torch.cuda.synchronize()
     with gpu.record() as graph:
         lin.run(x, 700, y)
