@@ -22,14 +22,15 @@ void pg_set_error(const char *fmt, ...)
 // Grows one of the context's device blocks.  Work already enqueued may still use the old block, so the stream is
 // drained first; a recorded graph may use it for as long as it lives, so with graphs alive the old block is parked
 // (pg_ctx::retired) instead of freed.
-static int32_t grow_block(pg_ctx *ctx, void **block, size_t *have, size_t bytes, const char *what, bool zeroed)
+// `recording`: also while a graph is being recorded, without a wait; the old block is parked then, and memory not `zeroed`.
+static int32_t grow_block(pg_ctx *ctx, void **block, size_t *have, size_t bytes, const char *what, bool zeroed, bool recording = false)
 {
     if (bytes <= *have) return PG_OK;
-    if (ctx->capturing)
+    if (ctx->capturing && !recording)
         PG_FAIL(PG_ERR_INVALID, "%s memory would have to grow while a graph is being recorded; run the call once before recording", what);
-    PG_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (!ctx->capturing) PG_CUDA(cudaStreamSynchronize(ctx->stream));
     if (*block) {
-        if (ctx->live_graphs > 0)
+        if (ctx->live_graphs > 0 || ctx->capturing)
             ctx->retired.push_back(*block);
         else
             PG_CUDA(cudaFree(*block));
@@ -38,13 +39,19 @@ static int32_t grow_block(pg_ctx *ctx, void **block, size_t *have, size_t bytes,
     *have = 0;
     size_t want = bytes + (bytes >> 2);
     want = (want + 255) & ~(size_t)255;
-    PG_CUDA(cudaMalloc(block, want));
+    // (a recording of this thread's forbids cudaMalloc unless the thread's mode says that it knows)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (ctx->capturing) PG_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaMalloc(block, want);
+    if (ctx->capturing) PG_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    PG_CUDA(e);
     if (zeroed) PG_CUDA(cudaMemsetAsync(*block, 0, want, ctx->stream));
     *have = want;
     return PG_OK;
 }
 
 int32_t pg_scratch_reserve(pg_ctx *ctx, size_t bytes) { return grow_block(ctx, &ctx->scratch, &ctx->scratch_bytes, bytes, "scratch", false); }
+int32_t pg_scratch_reserve_recording(pg_ctx *ctx, size_t bytes) { return grow_block(ctx, &ctx->scratch, &ctx->scratch_bytes, bytes, "scratch", false, true); }
 int32_t pg_staging_reserve(pg_ctx *ctx, size_t bytes) { return grow_block(ctx, &ctx->staging, &ctx->staging_bytes, bytes, "staging", false); }
 int32_t pg_splitk_reserve(pg_ctx *ctx, size_t bytes) { return grow_block(ctx, &ctx->splitk, &ctx->splitk_bytes, bytes, "split-K workspace", true); }
 

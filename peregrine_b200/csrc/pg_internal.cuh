@@ -376,6 +376,7 @@ __device__ __forceinline__ void pg_peer_store4(const PgPeerOut &o, int64_t m, in
 #endif
 
 int32_t pg_scratch_reserve(pg_ctx *ctx, size_t bytes);
+int32_t pg_scratch_reserve_recording(pg_ctx *ctx, size_t bytes);   // also while a graph is being recorded
 int32_t pg_pinned_reserve(pg_ctx *ctx, size_t bytes);
 int32_t pg_staging_reserve(pg_ctx *ctx, size_t bytes);
 int32_t pg_splitk_reserve(pg_ctx *ctx, size_t bytes);

@@ -27,7 +27,7 @@ constexpr int FN = 128;                // columns of y (rows of W) per tile
 constexpr int FK = 64;                 // elements of K per stage = one 128-byte swizzle span
 constexpr int F_THREADS = 192;
 constexpr int F_ROWS = 128;            // rows for which the planes always find room (pg_linear_wrap)
-constexpr int64_t F_SLABS = 64 << 20;  // most bytes of slabs
+constexpr int64_t F_PLANES = 100 << 20, F_SLABS = 64 << 20;   // most bytes of planes (they stay in L2; longer calls go in portions), of slabs
 
 template <int MT>
 struct FCfg {
@@ -450,18 +450,14 @@ int32_t pgk_linear_f32(pg_ctx *ctx, const pg_linear *lin, const float *a, int64_
     PG_REQUIRE(m < (1ll << 31) - 256 && lin->experts * lin->n < (1ll << 31) - 256, "linear: too many rows");
     const PgRouted none = {};
     const PgRouted &rt = routed ? *routed : none;
-    // all rows at once if there is room for their planes; while a graph is recorded the workspace cannot grow, and what
-    // pg_linear_wrap has reserved then takes them in portions
+    // Rows in portions whose planes stay below F_PLANES: the same outputs as all at once.  While a graph is recorded, what there is of
+    // the workspace takes them, and there is always some (pg_linear_wrap, or this call where another context made the weight)
     const int64_t row_bytes = lin->k * 3 * (int64_t)sizeof(bf16);
-    int64_t portion = m;
-    if ((size_t)(m * row_bytes) > ctx->scratch_bytes) {
-        if (ctx->capturing) {
-            portion = (int64_t)(ctx->scratch_bytes / (size_t)row_bytes) / F_ROWS * F_ROWS;
-            PG_REQUIRE(portion > 0, "linear: the context has no workspace for the f32 form");
-        } else {
-            const int32_t rc = pg_scratch_reserve(ctx, (size_t)(m * row_bytes));
-            if (rc != PG_OK) return rc;
-        }
+    int64_t portion = std::min(m, std::max<int64_t>(F_ROWS, F_PLANES / row_bytes / F_ROWS * F_ROWS));
+    if ((size_t)(portion * row_bytes) > ctx->scratch_bytes) {
+        if (ctx->capturing) portion = std::min(portion, std::max<int64_t>(F_ROWS, (int64_t)(ctx->scratch_bytes / (size_t)row_bytes) / F_ROWS * F_ROWS));
+        const int32_t rc = pg_scratch_reserve_recording(ctx, (size_t)(portion * row_bytes));
+        if (rc != PG_OK) return rc;
     }
     bf16 *planes = reinterpret_cast<bf16 *>(ctx->scratch);
     for (int64_t r0 = 0; r0 < m; r0 += portion) {

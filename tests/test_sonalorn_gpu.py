@@ -137,6 +137,54 @@ def test_f32_product_rows_do_not_depend_on_each_other(lm, n, k):
     lin.free()
 
 
+def test_f32_product_of_many_rows_goes_in_portions(lm):
+    """The workspace of a call is bounded; its outputs are those of its portions."""
+    from peregrine_b200.layers import Linear
+    from peregrine_b200.runtime import GpuContext
+
+    gpu = GpuContext(component="lm")
+    d = device(gpu, "float32", 20000)
+    g = rng(4)
+    lin = Linear(d, d.bf16(t.bf16_values(g.standard_normal((72, 1024)))))
+    x, y, z = d.torch.randn(20000, 1024, device=d.dev), d.torch.zeros(20000, 72, device=d.dev), d.torch.zeros(50, 72, device=d.dev)
+    d.torch.cuda.synchronize()
+    lin.run(x, 20000, y)
+    for r0 in (0, 10000, 17000, 19950):
+        lin.run(x[r0:], 50, z)
+        gpu.sync()
+        assert d.torch.equal(z, y[r0:r0 + 50]), r0
+    assert gpu.lib.pg_ctx_scratch_bytes(gpu.handle) < 220 << 20 and gpu.device_status() == 0
+    lin.free()
+    gpu.close()
+
+
+def test_f32_product_is_recorded_by_another_context(lm):
+    """A matrix belongs to no context: one that has no workspace yet records products with it too, before and behind others."""
+    from peregrine_b200.layers import Linear
+    from peregrine_b200.runtime import GpuContext
+
+    d = device(lm, "float32", 320)
+    g = rng(5)
+    lins = [Linear(d, d.bf16(t.bf16_values(g.standard_normal((200, k))))) for k in (192, 4096)]
+    x = [act(d, g.standard_normal((300, lin.k)).astype(np.float32)) for lin in lins]
+    y, z = ([d.torch.zeros(300, 200, device=d.dev) for _ in lins] for _ in range(2))
+    d.torch.cuda.synchronize()
+    for i, lin in enumerate(lins):
+        lin.run(x[i], 300, y[i])
+    lm.sync()
+    gpu = GpuContext(component="lm")
+    with gpu.record() as graph:
+        for i, lin in enumerate(lins):
+            d.check(d.lib.pg_linear_run(gpu.handle, lin.handle, x[i].data_ptr(), d.code, 300, 0, 0.0, z[i].data_ptr(), d.code, 200))
+    graph.launch()
+    gpu.sync()
+    assert all(d.torch.equal(a, b) for a, b in zip(y, z)) and gpu.device_status() == 0
+    graph.free()
+    gpu.close()
+    for lin in lins:
+        lin.free()
+
+
 @pytest.mark.parametrize("k", [192, 4096])
 def test_f32_product_is_recorded_without_a_run_before(lm, k):
     """The workspace does not grow for all rows in a recording: they go through what there is in portions, with the same results, also
