@@ -556,8 +556,8 @@ int32_t pg_gguf_upload(pg_ctx *ctx, int32_t type, const uint8_t *raw, size_t raw
         e = cudaMemcpyAsync(d_raw, raw + (size_t)row_begin * nblk * bs, blocks * bs, cudaMemcpyHostToDevice, ctx->stream);
     int32_t rc = PG_OK;
     if (e == cudaSuccess) rc = pgk_gguf_repack(ctx, type, (const uint8_t *)d_raw, nr, k, w);
-    // now, since the workspaces cannot grow while a step is being recorded
-    if (e == cudaSuccess && rc == PG_OK && w->tiled) rc = pgk_gguf_tc_reserve(ctx, k);
+    // now, since the workspaces cannot grow while a step is being recorded (without them products take the streaming form)
+    if (e == cudaSuccess && rc == PG_OK && w->tiled) (void)pgk_gguf_tc_reserve(ctx, k);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cudaFree(d_raw);
     if (e != cudaSuccess || rc != PG_OK) {

@@ -44,7 +44,11 @@ static int32_t grow_block(pg_ctx *ctx, void **block, size_t *have, size_t bytes,
     if (ctx->capturing) PG_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
     const cudaError_t e = cudaMalloc(block, want);
     if (ctx->capturing) PG_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-    PG_CUDA(e);
+    if (e != cudaSuccess) {
+        cudaGetLastError();                       // (the caller may do without)
+        *block = nullptr;
+        PG_CUDA(e);
+    }
     if (zeroed) PG_CUDA(cudaMemsetAsync(*block, 0, want, ctx->stream));
     *have = want;
     return PG_OK;

@@ -38,6 +38,7 @@ namespace {
 constexpr int GT_N = 128;                         // rows of W per tile
 constexpr int GT_ROWS = 64;                       // rows for which the planes always find room (pgk_gguf_tc_reserve)
 constexpr size_t GT_TICKET_BYTES = 64 * 1024;     // as in the int8 kernel: tickets, zero between calls, then slabs
+constexpr int64_t GT_PLANES = 100 << 20;          // most bytes of planes (they stay in L2; longer calls go in portions)
 
 template <int TYPE, int MT>
 struct GtCfg {
@@ -473,17 +474,18 @@ int32_t gt_launch(pg_ctx *ctx, const pg_gguf_weight *w, const void *planes, cons
                       (int)(w->k / 256), (int)m, us, y, kp, ctx->d_status, ctx->wait_limit_ns);
 }
 
-template <int TYPE>
-int32_t gt_run(pg_ctx *ctx, const pg_gguf_weight *w, const void *planes, const float *us, int64_t m, float *y)
+// rows of slabs that a context keeps for every product
+int64_t gt_slab_rows(const pg_ctx *ctx) { return (int64_t)ctx->sm_count * 3 * 64; }
+
+// Rows per tile and parts of K, by the shape alone (a portion of a call has those of the whole call): the fewest cycles by count --
+// slices of the busiest CTA and what a tile costs at its end, more where slabs meet.  Measured at N 14336, K 4096, a block of 32 k takes
+// 350 / 430 / 570 / 800 / 930 cycles with 16 / 32 / 64 / 128 / 160 rows.
+GtParts gt_plan(const pg_ctx *ctx, const pg_gguf_weight *w, int64_t m, int *mt)
 {
-    // rows per tile and parts of K: the fewest cycles by count -- slices of the busiest CTA and what a tile costs at its end, more
-    // where slabs meet.  Measured at N 14336, K 4096, a block of 32 k takes 350 / 430 / 570 / 800 / 930 cycles with 16 / 32 / 64 / 128 /
-    // 160 rows.
     const int64_t nslices = w->k / 256, tiles_n = (w->n + GT_N - 1) / GT_N;
-    const int64_t room = (int64_t)(ctx->splitk_bytes > GT_TICKET_BYTES ? ctx->splitk_bytes - GT_TICKET_BYTES : 0) / (GT_N * (int64_t)sizeof(float));
     static const int sizes[] = {16, 32, 64, 128, 160};
     double best = 0;
-    int mt = 16;
+    *mt = 16;
     GtParts kp = {1, (int)nslices, nullptr, nullptr};
     for (int cand : sizes) {
         if (cand < 64 && cand < m) continue;
@@ -492,17 +494,23 @@ int32_t gt_run(pg_ctx *ctx, const pg_gguf_weight *w, const void *planes, const f
         for (int64_t parts = 1; parts <= std::min<int64_t>(16, nslices); parts++) {
             const int64_t slices = (nslices + parts - 1) / parts;
             if ((nslices + slices - 1) / slices != parts) continue;
-            if (parts > 1 && (tiles * parts * cand > room || tiles * 8 * (int64_t)sizeof(int) > (int64_t)GT_TICKET_BYTES)) break;
+            if (parts > 1 && (tiles * parts * cand > gt_slab_rows(ctx) || tiles * 8 * (int64_t)sizeof(int) > (int64_t)GT_TICKET_BYTES)) break;
             const int64_t rounds = (tiles * parts + ctx->sm_count - 1) / ctx->sm_count;
             const double cost = rounds * (slices * 8.0 * (280.0 + cand * 4.0) + 1500.0 + cand * 8.0 + (parts > 1 ? 2500.0 + cand * parts * 4.0 : 0.0));
             if (best == 0 || cost < best) {
                 best = cost;
-                mt = cand;
+                *mt = cand;
                 kp.parts = (int)parts;
                 kp.slices = (int)slices;
             }
         }
     }
+    return kp;
+}
+
+template <int TYPE>
+int32_t gt_run(pg_ctx *ctx, const pg_gguf_weight *w, const void *planes, const float *us, int64_t m, float *y, int mt, const GtParts &kp)
+{
     if (mt == 160) return gt_launch<TYPE, 160>(ctx, w, planes, us, m, y, kp);
     if (mt == 128) return gt_launch<TYPE, 128>(ctx, w, planes, us, m, y, kp);
     if (mt == 64) return gt_launch<TYPE, 64>(ctx, w, planes, us, m, y, kp);
@@ -530,22 +538,24 @@ int32_t pgk_gguf_tc_reserve(pg_ctx *ctx, int64_t k)
 {
     const int32_t rc = pg_scratch_reserve(ctx, (size_t)(GT_ROWS * gt_row_bytes(k)));
     if (rc != PG_OK) return rc;
-    return pg_splitk_reserve(ctx, GT_TICKET_BYTES + (size_t)ctx->sm_count * 3 * 64 * GT_N * sizeof(float));
+    return pg_splitk_reserve(ctx, GT_TICKET_BYTES + (size_t)(gt_slab_rows(ctx) * GT_N) * sizeof(float));
 }
 
 int32_t pgk_matmul_gguf_tc(pg_ctx *ctx, const float *d_x, int64_t m, const pg_gguf_weight *w, float *d_y)
 {
-    // all rows at once if there is room for their planes; while a graph is recorded the workspace cannot grow, and what the upload
-    // has reserved then takes them in portions
-    int64_t portion = m;
-    if ((size_t)(m * gt_row_bytes(w->k)) > ctx->scratch_bytes) {
-        if (ctx->capturing) {
-            portion = (int64_t)(ctx->scratch_bytes / (size_t)gt_row_bytes(w->k)) / 16 * 16;
-            PG_REQUIRE(portion > 0, "matmul_gguf: the context has no workspace for %lld rows", (long long)m);
-        } else {
-            const int32_t rc = pg_scratch_reserve(ctx, (size_t)(m * gt_row_bytes(w->k)));
-            if (rc != PG_OK) return rc;
-        }
+    // Rows in portions whose planes stay below GT_PLANES; while a graph is recorded the workspace cannot grow, and what there is (an
+    // upload reserves some in its context) takes them.  Where there is none to be had, the streaming form does without.
+    int mt;
+    const GtParts kp = gt_plan(ctx, w, m, &mt);
+    const int64_t row_bytes = gt_row_bytes(w->k);
+    int64_t portion = std::min(m, std::max<int64_t>(GT_ROWS, GT_PLANES / row_bytes / mt * mt));
+    if (ctx->capturing) {
+        const int64_t fit = (int64_t)(ctx->scratch_bytes / (size_t)row_bytes), step = fit >= mt ? mt : 16;
+        if (fit < portion) portion = fit / step * step;
+        if (portion == 0 || (kp.parts > 1 && ctx->splitk_bytes < GT_TICKET_BYTES + (size_t)(gt_slab_rows(ctx) * GT_N) * sizeof(float)))
+            return pgk_matmul_gguf_stream(ctx, d_x, m, w, d_y);
+    } else if (pg_scratch_reserve(ctx, (size_t)(portion * row_bytes)) != PG_OK || pgk_gguf_tc_reserve(ctx, w->k) != PG_OK) {
+        return pgk_matmul_gguf_stream(ctx, d_x, m, w, d_y);
     }
     for (int64_t r0 = 0; r0 < m; r0 += portion) {
         const int64_t rows = std::min(portion, m - r0);
@@ -557,8 +567,8 @@ int32_t pgk_matmul_gguf_tc(pg_ctx *ctx, const float *d_x, int64_t m, const pg_gg
                          ? launch_pdl(ctx, gguf_planes_kernel<true>, grid, dim3(256), 0, d_x, (int)r0, (int)rows, (int)w->k, planes, us)
                          : launch_pdl(ctx, gguf_planes_kernel<false>, grid, dim3(256), 0, d_x, (int)r0, (int)rows, (int)w->k, planes, us);
         if (rc != PG_OK) return rc;
-        rc = w->type == PG_GGUF_Q4_0 ? gt_run<PG_GGUF_Q4_0>(ctx, w, planes, us, rows, d_y + r0 * w->n)
-                                     : gt_run<PG_GGUF_Q8_0>(ctx, w, planes, us, rows, d_y + r0 * w->n);
+        rc = w->type == PG_GGUF_Q4_0 ? gt_run<PG_GGUF_Q4_0>(ctx, w, planes, us, rows, d_y + r0 * w->n, mt, kp)
+                                     : gt_run<PG_GGUF_Q8_0>(ctx, w, planes, us, rows, d_y + r0 * w->n, mt, kp);
         if (rc != PG_OK) return rc;
     }
     return PG_OK;

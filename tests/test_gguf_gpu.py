@@ -209,7 +209,8 @@ def test_matmul_gguf_few_rows_long_k(pg, gpu, oracle_mt, kind, m, n, k):
 
 
 def test_matmul_gguf_many_rows_recorded_without_a_run_before(pg, oracle_mt):
-    """The workspace cannot grow in a recording: the rows then go through what the upload has reserved, in portions."""
+    """The workspace cannot grow in a recording: the rows then go through what the upload has reserved, in portions, with the same
+    results."""
     import torch
 
     g = pg.GpuContext()
@@ -224,9 +225,47 @@ def test_matmul_gguf_many_rows_recorded_without_a_run_before(pg, oracle_mt):
     g.sync()
     w.matmul_device(x, m, z)
     g.sync()
-    # (portions may divide K otherwise)
-    assert graph.kernels > 2 and torch.allclose(y, z, rtol=0, atol=1e-5 * z.abs().max().item()) and g.device_status() == 0
+    assert graph.kernels > 2 and torch.equal(y, z) and g.device_status() == 0
     graph.free()
+    w.free()
+    g.close()
+
+
+@pytest.mark.parametrize("kind", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("m,n,k", [(9, 200, 512), (130, 72, 4352), (3, 40, 12544)])
+def test_matmul_gguf_recorded_by_a_context_without_workspace(pg, gpu, oracle_mt, kind, m, n, k):
+    """A weight belongs to no context: another one, which has uploaded nothing, records products with it."""
+    import torch
+
+    raw = oracle_mt.encode(kind, normal(rng(9), (n, k), 0.02))
+    w = pg.gguf.GgufWeight(kind, raw, n, k, gpu)
+    g = pg.GpuContext()
+    x, y = torch.randn(m, k, device="cuda"), torch.zeros(m, n, device="cuda")
+    torch.cuda.synchronize()
+    with g.record() as graph:
+        pg._lib.check(g.lib.pg_matmul_gguf(g.handle, x.data_ptr(), m, w.handle, y.data_ptr()))
+    graph.launch()
+    g.sync()
+    want = x.double().cpu().numpy() @ oracle_mt.dequant(kind, raw, n * k).reshape(n, k).astype(np.float64).T
+    assert np.abs(y.cpu().numpy() - want).max() <= REL_TOL * np.abs(want).max() and g.device_status() == 0
+    graph.free()
+    w.free()
+    g.close()
+
+
+def test_matmul_gguf_of_many_rows_goes_in_portions(pg, oracle_mt):
+    """The workspace of a call is bounded; its outputs are those of its portions."""
+    import torch
+
+    g = pg.GpuContext()
+    n, k, m = 40, 1024, 40000
+    w = pg.gguf.GgufWeight("q8_0", oracle_mt.encode("q8_0", normal(rng(10), (n, k), 0.02)), n, k, g)
+    x, y, z = torch.randn(m, k, device="cuda"), torch.zeros(m, n, device="cuda"), torch.zeros(m // 2, n, device="cuda")
+    torch.cuda.synchronize()
+    w.matmul_device(x, m, y)
+    w.matmul_device(x[m // 2:], m // 2, z)
+    g.sync()
+    assert torch.equal(y[m // 2:], z) and g.lib.pg_ctx_scratch_bytes(g.handle) < 160 << 20 and g.device_status() == 0
     w.free()
     g.close()
 
