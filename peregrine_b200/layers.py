@@ -41,10 +41,7 @@ class Device:
         self.act = torch.bfloat16 if dtype == "bfloat16" else torch.float32
         self.rows = int(step_rows)
         self._buffers = {}
-        # a batch may be the first thing that follows: torch has cleared its arrays, on a stream of its own, before the context's
-        # stream writes to them
         self.buffer("batch", 1, BATCH_WORDS(self.rows), torch.int32)
-        torch.cuda.current_stream(self.dev).synchronize()
 
     def f32(self, a):
         """Host array (f32, or bf16 bits as uint16) or torch tensor -> f32 on the device."""
@@ -68,6 +65,8 @@ class Device:
         t = self._buffers.get(key)
         if t is None or t.shape[0] < rows:
             t = self._buffers[key] = self.torch.zeros(rows, cols, dtype=dtype, device=self.dev)
+            # torch clears it on a stream of its own, and the context's stream may be the next to write to it
+            self.torch.cuda.current_stream(self.dev).synchronize()
         return t
 
     def rotation(self, base: float, dims: int, positions: int):

@@ -25,6 +25,8 @@ class SlotPool:
         import torch
 
         t = torch.zeros((self.slots, *shape), dtype=dtype, device=self.device)
+        if t.is_cuda:       # cleared on torch's stream, before the context's stream writes to it
+            torch.cuda.current_stream(t.device).synchronize()
         self.bytes += t.numel() * t.element_size()
         return t
 

@@ -357,6 +357,19 @@ def test_first_batch_of_a_device_outlives_the_clearing_of_its_buffer(lm):
     assert b.mem.flatten().cpu().tolist()[:12] == [7, 8, 9, 5, 6, 7, 0, 0, 0, 0, 3, 2]
 
 
+def test_buffers_are_cleared_before_another_stream_writes_to_them(lm):
+    """Any buffer, one that grows too: torch's clearing, held up by other work, must not come behind a write of the context's."""
+    d = device(lm, "bfloat16", 16)
+    for rows in (4, 16):
+        d.torch.cuda._sleep(200_000_000)
+        b = d.buffer("something", 8, rows, d.torch.int32)
+        host = np.arange(8 * rows, dtype=np.int32)
+        d.check(d.lib.pg_mem_upload(lm.handle, b.data_ptr(), host.ctypes.data, host.nbytes))
+        lm.sync()
+        d.torch.cuda.synchronize()
+        assert b.flatten().cpu().tolist() == host.tolist()
+
+
 def run_mixer(lm, d, mixer, width, x, cuts, slot=1, between=None):
     """x [T, width] in portions -> [T, width] outputs; `between` is called before every portion."""
     from peregrine_b200.layers import Batch, up
