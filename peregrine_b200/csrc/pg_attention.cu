@@ -789,7 +789,7 @@ int32_t pgk_attention_f32(pg_ctx *ctx, const AttnShape &s, const pg_batch *bt, c
     PG_REQUIRE(bt->rows <= 65535, "attention: too many rows for the f32 form");
     PG_REQUIRE(s.V <= 8 * AF_T && (s.dp + AF_T) * 4 <= 48 * 1024, "attention: heads too wide for the f32 form");
     // (tokens of different sequences share nothing)
-    if (bt->max_len > 1 && AF_Q * (s.dp + AF_T) * 4 <= 48 * 1024)
+    if (bt->max_len > 1 && AF_Q * (s.dp + AF_T) * 4 <= 48 * 1024 && bt->rows / AF_Q + bt->seqs <= 65535)
         return launch_pdl(ctx, attn_f32_kernel<AF_Q>, dim3((unsigned)s.H, (unsigned)(bt->rows / AF_Q + bt->seqs)), dim3(AF_T), (size_t)AF_Q * (s.dp + AF_T) * 4, s,
                           *bt, q, kc, vc, out, ldo);
     return launch_pdl(ctx, attn_f32_kernel<1>, dim3((unsigned)s.H, (unsigned)bt->rows), dim3(AF_T), (size_t)(s.dp + AF_T) * 4, s, *bt, q, kc, vc, out, ldo);

@@ -590,6 +590,26 @@ def planted(p, width, T, far, at):
     return t.bf16_values(x), W
 
 
+def test_attention_f32_of_very_many_sequences(lm):
+    """As many rows as there were before tokens went together (a launch has 65535 groups at most)."""
+    from peregrine_b200.layers import Attention, Batch
+    from peregrine_b200.state import SlotPool
+
+    p, width, seqs = t.attention(1, 1, 16, 16, 0.3), 64, 55000
+    d = device(lm, "float32", 60000)
+    g = rng(10)
+    mixer = Attention(d, p, {k: t.bf16_values(v) for k, v in t.mixer_weights(g, "attention", p, width).items()}, width, 1e-4, 32, seqs)
+    x = t.bf16_values(g.standard_normal((1, width)))
+    lengths = [1] * (seqs - 2) + [2, 2]
+    y = d.torch.zeros(d.rows, width, device=d.dev)
+    mixer.run(Batch(d, [(i, 0, [0] * n) for i, n in enumerate(lengths)]), act(d, np.repeat(x, sum(lengths), 0)), mixer.new_state(SlotPool(seqs, 32, d.dev)), y)
+    lm.sync()
+    one, _ = run_mixer(lm, d, mixer, width, x, [1])
+    first = y[:sum(lengths)].cpu().numpy()[np.concatenate([[0], np.cumsum(lengths)[:-1]])]
+    assert (first == one).all() and lm.device_status() == 0
+    mixer.free()
+
+
 def test_attention_f32_tokens_of_several_sequences(lm):
     """f32: up to four tokens of a sequence share a CTA; whatever the lengths, each sequence is as if it were alone (products of other row counts aside)."""
     from peregrine_b200.layers import Attention, Batch, up
