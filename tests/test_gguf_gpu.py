@@ -192,10 +192,11 @@ def test_matmul_gguf_many_rows(pg, gpu, oracle_mt, kind, n, k):
 
 
 @pytest.mark.parametrize("kind", ["q4_0", "q8_0"])
-@pytest.mark.parametrize("m,n,k", [(3, 300, 12544), (4, 260, 8448), (5, 129, 4352), (7, 200, 2304), (8, 5000, 6400), (6, 131, 16640)])
-def test_matmul_gguf_few_rows_long_k(pg, gpu, oracle_mt, kind, m, n, k):
+@pytest.mark.parametrize("m,n,k,digits", [(3, 300, 12544, 39), (4, 260, 8448, 39), (5, 129, 4352, 39), (7, 200, 2304, 39), (8, 5000, 6400, 39), (6, 131, 16640, 39),
+                                          (2, 300, 12544, 22), (5, 200, 2304, 22), (8, 5000, 4096, 22)])
+def test_matmul_gguf_few_rows_long_k(pg, gpu, oracle_mt, kind, m, n, k, digits):
     """Up to eight rows, on both sides of the line between the streaming form and the tensor cores: the bound of the latter's planes and
-    sums (above) holds for both but for the streaming form's three digits of 7 bits of the row's largest element."""
+    sums (above), whose planes hold 2^-39 of a row's largest element; the streaming form has whole numbers of 23 bits with their sign."""
     g = rng(n + k + m)
     raw = oracle_mt.encode(kind, normal(g, (n, k), 0.02))
     w64 = oracle_mt.dequant(kind, raw, n * k).reshape(n, k).astype(np.float64)
@@ -203,7 +204,7 @@ def test_matmul_gguf_few_rows_long_k(pg, gpu, oracle_mt, kind, m, n, k):
     x = normal(g, (m, k))
     got = w.matmul(x, m)
     x64 = np.abs(x).astype(np.float64)
-    bound = x64 @ np.abs(w64).T * (2.0 ** -22 + 4 * 2.0 ** -23 + (k // 32 + 18) * 2.0 ** -24) + x64.max(1, keepdims=True) * 2.0 ** -20 * np.abs(w64).sum(1)
+    bound = x64 @ np.abs(w64).T * (2.0 ** -22 + 4 * 2.0 ** -23 + (k // 32 + 18) * 2.0 ** -24) + x64.max(1, keepdims=True) * 2.0 ** -digits * np.abs(w64).sum(1)
     assert (np.abs(got - x.astype(np.float64) @ w64.T) <= bound).all() and gpu.device_status() == 0
     w.free()
 

@@ -293,7 +293,7 @@ def test_tcgen05_small_row_counts(pg, gpu, oracle_mt, m, bn):
 
 @pytest.mark.parametrize("m,k,n", [(17, 4096, 14336), (48, 4096, 6144), (64, 14336, 4096), (100, 4096, 4096), (24, 1040, 12000)])
 def test_mid_batch_dispatch(pg, gpu, oracle_mt, m, k, n):
-    """17 <= M <= 128 with the automatic kernel choice (tcgen05 with the modelled tile width, or the FIFO kernel)."""
+    """17 <= M <= 128 with the automatic kernel choice (K over a cluster, or the tile kernel on wide layers)."""
     x, w = linear_inputs(m, k, n, 40 + m)
     _check_product(pg, gpu, oracle_mt, x, w, m, k, n, ["naive"])
 
@@ -341,9 +341,11 @@ def test_tcgen05_k_split_over_ctas(pg, gpu, oracle_mt, m, k, n, bn, split):
         gpu.lib.pg_tune_tcgen05_bn(0)
 
 
-@pytest.mark.parametrize("m,k,n", [(256, 128, 256), (512, 1024, 768), (300, 1040, 520), (1000, 4096, 1000), (129, 144, 257)])
+@pytest.mark.parametrize("m,k,n", [(256, 128, 256), (512, 1024, 768), (300, 1040, 520), (1000, 4096, 1000), (129, 144, 257),
+                                   (1024, 272, 4100), (900, 1040, 4099), (520, 272, 14300), (700, 400, 14250)])
 def test_tcgen05_cta_pairs(pg, gpu, oracle_mt, m, k, n):
-    """cta_group::2: two CTAs share one 256 x 256 tile; full and ragged tiles in M, N and K."""
+    """cta_group::2: two CTAs share a tile, full and ragged in M, N and K; of 192 columns in one round of tiles, 256 in the sixth and
+    seventh, 224 in the last two."""
     x, w = linear_inputs(m, k, n, 900 + m + n)
     gpu.lib.pg_tune_tcgen05_pair(2)
     try:
