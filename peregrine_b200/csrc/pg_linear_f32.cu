@@ -1,6 +1,6 @@
 // y = a W^T in f32 accuracy on the 5th-generation tensor cores: bf16 weights as they are, f32 activations as three bf16 pieces.
 //
-//   * a = a1 + a2 + a3 with each piece the next eight significant bits (cut off, not rounded): exact, and so is every product
+//   * a = a1 + a2 + a3 with each piece the next eight significant bits (cut off, not rounded, and none zero): exact, and so is every product
 //     with a bf16 weight.  `linear_split_kernel` writes the pieces as three planes (routed rows in the order of the route).
 //   * D[n][m] = W (128 rows) x A^T (MT rows of a, all three planes): weights are the M side of the instruction, so that a lane of
 //     the epilogue owns a column of y and 32 lanes store 128 contiguous bytes of a row.
@@ -73,8 +73,11 @@ __global__ void __launch_bounds__(256)
                 const uint32_t bits = __float_as_uint(x[i]);
                 const bool finite = (bits & 0x7f800000u) != 0x7f800000u;
                 p[0][i] = finite || (bits & 0x007fffffu) == 0 ? bits & 0xffff0000u : bits | 0x00400000u;   // (a NaN stays one)
+                // no piece of a number is zero, since an infinite weight times one would be NaN: one with nothing left gives up its last bit
+                if (finite && x[i] == __uint_as_float(p[0][i]) && x[i] != 0.0f) p[0][i] -= 0x10000u;
                 const float r1 = finite ? x[i] - __uint_as_float(p[0][i]) : 0.0f;
                 p[1][i] = __float_as_uint(r1) & 0xffff0000u;
+                if (r1 == __uint_as_float(p[1][i]) && r1 != 0.0f) p[1][i] -= 0x10000u;
                 p[2][i] = __float_as_uint(r1 - __uint_as_float(p[1][i]));
             }
 #pragma unroll

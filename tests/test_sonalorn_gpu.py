@@ -119,6 +119,33 @@ def test_f32_product_is_f32(lm, m, n, k):
     lin.free()
 
 
+def test_f32_product_with_infinite_weights(lm):
+    """As in f32 arithmetic: infinite times a number is infinite, whatever bits the number has, and times zero NaN."""
+    from peregrine_b200.layers import Linear
+
+    d = device(lm, "float32", 16)
+    g = rng(11)
+    w = t.bf16_values(g.standard_normal((130, 128)))
+    w[3, 5], w[129, 127] = np.inf, -np.inf
+    a = g.standard_normal((7, 128)).astype(np.float32)
+    a[:, 5] = [1.0, -2.0, 0.0, 1.5, 3.14159274, -1.00390625, 0.333]
+    a[:, 127] = [-1.0, 2.0 ** -60, 3.0, 0.0, 1e30, 1.0 + 2.0 ** -16, -1.0 - 2.0 ** -23]
+    lin = Linear(d, d.bf16(w))
+    y = d.torch.zeros(7, 136, device=d.dev)
+    lin.run(act(d, a), 7, y)
+    lm.sync()
+    with np.errstate(invalid="ignore"):
+        want = a.astype(np.float64) @ w.T.astype(np.float64)
+    got = y[:, :130].cpu().numpy()
+    for c in (3, 129):
+        assert np.array_equal(got[:, c], want[:, c].astype(np.float32), equal_nan=True)
+    assert np.isinf(got[:, 3]).sum() == 6 and np.isnan(got[2, 3]) and np.isnan(got[3, 129])
+    keep = [c for c in range(130) if c not in (3, 129)]
+    bound = np.abs(a).astype(np.float64) @ np.abs(w[keep]).T.astype(np.float64) * (12 * 2.0 ** -23 + 18 * 2.0 ** -24)
+    assert (np.abs(got[:, keep] - want[:, keep]) <= bound).all()
+    lin.free()
+
+
 @pytest.mark.parametrize("n,k", [(200, 4096), (4100, 1024), (136, 14336), (20000, 512)])
 def test_f32_product_rows_do_not_depend_on_each_other(lm, n, k):
     """A row's outputs are the same bits whatever other rows there are, in tiles of any height and with K divided in any way."""
