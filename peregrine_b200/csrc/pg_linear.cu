@@ -15,11 +15,9 @@ PG_API int32_t pg_linear_wrap(pg_ctx *ctx, const void *d_w_bf16, int64_t n, int6
     PG_REQUIRE(k % 64 == 0 && ((uintptr_t)d_w_bf16 & 15) == 0, "linear_wrap: K must be a multiple of 64 (K = %lld) and the weights 16-byte aligned",
                (long long)k);
     PG_REQUIRE(n < (1 << 30) && k < (1 << 30), "linear_wrap: shape too large");
-    // now, since the workspaces cannot grow while a step is being recorded
+    // now, since this workspace cannot grow while a step is being recorded
     const int32_t rc = pg_splitk_reserve(ctx, std::max(pgk_linear_gemv_workspace(n, k), PG_LM_TICKET_BYTES + (size_t)ctx->sm_count * 128 * 128 * sizeof(float)));
     if (rc != PG_OK) return rc;
-    const int32_t rs = pg_scratch_reserve(ctx, pgk_linear_f32_workspace(k));
-    if (rs != PG_OK) return rs;
     pg_linear *l = new (std::nothrow) pg_linear();
     if (!l) PG_FAIL(PG_ERR_NOMEM, "out of host memory");
     l->w = (const bf16 *)d_w_bf16;
@@ -82,7 +80,7 @@ PG_API int32_t pg_linear_run_routed(pg_ctx *ctx, pg_linear *lin, pg_route *route
     if (by_token) {
         // the tokens' rows in the order of the route
         const size_t row_bytes = (size_t)lin->k * 2;
-        const int32_t rr = pg_scratch_reserve(ctx, (size_t)rows * row_bytes);
+        const int32_t rr = pg_scratch_reserve_recording(ctx, (size_t)rows * row_bytes);
         if (rr != PG_OK) return rr;
         const int32_t rc = pgk_route_gather(ctx, route, d_a, row_bytes, ctx->scratch);
         if (rc != PG_OK) return rc;

@@ -26,7 +26,7 @@ namespace {
 constexpr int FN = 128;                // columns of y (rows of W) per tile
 constexpr int FK = 64;                 // elements of K per stage = one 128-byte swizzle span
 constexpr int F_THREADS = 192;
-constexpr int F_ROWS = 128;            // rows for which the planes always find room (pg_linear_wrap)
+constexpr int F_ROWS = 128;            // rows for which a call finds room also while a graph is recorded
 constexpr int64_t F_PLANES = 100 << 20, F_SLABS = 64 << 20;   // most bytes of planes (they stay in L2; longer calls go in portions), of slabs
 
 template <int MT>
@@ -443,8 +443,6 @@ int32_t dispatch(pg_ctx *ctx, const pg_linear *lin, const bf16 *planes, int64_t 
 
 }  // namespace
 
-size_t pgk_linear_f32_workspace(int64_t k) { return (size_t)F_ROWS * k * 3 * sizeof(bf16); }
-
 int32_t pgk_linear_f32(pg_ctx *ctx, const pg_linear *lin, const float *a, int64_t lda, int64_t m, int act, float limit, void *y, int y_dtype, int64_t ldy,
                        const PgRouted *routed)
 {
@@ -454,7 +452,7 @@ int32_t pgk_linear_f32(pg_ctx *ctx, const pg_linear *lin, const float *a, int64_
     const PgRouted none = {};
     const PgRouted &rt = routed ? *routed : none;
     // Rows in portions whose planes stay below F_PLANES: the same outputs as all at once.  While a graph is recorded, what there is of
-    // the workspace takes them, and there is always some (pg_linear_wrap, or this call where another context made the weight)
+    // the workspace takes them, and at least F_ROWS at a time
     const int64_t row_bytes = lin->k * 3 * (int64_t)sizeof(bf16);
     int64_t portion = std::min(m, std::max<int64_t>(F_ROWS, F_PLANES / row_bytes / F_ROWS * F_ROWS));
     if ((size_t)(portion * row_bytes) > ctx->scratch_bytes) {

@@ -56,8 +56,7 @@ int32_t pgk_linear_gemv(pg_ctx *ctx, const pg_linear *lin, const bf16 *a, int64_
 // pg_linear_tc.cu
 int32_t pgk_linear_tc(pg_ctx *ctx, pg_linear *lin, const bf16 *a, int64_t lda, int64_t m, int act, float limit, void *y, int y_dtype, int64_t ldy,
                       const PgRouted *routed);
-// pg_linear_f32.cu; the workspace that pg_linear_wrap reserves for it
-size_t pgk_linear_f32_workspace(int64_t k);
+// pg_linear_f32.cu
 int32_t pgk_linear_f32(pg_ctx *ctx, const pg_linear *lin, const float *a, int64_t lda, int64_t m, int act, float limit, void *y, int y_dtype, int64_t ldy,
                        const PgRouted *routed);
 // pg_route.cu: rows of h in the order of the route (many-token form)

@@ -164,6 +164,19 @@ def test_f32_product_rows_do_not_depend_on_each_other(lm, n, k):
     lin.free()
 
 
+def test_wrapping_a_matrix_takes_nothing_for_f32_steps(lm):
+    """Planes of f32 activations (11 MB for 128 rows of this K) are the matter of a step in f32; slabs are a tile of 128 x 128 per SM."""
+    from peregrine_b200.layers import Linear
+    from peregrine_b200.runtime import GpuContext
+
+    gpu = GpuContext(component="lm")
+    d = device(gpu, "bfloat16", 16)
+    lin = Linear(d, d.torch.zeros(64, 14336, dtype=d.torch.bfloat16, device=d.dev))
+    assert gpu.lib.pg_ctx_scratch_bytes(gpu.handle) < 16 << 20
+    lin.free()
+    gpu.close()
+
+
 def test_f32_product_of_many_rows_goes_in_portions(lm):
     """The workspace of a call is bounded; its outputs are those of its portions."""
     from peregrine_b200.layers import Linear
