@@ -112,9 +112,9 @@ __device__ __forceinline__ float2 scale_of(float bound, int to)
 // block.  The blocks are mma.sync products of transposed tiles, X^T [sixteen columns][64 rows]: the sums of one are the left operand
 // of the next without leaving the warp's registers.  The last chunks come first, so that the chain finds the first ones in L2.
 //
-// Bound by instructions: 55000 cycles a CTA at 4096 tokens, 20000 of them the convolution, 15000 the substitution (before the sums
-// went apart, which took the two kernels from 395 to 444 us).  4096 tokens of 32 heads (430 MB in and out): 212 us; with f32 multiply-adds over columns in place of the tiles 290, with all 64 rows of two columns in
-// a thread's registers, unrolled, 448 (code that runs once is waited for).
+// Bound by instructions: 59000 cycles a CTA at 4096 tokens, 20000 of them the convolution, 15000 the substitution.  4096 tokens of 32
+// heads (430 MB in and out): 227 us, 212 with all products of a sum in one accumulator.  Then, with f32 multiply-adds over columns in place
+// of the tiles 290, with all 64 rows of two columns in a thread's registers, unrolled, 448 (code that runs once is waited for).
 constexpr int V_PITCH = 132, DIAG_PITCH = 20, T_PITCH = 48;
 struct ChunkSmem {
     unsigned char k[4 * TILE];
@@ -579,8 +579,9 @@ __global__ void __launch_bounds__(512, 1)
 // O, run beside it.  Operands come through a ring of 16 KB slots, seven a chunk, as soon as a slot is free, and are asked for in L2
 // some chunks ahead (the four CTAs of a head share that).
 //
-// Bound by that chain: 4000 cycles a chunk and more, 1200 of them the first product, whose operands are 96 KB of shared memory.  4096 tokens of
-// 32 heads 145 us before its accumulators were divided (192 with two fixed buffers and eight warps; delta_scan_kernel, four tokens at a time, 820).
+// Bound by that chain: 4600 cycles a chunk, 1200 of them the first product, whose operands are 96 KB of shared memory.  4096 tokens of
+// 32 heads 167 us; 145 with one accumulator a product (192 with two fixed buffers and eight warps); delta_scan_kernel, four tokens at a
+// time, 820.
 constexpr int CHAIN_WARPS = 16, CHAIN_THREADS = (CHAIN_WARPS + 2) * 32, COLS = 32, PART = 8;
 constexpr int SLOT = 2 * TILE, SLOTS = 12, PER_CHUNK = 7, AHEAD = 3;
 constexpr int S_SM = 0, U_SM = 2 * TILE, RING_SM = 3 * TILE, OWN_SM = RING_SM + SLOTS * SLOT, BARS_SM = OWN_SM + CT * COLS * 4;
