@@ -88,7 +88,6 @@ class Engine:
                 raise RequestError(f"request {key!r}: a wanted place outside its tokens")
         if len(seen - set(self.live)) > self.model.pool.free:
             raise OutOfSlots(f"{len(seen - set(self.live))} new requests, {self.model.pool.free} free slots")
-        out = []
         # rows of one step are limited: what does not fit follows in further steps
         todo = [[key, self._request(key), list(tokens), sorted(set(want)), 0] for key, tokens, want in entries]
         got: Dict[Tuple[Hashable, int], np.ndarray] = {}
@@ -107,14 +106,18 @@ class Engine:
                         wanted.append(at + w - lo)
                         rows.append((item[0], w))
                 at += n
-            got.update(zip(rows, self.model.run([(item[1].slot, item[1].length, item[2][lo:lo + n]) for item, lo, n in parts], wanted)))
+            logits = self.model.run([(item[1].slot, item[1].length, item[2][lo:lo + n]) for item, lo, n in parts], wanted)
+            got.update(zip(rows, logits))
             for item, lo, n in parts:
                 item[1].length += n
                 item[4] = lo + n
             todo = [item for item in todo if item[4] < len(item[2])]
-        for key, _tokens, want in entries:
-            out += [got[(key, w)] for w in want]
-        return np.stack(out) if out else np.zeros((0, self.model.vocab), np.float32)
+        order = [(key, w) for key, _tokens, want in entries for w in want]
+        if order and order == rows:
+            # one run brought them all, in this order: its array is the answer (a copy of 16 rows of 32768 took 190 us, and up to 1.8 ms where
+            # the allocator gave both arrays' pages back to the system between steps)
+            return logits
+        return np.stack([got[at] for at in order]) if order else np.zeros((0, self.model.vocab), np.float32)
 
     # ---- generation ----------------------------------------------------------------------------------------------
     def generate(self, prompts: Sequence[Sequence[int]], max_new: int, stop: Sequence[int] = ()) -> List[List[int]]:

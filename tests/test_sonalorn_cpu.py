@@ -250,3 +250,33 @@ def test_command_line_help_and_bad_model(tmp_path):
     (tmp_path / "config.json").write_text(json.dumps({"architecture": "Unheard"}))
     r = run("generate", "--model", str(tmp_path), "--prompt", "1,2")
     assert r.returncode != 0 and "Unheard" in r.stderr
+
+
+class CountingModel:
+    """Logits that name their row: (slot, position, token) in the first columns."""
+
+    vocab, capacity, step_rows = 5, 64, 6
+
+    def __init__(self):
+        self.pool = SlotPool(3, self.capacity, "cpu")
+
+    def run(self, entries, wanted):
+        rows = [(slot, pos + i, t) for slot, pos, tokens in entries for i, t in enumerate(tokens)]
+        out = np.zeros((len(wanted), self.vocab), np.float32)
+        for o, w in zip(out, wanted):
+            o[:3] = rows[w]
+        return out
+
+
+@pytest.mark.parametrize("portion", [0, 4])          # 0: as many rows as a step of the model takes
+@pytest.mark.parametrize("wants", [[[0], [2], [1]], [[], [0, 1, 2], [0]], [[], [2, 0], [1]], [[0], [1, 1], []], [[], [], []]])
+def test_step_returns_the_wanted_rows_in_their_order(portion, wants):
+    """Whether one run brings them all, in their order or another one, or several runs do; and results of their own each time."""
+    e = Engine(CountingModel(), portion)
+    tokens = [[4], [1, 2, 3], [3, 1]]
+    entries = [(k, t, w) for k, t, w in zip("abc", tokens, wants)]
+    first = e.step(entries)
+    expect = lambda pos: np.array([[s, pos[s] + w, tokens[s][w], 0, 0] for s in range(3) for w in wants[s]], np.float32).reshape(-1, 5)
+    assert first.dtype == np.float32 and np.array_equal(first, expect([0, 0, 0]))
+    again = e.step(entries)
+    assert np.array_equal(again, expect([1, 3, 2])) and np.array_equal(first, expect([0, 0, 0]))
