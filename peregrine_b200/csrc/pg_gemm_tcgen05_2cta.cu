@@ -346,14 +346,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
                         }
                         pg_store_block_32x32(reinterpret_cast<uint32_t *>(y + off0), N, M - row_base, N - (n0 + c), stage_buf, lane, o);
                     }
-                } else if (row < M) {
-                    const int64_t off = off0 + (int64_t)lane * N;
+                } else {
+                    if (acc_out) pg_store_block_words(reinterpret_cast<uint32_t *>(acc_out + off0), N, M - row_base, N - (n0 + c), stage_buf, lane, v);
+                    if (y) {
+                        uint32_t o[32];
 #pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        if (n0 + c + j < N) {
-                            if (acc_out) acc_out[off + j] = (int)v[j];
-                            if (y) y[off + j] = __fmul_rn(__fmul_rn(__int2float_rn((int)v[j]), as), __ldg(w_scales + n0 + c + j));
-                        }
+                        for (int j = 0; j < 32; j++)
+                            o[j] = __float_as_uint(__fmul_rn(__fmul_rn(__int2float_rn((int)v[j]), as), n0 + c + j < N ? __ldg(w_scales + n0 + c + j) : 0.0f));
+                        pg_store_block_words(reinterpret_cast<uint32_t *>(y + off0), N, M - row_base, N - (n0 + c), stage_buf, lane, o);
                     }
                 }
             }

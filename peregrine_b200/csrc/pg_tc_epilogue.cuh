@@ -39,3 +39,25 @@ __device__ __forceinline__ void pg_store_block_32x32(uint32_t *dst, int64_t ld, 
     __syncwarp();
 }
 
+
+// The same where rows do not start on 16-byte boundaries (or the last columns are no multiple of four): a store instruction writes 32
+// consecutive words of one row.
+__device__ __forceinline__ void pg_store_block_words(uint32_t *dst, int64_t ld, int rows_left, int cols_left, uint32_t stage, int lane,
+                                                     const uint32_t (&vals)[32])
+{
+    const uint32_t mine = stage + (uint32_t)lane * (PG_EPI_STRIDE * 4);
+#pragma unroll
+    for (int j = 0; j < 32; j += 4)
+        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(mine + j * 4), "r"(vals[j]), "r"(vals[j + 1]), "r"(vals[j + 2]),
+                     "r"(vals[j + 3])
+                     : "memory");
+    __syncwarp();
+    const int rows = min(rows_left, 32);
+#pragma unroll 8
+    for (int r = 0; r < rows; r++) {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(stage + (uint32_t)(r * PG_EPI_STRIDE + lane) * 4));
+        if (lane < cols_left) dst[(int64_t)r * ld + lane] = v;
+    }
+    __syncwarp();
+}

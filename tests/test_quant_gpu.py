@@ -355,6 +355,19 @@ def test_tcgen05_cta_pairs(pg, gpu, oracle_mt, m, k, n):
         gpu.lib.pg_tune_tcgen05_pair(0)
 
 
+@pytest.mark.parametrize("pair", [1, 2])
+@pytest.mark.parametrize("m,n", [(129, 31), (130, 33), (160, 1), (257, 255), (300, 259), (290, 1537)])
+def test_tcgen05_rows_of_outputs_of_any_length(pg, gpu, oracle_mt, m, n, pair):
+    """Output rows that do not start on 16-byte boundaries, and last columns that are no multiple of four: one CTA a tile, and pairs."""
+    x, w = linear_inputs(m, 272, n, 1300 + m + n)
+    gpu.lib.pg_tune_tcgen05_pair(pair)
+    try:
+        _check_product(pg, gpu, oracle_mt, x, w, m, 272, n, ["tcgen05"])
+        assert gpu.device_status() == 0
+    finally:
+        gpu.lib.pg_tune_tcgen05_pair(0)
+
+
 def test_threads_share_a_weight(pg, gpu):
     """Two contexts on two threads multiply with one weight, each with tiles of another width: calls share nothing that a call writes.
     (1024, 300 and 40 rows of 4100 columns: 256 and 192 columns a tile, and the kernel of few rows)"""
