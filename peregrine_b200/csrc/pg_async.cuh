@@ -51,6 +51,31 @@ __device__ __forceinline__ bool pg_mbar_wait(uint32_t bar, uint32_t parity, vola
         }
     }
 }
+// The whole warp waits: a vote makes the outcome uniform, so that the way past a barrier that is complete holds no divergent branch
+// (about 60 cycles; pg_mbar_wait by every lane and a vote behind it, 220).
+__device__ __forceinline__ bool pg_mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag, int32_t *status, unsigned long long limit_ns)
+{
+    unsigned long long t0 = 0;
+    for (uint32_t it = 1;; ++it) {
+        if (__all_sync(0xffffffffu, pg_mbar_try(bar, parity))) return true;
+        if ((it & 0xff) == 0) {
+            if (__any_sync(0xffffffffu, *abort_flag)) return false;
+            const unsigned long long now = pg_globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            if (__any_sync(0xffffffffu, now - t0 > limit_ns)) {
+                *abort_flag = 1;
+                atomicExch(status, (int32_t)PG_ERR_DEVICE_TIMEOUT);
+                return false;
+            }
+        }
+    }
+}
+// lane 0 arrives for its warp (a predicate, not a branch)
+__device__ __forceinline__ void pg_mbar_arrive_warp(uint32_t bar, int lane)
+{
+    __syncwarp();
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"(lane) : "memory");
+}
 __device__ __forceinline__ void pg_bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
 {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),

@@ -5,15 +5,18 @@
 //   * D[n][m] = W (128 rows) x A^T (MT rows of a, all three planes): weights are the M side of the instruction, so that a lane of
 //     the epilogue owns a column of y and 32 lanes store 128 contiguous bytes of a row.
 //   * the sums: tcgen05's f32 accumulator cuts off what falls below its last bit, always towards zero, and a chain over a whole K
-//     would add that up.  An accumulator therefore only lives for one block of 64 k (smallest pieces first); four warps add the
-//     blocks in registers, rounded, while the next block's products run in the other accumulator.  MT = 128: twelve products of 64
-//     cycles a block, against about 300 cycles for the 128 additions per lane.
+//     would add that up.  An accumulator therefore only lives for one block of 64 k (smallest pieces first); four warps, eight from
+//     64 rows on, add the blocks in registers, rounded, while the next block's products run in the other accumulator.  A warp's chain per block
+//     -- barrier, some 100 cycles for every 32 columns of TMEM, back to the products -- is what four warps could not hide at 128 rows (1413
+//     cycles a block).  Two warps issue the products, a block each in turn, so that one's waits and commits lie beside the other's products.
 //   * K has parts, whose number follows from the matrix alone (f32_parts): each part is summed up by itself, and the parts are added in
 //     their order.  With few tiles they are spread over CTAs and meet in slabs, with tickets, as in linear_tc_kernel; else a CTA goes
 //     through them one after the other and keeps the sum so far in TMEM.  So a row's outputs are the same whatever rows are beside it,
 //     however a call is divided, and whatever workspace there is.
 //
-// What bounds it: the tensor cores at three products for each of the bf16 form's, from about 64 rows; the stream of W below.
+// What bounds it: from about 64 rows shared memory, where a block of 64 k brings 64 KB and its twelve products read 96 KB (1250 cycles at 128
+// bytes each, 768 of products; 1318 measured); the stream of W below.  Products of a prompt of 333 tokens, four dense layers: 2150 -> 1865 us with
+// eight warps of sums, two of products and one copy for the three planes (a copy costs its thread 230 ... 400 cycles).
 // Every mbarrier wait is bounded (pg_async.cuh).
 #include <algorithm>
 
@@ -25,7 +28,6 @@ namespace {
 
 constexpr int FN = 128;                // columns of y (rows of W) per tile
 constexpr int FK = 64;                 // elements of K per stage = one 128-byte swizzle span
-constexpr int F_THREADS = 192;
 constexpr int F_ROWS = 128;            // rows for which a call finds room also while a graph is recorded
 constexpr int64_t F_PLANES = 100 << 20, F_SLABS = 64 << 20;   // most bytes of planes (they stay in L2; longer calls go in portions), of slabs
 
@@ -38,6 +40,10 @@ struct FCfg {
     static constexpr int STAGES = ROOM / STAGE > 10 ? 10 : ROOM / STAGE;
     static constexpr int ACC = MT < 32 ? 32 : MT;          // TMEM columns of an accumulator
     static constexpr int COLS = 4 * ACC;                   // two accumulators, the sum so far, and up to a power of two
+    static constexpr int MW = 2;                           // warps that issue products, a block of K in turn
+    static constexpr int EW = MT >= 64 ? 2 : 1;            // warps of the epilogue per TMEM quarter
+    static constexpr int PART = MT / EW;                   // rows of a per such warp
+    static constexpr int THREADS = (4 + 4 * EW) * 32;      // copies, products, a warp without work, epilogue
     static constexpr size_t SMEM = (size_t)STAGES * STAGE + 1024 + 256;
 };
 
@@ -45,7 +51,7 @@ struct FParts {
     int parts, blocks;       // K in `parts` parts of `blocks` 64-element blocks
     int runs, run;           // a unit takes `run` parts that follow each other; `runs` units make a tile
     float *slabs;            // [tile][part][MT][128]
-    unsigned int *tickets;   // one per (tile, quarter), zero between calls
+    unsigned int *tickets;   // one per (tile, warp of the epilogue), zero between calls
 };
 
 // ---- the three planes of rows row0 .. of a: planes [3][rows][K] --------------------------------------------------------
@@ -101,7 +107,7 @@ __device__ __forceinline__ void f32_keep(uint32_t taddr, const uint32_t (&v)[32]
 }
 
 template <int MT, int ACT>
-__global__ void __launch_bounds__(F_THREADS, 1)
+__global__ void __launch_bounds__(FCfg<MT>::THREADS, 1)
     linear_f32_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, int M, int N, int K, float limit,
                       float *__restrict__ y, int64_t ldy, const PgRouted rt, int block0, const FParts kp, int32_t *status, unsigned long long limit_ns)
 {
@@ -127,7 +133,7 @@ __global__ void __launch_bounds__(F_THREADS, 1)
         }
         for (int i = 0; i < 2; i++) {
             pg_mbar_init(bar_tfull + 8 * i, 1);
-            pg_mbar_init(bar_tempty + 8 * i, 4);   // one arrival per epilogue warp
+            pg_mbar_init(bar_tempty + 8 * i, 4 * C::EW);   // one arrival per epilogue warp
         }
         *abort_flag = 0;
         pg_mbar_fence();
@@ -181,8 +187,7 @@ __global__ void __launch_bounds__(F_THREADS, 1)
                         pg_mbar_expect(bar_full + 8 * stage, C::STAGE);
                         tma_load_2d(at, &tmap_w, bar_full + 8 * stage, kb * FK, w0);
                     }
-#pragma unroll
-                    for (int l = 0; l < 3; l++) tma_load_3d(at + C::STAGE_W + l * C::PLANE, &tmap_a, bar_full + 8 * stage, kb * FK, m0, l);
+                    tma_load_3d(at + C::STAGE_W, &tmap_a, bar_full + 8 * stage, kb * FK, m0, 0);   // all three planes
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
@@ -196,66 +201,61 @@ __global__ void __launch_bounds__(F_THREADS, 1)
                 }
             }
         }
-    } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issuer (the whole warp; one lane's products count)
-        const uint32_t on = pg_elect();
-        constexpr uint32_t idesc = make_idesc(FN, MT);
-        uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-        bool ok = true;
-        for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
-            for (int kb = k_first(u), end = k_end(u); kb < end; kb++) {
-                ok = pg_mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, status, limit_ns);
-                ok = ok && pg_mbar_wait(bar_full + 8 * stage, phase, abort_flag, status, limit_ns);
-                if (!(ok = __all_sync(0xffffffffu, ok))) break;
-                tc_fence_after();
-                const uint32_t at = base + stage * C::STAGE, d_tmem = tmem_base + acc * C::ACC;
-                const uint64_t dw = make_smem_desc(at), da = make_smem_desc(at + C::STAGE_W);
+    } else if (warp < 4) {
+        // ---------------------------------------------------------------- MMA issuers (the whole warp; one lane's products count): each has
+        // every other block of K and one of the accumulators.  (An accumulator is waited for before a stage: the epilogue gives it back
+        // in the order of the blocks, so that no stage is waited for whose use before last is still to be filled.)
+        if (warp <= C::MW) {
+            const uint32_t on = pg_elect();
+            constexpr uint32_t idesc = make_idesc(FN, MT);
+            uint32_t count = 0;
+            bool ok = true;
+            for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+                for (int kb = k_first(u), end = k_end(u); kb < end; kb++, count++) {
+                    const uint32_t acc = count & 1, stage = count % STAGES;
+                    if ((int)acc != warp - 1) continue;
+                    ok = pg_mbar_wait_warp(bar_tempty + 8 * acc, (count / 2 & 1) ^ 1, abort_flag, status, limit_ns);
+                    if (!ok || !(ok = pg_mbar_wait_warp(bar_full + 8 * stage, count / STAGES & 1, abort_flag, status, limit_ns))) break;
+                    tc_fence_after();
+                    const uint32_t at = base + stage * C::STAGE, d_tmem = tmem_base + acc * C::ACC;
+                    const uint64_t dw = make_smem_desc(at), da = make_smem_desc(at + C::STAGE_W);
 #pragma unroll
-                for (int l = 2; l >= 0; l--)
+                    for (int l = 2; l >= 0; l--)
 #pragma unroll
-                    for (int j = 0; j < FK / 16; j++)
-                        umma_f16(d_tmem, dw + (uint64_t)(j * 2), da + (uint64_t)(l * (C::PLANE >> 4) + j * 2), idesc, l != 2 || j != 0 ? 1u : 0u, on);
-                umma_commit(bar_empty + 8 * stage, on);     // stage reusable once these products have read it
-                umma_commit(bar_tfull + 8 * acc, on);
-                if (++stage == STAGES) {
-                    stage = 0;
-                    phase ^= 1;
-                }
-                if (++acc == 2) {
-                    acc = 0;
-                    acc_phase ^= 1;
+                        for (int j = 0; j < FK / 16; j++)
+                            umma_f16(d_tmem, dw + (uint64_t)(j * 2), da + (uint64_t)(l * (C::PLANE >> 4) + j * 2), idesc, l != 2 || j != 0 ? 1u : 0u, on);
+                    umma_commit(bar_empty + 8 * stage, on);     // stage reusable once these products have read it
+                    umma_commit(bar_tfull + 8 * acc, on);
                 }
             }
         }
     } else {
         // ---------------------------------------------------------------- sums and outputs: lane = column of y
-        const int q = warp & 3;                             // TMEM lane quarter this warp may read
+        const int q = warp & 3, half = (warp - 4) >> 2;     // TMEM lane quarter this warp may read, its rows of a
         if (!routed) asm volatile("griddepcontrol.wait;" ::: "memory");   // y may still be read by the predecessor
         const int rows = routed ? tiles_m * MT : M;
         uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
         for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
             const int tile = u / sp;
-            const int m0 = (tile % tiles_m) * MT, n0 = (tile / tiles_m) * FN;
-            const uint32_t lanes = tmem_base + ((uint32_t)(q * 32) << 16), so_far = lanes + 2 * C::ACC;
-            float sum[MT] = {};
+            const int m0 = (tile % tiles_m) * MT + half * C::PART, n0 = (tile / tiles_m) * FN;
+            const uint32_t lanes = tmem_base + ((uint32_t)(q * 32) << 16), so_far = lanes + 2 * C::ACC + half * C::PART;
+            float sum[C::PART] = {};
             int part = (u % sp) * kp.run, next = k_first(u) + kp.blocks;   // the part under way, and the block behind it
             for (int kb = k_first(u), end = k_end(u); kb < end; kb++) {
-                ok = pg_mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, status, limit_ns);
-                if (!(ok = __all_sync(0xffffffffu, ok))) break;
+                if (!(ok = pg_mbar_wait_warp(bar_tfull + 8 * acc, acc_phase, abort_flag, status, limit_ns))) break;
                 tc_fence_after();
-                const uint32_t taddr = lanes + acc * C::ACC;
+                const uint32_t taddr = lanes + acc * C::ACC + half * C::PART;
 #pragma unroll
-                for (int c = 0; c < C::ACC; c += 32) {
+                for (int c = 0; c < C::ACC / C::EW; c += 32) {
                     uint32_t v[32];
                     tmem_ld32(taddr + c, v);
 #pragma unroll
                     for (int j = 0; j < 32; j++)
-                        if (c + j < MT) sum[c + j] += __uint_as_float(v[j]);
+                        if (c + j < C::PART) sum[c + j] += __uint_as_float(v[j]);
                 }
                 tc_fence_before();
-                __syncwarp();
-                if (lane == 0) pg_mbar_arrive(bar_tempty + 8 * acc);
+                pg_mbar_arrive_warp(bar_tempty + 8 * acc, lane);
                 if (++acc == 2) {
                     acc = 0;
                     acc_phase ^= 1;
@@ -263,33 +263,33 @@ __global__ void __launch_bounds__(F_THREADS, 1)
                 if (kp.parts > 1 && (kb + 1 == next || kb + 1 == end)) {
                     // the end of a part: to its slab, or onto the sum of those in front of it
                     if (sp > 1) {
-                        float *slab = kp.slabs + ((int64_t)tile * kp.parts + part) * MT * FN + q * 32 + lane;
+                        float *slab = kp.slabs + (((int64_t)tile * kp.parts + part) * MT + half * C::PART) * FN + q * 32 + lane;
 #pragma unroll
-                        for (int j = 0; j < MT; j++) __stcg(slab + j * FN, sum[j]);
+                        for (int j = 0; j < C::PART; j++) __stcg(slab + j * FN, sum[j]);
                     } else {
                         if (part > 0) {
 #pragma unroll
-                            for (int c = 0; c < C::ACC; c += 32) {
+                            for (int c = 0; c < C::ACC / C::EW; c += 32) {
                                 uint32_t v[32];
                                 tmem_ld32(so_far + c, v);
 #pragma unroll
                                 for (int j = 0; j < 32; j++)
-                                    if (c + j < MT) sum[c + j] = __uint_as_float(v[j]) + sum[c + j];
+                                    if (c + j < C::PART) sum[c + j] = __uint_as_float(v[j]) + sum[c + j];
                             }
                         }
                         if (kb + 1 < end) {
 #pragma unroll
-                            for (int c = 0; c < C::ACC; c += 32) {
+                            for (int c = 0; c < C::ACC / C::EW; c += 32) {
                                 uint32_t v[32];
 #pragma unroll
-                                for (int j = 0; j < 32; j++) v[j] = c + j < MT ? __float_as_uint(sum[c + j]) : 0u;
+                                for (int j = 0; j < 32; j++) v[j] = c + j < C::PART ? __float_as_uint(sum[c + j]) : 0u;
                                 f32_keep(so_far + c, v);
                             }
                         }
                     }
                     if (kb + 1 < end) {
 #pragma unroll
-                        for (int j = 0; j < MT; j++) sum[j] = 0.0f;
+                        for (int j = 0; j < C::PART; j++) sum[j] = 0.0f;
                     }
                     part++;
                     next += kp.blocks;
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(F_THREADS, 1)
             const int n = n0 + q * 32 + lane;
             bool mine = true;
             if (sp > 1) {
-                unsigned int *ticket = kp.tickets + tile * 4 + q;
+                unsigned int *ticket = kp.tickets + (tile * C::EW + half) * 4 + q;
                 __threadfence();
                 __syncwarp();
                 const unsigned int before = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(ticket, 1u) : 0u, 0);
@@ -308,13 +308,13 @@ __global__ void __launch_bounds__(F_THREADS, 1)
                     // the last part of these columns to finish adds all parts up, in their order
                     __threadfence();
                     if (lane == 0) *ticket = 0;
-                    const float *slab = kp.slabs + (int64_t)tile * kp.parts * MT * FN + q * 32 + lane;
+                    const float *slab = kp.slabs + ((int64_t)tile * kp.parts * MT + half * C::PART) * FN + q * 32 + lane;
 #pragma unroll
-                    for (int j = 0; j < MT; j++) sum[j] = __ldcg(slab + j * FN);
+                    for (int j = 0; j < C::PART; j++) sum[j] = __ldcg(slab + j * FN);
                     for (int p = 1; p < kp.parts; p++) {
                         slab += MT * FN;
 #pragma unroll
-                        for (int j = 0; j < MT; j++) sum[j] += __ldcg(slab + j * FN);
+                        for (int j = 0; j < C::PART; j++) sum[j] += __ldcg(slab + j * FN);
                     }
                 }
             }
@@ -323,14 +323,14 @@ __global__ void __launch_bounds__(F_THREADS, 1)
                 if (n < N) {
                     float *dst = y + (int64_t)m0 * ldy + n;
 #pragma unroll
-                    for (int j = 0; j < MT; j++)
+                    for (int j = 0; j < C::PART; j++)
                         if (m0 + j < rows) dst[j * ldy] = sum[j];
                 }
             } else {
                 // columns [8 gates | 8 ups] twice per warp; N is a multiple of 16
                 float *dst = y + (int64_t)m0 * ldy + (n0 + q * 32) / 2 + (lane >> 4) * 8 + (lane & 7);
 #pragma unroll
-                for (int j = 0; j < MT; j++) {
+                for (int j = 0; j < C::PART; j++) {
                     const float u2 = __shfl_down_sync(0xffffffffu, sum[j], 8);
                     if (!(lane & 8) && n < N && m0 + j < rows) dst[j * ldy] = pg_glu<ACT>(sum[j], u2, limit);
                 }
@@ -358,7 +358,7 @@ int32_t launch(pg_ctx *ctx, const pg_linear *lin, const bf16 *planes, int64_t m,
     int32_t rc = pg_encode_bf16(&tw, lin->w, 2, wd, ws, wb);
     if (rc != PG_OK) return rc;
     const cuuint64_t ad[3] = {(cuuint64_t)lin->k, (cuuint64_t)m, 3}, as[2] = {(cuuint64_t)lin->k * 2, (cuuint64_t)(lin->k * m) * 2};
-    const cuuint32_t ab[3] = {FK, MT, 1};
+    const cuuint32_t ab[3] = {FK, MT, 3};
     rc = pg_encode_bf16(&ta, planes, 3, ad, as, ab);
     if (rc != PG_OK) return rc;
     auto kern = linear_f32_kernel<MT, ACT>;
@@ -367,7 +367,7 @@ int32_t launch(pg_ctx *ctx, const pg_linear *lin, const bf16 *planes, int64_t m,
     const int64_t units = ((m + MT - 1) / MT) * ((lin->n + FN - 1) / FN) * kp.runs;
     kp.tickets = reinterpret_cast<unsigned int *>(ctx->splitk);
     kp.slabs = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(ctx->splitk) + PG_LM_TICKET_BYTES);
-    return launch_pdl(ctx, kern, dim3((unsigned)std::min<int64_t>(units, ctx->sm_count)), dim3(F_THREADS), C::SMEM, tw, ta, (int)m, (int)lin->n, (int)lin->k,
+    return launch_pdl(ctx, kern, dim3((unsigned)std::min<int64_t>(units, ctx->sm_count)), dim3(C::THREADS), C::SMEM, tw, ta, (int)m, (int)lin->n, (int)lin->k,
                       limit, y, ldy, rt, block0, kp, ctx->d_status, ctx->wait_limit_ns);
 }
 
@@ -388,7 +388,7 @@ void f32_parts(const pg_ctx *ctx, const pg_linear *lin, FParts *kp)
     double best = 0;
     for (int64_t parts = 1; parts <= std::max<int64_t>(1, std::min<int64_t>(8, kblocks / 4)); parts++) {
         const int64_t blocks = (kblocks + parts - 1) / parts;
-        if ((kblocks + blocks - 1) / blocks != parts || tiles * 4 * (int64_t)sizeof(int) > (int64_t)PG_LM_TICKET_BYTES) continue;
+        if ((kblocks + blocks - 1) / blocks != parts || tiles * 8 * (int64_t)sizeof(int) > (int64_t)PG_LM_TICKET_BYTES) continue;
         const double cost = f32_cost((tiles * parts + ctx->sm_count - 1) / ctx->sm_count, blocks, 16, parts, parts > 1);
         if (best == 0 || cost < best) {
             best = cost;
@@ -419,7 +419,7 @@ int32_t dispatch(pg_ctx *ctx, const pg_linear *lin, const bf16 *planes, int64_t 
             const int64_t tiles = tiles_n * ((m + cand - 1) / cand);
             for (int64_t run = kp.parts; run >= 1; run--) {
                 const int64_t runs = (kp.parts + run - 1) / run;
-                if (runs > 1 && (tiles * kp.parts * cand * slab > room || tiles * 4 * (int64_t)sizeof(int) > (int64_t)PG_LM_TICKET_BYTES)) break;
+                if (runs > 1 && (tiles * kp.parts * cand * slab > room || tiles * 8 * (int64_t)sizeof(int) > (int64_t)PG_LM_TICKET_BYTES)) break;
                 const double cost = f32_cost((tiles * runs + ctx->sm_count - 1) / ctx->sm_count, run * kp.blocks, cand, kp.parts, runs > 1);
                 if (best == 0 || cost < best) {
                     best = cost;
