@@ -82,8 +82,9 @@ __global__ void __launch_bounds__(256) f16_to_f32_kernel(const uint16_t *__restr
 // slice of 8 blocks), FILL = 16 * SEG + 256 bytes with SEG = 8 * {16, 32} quant bytes per row:
 //   row r of the tile at r * SEG, as 16-byte pieces; piece p of a row holds what lane t = p % 4 of a tensor-core fragment
 //   needs of block group p / 4 -- Q4_0: word t (elements 8t..8t+7) of the group's four blocks; Q8_0: bytes 8t..8t+7 of
-//   the group's two blocks -- and is stored at position p ^ ((r & 1) << 2), so that the eight lanes of a quarter warp
-//   (two rows, four pieces each) hit all 32 banks when the fill lies in shared memory as it lies in global memory;
+//   the group's two blocks -- and is stored at position p ^ (((r & 1) << 2) | ((r >> 1) & 3)), so that the eight lanes of a
+//   quarter warp hit all 32 banks when the fill lies in shared memory as it lies in global memory, whether they read four
+//   pieces of two rows or the same piece of eight;
 //   then the scales: row r's eight f16 at 16 * SEG + r * 16.
 __device__ __forceinline__ int64_t tiled_index(int type, int64_t row, int64_t nslices, int blk_in_row, int byte, bool scale)
 {
@@ -100,7 +101,7 @@ __device__ __forceinline__ int64_t tiled_index(int type, int64_t row, int64_t ns
         piece = (bl >> 2) * 4 + (byte >> 2);
         within = (bl & 3) * 4 + (byte & 3);
     }
-    return base + (int64_t)r * seg + ((piece ^ ((r & 1) << 2)) * 16) + within;
+    return base + (int64_t)r * seg + ((piece ^ (((r & 1) << 2) | ((r >> 1) & 3))) * 16) + within;
 }
 
 __global__ void __launch_bounds__(256) repack_kernel(int type, int tiled, const uint8_t *__restrict__ raw, int64_t num_blocks, int nblk_row,

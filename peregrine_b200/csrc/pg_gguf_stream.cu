@@ -36,9 +36,9 @@
 //
 // Layout of a fill (made at upload, csrc/pg_gguf.cu: repack_kernel): row r of the tile at r * SEG as 16-byte pieces;
 // piece p = (block group) * 4 + t holds, for lane t of a fragment, Q4_0: word t (elements 8t..8t+7) of the group's four
-// blocks; Q8_0: bytes 8t..8t+7 of the group's two blocks; it is stored at position p ^ ((r & 1) << 2), which makes the
-// 128-bit reads of a quarter warp (two rows, four pieces each) free of bank conflicts without padding.  The scales
-// follow at 16 * SEG + r * 16.
+// blocks; Q8_0: bytes 8t..8t+7 of the group's two blocks; it is stored at position p ^ (((r & 1) << 2) | ((r >> 1) & 3)),
+// which makes the 128-bit reads of a quarter warp (two rows, four pieces each; in csrc/pg_gguf_tc.cu one piece of eight rows
+// too) free of bank conflicts without padding.  The scales follow at 16 * SEG + r * 16.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(W * 32, 1)
                     constexpr int BPL = (TYPE == PG_GGUF_Q4_0) ? 4 : 2;     // blocks per 128-bit load of a row
 #pragma unroll
                     for (int b4 = 0; b4 < GS_SLICE / BPL; b4++) {
-                        const uint32_t piece = (uint32_t)(((b4 * 4 + t) ^ ((g & 1) << 2)) * 16);
+                        const uint32_t piece = (uint32_t)((t ^ (g >> 1)) * 16 + ((b4 * 4) ^ ((g & 1) << 2)) * 16);
                         const uint4 qa = gs_lds128(slot + (uint32_t)g * C::SEG + piece);
                         const uint4 qb = gs_lds128(slot + (uint32_t)(g + 8) * C::SEG + piece);
                         const uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w}, wb[4] = {qb.x, qb.y, qb.z, qb.w};

@@ -10,20 +10,28 @@
 //   * a row that holds a NaN or an infinity gives NaN, as in the streaming form (2^-s is then a NaN).
 //
 // Weights are the M side of the instruction (128 rows of W), rows of x the N side (MT): a lane of the epilogue owns a row of W, so
-// that a block's scale is one register, and 32 lanes store 128 contiguous bytes of a row of y.  A CTA (15 or 19 warps, one per SM):
-//   warps 0, 10   copies: blocks of 64 k of both planes by TMA; slices of W as they lie in memory (eight fills of 16 rows x 256 k)
-//   warp 1        products: two planes x two steps of 16 k per block of W into an accumulator of its own; up to 64 rows the planes lie
-//                 side by side in one product, whose issue (not its time in the tensor core) is what counts there
+// that a block's scale is one register, and 32 lanes store 128 contiguous bytes of a row of y.  With few tiles K is divided over CTAs;
+// the last part of a tile to finish adds all parts in their order.
+//
+// Up to 32 rows, gguf_tc_kernel (19 warps):
+//   warps 0, 10   copies: blocks of 128 k of both planes by TMA; slices of W as they lie in memory (eight fills of 16 rows x 256 k)
+//   warp 1        products: two steps of 16 k per block of W into an accumulator of its own; the planes lie side by side in one product,
+//                 whose issue (not its time in the tensor core) is what counts here
 //   warps 2-9     two per TMEM quarter, half of the columns each: sum += d * accumulator
 //   warps 11-     quants -> f16 in the 128-byte-swizzled tiles that the products read, 128 k at a time, two such buffers
-// With few tiles K is divided over CTAs; the last part of a tile to finish adds all parts in their order.
 //
-// What bounds it: shared memory, then the epilogue's way through TMEM.  At MT = 128 a block of 32 k takes 256 cycles of products, which
-// read 32 KB of it, while 16 KB of planes come in, 8 KB of f16 weights are written and 2 KB of quants read: 470 cycles at 128 bytes
-// each, about 460 of the warp that issues the products (800 with its waits).  N 14336, K 4096, 9 / 16 / 33 / 64 / 300 rows: Q4_0 25 / 26 /
-// 39 / 43 / 126 us, where eight rows at a time through the streaming form took 31 / 42 / 92 / 167 / 787; error against 64 bits 2e-7 ...
-// 3e-7 with 1 % of the channels x 20 (1.2e-6).  At eight rows
-// and K 4096 the streaming form is the faster one (21 against 25 us).
+// Above, gguf_tc_wide_kernel (23 warps): the quants go to TMEM as f16 and the products take them from there, which leaves shared memory to
+// the planes and makes a product of few columns cheaper (M 128, N 64: 37 cycles, 55 with the weights in shared memory).
+//   warps 0, 1    one copy per stage of the planes, one per slice of W (a copy costs its thread 250 ... 600 cycles, whatever it brings)
+//   warp 2        products: two planes x two steps of 16 k per block of W
+//   warps 3-6     quants -> f16, a lane per row of W, 128 k at a time, two such buffers
+//   warps 7-22    sum += d * accumulator, four warps per TMEM quarter
+//
+// What bounds it: the epilogue's chain per block -- barrier, some 100 cycles to read 32 columns of TMEM, back to the products -- at two or
+// three accumulators in flight; at MT = 160 a block takes 685 cycles, 320 of them products.  Waits by the whole warp that end in one
+// vote (pg_mbar_wait_warp) took a third off it.  Q4_0, N 14336, K 4096, us, 9 / 16 / 33 / 64 / 128 / 300 / 512 rows: 25 / 26 / 37 / 37 / 47 / 100 / 160
+// (33 rows and more with the quants in shared memory and two warps per quarter: 39 / 42 / 53 / 126 / 194).  Error against 64 bits 2e-7 ... 3e-7 with 1 %
+// of the channels x 20 (1.2e-6).  At eight rows and K 4096 the streaming form is the faster one (21 against 25 us).
 // Every mbarrier wait is bounded (pg_async.cuh).
 #include <algorithm>
 
@@ -40,6 +48,7 @@ constexpr int GT_ROWS = 64;                       // rows for which the planes a
 constexpr size_t GT_TICKET_BYTES = 64 * 1024;     // as in the int8 kernel: tickets, zero between calls, then slabs
 constexpr int64_t GT_PLANES = 100 << 20;          // most bytes of planes (they stay in L2; longer calls go in portions)
 
+// ---- up to 32 rows ----------------------------------------------------------------------------------------------------------
 template <int TYPE, int MT>
 struct GtCfg {
     static constexpr int SEG = TYPE == PG_GGUF_Q4_0 ? 128 : 256;   // quant bytes per row and slice
@@ -47,19 +56,18 @@ struct GtCfg {
     static constexpr int RAW = 8 * FILL;                           // a slice (256 k) of 128 rows
     static constexpr int A_TILE = GT_N * 64 * 2;                   // 64 k of 128 rows in f16
     static constexpr int A_BYTES = 4 * A_TILE;                     // two buffers of 128 k
-    static constexpr bool STACK = MT <= 64;                        // both planes as columns of one product, added up in the epilogue
-    static constexpr int COLS = STACK ? 2 * MT : MT;               // accumulator columns of a block
+    static constexpr int COLS = 2 * MT;                            // accumulator columns of a block: one product for both planes, added up in the epilogue
     static constexpr int PLANE = MT * 64 * 2;
-    static constexpr int BK64 = MT <= 64 ? 2 : 1;                  // 64-k blocks of the planes per stage
+    static constexpr int BK64 = 2;                                 // 64-k blocks of the planes per stage
     static constexpr int B_STAGE = BK64 * 2 * PLANE;
     static constexpr int ROOM = 232448 - 1024 - 512;
-    static constexpr int BST = MT >= 160 ? 2 : MT >= 64 ? (TYPE == PG_GGUF_Q4_0 ? 3 : 2) : MT == 32 ? 4 : 6;
+    static constexpr int BST = MT == 32 ? 4 : 6;
     static constexpr int FIT = (ROOM - A_BYTES - BST * B_STAGE) / RAW;
     static constexpr int RST = FIT > 7 ? 7 : FIT;
-    static constexpr int GB = MT <= 32 ? 4 : MT <= 128 ? 2 : 1;    // blocks per group of accumulators
+    static constexpr int GB = 4;                                   // blocks per group of accumulators
     static constexpr int NBUF = 512 / (GB * COLS) > 4 ? 4 : 512 / (GB * COLS);
     static constexpr int HALF = MT / 2;                            // rows of x per warp of the epilogue
-    static constexpr int DW = MT <= 64 ? 8 : 4;                    // warps that turn quants into f16 (the wide tiles' registers leave room for four)
+    static constexpr int DW = 8;                                   // warps that turn quants into f16
     static constexpr int THREADS = (11 + DW) * 32;
     static constexpr size_t SMEM = (size_t)A_BYTES + BST * B_STAGE + RST * RAW + 1024 + 512;
     static_assert(RST >= 2 && NBUF >= 2, "shared memory or TMEM too small");
@@ -274,16 +282,8 @@ __global__ void __launch_bounds__(GtCfg<TYPE, MT>::THREADS, 1)
                     const uint32_t d = tmem + (ts * C::GB + blk % C::GB) * C::COLS;
                     const uint64_t da = desc_a + (uint64_t)((as * 2 + (blk >> 1)) * (C::A_TILE >> 4) + (blk & 1) * 4);
                     const uint64_t db = desc_b + (uint64_t)(bs * (C::B_STAGE >> 4) + (blk % PER_B >> 1) * (2 * C::PLANE >> 4) + (blk & 1) * 4);
-                    if constexpr (C::STACK) {
 #pragma unroll
-                        for (int j = 0; j < 2; j++) umma_f16(d, da + (uint64_t)(j * 2), db + (uint64_t)(j * 2), idesc, j != 0 ? 1u : 0u, on);
-                    } else {
-#pragma unroll
-                        for (int l = 1; l >= 0; l--)
-#pragma unroll
-                            for (int j = 0; j < 2; j++)
-                                umma_f16(d, da + (uint64_t)(j * 2), db + (uint64_t)(l * (C::PLANE >> 4) + j * 2), idesc, l != 1 || j != 0 ? 1u : 0u, on);
-                    }
+                    for (int j = 0; j < 2; j++) umma_f16(d, da + (uint64_t)(j * 2), db + (uint64_t)(j * 2), idesc, j != 0 ? 1u : 0u, on);
                     if ((blk + 1) % C::GB == 0) {
                         umma_commit(t_full + 8 * ts, on);
                         if (++ts == C::NBUF) {
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(GtCfg<TYPE, MT>::THREADS, 1)
         const int row0 = (warp - 11) * (GT_N / C::DW) + (lane >> 2), t = lane & 3;
         // lane: row r, quarter t of the blocks; rows of odd number take their blocks in the other order, so that two rows never write
         // to the same banks (and the layout has them read from different ones)
-        const int odd = row0 & 1;
+        const int odd = row0 & 1, sw = (odd << 2) | ((row0 >> 1) & 3);   // (rows eight apart have the same)
         uint32_t rs = 0, rp = 0, as = 0, ap = 0;
         for (int u = blockIdx.x; ok && u < total; u += gridDim.x)
             for (int s = s_first(u), end = s_end(u); ok && s < end; s++) {
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(GtCfg<TYPE, MT>::THREADS, 1)
                         const int r = row0 + i * 8;
                         const uint32_t src = r_at + rs * C::RAW + (uint32_t)(r >> 4) * C::FILL + (uint32_t)(r & 15) * C::SEG;
 #pragma unroll
-                        for (int p = 0; p < LOADS; p++) q[i][p] = pg_lds128(src + (uint32_t)((((h * LOADS + p) * 4 + t) ^ (odd << 2)) * 16));
+                        for (int p = 0; p < LOADS; p++) q[i][p] = pg_lds128(src + (uint32_t)((((h * LOADS + p) * 4 + t) ^ sw) * 16));
                     }
                     ok = __all_sync(0xffffffffu, pg_mbar_wait(a_empty + 8 * as, ap ^ 1, abort_flag, status, limit_ns));
                     if (!ok) break;
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(GtCfg<TYPE, MT>::THREADS, 1)
                     const __half2 hh = *reinterpret_cast<const __half2 *>(&scw[b >> 1]);
                     const float d = (b & 1) ? __high2float(hh) : __low2float(hh);
                     const uint32_t at = taddr + (ts * C::GB + b % C::GB) * C::COLS;
-                    if constexpr (C::STACK) gt_add<C::HALF>(at + MT, d, sum);
+                    gt_add<C::HALF>(at + MT, d, sum);
                     gt_add<C::HALF>(at, d, sum);
                     if ((b + 1) % C::GB == 0) {
                         tc_fence_before();
@@ -452,6 +452,380 @@ __global__ void __launch_bounds__(GtCfg<TYPE, MT>::THREADS, 1)
     }
 }
 
+// asks for NC columns of this lane's TMEM row (8, 16, 32, or pieces of them)
+template <int NC>
+__device__ __forceinline__ void gt_ask(uint32_t taddr, uint32_t *t)
+{
+    if constexpr (NC >= 32) {
+        tmem_ld32_async(taddr, *reinterpret_cast<uint32_t (*)[32]>(t));
+        if constexpr (NC > 32) gt_ask<NC - 32>(taddr + 32, t + 32);
+    } else if constexpr (NC >= 16) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7]), "=r"(t[8]), "=r"(t[9]), "=r"(t[10]),
+              "=r"(t[11]), "=r"(t[12]), "=r"(t[13]), "=r"(t[14]), "=r"(t[15])
+            : "r"(taddr)
+            : "memory");
+        if constexpr (NC > 16) gt_ask<NC - 16>(taddr + 16, t + 16);
+    } else {
+        static_assert(NC == 8, "pieces of 32, 16 and 8 columns");
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7])
+                     : "r"(taddr)
+                     : "memory");
+    }
+}
+__device__ __forceinline__ void gt_load_4d(uint32_t dst, const CUtensorMap *tmap, uint32_t bar, int x, int y, int z, int w)
+{
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst),
+                 "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w)
+                 : "memory");
+}
+// ---- more than 32 rows -------------------------------------------------------------------------------------------------------
+template <int TYPE, int MT>
+struct GwCfg {
+    static constexpr int SEG = TYPE == PG_GGUF_Q4_0 ? 128 : 256;   // quant bytes per row and slice
+    static constexpr int FILL = 16 * SEG + 256;
+    static constexpr int RAW = 8 * FILL;                           // a slice (256 k) of 128 rows
+    static constexpr int PLANE = MT * 128;                         // 64 k of a plane
+    static constexpr int BK64 = MT == 64 ? 2 : 1;                  // 64-k blocks of the planes per stage
+    static constexpr int PER_B = 2 * BK64;                         // blocks of W per stage
+    static constexpr int B_STAGE = BK64 * 2 * PLANE;
+    static constexpr int GB = MT == 64 ? 2 : 1;                    // blocks of W per group of accumulators
+    static constexpr int SETS = GB;                                // groups go to SETS sets of 4 / SETS warps per TMEM quarter in turn
+    static constexpr int PART = MT * SETS / 4;                     // rows of x per warp of the epilogue
+    static constexpr int COMB = SETS == 1 ? 0 : 2 * PART * GT_N * 4;   // where the sets' sums meet
+    static constexpr int ROOM = 232448 - 1024 - 512 - COMB;
+    static constexpr int BST = TYPE == PG_GGUF_Q8_0 && MT == 64 ? 2 : 3;
+    static constexpr int FIT = (ROOM - BST * B_STAGE) / RAW;
+    static constexpr int RST = FIT > 8 ? 8 : FIT;
+    static constexpr int NA = 2;                                   // f16 buffers: 64 columns of TMEM, 128 k of 128 rows of W
+    static constexpr int A_COL = 512 - 64 * NA;
+    static constexpr int NBUF = A_COL / (GB * MT);
+    static constexpr int DW0 = 3, EW0 = 7;                         // first warps of the quants (four), of the epilogue (sixteen)
+    static constexpr int THREADS = (EW0 + 16) * 32;
+    static constexpr int BARS = 2 * (RST + BST + NA + NBUF) + 8;
+    static constexpr size_t SMEM = (size_t)BST * B_STAGE + RST * RAW + COMB + 1024 + 512;
+    static_assert(RST >= 2 && NBUF >= 2 && BARS * 8 + 8 <= 512, "shared memory or TMEM too small");
+};
+
+template <int TYPE, int MT>
+__global__ void __launch_bounds__(GwCfg<TYPE, MT>::THREADS, 1)
+    gguf_tc_wide_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, int64_t N, int nslices, int M,
+                   const float *__restrict__ us, float *__restrict__ y, const GtParts kp, int32_t *status, unsigned long long limit_ns)
+{
+    using C = GwCfg<TYPE, MT>;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw_addr = pg_smem(smem_raw);
+    const uint32_t base = (raw_addr + 1023u) & ~1023u;
+    const uint32_t b_at = base, r_at = b_at + C::BST * C::B_STAGE, c_at = r_at + C::RST * C::RAW;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw + (c_at - raw_addr) + C::COMB);
+    const uint32_t bar = pg_smem(bars);
+    // full and empty of: slices, blocks of the planes, f16 buffers, groups of accumulators; then the meeting of sums, by quarter
+    const uint32_t r_full = bar, r_empty = r_full + 8 * C::RST, b_full = r_empty + 8 * C::RST, b_empty = b_full + 8 * C::BST;
+    const uint32_t a_full = b_empty + 8 * C::BST, a_empty = a_full + 8 * C::NA, t_full = a_empty + 8 * C::NA, t_empty = t_full + 8 * C::NBUF;
+    const uint32_t c_full = t_empty + 8 * C::NBUF, c_free = c_full + 32;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + C::BARS);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < C::RST; i++) {
+            pg_mbar_init(r_full + 8 * i, 1);
+            pg_mbar_init(r_empty + 8 * i, 16 + 4);   // the scales, the quants
+        }
+        for (int i = 0; i < C::BST; i++) {
+            pg_mbar_init(b_full + 8 * i, 1);
+            pg_mbar_init(b_empty + 8 * i, 1);
+        }
+        for (int i = 0; i < C::NA; i++) {
+            pg_mbar_init(a_full + 8 * i, 4);
+            pg_mbar_init(a_empty + 8 * i, 1);
+        }
+        for (int i = 0; i < C::NBUF; i++) {
+            pg_mbar_init(t_full + 8 * i, 1);
+            pg_mbar_init(t_empty + 8 * i, 16 / C::SETS);
+        }
+        for (int i = 0; i < 4; i++) {
+            pg_mbar_init(c_full + 8 * i, 2);
+            pg_mbar_init(c_free + 8 * i, 2);
+        }
+        *abort_flag = 0;
+        pg_mbar_fence();
+    }
+    __syncwarp();
+    if (warp == 2) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pg_smem(tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    const int tiles_m = (M + MT - 1) / MT, tiles_n = (int)((N + GT_N - 1) / GT_N);
+    const int sp = kp.parts, total = tiles_m * tiles_n * sp;   // unit u: part u % sp of tile u / sp; the tiles of a row of W follow each other
+    auto s_first = [&](int u) { return (u % sp) * kp.slices; };
+    auto s_end = [&](int u) { return min(nslices, (u % sp + 1) * kp.slices); };
+    auto wait = [&](uint32_t b, uint32_t parity) { return pg_mbar_wait_warp(b, parity & 1, abort_flag, status, limit_ns); };
+    bool ok = true;
+
+    if (warp == 0) {
+        // ---------------------------------------------------------------- planes of x: a copy per stage
+        if (lane == 0) {
+            uint32_t bs = 0, bp = 1;
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+                const int m0 = (u / sp % tiles_m) * MT;
+                for (int kb = 4 * s_first(u), end = 4 * s_end(u); kb < end; kb += C::BK64) {
+                    if (!(ok = pg_mbar_wait(b_empty + 8 * bs, bp, abort_flag, status, limit_ns))) break;
+                    pg_mbar_expect(b_full + 8 * bs, C::B_STAGE);
+                    gt_load_4d(b_at + bs * C::B_STAGE, &tmap_x, b_full + 8 * bs, 0, m0, 0, kb);
+                    if (++bs == C::BST) {
+                        bs = 0;
+                        bp ^= 1;
+                    }
+                }
+            }
+            if (!ok) gt_settle();
+        }
+    } else if (warp == 1) {
+        // ---------------------------------------------------------------- slices of W, which no kernel writes: no wait for the preceding one
+        if (lane == 0) {
+            uint32_t rs = 0, rp = 1;
+            for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+                const int f0 = u / sp / tiles_m * (GT_N / 16);      // (fills behind the last one are zeros)
+                for (int s = s_first(u), end = s_end(u); s < end; s++) {
+                    if (!(ok = pg_mbar_wait(r_empty + 8 * rs, rp, abort_flag, status, limit_ns))) break;
+                    pg_mbar_expect(r_full + 8 * rs, C::RAW);
+                    gt_load_4d(r_at + rs * C::RAW, &tmap_w, r_full + 8 * rs, 0, 0, s, f0);
+                    if (++rs == C::RST) {
+                        rs = 0;
+                        rp ^= 1;
+                    }
+                }
+            }
+            if (!ok) gt_settle();
+        }
+    } else if (warp == 2) {
+        // ---------------------------------------------------------------- products (the whole warp; one lane's count)
+        const uint32_t on = pg_elect();
+        constexpr uint32_t idesc = gt_idesc(GT_N, MT);
+        const uint64_t desc_b = make_smem_desc(b_at);
+        uint32_t bs = 0, bp = 0, as = 0, ap = 0, ts = 0, tp = 0;
+        for (int u = blockIdx.x; ok && u < total; u += gridDim.x)
+            for (int h = 2 * s_first(u), end = 2 * s_end(u); ok && h < end; h++) {
+                if (!(ok = wait(a_full + 8 * as, ap))) break;
+#pragma unroll
+                for (int blk = 0; blk < 4; blk++) {             // blocks of the 128 k
+                    if (blk % C::PER_B == 0 && !(ok = wait(b_full + 8 * bs, bp))) break;
+                    if (blk % C::GB == 0) {
+                        if (!(ok = wait(t_empty + 8 * ts, tp ^ 1))) break;
+                        tc_fence_after();
+                    }
+                    const uint32_t d = tmem + (ts * C::GB + blk % C::GB) * MT;
+                    const uint32_t a = tmem + C::A_COL + as * 64 + blk * 16;
+                    const uint64_t db = desc_b + (uint64_t)(bs * (C::B_STAGE >> 4) + (blk % C::PER_B >> 1) * (2 * C::PLANE >> 4) + (blk & 1) * 4);
+#pragma unroll
+                    for (int l = 1; l >= 0; l--)
+#pragma unroll
+                        for (int j = 0; j < 2; j++)
+                            umma_f16_ta(d, a + j * 8, db + (uint64_t)(l * (C::PLANE >> 4) + j * 2), idesc, l != 1 || j != 0 ? 1u : 0u, on);
+                    if ((blk + 1) % C::GB == 0) {
+                        umma_commit(t_full + 8 * ts, on);
+                        if (++ts == C::NBUF) {
+                            ts = 0;
+                            tp ^= 1;
+                        }
+                    }
+                    if ((blk + 1) % C::PER_B == 0) {
+                        umma_commit(b_empty + 8 * bs, on);
+                        if (++bs == C::BST) {
+                            bs = 0;
+                            bp ^= 1;
+                        }
+                    }
+                }
+                if (!ok) break;
+                umma_commit(a_empty + 8 * as, on);
+                as ^= 1;
+                if (as == 0) ap ^= 1;
+            }
+    } else if (warp < C::EW0) {
+        // ---------------------------------------------------------------- quants -> f16 in TMEM: lane = row of W.  A chunk of 128 k is announced
+        // when the next one's quants have been read: its stores take some 200 cycles to arrive.
+        const int q = warp & 3, row = q * 32 + lane, sw = ((row & 1) << 2) | ((row >> 1) & 3);
+        const uint32_t src0 = r_at + (uint32_t)(row >> 4) * C::FILL + (uint32_t)(row & 15) * C::SEG;
+        const uint32_t dst0 = tmem + ((uint32_t)(q * 32) << 16) + C::A_COL;
+        uint32_t rs = 0, rp = 0, as = 0, ap = 1;
+        bool stored = false;                                    // a chunk in the other buffer waits to be announced
+        auto announce = [&] {
+            tmem_wait_st();
+            tc_fence_before();
+            pg_mbar_arrive_warp(a_full + 8 * (as ^ 1), lane);
+        };
+        for (int u = blockIdx.x; ok && u < total; u += gridDim.x)
+            for (int s = s_first(u), end = s_end(u); ok && s < end; s++) {
+                ok = wait(r_full + 8 * rs, rp);
+                for (int h = 0; ok && h < 2; h++) {
+                    const uint32_t src = src0 + rs * C::RAW;
+                    uint4 w[4];                                 // Q4_0: word t of four blocks; Q8_0: bytes 8 t .. of two
+                    auto read = [&](int g) {
+#pragma unroll
+                        for (int t = 0; t < 4; t++) w[t] = pg_lds128(src + (uint32_t)(((g * 4 + t) ^ sw) * 16));
+                    };
+                    read(TYPE == PG_GGUF_Q4_0 ? h : 2 * h);
+                    if (stored) announce();
+                    if (!(ok = wait(a_empty + 8 * as, ap))) break;
+                    tc_fence_after();
+#pragma unroll
+                    for (int p = 0; p < 2; p++) {               // blocks 2 p and 2 p + 1
+                        if (TYPE != PG_GGUF_Q4_0 && p == 1) read(2 * h + 1);
+                        uint32_t v[32];
+#pragma unroll
+                        for (int t = 0; t < 4; t++)
+#pragma unroll
+                            for (int b = 0; b < 2; b++) {
+                                uint32_t f[4];
+                                if constexpr (TYPE == PG_GGUF_Q4_0)
+                                    gguf_nibbles_f16(p ? (b ? w[t].w : w[t].z) : (b ? w[t].y : w[t].x), f);
+                                else
+                                    gguf_bytes_f16(b ? w[t].z : w[t].x, b ? w[t].w : w[t].y, f);
+#pragma unroll
+                                for (int e = 0; e < 4; e++) v[16 * b + 4 * t + e] = f[e];
+                            }
+                        tmem_st32(dst0 + as * 64 + p * 32, v);
+                    }
+                    stored = true;
+                    if (h == 1) pg_mbar_arrive_warp(r_empty + 8 * rs, lane);
+                    as ^= 1;
+                    if (as == 0) ap ^= 1;
+                }
+                if (++rs == C::RST) {
+                    rs = 0;
+                    rp ^= 1;
+                }
+            }
+        if (ok && stored) announce();
+    } else {
+        // ---------------------------------------------------------------- sums and outputs: lane = row of W.  With 64 rows of x, two of a quarter's
+        // four warps take a group of accumulators, half of the rows each, the other two the next one; above, all four take every group
+        const int q = warp & 3, e = (warp - C::EW0) >> 2, row = q * 32 + lane;
+        const int part = C::SETS == 2 ? e & 1 : e, set = C::SETS == 2 ? e >> 1 : 0;
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + part * C::PART;
+        const uint32_t scales = r_at + (uint32_t)(row >> 4) * C::FILL + 16 * C::SEG + (uint32_t)(row & 15) * 16;
+        const uint32_t meet = c_at + (uint32_t)(part * C::PART * GT_N + row) * 4;
+        asm volatile("griddepcontrol.wait;" ::: "memory");     // y may still be read by the predecessor
+        uint32_t rs = 0, ts = set, tp = 0, cp = 0;
+        for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+            const int tile = u / sp;
+            float sum[C::PART];
+#pragma unroll
+            for (int j = 0; j < C::PART; j++) sum[j] = 0.0f;
+            for (int s = s_first(u), end = s_end(u); ok && s < end; s++) {
+#pragma unroll
+                for (int g = 0; g < 8 / C::GB; g++) {
+                    if (C::SETS == 2 && (g & 1) != set) continue;
+                    if (!(ok = wait(t_full + 8 * ts, tp))) break;
+                    tc_fence_after();
+                    // (the slice's scales are there too: the products' quants came with them)
+                    const uint32_t sc = scales + rs * C::RAW + g * C::GB * 2;
+                    float d[C::GB];
+#pragma unroll
+                    for (int b = 0; b < C::GB; b++) {
+                        uint16_t bits;
+                        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(bits) : "r"(sc + b * 2));
+                        d[b] = __half2float(__ushort_as_half(bits));
+                    }
+                    constexpr int P = C::PART <= 32 ? C::PART : 16;   // columns at a time
+#pragma unroll
+                    for (int b = 0; b < C::GB; b++)
+#pragma unroll
+                        for (int c = 0; c < C::PART; c += P) {
+                            constexpr int LAST = C::PART % P ? C::PART % P : P;
+                            const bool last = c + P >= C::PART;
+                            uint32_t v[P];
+                            if (last)
+                                gt_ask<LAST>(taddr + (ts * C::GB + b) * MT + c, v);
+                            else
+                                gt_ask<P>(taddr + (ts * C::GB + b) * MT + c, v);
+                            tmem_wait_ld();
+                            if (last && b == C::GB - 1) {
+                                tc_fence_before();
+                                pg_mbar_arrive_warp(t_empty + 8 * ts, lane);
+                                if (g >= 8 / C::GB - C::SETS) pg_mbar_arrive_warp(r_empty + 8 * rs, lane);   // (this warp's last group of the slice)
+                            }
+#pragma unroll
+                            for (int j = 0; j < P; j++)
+                                if (!last || j < LAST) sum[c + j] = fmaf(d[b], __uint_as_float(v[j]), sum[c + j]);
+                        }
+                    ts += C::SETS;
+                    if (ts >= C::NBUF) {
+                        ts -= C::NBUF;
+                        tp ^= 1;
+                    }
+                }
+                if (++rs == C::RST) rs = 0;
+            }
+            if (!ok) break;
+            if constexpr (C::SETS == 2) {
+                // the sets' sums meet in the first one
+                if (set == 1) {
+                    if (!(ok = wait(c_free + 8 * q, cp + 1))) break;
+#pragma unroll
+                    for (int j = 0; j < C::PART; j++) asm volatile("st.shared.f32 [%0], %1;" ::"r"(meet + j * GT_N * 4), "f"(sum[j]) : "memory");
+                    pg_mbar_arrive_warp(c_full + 8 * q, lane);
+                    cp ^= 1;
+                    continue;
+                }
+                if (!(ok = wait(c_full + 8 * q, cp))) break;
+#pragma unroll
+                for (int j = 0; j < C::PART; j++) {
+                    float f;
+                    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(meet + j * GT_N * 4));
+                    sum[j] += f;
+                }
+                pg_mbar_arrive_warp(c_free + 8 * q, lane);
+                cp ^= 1;
+            }
+            if (sp > 1) {
+                float *slab = kp.slabs + ((int64_t)u * MT + part * C::PART) * GT_N + row;
+#pragma unroll
+                for (int j = 0; j < C::PART; j++) __stcg(slab + j * GT_N, sum[j]);
+                unsigned int *ticket = kp.tickets + tile * 16 + part * 4 + q;
+                __threadfence();
+                __syncwarp();
+                const unsigned int before = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(ticket, 1u) : 0u, 0);
+                if (before != (unsigned)(sp - 1)) continue;
+                __threadfence();
+                if (lane == 0) *ticket = 0;
+                slab = kp.slabs + ((int64_t)tile * sp * MT + part * C::PART) * GT_N + row;
+#pragma unroll
+                for (int j = 0; j < C::PART; j++) sum[j] = __ldcg(slab + j * GT_N);
+                for (int p = 1; p < sp; p++) {
+                    slab += MT * GT_N;
+#pragma unroll
+                    for (int j = 0; j < C::PART; j++) sum[j] += __ldcg(slab + j * GT_N);
+                }
+            }
+            const int64_t n = (int64_t)(tile / tiles_m) * GT_N + row;
+            const int m0 = (tile % tiles_m) * MT + part * C::PART;
+            if (n < N) {
+                float *dst = y + (int64_t)m0 * N + n;
+#pragma unroll
+                for (int j = 0; j < C::PART; j++)
+                    if (m0 + j < M) dst[j * N] = sum[j] * __ldcg(us + m0 + j);
+            }
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 2) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
 // ---------------------------------------------------------------- host side ----
 int64_t gt_row_bytes(int64_t k) { return 4 * k + 4; }    // two planes and 2^-s
 
@@ -474,12 +848,38 @@ int32_t gt_launch(pg_ctx *ctx, const pg_gguf_weight *w, const void *planes, cons
                       (int)(w->k / 256), (int)m, us, y, kp, ctx->d_status, ctx->wait_limit_ns);
 }
 
+template <int TYPE, int MT>
+int32_t gw_launch(pg_ctx *ctx, const pg_gguf_weight *w, const void *planes, const float *us, int64_t m, float *y, GtParts kp)
+{
+    using C = GwCfg<TYPE, MT>;
+    CUtensorMap tx, tw;
+    // x: 64 k of the rows of both planes, a stage's blocks of 64 k behind each other
+    const cuuint64_t xd[4] = {64, (cuuint64_t)m, 2, (cuuint64_t)w->k / 64}, xs[3] = {(cuuint64_t)w->k * 2, (cuuint64_t)(w->k * m) * 2, 128};
+    const cuuint32_t xb[4] = {64, MT, 2, C::BK64};
+    int32_t rc = pg_encode_bf16(&tx, planes, 4, xd, xs, xb);   // (f16: the copies only move it)
+    // W: the fills of a slice of eight tiles of 16 rows
+    const cuuint64_t nslices = (cuuint64_t)w->k / 256, tiles = (cuuint64_t)(w->n + 15) / 16;
+    const cuuint64_t wd[4] = {64, C::FILL / 256, nslices, tiles}, ws[3] = {256, C::FILL, nslices * C::FILL};
+    const cuuint32_t wb[4] = {64, C::FILL / 256, 1, 8};
+    if (rc == PG_OK) rc = pg_encode_map(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, w->d_qs, 4, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_NONE);
+    if (rc != PG_OK) return rc;
+    auto kern = gguf_tc_wide_kernel<TYPE, MT>;
+    static std::atomic<uint64_t> smem_set{0};
+    PG_CUDA(pg_max_smem_once(kern, (int)C::SMEM, ctx->device, smem_set));
+    const int64_t units = ((m + MT - 1) / MT) * ((w->n + GT_N - 1) / GT_N) * kp.parts;
+    kp.tickets = reinterpret_cast<unsigned int *>(ctx->splitk);
+    kp.slabs = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(ctx->splitk) + GT_TICKET_BYTES);
+    return launch_pdl(ctx, kern, dim3((unsigned)std::min<int64_t>(units, ctx->sm_count)), dim3(C::THREADS), C::SMEM, tx, tw, w->n, (int)nslices, (int)m, us,
+                      y, kp, ctx->d_status, ctx->wait_limit_ns);
+}
+
 // rows of slabs that a context keeps for every product
 int64_t gt_slab_rows(const pg_ctx *ctx) { return (int64_t)ctx->sm_count * 3 * 64; }
 
 // Rows per tile and parts of K, by the shape alone (a portion of a call has those of the whole call): the fewest cycles by count --
-// slices of the busiest CTA and what a tile costs at its end, more where slabs meet.  Measured at N 14336, K 4096, a block of 32 k takes
-// 350 / 430 / 570 / 800 / 930 cycles with 16 / 32 / 64 / 128 / 160 rows.
+// slices of the busiest CTA and what a tile costs at its end, more where slabs meet.  Measured, N 14336, K 4096: a block of 32 k takes 350 / 430
+// cycles with 16 / 32 rows, 440 / 575 / 685 with 64 / 128 / 160; N 4096, K 4096, four parts of K: what the parts cost is 10000 / 14000 / 20000 cycles
+// with 64 / 128 / 160 rows.
 GtParts gt_plan(const pg_ctx *ctx, const pg_gguf_weight *w, int64_t m, int *mt)
 {
     const int64_t nslices = w->k / 256, tiles_n = (w->n + GT_N - 1) / GT_N;
@@ -494,9 +894,11 @@ GtParts gt_plan(const pg_ctx *ctx, const pg_gguf_weight *w, int64_t m, int *mt)
         for (int64_t parts = 1; parts <= std::min<int64_t>(16, nslices); parts++) {
             const int64_t slices = (nslices + parts - 1) / parts;
             if ((nslices + slices - 1) / slices != parts) continue;
-            if (parts > 1 && (tiles * parts * cand > gt_slab_rows(ctx) || tiles * 8 * (int64_t)sizeof(int) > (int64_t)GT_TICKET_BYTES)) break;
+            if (parts > 1 && (tiles * parts * cand > gt_slab_rows(ctx) || tiles * 16 * (int64_t)sizeof(int) > (int64_t)GT_TICKET_BYTES)) break;
             const int64_t rounds = (tiles * parts + ctx->sm_count - 1) / ctx->sm_count;
-            const double cost = rounds * (slices * 8.0 * (280.0 + cand * 4.0) + 1500.0 + cand * 8.0 + (parts > 1 ? 2500.0 + cand * parts * 4.0 : 0.0));
+            const double block = cand < 64 ? 280.0 + cand * 4.0 : 300.0 + cand * 2.3;
+            const double meet = parts == 1 ? 0.0 : cand < 64 ? 2500.0 + cand * parts * 4.0 : 4000.0 + cand * parts * 25.0;
+            const double cost = rounds * (slices * 8.0 * block + 1500.0 + cand * 8.0 + meet);
             if (best == 0 || cost < best) {
                 best = cost;
                 *mt = cand;
@@ -511,9 +913,9 @@ GtParts gt_plan(const pg_ctx *ctx, const pg_gguf_weight *w, int64_t m, int *mt)
 template <int TYPE>
 int32_t gt_run(pg_ctx *ctx, const pg_gguf_weight *w, const void *planes, const float *us, int64_t m, float *y, int mt, const GtParts &kp)
 {
-    if (mt == 160) return gt_launch<TYPE, 160>(ctx, w, planes, us, m, y, kp);
-    if (mt == 128) return gt_launch<TYPE, 128>(ctx, w, planes, us, m, y, kp);
-    if (mt == 64) return gt_launch<TYPE, 64>(ctx, w, planes, us, m, y, kp);
+    if (mt == 160) return gw_launch<TYPE, 160>(ctx, w, planes, us, m, y, kp);
+    if (mt == 128) return gw_launch<TYPE, 128>(ctx, w, planes, us, m, y, kp);
+    if (mt == 64) return gw_launch<TYPE, 64>(ctx, w, planes, us, m, y, kp);
     if (mt == 32) return gt_launch<TYPE, 32>(ctx, w, planes, us, m, y, kp);
     return gt_launch<TYPE, 16>(ctx, w, planes, us, m, y, kp);
 }

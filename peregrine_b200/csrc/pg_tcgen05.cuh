@@ -138,7 +138,7 @@ typedef CUresult (*PgEncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32
 
 // the box's inner extent is one 128-byte swizzle span; reads past the edge give 0
 inline int32_t pg_encode_map(CUtensorMap *map, CUtensorMapDataType type, const void *ptr, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
-                             const cuuint32_t *box)
+                             const cuuint32_t *box, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B)
 {
     static PgEncodeTiledFn enc = nullptr;
     if (!enc) {
@@ -150,7 +150,7 @@ inline int32_t pg_encode_map(CUtensorMap *map, CUtensorMapDataType type, const v
     if (!enc) PG_FAIL(PG_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     const CUresult r = enc(map, type, (cuuint32_t)rank, const_cast<void *>(ptr), dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) PG_FAIL(PG_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
     return PG_OK;
 }

@@ -192,6 +192,26 @@ def test_matmul_gguf_many_rows(pg, gpu, oracle_mt, kind, n, k):
 
 
 @pytest.mark.parametrize("kind", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("m", [40, 64, 100, 128, 150, 161])
+def test_matmul_gguf_several_tiles_to_a_cta(pg, gpu, oracle_mt, kind, m):
+    """More tiles than SMs, the last of them ragged: each CTA goes through several, with tiles of 64, 128 and 160 rows.  Bound as above."""
+    n, k = 20100, 768
+    g = rng(m)
+    raw = oracle_mt.encode(kind, normal(g, (n, k), 0.02))
+    w64 = oracle_mt.dequant(kind, raw, n * k).reshape(n, k).astype(np.float64)
+    w = pg.gguf.GgufWeight(kind, raw, n, k, gpu)
+    x = normal(g, (m, k))
+    x64 = np.abs(x).astype(np.float64)
+    bound = x64 @ np.abs(w64).T * (2.0 ** -22 + 4 * 2.0 ** -23 + (k // 32 + 18) * 2.0 ** -24) + x64.max(1, keepdims=True) * 2.0 ** -39 * np.abs(w64).sum(1)
+    want = x.astype(np.float64) @ w64.T
+    got = w.matmul(x, m)
+    assert (np.abs(got - want) <= bound).all()
+    assert np.array_equal(w.matmul(x, m), got)
+    assert gpu.device_status() == 0
+    w.free()
+
+
+@pytest.mark.parametrize("kind", ["q4_0", "q8_0"])
 @pytest.mark.parametrize("m,n,k,digits", [(3, 300, 12544, 39), (4, 260, 8448, 39), (5, 129, 4352, 39), (7, 200, 2304, 39), (8, 5000, 6400, 39), (6, 131, 16640, 39),
                                           (2, 300, 12544, 22), (5, 200, 2304, 22), (8, 5000, 4096, 22)])
 def test_matmul_gguf_few_rows_long_k(pg, gpu, oracle_mt, kind, m, n, k, digits):
