@@ -7,7 +7,13 @@
 //   * products with fewer tiles than SMs: K is divided over `sp` CTAs.  Each writes its raw sums to a slab; the last warp of a
 //     32-row band to finish (a ticket per band) adds the slabs in a fixed order and writes the outputs.  Nobody waits;
 //   * routed products: an A tile of 128 rows belongs to one expert, whose weights start at row expert * N of the
-//     stacked [experts * N][K] matrix.  Number and experts of the tiles are read on the device.
+//     stacked [experts * N][K] matrix.  Number and experts of the tiles are read on the device;
+//   * pairs of CTAs (CG = 2) with 256 x 256 tiles: each stages its 128 rows of a and its half of W's, and the leader issues products over
+//     both (tcgen05.mma.cta_group::2).  Sums are those of one CTA, bit for bit.
+//
+// What bounds it: alone, shared memory -- a block of 64 k of a 128 x 256 tile brings 48 KB and its products read 48 KB, 750 cycles for 512 of
+// products; a pair's CTA takes 32 KB for the same products.  Back to back, us, one CTA / pairs: N 28672, K 4096, 200 / 512 / 2048 / 4096 rows 60 /
+// 106 / 361 / 697 against 53 / 93 / 314 / 590; K 14336, N 4096, 777 / 4096 rows 105 / 380 against 81 / 335 (then under the power cap).
 //
 // Every mbarrier wait is bounded (pg_async.cuh).
 #include <algorithm>
@@ -25,16 +31,25 @@ constexpr int BKB = BK * 2;
 constexpr int UMMA_KB = 32;            // bytes of K per instruction
 constexpr int TC_THREADS = 192;
 
-template <int BN>
+// CG = 2: a pair of CTAs has 256 rows of a, 128 each, and each stages half of the BN columns
+template <int BN, int CG>
 struct Cfg {
     static constexpr int STAGE_A = BM * BKB;
-    static constexpr int STAGE_B = BN * BKB;
+    static constexpr int STAGE_B = BN / CG * BKB;
     static constexpr int STAGE = STAGE_A + STAGE_B;
     static constexpr int ROOM = 232448 - (1024 + 256 + 4 * PG_EPI_WARP_BYTES);
     static constexpr int STAGES = ROOM / STAGE > 10 ? 10 : ROOM / STAGE;
     static constexpr int TMEM_COLS = (2 * BN < 32) ? 32 : 2 * BN;
     static constexpr size_t SMEM = (size_t)STAGES * STAGE + 1024 + 256 + 4 * PG_EPI_WARP_BYTES;
 };
+
+// (with one CTA to a tile the plain form is the faster one: K 14336, N 4096, 400 rows 108 us against 127; with pairs it is the other way round)
+template <int CG>
+__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int32_t *status, unsigned long long limit_ns)
+{
+    if constexpr (CG == 1) return __all_sync(0xffffffffu, pg_mbar_wait(bar, parity, abort_flag, status, limit_ns));
+    return pg_mbar_wait_warp(bar, parity, abort_flag, status, limit_ns);
+}
 
 // How K is divided: parts of `blocks` 64-element blocks; slab of (unit, quarter): [BN][32 rows]
 struct KParts {
@@ -83,12 +98,12 @@ __device__ __forceinline__ void store_row(TY *y, int64_t ldy, int row, int n0, i
     }
 }
 
-template <int BN, int ACT, typename TY>
+template <int BN, int CG, int ACT, typename TY>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, int M, int N, int K, float limit,
                      TY *__restrict__ y, int64_t ldy, const PgRouted rt, const KParts kp, int32_t *status, unsigned long long limit_ns)
 {
-    using C = Cfg<BN>;
+    using C = Cfg<BN, CG>;
     constexpr int STAGES = C::STAGES;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ uint8_t smem_raw[];
@@ -102,7 +117,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const uint32_t bar_tempty = bar_tfull + 16;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = CG == 2 ? (int)pg_cluster_rank() : 0;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -111,24 +126,23 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         }
         for (int i = 0; i < 2; i++) {
             pg_mbar_init(bar_tfull + 8 * i, 1);
-            pg_mbar_init(bar_tempty + 8 * i, 4);   // one arrival per epilogue warp
+            pg_mbar_init(bar_tempty + 8 * i, 4 * CG);   // one arrival per epilogue warp
         }
         *abort_flag = 0;
         pg_mbar_fence();
     }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pg_smem(tmem_slot)), "r"(C::TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+    __syncwarp();
+    if (warp == 1) tmem_alloc<CG>(pg_smem(tmem_slot), C::TMEM_COLS);
     tc_fence_before();
-    __syncthreads();
+    pg_group_sync<CG>();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const bool routed = rt.blocks != nullptr;
     if (routed) asm volatile("griddepcontrol.wait;" ::: "memory");   // the list of tiles comes from the preceding kernels
-    const int tiles_m = routed ? __ldcg(rt.blocks) : (M + BM - 1) / BM;
+    const int tiles_m = routed ? __ldcg(rt.blocks) : (M + CG * BM - 1) / (CG * BM);   // (routed only with CG = 1)
     const int tiles_n = (N + BN - 1) / BN;
     const int sp = kp.parts, total = tiles_m * tiles_n * sp;   // unit u: part u % sp of tile u / sp
+    const int unit0 = blockIdx.x / CG, units = gridDim.x / CG;
     const int kblocks = K / BK;
     auto k_first = [&](int u) { return (u % sp) * kp.blocks; };
     auto k_end = [&](int u) { return min(kblocks, (u % sp + 1) * kp.blocks); };
@@ -139,23 +153,24 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         if (lane == 0) {
             uint32_t stage = 0, phase = 0;
             bool ok = true;
+            const uint32_t full_l = pg_leader<CG>(bar_full);
             // without a route the weight tiles of the first stages are requested before the predecessor has finished
             int early = 0;
             if (!routed) {
-                if ((int)blockIdx.x < total) {
-                    const int n0 = ((int)blockIdx.x / sp / tiles_m) * BN, first = k_first(blockIdx.x);
-                    early = min(k_end(blockIdx.x) - first, STAGES);
+                if (unit0 < total) {
+                    const int n0 = (unit0 / sp / tiles_m) * BN + rank * (BN / CG), first = k_first(unit0);
+                    early = min(k_end(unit0) - first, STAGES);
                     for (int i = 0; i < early; i++) {
-                        pg_mbar_expect(bar_full + 8 * i, C::STAGE);
-                        tma_load_2d(base + i * C::STAGE + C::STAGE_A, &tmap_b, bar_full + 8 * i, (first + i) * BK, n0);
+                        if (rank == 0) pg_mbar_expect(bar_full + 8 * i, CG * C::STAGE);
+                        tma_load_2d_to<CG>(base + i * C::STAGE + C::STAGE_A, &tmap_b, full_l + 8 * i, (first + i) * BK, n0);
                     }
                 }
                 asm volatile("griddepcontrol.wait;" ::: "memory");
             }
-            for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+            for (int u = unit0; ok && u < total; u += units) {
                 const int tile = u / sp;
-                const int m0 = (tile % tiles_m) * BM;
-                const int n0 = (tile / tiles_m) * BN;
+                const int m0 = (tile % tiles_m * CG + rank) * BM;
+                const int n0 = (tile / tiles_m) * BN + rank * (BN / CG);
                 const int b0 = routed ? __ldcg(rt.block_expert + tile % tiles_m) * N + n0 : n0;
                 for (int kb = k_first(u), end = k_end(u); kb < end; kb++) {
                     if (!(ok = pg_mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, status, limit_ns))) break;
@@ -163,10 +178,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                     if (early > 0) {
                         early--;                            // announced and half filled above
                     } else {
-                        pg_mbar_expect(bar_full + 8 * stage, C::STAGE);
-                        tma_load_2d(sa + C::STAGE_A, &tmap_b, bar_full + 8 * stage, kb * BK, b0);
+                        if (rank == 0) pg_mbar_expect(bar_full + 8 * stage, CG * C::STAGE);
+                        tma_load_2d_to<CG>(sa + C::STAGE_A, &tmap_b, full_l + 8 * stage, kb * BK, b0);
                     }
-                    tma_load_2d(sa, &tmap_a, bar_full + 8 * stage, kb * BK, m0);
+                    tma_load_2d_to<CG>(sa, &tmap_a, full_l + 8 * stage, kb * BK, m0);
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
@@ -182,32 +197,32 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer (the whole warp; one lane's products count)
-        {
+        if (rank == 0) {
             const uint32_t on = pg_elect();
-            constexpr uint32_t idesc = make_idesc(BM, BN);
+            constexpr uint32_t idesc = make_idesc(CG * BM, BN);
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
             bool ok = true;
-            for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
-                if (!(ok = __all_sync(0xffffffffu, pg_mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, status, limit_ns)))) break;
+            for (int u = unit0; ok && u < total; u += units) {
+                if (!(ok = tc_wait<CG>(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, status, limit_ns))) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
                 const int first = k_first(u), end = k_end(u);
                 for (int kb = first; kb < end; kb++) {
-                    if (!(ok = __all_sync(0xffffffffu, pg_mbar_wait(bar_full + 8 * stage, phase, abort_flag, status, limit_ns)))) break;
+                    if (!(ok = tc_wait<CG>(bar_full + 8 * stage, phase, abort_flag, status, limit_ns))) break;
                     tc_fence_after();
                     const uint32_t sa = base + stage * C::STAGE;
                     const uint64_t da = make_smem_desc(sa), db = make_smem_desc(sa + C::STAGE_A);
 #pragma unroll
                     for (int j = 0; j < BKB / UMMA_KB; j++)
-                        umma_f16(d_tmem, da + (uint64_t)(j * (UMMA_KB >> 4)), db + (uint64_t)(j * (UMMA_KB >> 4)), idesc, kb != first || j != 0 ? 1u : 0u, on);
-                    umma_commit(bar_empty + 8 * stage, on);   // stage reusable once these MMAs have read it
+                        umma_f16_of<CG>(d_tmem, da + (uint64_t)(j * (UMMA_KB >> 4)), db + (uint64_t)(j * (UMMA_KB >> 4)), idesc, kb != first || j != 0 ? 1u : 0u, on);
+                    umma_commit_to<CG>(bar_empty + 8 * stage, on);   // stage reusable once these MMAs have read it
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
                 if (!ok) break;
-                umma_commit(bar_tfull + 8 * acc, on);         // accumulator complete
+                umma_commit_to<CG>(bar_tfull + 8 * acc, on);         // accumulator complete
                 if (++acc == 2) {
                     acc = 0;
                     acc_phase ^= 1;
@@ -219,15 +234,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         const int q = warp & 3;                           // TMEM lane quarter this warp may read
         if (!routed) asm volatile("griddepcontrol.wait;" ::: "memory");   // y may still be read by the predecessor
         uint32_t acc = 0, acc_phase = 0;
+        const uint32_t tempty_l = pg_leader<CG>(bar_tempty);
         const bool vec_ok = ACT == PG_ACT_NONE && sizeof(TY) == 4 && ((N & 3) == 0) && ((ldy & 3) == 0) && (((uintptr_t)y & 15) == 0);
         bool ok = true;
-        for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+        for (int u = unit0; ok && u < total; u += units) {
             const int tile = u / sp;
-            const int m0 = (tile % tiles_m) * BM;
+            const int m0 = (tile % tiles_m * CG + rank) * BM;
             const int n0 = (tile / tiles_m) * BN;
-            ok = pg_mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, status, limit_ns);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
+            if (!(ok = tc_wait<CG>(bar_tfull + 8 * acc, acc_phase, abort_flag, status, limit_ns))) break;
             tc_fence_after();
             const int row_base = m0 + q * 32, row = row_base + lane;
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
@@ -253,8 +267,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 }
             }
             tc_fence_before();
-            __syncwarp();
-            if (lane == 0) pg_mbar_arrive(bar_tempty + 8 * acc);
+            pg_arrive_leader_warp<CG>(tempty_l + 8 * acc, lane);
             if (sp > 1 && row_base < rows) {
                 unsigned int *ticket = kp.tickets + tile * 4 + q;
                 __threadfence();
@@ -295,12 +308,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         }
     }
 
+    // (neither CTA of a pair may leave while the other can still touch its shared memory, barriers or TMEM)
     __syncwarp();
     tc_fence_before();
-    __syncthreads();
+    pg_group_sync<CG>();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::TMEM_COLS) : "memory");
+        tmem_dealloc<CG>(tmem_base, C::TMEM_COLS);
     }
 }
 
@@ -313,27 +327,28 @@ int32_t encode_kmajor(CUtensorMap *map, const void *ptr, int64_t rows, int64_t k
     return pg_encode_bf16(map, ptr, 2, dims, strides, box);
 }
 
-template <int BN, int ACT, typename TY>
+template <int BN, int CG, int ACT, typename TY>
 int32_t launch(pg_ctx *ctx, pg_linear *lin, const bf16 *a, int64_t lda, int64_t m, float limit, TY *y, int64_t ldy, const PgRouted &rt,
                KParts kp)
 {
-    using C = Cfg<BN>;
+    using C = Cfg<BN, CG>;
     CUtensorMap ta;
     int32_t rc = encode_kmajor(&ta, a, m, lin->k, lda, BM);
     if (rc) return rc;
-    const int at = BN == 128 || BN == 32 ? 0 : 1;
-    if (lin->tmap_rows[at] != BN) {
-        rc = encode_kmajor(reinterpret_cast<CUtensorMap *>(lin->tmap[at]), lin->w, lin->experts * lin->n, lin->k, lin->k, BN);
+    constexpr int BOX = BN / CG;
+    const int at = BOX == 128 || BOX == 32 ? 0 : 1;
+    if (lin->tmap_rows[at] != BOX) {
+        rc = encode_kmajor(reinterpret_cast<CUtensorMap *>(lin->tmap[at]), lin->w, lin->experts * lin->n, lin->k, lin->k, BOX);
         if (rc) return rc;
-        lin->tmap_rows[at] = BN;
+        lin->tmap_rows[at] = BOX;
     }
-    auto kern = linear_tc_kernel<BN, ACT, TY>;
+    auto kern = linear_tc_kernel<BN, CG, ACT, TY>;
     static std::atomic<uint64_t> smem_set{0};
     PG_CUDA(pg_max_smem_once(kern, (int)C::SMEM, ctx->device, smem_set));
-    const int64_t tiles = ((m + BM - 1) / BM) * ((lin->n + BN - 1) / BN) * kp.parts;
+    const int64_t tiles = ((m + CG * BM - 1) / (CG * BM)) * ((lin->n + BN - 1) / BN) * kp.parts;
     kp.tickets = reinterpret_cast<unsigned int *>(ctx->splitk);
     kp.slabs = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(ctx->splitk) + PG_LM_TICKET_BYTES);
-    return launch_pdl(ctx, kern, dim3((unsigned)std::min<int64_t>(tiles, ctx->sm_count)), dim3(TC_THREADS), C::SMEM, ta,
+    return launch_pdl_cluster(ctx, kern, dim3((unsigned)(std::min<int64_t>(tiles, ctx->sm_count / CG) * CG)), dim3(TC_THREADS), C::SMEM, CG, ta,
                       *reinterpret_cast<CUtensorMap *>(lin->tmap[at]), (int)m, (int)lin->n, (int)lin->k, limit, y, ldy, rt, kp, ctx->d_status,
                       ctx->wait_limit_ns);
 }
@@ -368,10 +383,17 @@ int32_t dispatch(pg_ctx *ctx, pg_linear *lin, const bf16 *a, int64_t lda, int64_
             if (rc != PG_OK) return rc;
         }
     }
-    if (bn == 256) return launch<256, ACT, TY>(ctx, lin, a, lda, m, limit, y, ldy, rt, kp);
-    if (bn == 128) return launch<128, ACT, TY>(ctx, lin, a, lda, m, limit, y, ldy, rt, kp);
-    if (bn == 64) return launch<64, ACT, TY>(ctx, lin, a, lda, m, limit, y, ldy, rt, kp);
-    return launch<32, ACT, TY>(ctx, lin, a, lda, m, limit, y, ldy, rt, kp);
+    if (rt.blocks == nullptr && kp.parts == 1 && bn >= 128) {
+        // Pairs of CTAs with 256 x 256 tiles, where the rounds of tiles do not cost more than they save.  A block of 64 k takes what shared
+        // memory takes for it, bytes in and bytes read by the products: 256 + 2 bn cycles, 512 in a pair (as long as its products).
+        auto rounds = [&](int64_t t, int64_t at_once) { return (t + at_once - 1) / at_once; };
+        const int64_t pairs = rounds(((m + 2 * BM - 1) / (2 * BM)) * ((lin->n + 255) / 256), ctx->sm_count / 2);
+        if (pairs * 540 < rounds(tiles(bn), ctx->sm_count) * (256 + 2 * bn)) return launch<256, 2, ACT, TY>(ctx, lin, a, lda, m, limit, y, ldy, rt, kp);
+    }
+    if (bn == 256) return launch<256, 1, ACT, TY>(ctx, lin, a, lda, m, limit, y, ldy, rt, kp);
+    if (bn == 128) return launch<128, 1, ACT, TY>(ctx, lin, a, lda, m, limit, y, ldy, rt, kp);
+    if (bn == 64) return launch<64, 1, ACT, TY>(ctx, lin, a, lda, m, limit, y, ldy, rt, kp);
+    return launch<32, 1, ACT, TY>(ctx, lin, a, lda, m, limit, y, ldy, rt, kp);
 }
 
 }  // namespace

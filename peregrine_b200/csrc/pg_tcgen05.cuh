@@ -71,6 +71,125 @@ __device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t on)
         "setp.ne.b32 q, %1, 0;\n\t"
         "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(on) : "memory");
 }
+// ---- one CTA (CG = 1), or a pair of CTAs in a cluster whose leader (rank 0) issues products over both (CG = 2) -------------------
+// In a pair each CTA stages its own rows of A and its half of B, and its TMEM receives the sums of its rows.  No load is multicast.
+__device__ __forceinline__ uint32_t pg_cluster_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+template <int CG>
+__device__ __forceinline__ uint32_t pg_leader(uint32_t addr)   // this offset in the leader's shared memory
+{
+    if constexpr (CG == 1) return addr;
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    return r;
+}
+// copies into this CTA's shared memory that complete on the leader's barrier
+template <int CG>
+__device__ __forceinline__ void tma_load_2d_to(uint32_t dst, const CUtensorMap *tmap, uint32_t leaders_bar, int x, int y)
+{
+    if constexpr (CG == 1)
+        tma_load_2d(dst, tmap, leaders_bar, x, y);
+    else
+        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+                     "l"(tmap), "r"(leaders_bar), "r"(x), "r"(y)
+                     : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void tma_load_3d_to(uint32_t dst, const CUtensorMap *tmap, uint32_t leaders_bar, int x, int y, int z)
+{
+    if constexpr (CG == 1)
+        tma_load_3d(dst, tmap, leaders_bar, x, y, z);
+    else
+        asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
+                     "l"(tmap), "r"(leaders_bar), "r"(x), "r"(y), "r"(z)
+                     : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void umma_f16_of(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t on)
+{
+    if constexpr (CG == 1)
+        umma_f16(d_tmem, desc_a, desc_b, idesc, accumulate, on);
+    else
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "setp.ne.b32 q, %5, 0;\n\t"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(on)
+            : "memory");
+}
+// A from TMEM, each CTA's rows from its own
+template <int CG>
+__device__ __forceinline__ void umma_f16_ta_of(uint32_t d_tmem, uint32_t a_tmem, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t on)
+{
+    if constexpr (CG == 1)
+        umma_f16_ta(d_tmem, a_tmem, desc_b, idesc, accumulate, on);
+    else
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "setp.ne.b32 q, %5, 0;\n\t"
+            "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+            ::"r"(d_tmem), "r"(a_tmem), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(on)
+            : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void umma_commit_to(uint32_t bar, uint32_t on)   // arrives on the barrier of this offset in every CTA of the group
+{
+    if constexpr (CG == 1) {
+        umma_commit(bar, on);
+    } else {
+        const uint16_t mask = 3;
+        asm volatile(
+            "{\n\t.reg .pred q;\n\t"
+            "setp.ne.b32 q, %2, 0;\n\t"
+            "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar), "h"(mask), "r"(on)
+            : "memory");
+    }
+}
+// lane 0 arrives for its warp on a barrier of the leader (without .release.cluster, which takes 320 cycles; what the barrier orders here
+// are TMEM accesses, by the tcgen05 fence in front)
+template <int CG>
+__device__ __forceinline__ void pg_arrive_leader_warp(uint32_t leaders_bar, int lane)
+{
+    if constexpr (CG == 1) {
+        pg_mbar_arrive_warp(leaders_bar, lane);
+    } else {
+        __syncwarp();
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}" ::"r"(leaders_bar), "r"(lane) : "memory");
+    }
+}
+template <int CG>
+__device__ __forceinline__ void pg_group_sync()
+{
+    if constexpr (CG == 1)
+        __syncthreads();
+    else
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <int CG>
+__device__ __forceinline__ void tmem_alloc(uint32_t slot, uint32_t cols)
+{
+    if constexpr (CG == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+}
+template <int CG>
+__device__ __forceinline__ void tmem_dealloc(uint32_t tmem, uint32_t cols)
+{
+    if constexpr (CG == 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+    else
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+}
 __device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, uint32_t (&v)[32])
 {
     asm volatile(
