@@ -14,9 +14,13 @@
 //     through them one after the other and keeps the sum so far in TMEM.  So a row's outputs are the same whatever rows are beside it,
 //     however a call is divided, and whatever workspace there is.
 //
-// What bounds it: from about 64 rows shared memory, where a block of 64 k brings 64 KB and its twelve products read 96 KB (1250 cycles at 128
-// bytes each, 768 of products; 1318 measured); the stream of W below.  Products of a prompt of 333 tokens, four dense layers: 2150 -> 1865 us with
-// eight warps of sums, two of products and one copy for the three planes (a copy costs its thread 230 ... 400 cycles).
+// From 64 rows on a pair of CTAs shares a tile's rows of a: each brings half of the planes and 128 rows of W of its own, which four more warps
+// put into TMEM, where the products of all three planes take them from.  With W in shared memory one CTA's block of 64 k brought 64 KB and its
+// products read 96 KB: 1250 cycles at 128 bytes each for 768 of products, 1318 measured; now 40 KB come in and some 64 KB are read.
+//
+// What bounds it: from about 64 rows the products and what is left of the ways through shared memory (1170 cycles a block); the stream of W
+// below.  us, N 28672, K 4096, 33 / 64 / 128 / 333 / 777 rows: 84 / 88 / 107 / 238 / 520 with one CTA and four warps of sums, 60 / 61 / 82 / 204 / 442 now; N 4096,
+// K 14336: 41 / 42 / 58 / 145 / 285 -> 36 / 37 / 53 / 128 / 250.
 // Every mbarrier wait is bounded (pg_async.cuh).
 #include <algorithm>
 
@@ -34,17 +38,23 @@ constexpr int64_t F_PLANES = 100 << 20, F_SLABS = 64 << 20;   // most bytes of p
 template <int MT>
 struct FCfg {
     static constexpr int STAGE_W = FN * FK * 2;
-    static constexpr int PLANE = MT * FK * 2;
+    static constexpr int CG = MT >= 64 ? 2 : 1;            // CTAs that share a tile's rows of a, each with 128 columns of y of its own
+    static constexpr int PLANE = MT / CG * FK * 2;         // a CTA's part of a plane
     static constexpr int STAGE = STAGE_W + 3 * PLANE;
-    static constexpr int ROOM = 232448 - (1024 + 256);
+    static constexpr int ROOM = 232448 - (1024 + 512);
     static constexpr int STAGES = ROOM / STAGE > 10 ? 10 : ROOM / STAGE;
     static constexpr int ACC = MT < 32 ? 32 : MT;          // TMEM columns of an accumulator
     static constexpr int COLS = 4 * ACC;                   // two accumulators, the sum so far, and up to a power of two
     static constexpr int MW = 2;                           // warps that issue products, a block of K in turn
     static constexpr int EW = MT >= 64 ? 2 : 1;            // warps of the epilogue per TMEM quarter
     static constexpr int PART = MT / EW;                   // rows of a per such warp
-    static constexpr int THREADS = (4 + 4 * EW) * 32;      // copies, products, a warp without work, epilogue
-    static constexpr size_t SMEM = (size_t)STAGES * STAGE + 1024 + 256;
+    // From 64 rows on the weights go from shared memory to TMEM (32 columns a block, two such buffers), and the products take them from there:
+    // three products read each piece of W, which is more than shared memory gives.
+    static constexpr bool TA = CG == 2;
+    static constexpr int A_COL = 3 * ACC;
+    static constexpr int EW0 = TA ? 8 : 4;                 // first warp of the epilogue; copies, products, a warp without work, W to TMEM
+    static constexpr int THREADS = (EW0 + 4 * EW) * 32;
+    static constexpr size_t SMEM = (size_t)STAGES * STAGE + 1024 + 512;
 };
 
 struct FParts {
@@ -112,7 +122,7 @@ __global__ void __launch_bounds__(FCfg<MT>::THREADS, 1)
                       float *__restrict__ y, int64_t ldy, const PgRouted rt, int block0, const FParts kp, int32_t *status, unsigned long long limit_ns)
 {
     using C = FCfg<MT>;
-    constexpr int STAGES = C::STAGES;
+    constexpr int STAGES = C::STAGES, CG = C::CG;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = pg_smem(smem_raw);
@@ -122,35 +132,37 @@ __global__ void __launch_bounds__(FCfg<MT>::THREADS, 1)
     const uint32_t bar_empty = bar_full + 8 * STAGES;
     const uint32_t bar_tfull = bar_empty + 8 * STAGES;
     const uint32_t bar_tempty = bar_tfull + 16;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
+    const uint32_t bar_a = bar_tempty + 16, bar_afree = bar_a + 16, bar_w = bar_afree + 16;   // TMEM's buffers of W; this CTA's own tiles of W
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * STAGES + 8);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = CG == 2 ? (int)pg_cluster_rank() : 0;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
             pg_mbar_init(bar_full + 8 * s, 1);
             pg_mbar_init(bar_empty + 8 * s, 1);
+            pg_mbar_init(bar_w + 8 * s, 1);
         }
         for (int i = 0; i < 2; i++) {
             pg_mbar_init(bar_tfull + 8 * i, 1);
-            pg_mbar_init(bar_tempty + 8 * i, 4 * C::EW);   // one arrival per epilogue warp
+            pg_mbar_init(bar_tempty + 8 * i, 4 * C::EW * CG);   // one arrival per epilogue warp
+            pg_mbar_init(bar_a + 8 * i, 4 * CG);
+            pg_mbar_init(bar_afree + 8 * i, 1);
         }
         *abort_flag = 0;
         pg_mbar_fence();
     }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(pg_smem(tmem_slot)), "r"(C::COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+    __syncwarp();
+    if (warp == 1) tmem_alloc<CG>(pg_smem(tmem_slot), C::COLS);
     tc_fence_before();
-    __syncthreads();
+    pg_group_sync<CG>();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const bool routed = rt.blocks != nullptr;
     if (routed) asm volatile("griddepcontrol.wait;" ::: "memory");   // the list of tiles comes from the preceding kernels
     constexpr int PER_BLOCK = PG_ROUTE_BLOCK / MT < 1 ? 1 : PG_ROUTE_BLOCK / MT;
     const int tiles_m = routed ? max(0, min(__ldcg(rt.blocks) - block0, M / PG_ROUTE_BLOCK)) * PER_BLOCK : (M + MT - 1) / MT;
-    const int tiles_n = (N + FN - 1) / FN;
+    const int tiles_n = (N + CG * FN - 1) / (CG * FN), unit0 = blockIdx.x / CG, units = gridDim.x / CG;
     const int sp = kp.runs, total = tiles_m * tiles_n * sp;    // unit u: run u % sp of tile u / sp
     const int kblocks = K / FK, per = kp.run * kp.blocks;
     auto k_first = [&](int u) { return (u % sp) * per; };
@@ -161,33 +173,40 @@ __global__ void __launch_bounds__(FCfg<MT>::THREADS, 1)
         if (lane == 0) {
             uint32_t stage = 0, phase = 0;
             bool ok = true;
+            const uint32_t full_l = pg_leader<CG>(bar_full);
+            // a tile of W, and what the stage's barrier counts: where W goes on to TMEM, W has a barrier of its own in each CTA
+            auto ask_w = [&](int stage, int kb, int row) {
+                if (C::TA) {
+                    pg_mbar_expect(bar_w + 8 * stage, C::STAGE_W);
+                    tma_load_2d(base + stage * C::STAGE, &tmap_w, bar_w + 8 * stage, kb * FK, row);
+                    if (rank == 0) pg_mbar_expect(bar_full + 8 * stage, CG * 3 * C::PLANE);
+                } else {
+                    pg_mbar_expect(bar_full + 8 * stage, C::STAGE);
+                    tma_load_2d(base + stage * C::STAGE, &tmap_w, bar_full + 8 * stage, kb * FK, row);
+                }
+            };
             // without a route the weight tiles of the first stages are requested before the predecessor has finished
             int early = 0;
             if (!routed) {
-                if ((int)blockIdx.x < total) {
-                    const int n0 = ((int)blockIdx.x / sp / tiles_m) * FN, first = k_first(blockIdx.x);
-                    early = min(k_end(blockIdx.x) - first, STAGES);
-                    for (int i = 0; i < early; i++) {
-                        pg_mbar_expect(bar_full + 8 * i, C::STAGE);
-                        tma_load_2d(base + i * C::STAGE, &tmap_w, bar_full + 8 * i, (first + i) * FK, n0);
-                    }
+                if (unit0 < total) {
+                    const int n0 = (unit0 / sp / tiles_m * CG + rank) * FN, first = k_first(unit0);
+                    early = min(k_end(unit0) - first, STAGES);
+                    for (int i = 0; i < early; i++) ask_w(i, first + i, n0);
                 }
                 asm volatile("griddepcontrol.wait;" ::: "memory");
             }
-            for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+            for (int u = unit0; ok && u < total; u += units) {
                 const int tile = u / sp;
-                const int m0 = (tile % tiles_m) * MT, n0 = (tile / tiles_m) * FN;
+                const int m0 = (tile % tiles_m) * MT, n0 = (tile / tiles_m * CG + rank) * FN;
                 const int w0 = routed ? __ldcg(rt.block_expert + block0 + m0 / PG_ROUTE_BLOCK) * N + n0 : n0;
                 for (int kb = k_first(u), end = k_end(u); kb < end; kb++) {
                     if (!(ok = pg_mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, status, limit_ns))) break;
                     const uint32_t at = base + stage * C::STAGE;
-                    if (early > 0) {
+                    if (early > 0)
                         early--;                            // announced and half filled above
-                    } else {
-                        pg_mbar_expect(bar_full + 8 * stage, C::STAGE);
-                        tma_load_2d(at, &tmap_w, bar_full + 8 * stage, kb * FK, w0);
-                    }
-                    tma_load_3d(at + C::STAGE_W, &tmap_a, bar_full + 8 * stage, kb * FK, m0, 0);   // all three planes
+                    else
+                        ask_w(stage, kb, w0);
+                    tma_load_3d_to<CG>(at + C::STAGE_W, &tmap_a, full_l + 8 * stage, kb * FK, m0 + rank * (MT / CG), 0);   // all three planes
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
@@ -205,40 +224,72 @@ __global__ void __launch_bounds__(FCfg<MT>::THREADS, 1)
         // ---------------------------------------------------------------- MMA issuers (the whole warp; one lane's products count): each has
         // every other block of K and one of the accumulators.  (An accumulator is waited for before a stage: the epilogue gives it back
         // in the order of the blocks, so that no stage is waited for whose use before last is still to be filled.)
-        if (warp <= C::MW) {
+        if (warp <= C::MW && rank == 0) {
             const uint32_t on = pg_elect();
-            constexpr uint32_t idesc = make_idesc(FN, MT);
+            constexpr uint32_t idesc = make_idesc(CG * FN, MT);
             uint32_t count = 0;
             bool ok = true;
-            for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+            for (int u = unit0; ok && u < total; u += units) {
                 for (int kb = k_first(u), end = k_end(u); kb < end; kb++, count++) {
                     const uint32_t acc = count & 1, stage = count % STAGES;
                     if ((int)acc != warp - 1) continue;
                     ok = pg_mbar_wait_warp(bar_tempty + 8 * acc, (count / 2 & 1) ^ 1, abort_flag, status, limit_ns);
                     if (!ok || !(ok = pg_mbar_wait_warp(bar_full + 8 * stage, count / STAGES & 1, abort_flag, status, limit_ns))) break;
+                    if (C::TA && !(ok = pg_mbar_wait_warp(bar_a + 8 * acc, count / 2 & 1, abort_flag, status, limit_ns))) break;
                     tc_fence_after();
                     const uint32_t at = base + stage * C::STAGE, d_tmem = tmem_base + acc * C::ACC;
                     const uint64_t dw = make_smem_desc(at), da = make_smem_desc(at + C::STAGE_W);
 #pragma unroll
                     for (int l = 2; l >= 0; l--)
 #pragma unroll
-                        for (int j = 0; j < FK / 16; j++)
-                            umma_f16(d_tmem, dw + (uint64_t)(j * 2), da + (uint64_t)(l * (C::PLANE >> 4) + j * 2), idesc, l != 2 || j != 0 ? 1u : 0u, on);
-                    umma_commit(bar_empty + 8 * stage, on);     // stage reusable once these products have read it
-                    umma_commit(bar_tfull + 8 * acc, on);
+                        for (int j = 0; j < FK / 16; j++) {
+                            const uint64_t dp = da + (uint64_t)(l * (C::PLANE >> 4) + j * 2);
+                            if (C::TA)
+                                umma_f16_ta_of<CG>(d_tmem, tmem_base + C::A_COL + acc * 32 + j * 8, dp, idesc, l != 2 || j != 0 ? 1u : 0u, on);
+                            else
+                                umma_f16(d_tmem, dw + (uint64_t)(j * 2), dp, idesc, l != 2 || j != 0 ? 1u : 0u, on);
+                        }
+                    if (C::TA) umma_commit_to<CG>(bar_afree + 8 * acc, on);
+                    umma_commit_to<CG>(bar_empty + 8 * stage, on);     // stage reusable once these products have read it
+                    umma_commit_to<CG>(bar_tfull + 8 * acc, on);
                 }
+            }
+        }
+    } else if (warp < C::EW0) {
+        // ---------------------------------------------------------------- W to TMEM: lane = row of W
+        const int row = (warp & 3) * 32 + lane;
+        const uint32_t dst = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + C::A_COL, a_l = pg_leader<CG>(bar_a);
+        uint32_t count = 0;
+        bool ok = true;
+        for (int u = unit0; ok && u < total; u += units) {
+            for (int kb = k_first(u), end = k_end(u); kb < end; kb++, count++) {
+                const uint32_t buf = count & 1, stage = count % STAGES, src = base + stage * C::STAGE + (uint32_t)row * 128;
+                if (!(ok = pg_mbar_wait_warp(bar_w + 8 * stage, count / STAGES & 1, abort_flag, status, limit_ns))) break;
+                uint32_t v[32];
+#pragma unroll
+                for (int p = 0; p < 8; p++) {
+                    const uint4 w = pg_lds128(src + (uint32_t)((p ^ (row & 7)) * 16));
+                    v[4 * p] = w.x, v[4 * p + 1] = w.y, v[4 * p + 2] = w.z, v[4 * p + 3] = w.w;
+                }
+                if (!(ok = pg_mbar_wait_warp(bar_afree + 8 * buf, (count / 2 & 1) ^ 1, abort_flag, status, limit_ns))) break;
+                tc_fence_after();
+                tmem_st32(dst + buf * 32, v);
+                tmem_wait_st();
+                tc_fence_before();
+                pg_arrive_leader_warp<CG>(a_l + 8 * buf, lane);
             }
         }
     } else {
         // ---------------------------------------------------------------- sums and outputs: lane = column of y
-        const int q = warp & 3, half = (warp - 4) >> 2;     // TMEM lane quarter this warp may read, its rows of a
+        const int q = warp & 3, half = (warp - C::EW0) >> 2;     // TMEM lane quarter this warp may read, its rows of a
         if (!routed) asm volatile("griddepcontrol.wait;" ::: "memory");   // y may still be read by the predecessor
         const int rows = routed ? tiles_m * MT : M;
+        const uint32_t tempty_l = pg_leader<CG>(bar_tempty);
         uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
-        for (int u = blockIdx.x; ok && u < total; u += gridDim.x) {
+        for (int u = unit0; ok && u < total; u += units) {
             const int tile = u / sp;
-            const int m0 = (tile % tiles_m) * MT + half * C::PART, n0 = (tile / tiles_m) * FN;
+            const int m0 = (tile % tiles_m) * MT + half * C::PART, n0 = (tile / tiles_m * CG + rank) * FN, mine_at = tile * CG + rank;
             const uint32_t lanes = tmem_base + ((uint32_t)(q * 32) << 16), so_far = lanes + 2 * C::ACC + half * C::PART;
             float sum[C::PART] = {};
             int part = (u % sp) * kp.run, next = k_first(u) + kp.blocks;   // the part under way, and the block behind it
@@ -255,7 +306,7 @@ __global__ void __launch_bounds__(FCfg<MT>::THREADS, 1)
                         if (c + j < C::PART) sum[c + j] += __uint_as_float(v[j]);
                 }
                 tc_fence_before();
-                pg_mbar_arrive_warp(bar_tempty + 8 * acc, lane);
+                pg_arrive_leader_warp<CG>(tempty_l + 8 * acc, lane);
                 if (++acc == 2) {
                     acc = 0;
                     acc_phase ^= 1;
@@ -263,7 +314,7 @@ __global__ void __launch_bounds__(FCfg<MT>::THREADS, 1)
                 if (kp.parts > 1 && (kb + 1 == next || kb + 1 == end)) {
                     // the end of a part: to its slab, or onto the sum of those in front of it
                     if (sp > 1) {
-                        float *slab = kp.slabs + (((int64_t)tile * kp.parts + part) * MT + half * C::PART) * FN + q * 32 + lane;
+                        float *slab = kp.slabs + (((int64_t)mine_at * kp.parts + part) * MT + half * C::PART) * FN + q * 32 + lane;
 #pragma unroll
                         for (int j = 0; j < C::PART; j++) __stcg(slab + j * FN, sum[j]);
                     } else {
@@ -299,7 +350,7 @@ __global__ void __launch_bounds__(FCfg<MT>::THREADS, 1)
             const int n = n0 + q * 32 + lane;
             bool mine = true;
             if (sp > 1) {
-                unsigned int *ticket = kp.tickets + (tile * C::EW + half) * 4 + q;
+                unsigned int *ticket = kp.tickets + (mine_at * C::EW + half) * 4 + q;
                 __threadfence();
                 __syncwarp();
                 const unsigned int before = __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(ticket, 1u) : 0u, 0);
@@ -308,7 +359,7 @@ __global__ void __launch_bounds__(FCfg<MT>::THREADS, 1)
                     // the last part of these columns to finish adds all parts up, in their order
                     __threadfence();
                     if (lane == 0) *ticket = 0;
-                    const float *slab = kp.slabs + ((int64_t)tile * kp.parts * MT + half * C::PART) * FN + q * 32 + lane;
+                    const float *slab = kp.slabs + ((int64_t)mine_at * kp.parts * MT + half * C::PART) * FN + q * 32 + lane;
 #pragma unroll
                     for (int j = 0; j < C::PART; j++) sum[j] = __ldcg(slab + j * FN);
                     for (int p = 1; p < kp.parts; p++) {
@@ -338,12 +389,13 @@ __global__ void __launch_bounds__(FCfg<MT>::THREADS, 1)
         }
     }
 
+    // (neither CTA of a pair may leave while the other can still touch its shared memory, barriers or TMEM)
     __syncwarp();
     tc_fence_before();
-    __syncthreads();
+    pg_group_sync<CG>();
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::COLS) : "memory");
+        tmem_dealloc<CG>(tmem_base, C::COLS);
     }
 }
 
@@ -358,20 +410,20 @@ int32_t launch(pg_ctx *ctx, const pg_linear *lin, const bf16 *planes, int64_t m,
     int32_t rc = pg_encode_bf16(&tw, lin->w, 2, wd, ws, wb);
     if (rc != PG_OK) return rc;
     const cuuint64_t ad[3] = {(cuuint64_t)lin->k, (cuuint64_t)m, 3}, as[2] = {(cuuint64_t)lin->k * 2, (cuuint64_t)(lin->k * m) * 2};
-    const cuuint32_t ab[3] = {FK, MT, 3};
+    const cuuint32_t ab[3] = {FK, MT / C::CG, 3};
     rc = pg_encode_bf16(&ta, planes, 3, ad, as, ab);
     if (rc != PG_OK) return rc;
     auto kern = linear_f32_kernel<MT, ACT>;
     static std::atomic<uint64_t> smem_set{0};
     PG_CUDA(pg_max_smem_once(kern, (int)C::SMEM, ctx->device, smem_set));
-    const int64_t units = ((m + MT - 1) / MT) * ((lin->n + FN - 1) / FN) * kp.runs;
+    const int64_t units = ((m + MT - 1) / MT) * ((lin->n + C::CG * FN - 1) / (C::CG * FN)) * kp.runs;
     kp.tickets = reinterpret_cast<unsigned int *>(ctx->splitk);
     kp.slabs = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(ctx->splitk) + PG_LM_TICKET_BYTES);
-    return launch_pdl(ctx, kern, dim3((unsigned)std::min<int64_t>(units, ctx->sm_count)), dim3(C::THREADS), C::SMEM, tw, ta, (int)m, (int)lin->n, (int)lin->k,
-                      limit, y, ldy, rt, block0, kp, ctx->d_status, ctx->wait_limit_ns);
+    return launch_pdl_cluster(ctx, kern, dim3((unsigned)(std::min<int64_t>(units, ctx->sm_count / C::CG) * C::CG)), dim3(C::THREADS), C::SMEM, C::CG, tw, ta, (int)m,
+                              (int)lin->n, (int)lin->k, limit, y, ldy, rt, block0, kp, ctx->d_status, ctx->wait_limit_ns);
 }
 
-// Cycles by count: blocks of the busiest CTA, which its copies bound (695 / 1004 / 1413 cycles with 16 / 64 / 128 rows), and what a tile
+// Cycles by count: blocks of the busiest CTA (695 / 1004 / 1413 cycles with 16 / 64 / 128 rows and one CTA to a tile; pairs take 0.8 of that), and what a tile
 // costs at its end, much more where parts meet.  K = N = 4096, four parts one after the other / two by two / all apart: 128 rows 50 / 42 / 32 us,
 // 333 rows 54 / 73 / 77, 1000 rows 97 / 140 / 179.
 double f32_cost(int64_t rounds, int64_t blocks, int rows, int64_t parts, bool slabs)
@@ -416,7 +468,7 @@ int32_t dispatch(pg_ctx *ctx, const pg_linear *lin, const bf16 *planes, int64_t 
         int64_t need = 0;
         double best = 0;
         for (int cand = full; cand >= std::min(full, 64); cand /= 2) {
-            const int64_t tiles = tiles_n * ((m + cand - 1) / cand);
+            const int64_t cg = cand >= 64 ? 2 : 1, tiles = (tiles_n + cg - 1) / cg * cg * ((m + cand - 1) / cand);   // (pairs have two each)
             for (int64_t run = kp.parts; run >= 1; run--) {
                 const int64_t runs = (kp.parts + run - 1) / run;
                 if (runs > 1 && (tiles * kp.parts * cand * slab > room || tiles * 8 * (int64_t)sizeof(int) > (int64_t)PG_LM_TICKET_BYTES)) break;
