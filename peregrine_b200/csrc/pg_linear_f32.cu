@@ -65,7 +65,8 @@ struct FParts {
 };
 
 // ---- the three planes of rows row0 .. of a: planes [3][rows][K] --------------------------------------------------------
-// rt.row_pair (by token): row r takes token row_pair[r] / top, zeros where it is -1; rows behind the route's blocks are left out
+// rt.row_pair: row r takes token row_pair[r] / top (by token), or row r.  Rows without a pair, and those behind the route's blocks, are left
+// out: nobody reads what comes of them, and rows do not touch each other.  (64 experts with a row or two each: 8192 rows of zeros took 10 us.)
 __global__ void __launch_bounds__(256)
     linear_split_kernel(const float *__restrict__ a, int64_t lda, int row0, int rows, int K, const PgRouted rt, uint2 *__restrict__ planes)
 {
@@ -75,13 +76,13 @@ __global__ void __launch_bounds__(256)
     const int64_t plane = (int64_t)rows * quads;
     for (int r = blockIdx.y; r < limit; r += gridDim.y) {
         int64_t src = row0 + r;
-        if (rt.blocks && rt.by_token) {
+        if (rt.blocks) {
             const int pair = __ldcg(rt.row_pair + row0 + r);
-            src = pair < 0 ? -1 : pair / rt.top;
+            if (pair < 0) continue;
+            if (rt.by_token) src = pair / rt.top;
         }
         for (int c = blockIdx.x * 256 + threadIdx.x; c < quads; c += gridDim.x * 256) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (src >= 0) v = __ldcg(reinterpret_cast<const float4 *>(a + src * lda) + c);
+            const float4 v = __ldcg(reinterpret_cast<const float4 *>(a + src * lda) + c);
             const float x[4] = {v.x, v.y, v.z, v.w};
             uint32_t p[3][4];
 #pragma unroll
