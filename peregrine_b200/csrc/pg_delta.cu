@@ -241,14 +241,15 @@ __device__ __forceinline__ void store_lanes(float *p, const Lanes<V> &r)
         *p = r.v[0];
 }
 
-// grid (ceil(longest / 4), seqs).  TAPS: the number of taps, 0 = any; V: channels per thread and round (4 where rows and
-// groups of channels start on 16-byte boundaries)
+// grid (ceil(longest / 4), seqs, parts): a part of the key / value heads with the heads that read them.  TAPS: the number of taps, 0 = any; V:
+// channels per thread and round (4 where rows and groups of channels start on 16-byte boundaries).  What bounds it is the chain of one
+// CTA -- rounds of channels, norms, products of pairs, gates -- not the GPU: 28 us with one part to a block of tokens, for 25 tokens as for 777.
 template <int TAPS, int V>
 __global__ void __launch_bounds__(256)
     delta_prep_kernel(const DeltaShape s, const pg_batch bt, const float *__restrict__ proj, int64_t ldp, const float *__restrict__ ring, const DeltaWork w,
                       int most)
 {
-    extern __shared__ __align__(16) float sm[];   // q and k channels [4][2 G D], then the pairs' products [G][16]
+    extern __shared__ __align__(16) float sm[];   // the part's q and k channels [4][2 GP D], then the pairs' products [GP][16]
     pg_pdl_begin();
     const int seq = gridDim.y - 1 - blockIdx.y, row0 = __ldcg(bt.d_seq_row0 + seq), T = __ldcg(bt.d_seq_row0 + seq + 1) - row0;
     const int t0 = blockIdx.x * BT, n = min(BT, T - t0), m0 = row0 + t0;
@@ -256,9 +257,12 @@ __global__ void __launch_bounds__(256)
     const int pos0 = __ldcg(bt.d_pos + row0);
     const float *row = proj + (int64_t)m0 * ldp;
     const float *rg = ring + (int64_t)__ldcg(bt.d_seq_slot + seq) * s.taps * s.C;
-    const int qk = 2 * s.G * s.D;
+    const int GP = s.G / gridDim.z, g0 = blockIdx.z * GP, rep = s.H / s.G;   // (the host takes parts that divide G)
+    const int one = GP * s.D, qk = 2 * one, all = qk + GP * rep * s.V;
     float *dots = sm + (size_t)BT * qk;
-    for (int c = threadIdx.x * V; c < s.C; c += 256 * V) {
+    for (int at = threadIdx.x * V; at < all; at += 256 * V) {
+        // channel `at` of the part: its q, its k, its v
+        const int c = at < one ? g0 * s.D + at : at < qk ? (s.G + g0) * s.D + at - one : 2 * s.G * s.D + g0 * rep * s.V + at - qk;
         Lanes<V> y[BT];
         if constexpr (TAPS > 0) {
             Lanes<V> x[TAPS - 1 + BT], wt[TAPS];
@@ -291,23 +295,23 @@ __global__ void __launch_bounds__(256)
         }
 #pragma unroll
         for (int a = 0; a < BT; a++) {
-            if (c < qk)
-                store_lanes<V>(sm + (size_t)a * qk + c, a < n ? y[a] : Lanes<V>{});
+            if (at < qk)
+                store_lanes<V>(sm + (size_t)a * qk + at, a < n ? y[a] : Lanes<V>{});
             else if (a < n)
-                store_lanes<V>(w.v + (int64_t)(m0 + a) * s.H * s.V + c - qk, y[a]);
+                store_lanes<V>(w.v + (int64_t)(m0 + a) * s.H * s.V + c - 2 * s.G * s.D, y[a]);
         }
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = warp; i < BT * 2 * s.G; i += 8) {        // unit norms: (token, q or k, head)
-        const int a = i / (2 * s.G), hd = i - a * 2 * s.G;
+    for (int i = warp; i < BT * 2 * GP; i += 8) {         // unit norms: (token, q or k, head)
+        const int a = i / (2 * GP), hd = i - a * 2 * GP;
         float *x = sm + (size_t)a * qk + hd * s.D;
         float ss = 0.0f;
         for (int d = lane; d < s.D; d += 32) ss += x[d] * x[d];
         ss = pg_warp_sum(ss);
-        const bool is_q = hd < s.G;
+        const bool is_q = hd < GP;
         const float inv = __fdiv_rn(is_q ? s.qscale : 1.0f, sqrtf(ss + s.unit_eps));
-        float *dst = (is_q ? w.q : w.k) + ((int64_t)(m0 + a) * s.G + (is_q ? hd : hd - s.G)) * s.D;
+        float *dst = (is_q ? w.q : w.k) + ((int64_t)(m0 + a) * s.G + g0 + (is_q ? hd : hd - GP)) * s.D;
         for (int d = lane; d < s.D; d += 32) {
             const float y = x[d] * inv;
             x[d] = y;
@@ -315,14 +319,14 @@ __global__ void __launch_bounds__(256)
         }
     }
     __syncthreads();
-    for (int g = warp; g < s.G; g += 8) {                 // the pairs' products
+    for (int g = warp; g < GP; g += 8) {                  // the pairs' products
         float p[16] = {};
         for (int d = lane; d < s.D; d += 32) {
             float q[BT], k[BT];
 #pragma unroll
             for (int a = 0; a < BT; a++) {
                 q[a] = sm[(size_t)a * qk + g * s.D + d];
-                k[a] = sm[(size_t)a * qk + (s.G + g) * s.D + d];
+                k[a] = sm[(size_t)a * qk + (GP + g) * s.D + d];
             }
 #pragma unroll
             for (int a = 0, i = 0, j = 6; a < BT; a++)
@@ -339,8 +343,8 @@ __global__ void __launch_bounds__(256)
         }
     }
     __syncthreads();
-    for (int h = threadIdx.x; h < s.H; h += 256) {
-        const float *dp = dots + h / (s.H / s.G) * 16;
+    for (int h = g0 * rep + threadIdx.x; h < (g0 + GP) * rep; h += 256) {
+        const float *dp = dots + (h / rep - g0) * 16;
         const float al = __ldg(s.a_log + h), db = __ldg(s.dt_bias + h);
         float g[BT], o[32];
 #pragma unroll
@@ -597,12 +601,16 @@ template <int TAPS, int V>
 int32_t run_prep_v(pg_ctx *ctx, const DeltaShape &s, const pg_batch *bt, const float *proj, int64_t ldp, const float *ring, const DeltaWork &w,
                    int most)
 {
-    const size_t smem = ((size_t)BT * 2 * s.G * s.D + 16 * s.G) * 4;
-    PG_REQUIRE(smem <= 220 * 1024, "delta: too many query / key channels");
+    // parts of the heads: up to four, with two key / value heads each, while the blocks of tokens alone are not several to an SM
+    const int64_t blocks = (int64_t)((std::min(bt->max_len, most) + BT - 1) / BT) * bt->seqs;
+    int parts = 1;
+    while (parts < 4 && s.G % (4 * parts) == 0 && (V == 1 || ((s.D | s.V) & 3) == 0) && blocks * parts < 4 * ctx->sm_count) parts *= 2;
+    PG_REQUIRE(((size_t)BT * 2 * s.G * s.D + 16 * s.G) * 4 <= 220 * 1024, "delta: too many query / key channels");
+    const size_t smem = ((size_t)BT * 2 * s.G * s.D + 16 * s.G) * 4 / parts;
     static std::atomic<uint64_t> set{0};
     PG_CUDA(pg_max_smem_once(delta_prep_kernel<TAPS, V>, 220 * 1024, ctx->device, set));
-    return launch_pdl(ctx, delta_prep_kernel<TAPS, V>, dim3((unsigned)((std::min(bt->max_len, most) + BT - 1) / BT), (unsigned)bt->seqs), dim3(256), smem, s, *bt, proj, ldp, ring, w,
-                      most);
+    return launch_pdl(ctx, delta_prep_kernel<TAPS, V>, dim3((unsigned)((std::min(bt->max_len, most) + BT - 1) / BT), (unsigned)bt->seqs, (unsigned)parts), dim3(256),
+                      smem, s, *bt, proj, ldp, ring, w, most);
 }
 
 template <int TAPS>
@@ -614,7 +622,7 @@ int32_t run_prep(pg_ctx *ctx, const DeltaShape &s, const pg_batch *bt, const flo
     return vec ? run_prep_v<TAPS, 4>(ctx, s, bt, proj, ldp, ring, w, most) : run_prep_v<TAPS, 1>(ctx, s, bt, proj, ldp, ring, w, most);
 }
 
-// a CTA per token: o / rms(o) * norm * silu(gate) per head; the sequence's last taps - 1 tokens also store their
+// grid (tokens, parts of the heads): o / rms(o) * norm * silu(gate) per head; the sequence's last taps - 1 tokens also store their
 // convolution inputs (everything that read the ring has run)
 template <typename TA>
 __global__ void __launch_bounds__(256)
@@ -625,7 +633,7 @@ __global__ void __launch_bounds__(256)
     const int m = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float *row = proj + (int64_t)m * ldp;
     if (vec) {                                            // V a multiple of 4, at most 128: a quad per lane
-        for (int h0 = warp; h0 < s.H; h0 += 16) {         // two heads at a time
+        for (int h0 = warp + 16 * blockIdx.y; h0 < s.H; h0 += 16 * gridDim.y) {   // two heads at a time
             float4 o[2], gt[2];
 #pragma unroll
             for (int i = 0; i < 2; i++) {
@@ -654,7 +662,7 @@ __global__ void __launch_bounds__(256)
             }
         }
     } else {
-        for (int h = warp; h < s.H; h += 8) {
+        for (int h = warp + 8 * blockIdx.y; h < s.H; h += 8 * gridDim.y) {
             const float *o = w.o + (int64_t)m * s.H * s.V + (int64_t)h * s.V;
             float ss = 0.0f;
             for (int c = lane; c < s.V; c += 32) {
@@ -670,7 +678,7 @@ __global__ void __launch_bounds__(256)
     const int seq = __ldcg(bt.d_row_seq + m);
     if (m >= __ldcg(bt.d_seq_row0 + seq + 1) - (s.taps - 1)) {
         float *rg = ring + ((int64_t)__ldcg(bt.d_seq_slot + seq) * s.taps + __ldcg(bt.d_pos + m) % s.taps) * s.C;
-        for (int c = threadIdx.x; c < s.C; c += 256) rg[c] = __ldcg(row + c);
+        for (int c = threadIdx.x + 256 * blockIdx.y; c < s.C; c += 256 * gridDim.y) rg[c] = __ldcg(row + c);
     }
 }
 
@@ -752,9 +760,11 @@ int32_t run_delta(pg_ctx *ctx, const pg_delta *p, const pg_batch *batch, const f
     if (rc != PG_OK) return rc;
     const bool vec = s.V % 4 == 0 && s.V <= 128 && s.C % 4 == 0 && ldp % 4 == 0 && ldo % 4 == 0 &&
                      (((uintptr_t)d_proj | (uintptr_t)d_out | (uintptr_t)s.norm | (uintptr_t)w.o) & 15) == 0;
+    // few tokens: several CTAs to each, for its heads and for the inputs that are stored (25 tokens of 32 heads: 20 us with one)
+    const int parts = M > 2 * (int64_t)ctx->sm_count ? 1 : std::max(1, std::min(4, std::max((s.H + (vec ? 15 : 7)) / (vec ? 16 : 8), s.C / 2048)));
     if (dtype == PG_BF16)
-        return launch_pdl(ctx, delta_out_kernel<bf16>, dim3((unsigned)M), dim3(256), 0, s, *batch, d_proj, ldp, w, d_ring, (bf16 *)d_out, ldo, vec);
-    return launch_pdl(ctx, delta_out_kernel<float>, dim3((unsigned)M), dim3(256), 0, s, *batch, d_proj, ldp, w, d_ring, (float *)d_out, ldo, vec);
+        return launch_pdl(ctx, delta_out_kernel<bf16>, dim3((unsigned)M, (unsigned)parts), dim3(256), 0, s, *batch, d_proj, ldp, w, d_ring, (bf16 *)d_out, ldo, vec);
+    return launch_pdl(ctx, delta_out_kernel<float>, dim3((unsigned)M, (unsigned)parts), dim3(256), 0, s, *batch, d_proj, ldp, w, d_ring, (float *)d_out, ldo, vec);
 }
 
 }  // namespace

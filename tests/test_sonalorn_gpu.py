@@ -451,6 +451,27 @@ def test_delta(lm, dtype, p):
     mixer.free()
 
 
+# key / value heads in one, two and four parts; widths of four channels at a time and of one; output heads in one to four parts
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("p", [t.delta(8, 4, 24, 40, 4), t.delta(16, 8, 16, 20, 3), t.delta(8, 8, 17, 5, 2), t.delta(12, 4, 32, 36, 5), t.delta(72, 8, 32, 128, 2),
+                               t.delta(6, 6, 20, 24, 4)])
+def test_delta_in_parts_of_its_heads(lm, dtype, p):
+    from peregrine_b200.layers import GatedDelta
+
+    width, T = 64, 41
+    d = device(lm, dtype)
+    g = rng(p["heads"] + p["vdim"])
+    W = {k: t.bf16_values(v) for k, v in t.mixer_weights(g, "delta", p, width).items()}
+    mixer = GatedDelta(d, p, W, width, 1e-4, chunks=False)
+    x = t.bf16_values(g.standard_normal((T, width)))
+    want, carried = so.delta_mixer(x.astype(np.float64), {k: v.astype(np.float64) for k, v in W.items()}, p, 1e-4, so.delta_start(p))
+    for cuts in ([41], [3, 18, 1, 19]):
+        got, state = run_mixer(lm, d, mixer, width, x, cuts)
+        close(got, want, 1e-4 if dtype == "float32" else 6e-2, f"cuts {cuts}")
+        close(state["state"][1].cpu().numpy()[:, :, :p["vdim"]], carried["S"], 1e-4 if dtype == "float32" else 6e-2, "state")
+    mixer.free()
+
+
 def test_delta_state_is_f32_over_a_long_sequence(lm):
     """Slow decay and small writes: a state kept in 16 bits, or a decay rounded to them, is far off after 600 tokens."""
     from peregrine_b200.layers import GatedDelta
