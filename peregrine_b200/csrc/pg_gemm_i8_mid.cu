@@ -25,6 +25,7 @@ constexpr int MD_K = 128;                     // bytes of K per stage: one swizz
 constexpr int MD_THREADS = 192, MD_WARPS = MD_THREADS / 32;
 constexpr int MD_ROOM = 232448 - 1024 - 512;
 constexpr int MD_MAX_PARTS = 8;
+constexpr int MD_TWO_FROM = 20;            // k-blocks a part with two threads for the copies
 
 // rows of x per tile
 __host__ __device__ inline int md_rows(int M) { return (M + 15) & ~15; }
@@ -44,6 +45,21 @@ __device__ __forceinline__ int4 md_peer_load(uint32_t local, uint32_t cta)
     return v;
 }
 
+// gives copies that are still in flight a bounded time to land before a CTA that gives up exits
+__device__ __forceinline__ void md_settle()
+{
+    const unsigned long long t0 = pg_globaltimer_ns();
+    while (pg_globaltimer_ns() - t0 < 2000000ull) {
+    }
+}
+
+// TWO: a copy costs the thread that asks for it 230 cycles, so in a long part of K x has a thread of its own.  It starts later than one thread
+// for both does, which a short part does not make up for; the line lies between the 16 and the 28 k-blocks measured.  us, one thread / two:
+//   32 k-blocks a part (K 4096, N 14336), 12 / 17 / 40 / 100 rows  14.4 / 14.7 / 16.0 / 19.6   13.4 / 13.5 / 14.7 / 19.1
+//   28 (K 14336, N 4096)                                           16.1 / 16.7 / 18.7 / 20.0   15.3 / 15.8 / 17.3 / 19.3
+//   16 (K 4096, N 6144)                                             8.9 /  9.3 /  9.8 / 12.2    9.4 /  9.6 /  9.9 / 12.1
+//    8 (K 4096, N 4096), 17 / 40 / 64 rows                                 7.8 /  8.4 /  9.0           8.3 /  8.8 /  9.3
+template <bool TWO>
 __global__ void __launch_bounds__(MD_THREADS, 1)
     gemm_i8_mid_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const float *__restrict__ a_scales,
                        const float *__restrict__ w_scales, int M, int N, int K, int parts, float *__restrict__ y, int32_t *__restrict__ acc_out,
@@ -81,7 +97,7 @@ __global__ void __launch_bounds__(MD_THREADS, 1)
     const int kb0 = min(kblocks, part * per), kb1 = min(kblocks, kb0 + per);   // (never empty: the host sees to it)
 
     bool ok = true;
-    if (warp == 0) {
+    if (warp == 0 && !TWO) {
         if (lane == 0) {
             const int early = min(kb1 - kb0, stages);           // weights do not depend on the preceding kernel
             for (int i = 0; i < early; i++) {
@@ -103,14 +119,30 @@ __global__ void __launch_bounds__(MD_THREADS, 1)
                     phase ^= 1;
                 }
             }
-            if (!ok) {
-                // give copies that are still in flight a bounded time to land before the CTA exits
-                const unsigned long long t0 = pg_globaltimer_ns();
-                while (pg_globaltimer_ns() - t0 < 2000000ull) {
-                }
+            if (!ok) md_settle();
+        }
+    } else if (TWO && (warp == 0 || warp == 2) && lane == 0) {
+        // a thread for the weights, and one for x, which announces a stage's bytes (its warp has nothing else to do until all sums are there)
+        if (warp == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
+        int stage = 0, phase = 1;
+        for (int kb = kb0; kb < kb1; kb++) {
+            const uint32_t at = base + stage * stage_bytes;
+            if (!(ok = pg_mbar_wait(bar_empty + 8 * stage, phase, abort_flag, status, limit_ns))) break;
+            if (warp == 0) {
+                tma_load_2d(at, &tmap_w, bar_full + 8 * stage, kb * MD_K, n0);
+            } else {
+                pg_mbar_expect(bar_full + 8 * stage, (uint32_t)stage_bytes);
+                tma_load_2d(at + MD_N * MD_K, &tmap_x, bar_full + 8 * stage, kb * MD_K, 0);
+            }
+            if (++stage == stages) {
+                stage = 0;
+                phase ^= 1;
             }
         }
-    } else if (warp == 1) {
+        if (!ok) md_settle();
+    }
+    if (TWO) __syncwarp();
+    if (warp == 1) {
         const uint32_t on = pg_elect();
         // kind::i8: D = s32 (2 at bit 4), A and B signed 8-bit (1 at bits 7 and 10), both K-major
         const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(rows >> 3) << 17) | ((uint32_t)(MD_N >> 4) << 24);
@@ -130,9 +162,9 @@ __global__ void __launch_bounds__(MD_THREADS, 1)
             }
         }
         if (ok) umma_commit(bar_done, on);
-    } else {
+    } else if (warp > 1) {
         // lane = column of y: its sums go to [row][128] in the ring, which nothing else uses any more
-        ok = __all_sync(0xffffffffu, pg_mbar_wait(bar_done, 0, abort_flag, status, limit_ns));
+        ok = __all_sync(0xffffffffu, (!TWO || ok) && pg_mbar_wait(bar_done, 0, abort_flag, status, limit_ns));
         if (ok) {
             tc_fence_after();
             const int q = warp & 3;
@@ -229,7 +261,7 @@ int32_t md_clusters(pg_ctx *ctx, int parts, int *fit)
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        PG_CUDA(cudaOccupancyMaxActiveClusters(&n, gemm_i8_mid_kernel, &cfg));
+        PG_CUDA(cudaOccupancyMaxActiveClusters(&n, gemm_i8_mid_kernel<false>, &cfg));
         v = n + 1;
         k.store(v, std::memory_order_relaxed);
     }
@@ -249,8 +281,9 @@ bool pgk_gemm_i8_mid_supports(pg_ctx *ctx, int64_t m, int64_t k, int64_t n)
 
 int32_t pgk_gemm_i8_mid(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64_t m, int64_t k, const pg_qtensor *w, float *d_y, int32_t *d_acc)
 {
-    static std::atomic<uint64_t> smem_set{0};
-    PG_CUDA(pg_max_smem_once(gemm_i8_mid_kernel, MD_ROOM + 1024 + 512, ctx->device, smem_set));
+    static std::atomic<uint64_t> smem_set{0}, smem_set_two{0};
+    PG_CUDA(pg_max_smem_once(gemm_i8_mid_kernel<false>, MD_ROOM + 1024 + 512, ctx->device, smem_set));
+    PG_CUDA(pg_max_smem_once(gemm_i8_mid_kernel<true>, MD_ROOM + 1024 + 512, ctx->device, smem_set_two));
     const int64_t n = w->cols, tiles = (n + MD_N - 1) / MD_N, kblocks = (k + MD_K - 1) / MD_K;
     // parts of K: as many as still have all their clusters on the GPU at once and at least four k-blocks each
     int parts = 1;
@@ -267,6 +300,7 @@ int32_t pgk_gemm_i8_mid(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int64
     int32_t rc = md_encode(&tw, w->d_data_i8_t, n, k, MD_N);
     if (rc == PG_OK) rc = md_encode(&tx, d_a, m, k, rows);
     if (rc != PG_OK) return rc;
-    return launch_pdl_cluster(ctx, gemm_i8_mid_kernel, dim3((unsigned)(tiles * parts)), dim3(MD_THREADS), (size_t)md_stages(rows) * md_stage(rows) + 1024 + 512, parts,
+    auto kern = (kblocks + parts - 1) / parts > MD_TWO_FROM ? gemm_i8_mid_kernel<true> : gemm_i8_mid_kernel<false>;
+    return launch_pdl_cluster(ctx, kern, dim3((unsigned)(tiles * parts)), dim3(MD_THREADS), (size_t)md_stages(rows) * md_stage(rows) + 1024 + 512, parts,
                               tw, tx, d_as, (const float *)w->d_scales, (int)m, (int)n, (int)k, parts, d_y, d_acc, ctx->d_status, ctx->wait_limit_ns);
 }

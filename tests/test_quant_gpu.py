@@ -298,6 +298,15 @@ def test_mid_batch_dispatch(pg, gpu, oracle_mt, m, k, n):
     _check_product(pg, gpu, oracle_mt, x, w, m, k, n, ["naive"])
 
 
+@pytest.mark.parametrize("m,k", [(17, 2560), (17, 2576), (48, 2688), (96, 2704), (33, 7680), (24, 5392)])
+def test_mid_batch_long_parts(pg, gpu, oracle_mt, m, k):
+    """Twenty 128-element blocks of K to a part, more and ragged ones: copies by one thread and by two."""
+    n = 9601                                      # 76 tiles of 128 columns, the last of one: no parts of K
+    x, w = linear_inputs(m, k, n, 1400 + m + k)
+    _check_product(pg, gpu, oracle_mt, x, w, m, k, n, ["naive"])
+    assert gpu.device_status() == 0
+
+
 @pytest.mark.parametrize("m,k,n", [(1, 4096, 10000), (8, 12800, 1600), (9, 4096, 5003), (16, 14336, 4096), (16, 3136, 7001), (9, 4096, 4096), (8, 4096, 12999)])
 def test_few_rows_dispatch(pg, gpu, oracle_mt, m, k, n):
     """Up to 16 rows with the automatic kernel choice, on both sides of its line: sums are whole numbers, the same from either kernel."""
