@@ -8,14 +8,18 @@
 //   of one tile overlaps the main loop of the next.
 //
 // One persistent CTA per SM, warp-specialised:
-//   warp 0   producer   TMA (cp.async.bulk.tensor, 128B swizzle) of a 128 x 128B tile of A and a
-//                       BN x 128B tile of B into a ring of shared-memory stages
+//   warps 0, 6 producers TMA (cp.async.bulk.tensor, 128B swizzle) of a 128 x 128B tile of A (warp 0) and a
+//                       BN x 128B tile of B (warp 6) into a ring of shared-memory stages
 //   warp 1   MMA        one elected lane issues tcgen05.mma.cta_group::1.kind::i8 (M=128, N=BN,
 //                       K=32 per instruction, four per stage); tcgen05.commit releases stages
 //                       and publishes finished accumulators
 //   warps 2-5 epilogue  tcgen05.ld of their TMEM lane quarter, then
 //                       `acc as f32 * a_scale[m] * w_scale[n]` as two rounded products, stored
 //                       straight to global memory (and the raw s32 sums when asked for)
+//
+// What bounds it: the copies.  One thread that asks for both tiles of a stage and one that issues the MMAs from a branch of its own kept the
+// tensor cores waiting; us, so / with two threads for the copies and a converged warp for the MMAs: 129 rows, K 4096, N 4096 15.9 / 14.3, K 14336
+// 38.2 / 33.3; 300 rows 25.0 / 22.1 and 68.5 / 58.4; 512 rows 25.5 / 22.5 and 72.0 / 61.9.
 //
 // Integer accumulation is exact, so the result is bit-identical to the scalar loop whatever the
 // tiling.  Rows/columns/K past the matrix edge are zero-filled by TMA and masked on store.
@@ -33,7 +37,7 @@ namespace {
 constexpr int BM = 128;
 constexpr int BK = 128;  // bytes of K per stage = one 128-byte swizzle span
 constexpr int UMMA_K = 32;
-constexpr int NUM_THREADS = 192;
+constexpr int NUM_THREADS = 224;   // warps: copies of A, MMAs, four of the epilogue, copies of B
 constexpr unsigned long long WAIT_LIMIT_NS = 1000ull * 1000ull * 1000ull;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -115,19 +119,23 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate)
+__device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate, uint32_t on)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(on)
         : "memory");
 }
 
-__device__ __forceinline__ void umma_commit(uint32_t bar)
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t on)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(on) : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32])
@@ -245,38 +253,27 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0) {
-        // ---------------------------------------------------------------- producer
+    if (warp == 0 || warp == 6) {
+        // ---------------------------------------------------------------- producers: a thread for A, which also announces a stage's bytes, and one
+        // for the weights, which do not wait for the predecessor.  (A copy of 16 KB costs the thread that asks for it 230 cycles.)
+        const bool weights = warp == 6;
         if (lane == 0) {
-            uint32_t stage = 0, phase = 0;
+            uint32_t stage = 0, phase = 1;
             bool ok = true;
-            // the weight tiles of the first stages of this CTA's first tile, before the predecessor has finished
-            int early = 0;
-            if ((int)blockIdx.x < total_tiles) {
-                const int u = (int)blockIdx.x, tile = u / splits, kb0 = (u - tile * splits) * kpb;
-                const int n0 = (tile / tiles_m) * BN;
-                const int mine = min(kblocks, kb0 + kpb) - kb0;
-                early = mine < STAGES ? mine : STAGES;
-                for (int i = 0; i < early; i++) {
-                    mbar_arrive_expect_tx(bar_full + 8 * i, C::STAGE);
-                    tma_load_2d(base + i * C::STAGE + C::STAGE_A, &tmap_b, bar_full + 8 * i, (kb0 + i) * BK, n0);
-                }
-            }
-            asm volatile("griddepcontrol.wait;" ::: "memory");
+            if (!weights) asm volatile("griddepcontrol.wait;" ::: "memory");
             for (int u = blockIdx.x; ok && u < total_tiles; u += gridDim.x) {
                 const int t = u / splits, kb0 = (u - t * splits) * kpb, kb1 = min(kblocks, kb0 + kpb);
                 const int m0 = (t % tiles_m) * BM;
                 const int n0 = (t / tiles_m) * BN;
                 for (int kb = kb0; kb < kb1; kb++) {
-                    if (!(ok = mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, status))) break;
+                    if (!(ok = mbar_wait(bar_empty + 8 * stage, phase, abort_flag, status))) break;
                     const uint32_t sa = base + stage * C::STAGE;
-                    if (early > 0) {
-                        early--;                            // announced and half filled above
+                    if (weights) {
+                        tma_load_2d(sa + C::STAGE_A, &tmap_b, bar_full + 8 * stage, kb * BK, n0);
                     } else {
                         mbar_arrive_expect_tx(bar_full + 8 * stage, C::STAGE);
-                        tma_load_2d(sa + C::STAGE_A, &tmap_b, bar_full + 8 * stage, kb * BK, n0);
+                        tma_load_2d(sa, &tmap_a, bar_full + 8 * stage, kb * BK, m0);
                     }
-                    tma_load_2d(sa, &tmap_a, bar_full + 8 * stage, kb * BK, m0);
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
@@ -291,19 +288,22 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
             }
         }
     } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        // ---------------------------------------------------------------- MMA issuer (the whole warp; one lane's count: issued from a branch that one
+        // thread is in, an MMA costs 110 cycles of issue)
+        {
+            uint32_t on;
+            asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(on));
             constexpr uint32_t idesc = make_idesc(BM, BN);
             uint32_t stage = 0, phase = 0;
             uint32_t acc = 0, acc_phase = 0;
             bool ok = true;
             for (int u = blockIdx.x; ok && u < total_tiles; u += gridDim.x) {
                 const int kb0 = (u % splits) * kpb, kb1 = min(kblocks, kb0 + kpb);
-                if (!(ok = mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, status))) break;
+                if (!(ok = __all_sync(0xffffffffu, mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, status)))) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
                 for (int kb = kb0; kb < kb1; kb++) {
-                    if (!(ok = mbar_wait(bar_full + 8 * stage, phase, abort_flag, status))) break;
+                    if (!(ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * stage, phase, abort_flag, status)))) break;
                     tc_fence_after();
                     const uint32_t sa = base + stage * C::STAGE;
                     const uint64_t da = make_smem_desc(sa);
@@ -312,16 +312,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
                     for (int j = 0; j < BK / UMMA_K; j++) {
                         // +32 bytes of K inside the swizzle span = +2 in the 16-byte address field
                         umma_i8(d_tmem, da + (uint64_t)(j * (UMMA_K >> 4)), db + (uint64_t)(j * (UMMA_K >> 4)), idesc,
-                                (kb != kb0 || j != 0) ? 1u : 0u);
+                                (kb != kb0 || j != 0) ? 1u : 0u, on);
                     }
-                    umma_commit(bar_empty + 8 * stage);  // stage reusable once these MMAs have read it
+                    umma_commit(bar_empty + 8 * stage, on);  // stage reusable once these MMAs have read it
                     if (++stage == STAGES) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
                 if (!ok) break;
-                umma_commit(bar_tfull + 8 * acc);  // accumulator complete
+                umma_commit(bar_tfull + 8 * acc, on);  // accumulator complete
                 if (++acc == 2) {
                     acc = 0;
                     acc_phase ^= 1;
