@@ -166,7 +166,8 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr)
 // kind::i8: D = s32, A/B = s8, K-major, N >> 3 at bit 17, M >> 4 at bit 24 (M = 256 over the pair)
 __host__ __device__ constexpr uint32_t make_idesc(int n) { return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24); }
 
-template <int TNH>
+// VEC: rows of y and of the sums start on 16-byte boundaries
+template <int TNH, bool VEC>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
     gemm_i8_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                                 const float *__restrict__ a_scales, const float *__restrict__ w_scales, int M, int N, int K,
@@ -309,8 +310,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         const int q = warp & 3;
         asm volatile("griddepcontrol.wait;" ::: "memory");   // a_scales come from the predecessor; y may still be read by it
         uint32_t acc = 0, acc_phase = 0;
-        const bool vec_ok = ((N & 3) == 0) && (((uintptr_t)y & 15) == 0) && (((uintptr_t)acc_out & 15) == 0) &&
-                            (((uintptr_t)w_scales & 15) == 0);
         bool ok = true;
         for (int t = pair; ok && t < total_tiles; t += npairs) {
             const int m0 = (t % tiles_m) * (2 * TM) + (int)rank * TM;
@@ -330,7 +329,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
                 tmem_ld32(taddr + c, v);
                 if (row_base >= M || n0 + c >= N) continue;   // uniform over the warp
                 const int64_t off0 = (int64_t)row_base * N + n0 + c;
-                if (vec_ok) {
+                if constexpr (VEC) {
                     // coalesced: the warp exchanges the block through shared memory and writes whole row segments
                     if (acc_out) pg_store_block_32x32(reinterpret_cast<uint32_t *>(acc_out + off0), N, M - row_base, N - (n0 + c), stage_buf, lane, v);
                     if (y) {
@@ -403,8 +402,8 @@ int32_t encode_kmajor(CUtensorMap *map, const void *ptr, int64_t rows, int64_t k
     return PG_OK;
 }
 
-template <int TNH>
-int32_t launch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, const pg_qtensor *w, float *d_y, int32_t *d_acc)
+template <int TNH, bool VEC>
+int32_t launch_as(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, const pg_qtensor *w, float *d_y, int32_t *d_acc)
 {
     using C = Cfg<TNH>;
     const int N = (int)w->cols;
@@ -413,7 +412,7 @@ int32_t launch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, 
     int32_t rc = encode_kmajor(&ta, d_a, M, K, TM);
     if (rc == PG_OK) rc = encode_kmajor(&tb, w->d_data_i8_t, N, K, TNH);
     if (rc) return rc;
-    auto kern = gemm_i8_tcgen05_2cta_kernel<TNH>;
+    auto kern = gemm_i8_tcgen05_2cta_kernel<TNH, VEC>;
     static std::atomic<uint64_t> smem_set{0};
     PG_CUDA(pg_max_smem_once(kern, (int)C::SMEM, ctx->device, smem_set));
     const int64_t tiles = (int64_t)((M + 2 * TM - 1) / (2 * TM)) * ((N + C::TN - 1) / C::TN);
@@ -436,6 +435,13 @@ int32_t launch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, 
                                ctx->d_status));
     PG_LAUNCHED();
     return PG_OK;
+}
+
+template <int TNH>
+int32_t launch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, int M, int K, const pg_qtensor *w, float *d_y, int32_t *d_acc)
+{
+    const bool vec = (w->cols & 3) == 0 && (((uintptr_t)d_y | (uintptr_t)d_acc | (uintptr_t)w->d_scales) & 15) == 0;
+    return vec ? launch_as<TNH, true>(ctx, d_a, d_as, M, K, w, d_y, d_acc) : launch_as<TNH, false>(ctx, d_a, d_as, M, K, w, d_y, d_acc);
 }
 
 }  // namespace

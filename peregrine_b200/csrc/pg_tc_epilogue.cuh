@@ -41,7 +41,8 @@ __device__ __forceinline__ void pg_store_block_32x32(uint32_t *dst, int64_t ld, 
 
 
 // The same where rows do not start on 16-byte boundaries (or the last columns are no multiple of four): a store instruction writes 32
-// consecutive words of one row.
+// consecutive words of one row.  W8A8 products, us, each lane with its own row / this: 2048 rows, K 4096, N 14335 237.9 / 122.1; 1132 rows, N 4097
+// 63.3 / 38.4; 729 rows, K 8640, N 3329 52.3 / 39.5; 300 rows, K 4096, N 5003 38.4 / 25.5.
 __device__ __forceinline__ void pg_store_block_words(uint32_t *dst, int64_t ld, int rows_left, int cols_left, uint32_t stage, int lane,
                                                      const uint32_t (&vals)[32])
 {
