@@ -32,7 +32,7 @@ SOURCES = CORE + [
     "pg_gemm_tcgen05.cu",
     "pg_gemm_tcgen05_2cta.cu",
     "pg_gguf.cu",
-    "pg_gguf_stream.cu", "pg_gguf_tc.cu",
+    "pg_gguf_stream.cu", "pg_gguf_few.cu", "pg_gguf_tc.cu",
     "pg_noalloc.cu",
     "pg_w8a32.cu",
     "pg_peer.cu",

@@ -295,6 +295,11 @@ int32_t pgk_matmul_gguf(pg_ctx *ctx, const float *d_x, int64_t m, const pg_gguf_
 {
     if (m == 0 || w->n == 0) return PG_OK;
     PG_REQUIRE(((uintptr_t)d_x & 15) == 0, "matmul_gguf: x must be 16-byte aligned");
+    if (pgk_matmul_gguf_few_supports(ctx, w, m)) {
+        bool taken;
+        const int32_t rc = pgk_matmul_gguf_few(ctx, d_x, m, w, d_y, &taken);
+        if (rc != PG_OK || taken) return rc;
+    }
     if (pgk_matmul_gguf_tc_supports(ctx, w, m)) return pgk_matmul_gguf_tc(ctx, d_x, m, w, d_y);
     if (w->tiled) return pgk_matmul_gguf_stream(ctx, d_x, m, w, d_y);
     switch (w->type) {

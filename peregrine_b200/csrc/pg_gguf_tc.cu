@@ -922,7 +922,8 @@ int32_t gt_run(pg_ctx *ctx, const pg_gguf_weight *w, const void *planes, const f
 
 }  // namespace
 
-// From nine rows on, and for fewer where the streaming form walks K in several chunks (it has room for 16384 elements of x in all),
+// From nine rows on, and for fewer -- where csrc/pg_gguf_few.cu finds no workspace or K is beyond it -- where the streaming form walks K in several
+// chunks (it has room for 16384 elements of x in all),
 // each with its own start: from four chunks on, from three on narrow layers, and from two with seven and eight rows there.  Q4_0, us,
 // streaming / this: K 14336, N 4096 at 2 / 3 / 5 / 8 rows 18.5 / 28.4 / 40.7 / 48.7 against 25.7 / 26.2 / 26.7 / 27.7; K 8192, N 8192 at 4 / 5 / 8
 // rows 23.3 / 29.4 / 34.2 against 28.2 / 28.3 / 28.9; K 6144, at 5 rows: N 4096 17.3 / 15.1, N 12000 29.7 / 32.9; K 4096, at 8 rows: N 4096

@@ -457,6 +457,9 @@ int32_t pgk_matmul_gguf(pg_ctx *ctx, const float *d_x, int64_t m, const pg_gguf_
 // pg_gguf_stream.cu
 bool pgk_matmul_gguf_stream_supports(const pg_gguf_weight *w, int64_t m);
 int32_t pgk_matmul_gguf_stream(pg_ctx *ctx, const float *d_x, int64_t m, const pg_gguf_weight *w, float *d_y);
+// pg_gguf_few.cu: up to eight rows
+bool pgk_matmul_gguf_few_supports(const pg_ctx *ctx, const pg_gguf_weight *w, int64_t m);
+int32_t pgk_matmul_gguf_few(pg_ctx *ctx, const float *d_x, int64_t m, const pg_gguf_weight *w, float *d_y, bool *taken);
 // pg_gguf_tc.cu: the same for several rows; the workspace that an upload reserves for it
 bool pgk_matmul_gguf_tc_supports(const pg_ctx *ctx, const pg_gguf_weight *w, int64_t m);
 int32_t pgk_gguf_tc_reserve(pg_ctx *ctx, int64_t k);

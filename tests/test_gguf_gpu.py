@@ -229,6 +229,30 @@ def test_matmul_gguf_few_rows_long_k(pg, gpu, oracle_mt, kind, m, n, k, digits):
     w.free()
 
 
+@pytest.mark.parametrize("kind", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("m,n,k", [(4, 17, 256), (4, 4100, 768), (5, 1, 2304), (8, 20100, 2304), (6, 130, 3584), (3, 300, 4352), (7, 2500, 9984), (2, 40, 12544),
+                                   (8, 33, 14592), (1, 50, 16640), (8, 15, 65536)])
+def test_matmul_gguf_few_rows(pg, gpu, oracle_mt, kind, m, n, k):
+    """A slice of K per warp: one warp to a tile and sixteen, parts of K in several CTAs with a shorter last one, ragged tiles, several tiles to a
+    CTA.  The bound of the planes and sums of many rows (above).  A row of x that holds an infinity or a NaN gives NaN and leaves the others alone."""
+    g = rng(n + k + m)
+    raw = oracle_mt.encode(kind, normal(g, (n, k), 0.02))
+    w64 = oracle_mt.dequant(kind, raw, n * k).reshape(n, k).astype(np.float64)
+    w = pg.gguf.GgufWeight(kind, raw, n, k, gpu)
+    x = normal(g, (m, k))
+    got = w.matmul(x, m)
+    x64 = np.abs(x).astype(np.float64)
+    bound = x64 @ np.abs(w64).T * (2.0 ** -22 + 4 * 2.0 ** -23 + (k // 32 + 18) * 2.0 ** -24) + x64.max(1, keepdims=True) * 2.0 ** -39 * np.abs(w64).sum(1)
+    assert (np.abs(got - x.astype(np.float64) @ w64.T) <= bound).all()
+    for value in (np.inf, np.nan):
+        bad = x.copy()
+        bad[m - 1, k - 3] = value
+        out = w.matmul(bad, m)
+        assert np.isnan(out[m - 1]).all() and np.array_equal(out[:m - 1], got[:m - 1])
+    assert gpu.device_status() == 0
+    w.free()
+
+
 def test_matmul_gguf_many_rows_recorded_without_a_run_before(pg, oracle_mt):
     """The workspace cannot grow in a recording: the rows then go through what the upload has reserved, in portions, with the same
     results."""
