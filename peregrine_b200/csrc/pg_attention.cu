@@ -124,16 +124,21 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---- f32: grid (H, rows), or (H, rows / 4 + seqs) with up to four tokens of one sequence a CTA ---------------------------
-// Bound by what it reads from L2: a key is a thread's, 16 bytes at a time, so four tokens share the keys and values that one read
-// (333 tokens of 32 heads of 128: 318 -> 182 us).  A token's sums are the same either way, to the last bit.
+// Four tokens share the keys and values that one reads (333 tokens of 32 heads of 128: 318 -> 182 us); a token's sums are the same either way, to
+// the last bit.  What bounds four tokens then is shared memory and L1 (67 % of their cycles; 41 % of the issue slots): keys come 16 columns at a time
+// in whole segments -- read by the thread that uses them, 16 bytes a key, an instruction touches 32 lines -- and values eight at a time
+// (182 -> 130 us).  One token alone waits for its loads instead, and reads its keys directly: through tiles, four sequences at 700 positions of a
+// model with keys of 576 columns took 1169 us a step instead of 1097.
 constexpr int AF_T = 128, AF_Q = 4;
-template <int QT>
+constexpr int AF_KT = 20;                     // floats between the keys of a tile of 16 columns: 128-bit reads of eight of them meet no bank twice
+template <int QT, int NV>                     // NV value columns per thread
 __global__ void __launch_bounds__(AF_T, QT > 1 ? 4 : 8)
     attn_f32_kernel(const AttnShape s, const pg_batch bt, const float *__restrict__ q, const float *__restrict__ kc, const float *__restrict__ vc,
                     float *__restrict__ out, int64_t ldo)
 {
     extern __shared__ __align__(16) float sm[];   // q[QT][dp] | p[QT][AF_T]
     __shared__ float red[QT][8];
+    __shared__ __align__(16) float tiles[AF_T * AF_KT];
     pg_pdl_begin();
     const int h = blockIdx.x, g = h / s.rep, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int m = blockIdx.y, n = 1;                    // the CTA's rows
@@ -154,7 +159,6 @@ __global__ void __launch_bounds__(AF_T, QT > 1 ? 4 : 8)
     if (pos < 0 || n <= 0) return;
     float *sq = sm, *sp = sm + QT * s.dp;
     const float slope = s.slopes ? __ldg(s.slopes + h) : 0.0f;
-    constexpr int NV = 8;                         // value columns per thread (vdim <= 1024)
     // (the rows of a group that lie in one chunk go together)
     for (int done = 0; done < n;) {
         const int low = attn_low(s, pos + done), nq = s.chunk ? min(n - done, s.chunk - (pos + done) % s.chunk) : n - done;
@@ -175,18 +179,48 @@ __global__ void __launch_bounds__(AF_T, QT > 1 ? 4 : 8)
             float sc[QT];
 #pragma unroll
             for (int u = 0; u < QT; u++) sc[u] = -INFINITY;
-            if (j < p0 + nq) {
-                // dp is a multiple of 16, zero behind D
+            // (dp is a multiple of 16, zero behind D)
+            if (QT > 1 || j < p0 + nq) {
                 float d[QT][8] = {};
-                for (int i = 0; i < s.dp; i += 8) {
-                    const float4 a = __ldcg(reinterpret_cast<const float4 *>(kb + (int64_t)j * s.dp + i));
-                    const float4 b = __ldcg(reinterpret_cast<const float4 *>(kb + (int64_t)j * s.dp + i + 4));
+                if constexpr (QT == 1) {
+                    for (int i = 0; i < s.dp; i += 8) {
+                        const float4 a = __ldcg(reinterpret_cast<const float4 *>(kb + (int64_t)j * s.dp + i));
+                        const float4 b = __ldcg(reinterpret_cast<const float4 *>(kb + (int64_t)j * s.dp + i + 4));
+                        const float4 x = *reinterpret_cast<const float4 *>(sq + i), y = *reinterpret_cast<const float4 *>(sq + i + 4);
+                        d[0][0] = fmaf(x.x, a.x, d[0][0]), d[0][1] = fmaf(x.y, a.y, d[0][1]), d[0][2] = fmaf(x.z, a.z, d[0][2]), d[0][3] = fmaf(x.w, a.w, d[0][3]);
+                        d[0][4] = fmaf(y.x, b.x, d[0][4]), d[0][5] = fmaf(y.y, b.y, d[0][5]), d[0][6] = fmaf(y.z, b.z, d[0][6]), d[0][7] = fmaf(y.w, b.w, d[0][7]);
+                    }
+                } else {
+                    // the warp reads 16 columns of its 32 keys, eight keys at a time, the next ones while these are used, and hands each lane its key
+                    // through shared memory
+                    float *tile = tiles + warp * 32 * AF_KT;
+                    const int piece = (lane & 3) * 4, k0 = j0 + warp * 32 + (lane >> 2), last = p0 + nq;
+                    const float *from = kb + (int64_t)k0 * s.dp + piece;
+                    float4 c[4];
+                    auto fetch = [&](int i) {
 #pragma unroll
-                    for (int u = 0; u < QT; u++) {
-                        if (QT > 1 && u >= nq) break;
-                        const float4 x = *reinterpret_cast<const float4 *>(sq + u * s.dp + i), y = *reinterpret_cast<const float4 *>(sq + u * s.dp + i + 4);
-                        d[u][0] = fmaf(x.x, a.x, d[u][0]), d[u][1] = fmaf(x.y, a.y, d[u][1]), d[u][2] = fmaf(x.z, a.z, d[u][2]), d[u][3] = fmaf(x.w, a.w, d[u][3]);
-                        d[u][4] = fmaf(y.x, b.x, d[u][4]), d[u][5] = fmaf(y.y, b.y, d[u][5]), d[u][6] = fmaf(y.z, b.z, d[u][6]), d[u][7] = fmaf(y.w, b.w, d[u][7]);
+                        for (int e = 0; e < 4; e++)
+                            c[e] = k0 + 8 * e < last ? __ldcg(reinterpret_cast<const float4 *>(from + (int64_t)(8 * e) * s.dp + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    };
+                    fetch(0);
+#pragma unroll 1
+                    for (int i = 0; i < s.dp; i += 16) {
+                        __syncwarp();
+#pragma unroll
+                        for (int e = 0; e < 4; e++) *reinterpret_cast<float4 *>(tile + ((lane >> 2) + 8 * e) * AF_KT + piece) = c[e];
+                        __syncwarp();
+                        if (i + 16 < s.dp) fetch(i + 16);
+#pragma unroll
+                        for (int e = 0; e < 16; e += 8) {
+                            const float4 a = *reinterpret_cast<const float4 *>(tile + lane * AF_KT + e), b = *reinterpret_cast<const float4 *>(tile + lane * AF_KT + e + 4);
+#pragma unroll
+                            for (int u = 0; u < QT; u++) {    // (what comes out for rows from nq on is not used)
+                                const float *qu = sq + u * s.dp + i + e;
+                                const float4 x = *reinterpret_cast<const float4 *>(qu), y = *reinterpret_cast<const float4 *>(qu + 4);
+                                d[u][0] = fmaf(x.x, a.x, d[u][0]), d[u][1] = fmaf(x.y, a.y, d[u][1]), d[u][2] = fmaf(x.z, a.z, d[u][2]), d[u][3] = fmaf(x.w, a.w, d[u][3]);
+                                d[u][4] = fmaf(y.x, b.x, d[u][4]), d[u][5] = fmaf(y.y, b.y, d[u][5]), d[u][6] = fmaf(y.z, b.z, d[u][6]), d[u][7] = fmaf(y.w, b.w, d[u][7]);
+                            }
+                        }
                     }
                 }
 #pragma unroll
@@ -221,7 +255,8 @@ __global__ void __launch_bounds__(AF_T, QT > 1 ? 4 : 8)
                 l[u] = l[u] * corr[u] + ((red[u][4] + red[u][5]) + (red[u][6] + red[u][7]));
                 cnt[u] = u < nq ? min(AF_T, p0 + u + 1 - j0) : 0;
             }
-            const int all = min(AF_T, p0 + nq - j0);
+            // keys that every row sees (later rows see more), in eights; a row's others may hold anything, and are looked at one by one
+            const int all = min(AF_T, p0 + nq - j0), both = QT > 1 ? max(0, cnt[0]) & ~7 : 0;
 #pragma unroll
             for (int i = 0; i < NV; i++) {
                 const int c = tid + i * AF_T;
@@ -229,7 +264,19 @@ __global__ void __launch_bounds__(AF_T, QT > 1 ? 4 : 8)
                 float a[QT];
 #pragma unroll
                 for (int u = 0; u < QT; u++) a[u] = acc[i][u] * corr[u];
-                for (int k = 0; k < all; k++) {
+#pragma unroll 1
+                for (int k = 0; k < both; k += 8) {
+                    float v[8];
+#pragma unroll
+                    for (int e = 0; e < 8; e++) v[e] = __ldcg(vb + (int64_t)(j0 + k + e) * s.vp + c);
+#pragma unroll
+                    for (int u = 0; u < QT; u++) {
+                        const float4 x = *reinterpret_cast<const float4 *>(sp + u * AF_T + k), y = *reinterpret_cast<const float4 *>(sp + u * AF_T + k + 4);
+                        a[u] = fmaf(x.x, v[0], a[u]), a[u] = fmaf(x.y, v[1], a[u]), a[u] = fmaf(x.z, v[2], a[u]), a[u] = fmaf(x.w, v[3], a[u]);
+                        a[u] = fmaf(y.x, v[4], a[u]), a[u] = fmaf(y.y, v[5], a[u]), a[u] = fmaf(y.z, v[6], a[u]), a[u] = fmaf(y.w, v[7], a[u]);
+                    }
+                }
+                for (int k = both; k < all; k++) {
                     const float v = __ldcg(vb + (int64_t)(j0 + k) * s.vp + c);
 #pragma unroll
                     for (int u = 0; u < QT; u++)
@@ -787,12 +834,12 @@ int32_t run_step(pg_ctx *ctx, const AttnShape &s, const pg_batch *bt, const floa
 int32_t pgk_attention_f32(pg_ctx *ctx, const AttnShape &s, const pg_batch *bt, const float *q, const float *kc, const float *vc, float *out, int64_t ldo)
 {
     PG_REQUIRE(bt->rows <= 65535, "attention: too many rows for the f32 form");
-    PG_REQUIRE(s.V <= 8 * AF_T && (s.dp + AF_T) * 4 <= 48 * 1024, "attention: heads too wide for the f32 form");
+    PG_REQUIRE(s.V <= 8 * AF_T && (s.dp + AF_T + AF_T * AF_KT) * 4 < 48 * 1024, "attention: heads too wide for the f32 form");
     // (tokens of different sequences share nothing)
-    if (bt->max_len > 1 && AF_Q * (s.dp + AF_T) * 4 <= 48 * 1024 && bt->rows / AF_Q + bt->seqs <= 65535)
-        return launch_pdl(ctx, attn_f32_kernel<AF_Q>, dim3((unsigned)s.H, (unsigned)(bt->rows / AF_Q + bt->seqs)), dim3(AF_T), (size_t)AF_Q * (s.dp + AF_T) * 4, s,
-                          *bt, q, kc, vc, out, ldo);
-    return launch_pdl(ctx, attn_f32_kernel<1>, dim3((unsigned)s.H, (unsigned)bt->rows), dim3(AF_T), (size_t)(s.dp + AF_T) * 4, s, *bt, q, kc, vc, out, ldo);
+    if (bt->max_len > 1 && (AF_Q * (s.dp + AF_T) + AF_T * AF_KT) * 4 < 47 * 1024 && bt->rows / AF_Q + bt->seqs <= 65535)
+        return launch_pdl(ctx, s.V <= AF_T ? attn_f32_kernel<AF_Q, 1> : attn_f32_kernel<AF_Q, 8>, dim3((unsigned)s.H, (unsigned)(bt->rows / AF_Q + bt->seqs)),
+                          dim3(AF_T), (size_t)AF_Q * (s.dp + AF_T) * 4, s, *bt, q, kc, vc, out, ldo);
+    return launch_pdl(ctx, attn_f32_kernel<1, 8>, dim3((unsigned)s.H, (unsigned)bt->rows), dim3(AF_T), (size_t)(s.dp + AF_T) * 4, s, *bt, q, kc, vc, out, ldo);
 }
 
 extern "C" {

@@ -696,6 +696,24 @@ def test_attention_f32_tokens_of_several_sequences(lm):
     mixer.free()
 
 
+@pytest.mark.parametrize("heads", [(2, 1, 16, 128, 0.3), (2, 2, 48, 136, 0.3), (4, 2, 200, 256, 0.1)])
+def test_attention_f32_tiles_of_keys(lm, heads):
+    """Groups of four tokens, full and ragged, at the borders of a block of 128 keys; one tile of 16 columns and several, values up to and above 128."""
+    from peregrine_b200.layers import Attention
+
+    p, width, T = t.attention(*heads), 64, 262
+    d = device(lm, "float32", T)
+    g = rng(heads[2])
+    W = {k: t.bf16_values(v) for k, v in t.mixer_weights(g, "attention", p, width).items()}
+    x = t.bf16_values(g.standard_normal((T, width)))
+    want, _ = so.attention_mixer(x.astype(np.float64), {k: v.astype(np.float64) for k, v in W.items()}, p, 1e-4, so.attention_start(p), 0)
+    mixer = Attention(d, p, W, width, 1e-4, 300, 1)
+    for cuts in ([T], [127, 4, 1, 123, 7], [3, 126, 130, 3]):
+        got, _ = run_mixer(lm, d, mixer, width, x, cuts)
+        close(got, want, 3e-5, f"cuts {cuts}")
+    mixer.free()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("heads", [(4, 2, 32, 32, 0.5), (4, 2, 64, 64, 0.25), (8, 1, 128, 128, 0.13)])
 @pytest.mark.parametrize("far", [0, 1, 63, 64, 65, 127, 128, 300, 440, 447])
