@@ -425,7 +425,7 @@ int32_t launch(pg_ctx *ctx, const pg_linear *lin, const bf16 *planes, int64_t m,
 }
 
 // Cycles by count: blocks of the busiest CTA (695 / 1004 / 1413 cycles with 16 / 64 / 128 rows and one CTA to a tile; pairs take 0.8 of that), and what a tile
-// costs at its end, much more where parts meet.  K = N = 4096, four parts one after the other / two by two / all apart: 128 rows 50 / 42 / 32 us,
+// costs at its end, much more where parts meet.  K = N = 4096, four parts one after the other / two by two / all apart, one CTA to a tile: 128 rows 50 / 42 / 32 us,
 // 333 rows 54 / 73 / 77, 1000 rows 97 / 140 / 179.
 double f32_cost(int64_t rounds, int64_t blocks, int rows, int64_t parts, bool slabs)
 {
