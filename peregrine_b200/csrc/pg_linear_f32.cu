@@ -66,7 +66,8 @@ struct FParts {
 
 // ---- the three planes of rows row0 .. of a: planes [3][rows][K] --------------------------------------------------------
 // rt.row_pair: row r takes token row_pair[r] / top (by token), or row r.  Rows without a pair, and those behind the route's blocks, are left
-// out: nobody reads what comes of them, and rows do not touch each other.  (64 experts with a row or two each: 8192 rows of zeros took 10 us.)
+// out: nobody reads what comes of them, and rows do not touch each other.  (157 tokens, eight of 64 experts each, 1256 pairs in some 8000 rows:
+// K 2048 by token 41 -> 31 us, K 1024 by row 23 -> 17, a prompt of four layers 2266 -> 2211.)
 __global__ void __launch_bounds__(256)
     linear_split_kernel(const float *__restrict__ a, int64_t lda, int row0, int rows, int K, const PgRouted rt, uint2 *__restrict__ planes)
 {

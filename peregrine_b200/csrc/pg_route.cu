@@ -172,13 +172,16 @@ __global__ void __launch_bounds__(128)
     }
 }
 
-// count -> first row of every expert (in cursor), the experts of the row blocks, the number of row blocks; count back to 0
-__global__ void __launch_bounds__(1024) route_layout_kernel(int experts, int32_t *count, int32_t *cursor, int32_t *block_expert, int32_t *blocks)
+// count -> first row of every expert (in cursor), the experts of the row blocks, the number of row blocks; count back to 0; -1 to the rows
+// behind every expert's last pair, which else held pairs of an earlier step
+__global__ void __launch_bounds__(1024)
+    route_layout_kernel(int experts, int32_t *count, int32_t *cursor, int32_t *row_pair, int32_t *block_expert, int32_t *blocks)
 {
     __shared__ int part[32];
+    __shared__ int2 padding[RT_MAX];   // of every expert: its first row without a pair, and the end of its rows
     pg_pdl_begin();
     const int e = threadIdx.x, warp = e >> 5, lane = e & 31;
-    const int nb = e < experts ? (__ldcg(count + e) + PG_ROUTE_BLOCK - 1) / PG_ROUTE_BLOCK : 0;
+    const int pairs = e < experts ? __ldcg(count + e) : 0, nb = (pairs + PG_ROUTE_BLOCK - 1) / PG_ROUTE_BLOCK;
     int inc = nb;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -198,6 +201,10 @@ __global__ void __launch_bounds__(1024) route_layout_kernel(int experts, int32_t
         for (int i = 0; i < nb; i++) block_expert[at + i] = e;
     }
     if (e == 0) *blocks = all;
+    padding[e] = make_int2(at * PG_ROUTE_BLOCK + pairs, (at + nb) * PG_ROUTE_BLOCK);
+    __syncthreads();
+    for (int x = warp; x < experts; x += 32)
+        for (int r = padding[x].x + lane; r < padding[x].y; r += 32) row_pair[r] = -1;
 }
 
 __global__ void __launch_bounds__(256) route_place_kernel(int pairs, int experts, const int32_t *ids, int32_t *cursor, int32_t *pair_row, int32_t *row_pair)
@@ -336,7 +343,8 @@ PG_API int32_t pg_route_run(pg_ctx *ctx, pg_route *route, int32_t dtype, const f
 #undef PG_RT_SMALL
 #undef PG_RT_CHOOSE
     if (rc != PG_OK) return rc;
-    rc = launch_pdl(ctx, route_layout_kernel, dim3(1), dim3(1024), 0, (int)route->experts, route->count, route->cursor, route->block_expert, route->blocks);
+    rc = launch_pdl(ctx, route_layout_kernel, dim3(1), dim3(1024), 0, (int)route->experts, route->count, route->cursor, route->row_pair, route->block_expert,
+                    route->blocks);
     if (rc != PG_OK) return rc;
     const int64_t pairs = m * route->top;
     return launch_pdl(ctx, route_place_kernel, dim3((unsigned)((pairs + 255) / 256)), dim3(256), 0, (int)pairs, (int)route->experts,

@@ -350,14 +350,23 @@ def test_router(lm, dtype, experts, identity, top, groups):
 @pytest.mark.parametrize("width,mlp", [(96, t.moe(24, 0.8, 6, 3, 2, (3, 2))), (70, t.moe(17, 2.5, 5, 0, 3)), (320, t.moe(136, 1.1, 12, 12, 6, (6, 2))),
                                        (64, t.moe(8, 0.5, 1, 1, 2))])
 def test_experts(lm, dtype, width, mlp):
+    experts(lm, dtype, width, mlp, (1, 5, 16, 17, 290))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width,mlp", [(96, t.moe(24, 0.8, 6, 3, 2, (3, 2))), (64, t.moe(8, 0.5, 1, 1, 2))])
+def test_experts_of_smaller_steps_after_larger_ones(lm, dtype, width, mlp):
+    experts(lm, dtype, width, mlp, (290, 40, 17, 5, 30))
+
+
+def experts(lm, dtype, width, mlp, sizes):
     from peregrine_b200.layers import Batch, MoeFF
 
     d = device(lm, dtype, 290)
     g = rng(width)
     W = {k: t.bf16_values(v) for k, v in t.mlp_weights(g, mlp, width).items()}
     ff = MoeFF(d, mlp, W, width)
-    got = {}
-    for m in (1, 5, 16, 17, 290):
+    for m in sizes:
         x = t.bf16_values(g.standard_normal((m, width)))
         b = Batch(d, [(0, 0, [0] * m)])
         dx, dw, ds = d.f32(x), d.f32(np.ones(width, np.float32)), d.f32(np.ones(width, np.float32))
@@ -372,11 +381,51 @@ def test_experts(lm, dtype, width, mlp):
         lm.sync()
         want = x + so.rms_norm(so.moe_ff(x.astype(np.float64), {k: v.astype(np.float64) for k, v in W.items()}, mlp), 1.0, 1e-5)
         close(dx.cpu().numpy(), want, 1e-5 if dtype == "float32" else 5e-2, f"m {m}")
-        got[m] = dx.cpu().numpy()
         ids, w = ff.chosen(m)
         assert ids.shape == (m, mlp["router"]["top"]) and (w >= 0).all()
     assert lm.device_status() == 0
     ff.free()
+
+
+def test_rows_without_a_pair_take_no_part(lm):
+    """f32 steps of a route, each smaller than the one before: the rows behind an expert's last pair read neither pairs of the step before nor rows
+    behind the step's own.  A product of zeros in front leaves zeros where the rows are split, so that a row which is left out gives zeros."""
+    import ctypes as C
+
+    from peregrine_b200.layers import Linear, up
+
+    d = device(lm, "float32", 300)
+    E, top, k, n = 6, 2, 128, 40
+    g = rng(11)
+    w = t.bf16_values(g.standard_normal((E, n, k)) / k ** 0.5)
+    lin, other = Linear(d, d.bf16(w)), Linear(d, d.bf16(w[0]))
+    h = C.c_void_p()
+    d.check(d.lib.pg_route_create(lm.handle, 300, E, 0, top, C.byref(h)))
+    most = int(d.lib.pg_route_max_rows(h))
+    a = g.standard_normal((300, k)).astype(np.float32)
+    x, z, corr = act(d, a), d.f32(g.standard_normal((300, E)).astype(np.float32)), d.f32(np.zeros(E, np.float32))
+    nothing, y, unused = (d.torch.zeros(most, c, device=d.dev) for c in (k, n, n))
+    d.torch.cuda.synchronize()
+    for m in (300, 130, 20, 1):
+        rows = up(m * top + min(m * top, E) * 127, 128)          # of the routed product
+        d.check(d.lib.pg_route_run(lm.handle, h, d.code, z.data_ptr(), E, m, corr.data_ptr(), 1, 1))
+        other.run(nothing, rows, unused)
+        lin.run_routed(h, x, True, y)
+        ids, weights = np.zeros((m, top), np.int32), np.zeros((m, top), np.float32)
+        d.check(d.lib.pg_route_read(lm.handle, h, ids.ctypes.data, weights.ctypes.data))
+        got, at = y.cpu().numpy(), 0
+        for e in range(E):
+            want = a[np.nonzero((ids == e).any(1))[0]].astype(np.float64) @ w[e].T.astype(np.float64)
+            c, end = len(want), at + up(len(want), 128)
+            order = lambda v: v[np.argsort(v[:, 0])]                # (an expert's pairs come in any order)
+            if c:
+                close(order(got[at:at + c]), order(want), 5e-6, f"m {m} expert {e}")
+            assert (got[at + c:end] == 0).all(), f"m {m} expert {e}"
+            at = end
+    assert lm.device_status() == 0
+    d.lib.pg_route_free(lm.handle, h)
+    lin.free()
+    other.free()
 
 
 # ---- gated delta rule ------------------------------------------------------------------------------------------------
