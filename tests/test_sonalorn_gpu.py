@@ -277,6 +277,68 @@ def test_gated_products(lm, dtype, f, k):
     lin.free()
 
 
+# (rows, columns, K) whose tiles of 256 x 256 go to pairs of CTAs (from 148 tiles of 128 x 128 on): a second CTA with one row and with none, a last
+# tile of one column, ones that end in either CTA's half of the weights, several tiles to a pair, one block of K and more than there are stages
+PAIRS = [(129, 20000, 448), (300, 6400, 448), (384, 7300, 448), (1300, 20010, 64), (300, 8193, 512), (700, 4100, 1024)]
+
+
+@pytest.mark.parametrize("m,n,k", PAIRS)
+def test_bf16_product_on_pairs_of_ctas(lm, m, n, k):
+    """Element by element: an instruction adds 16 products to a sum and cuts each of the 17 off below 2^-23 of the largest.  128 rows alone take one
+    CTA to a tile (and K in parts from 512 on, whose sums are others): the same bits."""
+    from peregrine_b200.layers import Linear, up
+
+    d = device(lm, "bfloat16", 1300)
+    g = rng(m + n + k)
+    w, a = t.bf16_values(g.standard_normal((n, k), np.float32)), t.bf16_values(g.standard_normal((m, k), np.float32))
+    lin, x = Linear(d, d.bf16(w)), act(d, a)
+    a64, w64 = (d.torch.from_numpy(np.asarray(v, np.float64)).to(d.dev) for v in (a, w))
+    want, bound = a64 @ w64.T, a64.abs() @ w64.abs().T * (17 * k / 16 * 2.0 ** -23)
+    for out in ("float32", "bfloat16"):
+        y = d.torch.full((m, up(n, 8) + 8), 7.0, dtype=getattr(d.torch, out), device=d.dev)
+        parts = y.clone()
+        d.torch.cuda.synchronize()
+        lin.run(x, m, y)
+        lm.sync()
+        # (bf16 has eight significant bits: outputs are rounded to 2^-8 of themselves)
+        assert ((y[:, :n].double() - want).abs() <= bound + (want.abs() + bound) * (2.0 ** -8 if out == "bfloat16" else 0.0)).all()
+        assert (y[:, n:] == 7.0).all()
+        if k < 512:
+            for r in range(0, m - 16, 128):
+                lin.run(x[r:], min(128, m - r), parts[r:])
+            lm.sync()
+            same = m if m % 128 == 0 or m % 128 > 16 else m // 128 * 128
+            assert d.torch.equal(y[:same], parts[:same])
+    assert lm.device_status() == 0
+    lin.free()
+
+
+@pytest.mark.parametrize("m,f,k", [(300, 3200, 448), (700, 2051, 130)])
+def test_gated_bf16_product_on_pairs_of_ctas(lm, m, f, k):
+    from peregrine_b200 import _lib
+    from peregrine_b200.layers import Linear, up
+
+    d = device(lm, "bfloat16", 700)
+    g = rng(f * 7 + k)
+    gate, upw, a = (t.bf16_values(g.standard_normal((r, k)) * s / k ** 0.5) for r, s in ((f, 2), (f, 2), (m, k ** 0.5)))
+    lin, x = Linear(d, (d.bf16(gate), d.bf16(upw)), gated=True), act(d, a)
+    G, U = (a.astype(np.float64) @ b.T.astype(np.float64) for b in (gate, upw))
+    for code, limit, want in ((_lib.ACT_GELU_TANH_GLU, 0.0, so.gelu_tanh(G) * U),
+                              (_lib.ACT_CLAMPED_SWISH_GLU, 0.9, np.minimum(G, .9) * so.sigmoid(1.702 * np.minimum(G, .9)) * (np.clip(U, -.9, .9) + 1))):
+        y = d.torch.zeros(m, up(f, 64), dtype=d.act, device=d.dev)
+        parts = d.torch.zeros_like(y)
+        d.torch.cuda.synchronize()
+        lin.run(x, m, y, code, limit)
+        for r in range(0, m, 128):
+            lin.run(x[r:], min(128, m - r), parts[r:], code, limit)
+        lm.sync()
+        got = y.float().cpu().numpy()
+        close(got[:, :f], want, 1e-2 * 3, f"act {code}")      # (as in test_gated_products)
+        assert (got[:, f:] == 0.0).all() and d.torch.equal(y, parts)
+    assert lm.device_status() == 0
+    lin.free()
+
+
 # ---- residual rows ---------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("width", [5, 70, 256, 1030, 4096])
