@@ -11,7 +11,7 @@
 //                                   csrc/pg_attention_tc.cu, or attn_prompt_kernel (mma.sync) for short portions and for
 //                                   head widths that the former does not take.  Rows of a tile are (token, head of the
 //                                   group) pairs, which share the keys and values.
-//   f32                             attn_prep_kernel, then attn_f32_kernel (one CTA per token and head, FFMA)
+//   f32                             attn_prep_kernel, then attn_f32_kernel (a CTA per head and token, or up to four tokens of a sequence; FFMA)
 //
 // The sink is a score of 0 without a value: the running maximum starts at 0 and exp(-max) joins the denominator.
 #include <math.h>
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(AF_T, QT > 1 ? 4 : 8)
 {
     extern __shared__ __align__(16) float sm[];   // q[QT][dp] | p[QT][AF_T]
     __shared__ float red[QT][8];
-    __shared__ __align__(16) float tiles[AF_T * AF_KT];
+    __shared__ __align__(16) float tiles[QT > 1 ? AF_T * AF_KT : 4];
     pg_pdl_begin();
     const int h = blockIdx.x, g = h / s.rep, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int m = blockIdx.y, n = 1;                    // the CTA's rows
@@ -834,7 +834,7 @@ int32_t run_step(pg_ctx *ctx, const AttnShape &s, const pg_batch *bt, const floa
 int32_t pgk_attention_f32(pg_ctx *ctx, const AttnShape &s, const pg_batch *bt, const float *q, const float *kc, const float *vc, float *out, int64_t ldo)
 {
     PG_REQUIRE(bt->rows <= 65535, "attention: too many rows for the f32 form");
-    PG_REQUIRE(s.V <= 8 * AF_T && (s.dp + AF_T + AF_T * AF_KT) * 4 < 48 * 1024, "attention: heads too wide for the f32 form");
+    PG_REQUIRE(s.V <= 8 * AF_T && (s.dp + AF_T) * 4 < 48 * 1024, "attention: heads too wide for the f32 form");
     // (tokens of different sequences share nothing)
     if (bt->max_len > 1 && (AF_Q * (s.dp + AF_T) + AF_T * AF_KT) * 4 < 47 * 1024 && bt->rows / AF_Q + bt->seqs <= 65535)
         return launch_pdl(ctx, s.V <= AF_T ? attn_f32_kernel<AF_Q, 1> : attn_f32_kernel<AF_Q, 8>, dim3((unsigned)s.H, (unsigned)(bt->rows / AF_Q + bt->seqs)),
