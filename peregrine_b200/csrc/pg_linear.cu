@@ -72,8 +72,7 @@ PG_API int32_t pg_linear_run_routed(pg_ctx *ctx, pg_linear *lin, pg_route *route
         return pgk_linear_gemv(ctx, lin, (const bf16 *)d_a, lin->k, route->m, act, limit, d_y, y_dtype, ldy, &rt, pairs < route->experts ? pairs : route->experts);
     }
     // rows the route can have for this many tokens
-    const int64_t pairs = route->m * route->top;
-    const int64_t rows = pg_up(pairs + (pairs < route->experts ? pairs : route->experts) * (PG_ROUTE_BLOCK - 1), PG_ROUTE_BLOCK);
+    const int64_t rows = pg_route_rows(route->m * route->top, route->experts);
     PG_REQUIRE(rows <= route->max_rows, "linear: the route is larger than it was created for");
     if (dtype == PG_F32) return pgk_linear_f32(ctx, lin, (const float *)d_a, lin->k, rows, act, limit, d_y, y_dtype, ldy, &rt);
     const void *a = d_a;

@@ -37,6 +37,8 @@ struct pg_route {
 };
 
 inline int64_t pg_up(int64_t v, int64_t to) { return (v + to - 1) / to * to; }
+// most rows of the many-token form for this many pairs
+inline int64_t pg_route_rows(int64_t pairs, int64_t experts) { return pg_up(pairs + (pairs < experts ? pairs : experts) * (PG_ROUTE_BLOCK - 1), PG_ROUTE_BLOCK); }
 
 // what a routed product needs of a route
 struct PgRouted {

@@ -155,13 +155,16 @@ __global__ void __launch_bounds__(512)
     }
 }
 
+// All rows that the step can have are marked as without a pair here, beside the choice; route_place_kernel writes those that get one.  (In the
+// layout kernel, one CTA that the others wait for, it took 0.8 us a launch, 64 experts; here nothing.)
 template <int NV>
 __global__ void __launch_bounds__(128)
     route_choose_kernel(const float *__restrict__ logits, int64_t ld, int m, int experts, const float *__restrict__ correction, const Choice ch,
-                        int32_t *ids, float *weights, int32_t *count)
+                        int32_t *ids, float *weights, int32_t *count, int32_t *row_pair, int rows)
 {
     extern __shared__ uint32_t sm[];
     pg_pdl_begin();
+    for (int r = blockIdx.x * 128 + threadIdx.x; r < rows; r += gridDim.x * 128) row_pair[r] = -1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * 4 + warp;
     if (t >= m) return;
@@ -172,16 +175,13 @@ __global__ void __launch_bounds__(128)
     }
 }
 
-// count -> first row of every expert (in cursor), the experts of the row blocks, the number of row blocks; count back to 0; -1 to the rows
-// behind every expert's last pair, which else held pairs of an earlier step
-__global__ void __launch_bounds__(1024)
-    route_layout_kernel(int experts, int32_t *count, int32_t *cursor, int32_t *row_pair, int32_t *block_expert, int32_t *blocks)
+// count -> first row of every expert (in cursor), the experts of the row blocks, the number of row blocks; count back to 0
+__global__ void __launch_bounds__(1024) route_layout_kernel(int experts, int32_t *count, int32_t *cursor, int32_t *block_expert, int32_t *blocks)
 {
     __shared__ int part[32];
-    __shared__ int2 padding[RT_MAX];   // of every expert: its first row without a pair, and the end of its rows
     pg_pdl_begin();
     const int e = threadIdx.x, warp = e >> 5, lane = e & 31;
-    const int pairs = e < experts ? __ldcg(count + e) : 0, nb = (pairs + PG_ROUTE_BLOCK - 1) / PG_ROUTE_BLOCK;
+    const int nb = e < experts ? (__ldcg(count + e) + PG_ROUTE_BLOCK - 1) / PG_ROUTE_BLOCK : 0;
     int inc = nb;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -201,10 +201,6 @@ __global__ void __launch_bounds__(1024)
         for (int i = 0; i < nb; i++) block_expert[at + i] = e;
     }
     if (e == 0) *blocks = all;
-    padding[e] = make_int2(at * PG_ROUTE_BLOCK + pairs, (at + nb) * PG_ROUTE_BLOCK);
-    __syncthreads();
-    for (int x = warp; x < experts; x += 32)
-        for (int r = padding[x].x + lane; r < padding[x].y; r += 32) row_pair[r] = -1;
 }
 
 __global__ void __launch_bounds__(256) route_place_kernel(int pairs, int experts, const int32_t *ids, int32_t *cursor, int32_t *pair_row, int32_t *row_pair)
@@ -258,8 +254,8 @@ PG_API int32_t pg_route_create(pg_ctx *ctx, int64_t max_tokens, int64_t experts,
     r->experts = experts;
     r->identity = identity;
     r->top = top;
-    const int64_t pairs = max_tokens * top, used = pairs < experts ? pairs : experts;
-    r->max_rows = pg_up(pairs + used * (PG_ROUTE_BLOCK - 1), PG_ROUTE_BLOCK);
+    const int64_t pairs = max_tokens * top;
+    r->max_rows = pg_route_rows(pairs, experts);
     const int64_t nblk = r->max_rows / PG_ROUTE_SMALL;
     const int64_t words = 3 * pg_up(pairs, 32) + pg_up(r->max_rows, 32) + 2 * pg_up(experts, 32) + pg_up(nblk, 32) + 32;
     const cudaError_t e = cudaMalloc(&r->mem, (size_t)words * 4);
@@ -322,7 +318,7 @@ PG_API int32_t pg_route_run(pg_ctx *ctx, pg_route *route, int32_t dtype, const f
     } while (0)
 #define PG_RT_CHOOSE(NV)                                                                                                                                 \
     launch_pdl(ctx, route_choose_kernel<NV>, dim3((unsigned)((m + 3) / 4)), dim3(128), (size_t)4 * groups * 4, d_logits, ld, (int)m, (int)route->experts, \
-               d_correction, ch, route->ids, route->weights, route->count)
+               d_correction, ch, route->ids, route->weights, route->count, route->row_pair, (int)rows)
     if (small) {
         const size_t smem = ((size_t)16 * groups + 2 * m * route->top + route->experts) * 4;
         PG_REQUIRE(smem <= 220 * 1024, "route: too many choices for the one-CTA form");
@@ -331,6 +327,7 @@ PG_API int32_t pg_route_run(pg_ctx *ctx, pg_route *route, int32_t dtype, const f
         if (n <= 256) PG_RT_SMALL(8);
         PG_RT_SMALL(32);
     }
+    const int64_t pairs = m * route->top, rows = pg_route_rows(pairs, route->experts);
     int32_t rc;
     if (n <= 32)
         rc = PG_RT_CHOOSE(1);
@@ -343,10 +340,8 @@ PG_API int32_t pg_route_run(pg_ctx *ctx, pg_route *route, int32_t dtype, const f
 #undef PG_RT_SMALL
 #undef PG_RT_CHOOSE
     if (rc != PG_OK) return rc;
-    rc = launch_pdl(ctx, route_layout_kernel, dim3(1), dim3(1024), 0, (int)route->experts, route->count, route->cursor, route->row_pair, route->block_expert,
-                    route->blocks);
+    rc = launch_pdl(ctx, route_layout_kernel, dim3(1), dim3(1024), 0, (int)route->experts, route->count, route->cursor, route->block_expert, route->blocks);
     if (rc != PG_OK) return rc;
-    const int64_t pairs = m * route->top;
     return launch_pdl(ctx, route_place_kernel, dim3((unsigned)((pairs + 255) / 256)), dim3(256), 0, (int)pairs, (int)route->experts,
                       (const int32_t *)route->ids, route->cursor, route->pair_row, route->row_pair);
 }
