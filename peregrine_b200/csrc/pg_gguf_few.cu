@@ -7,8 +7,8 @@
 //   * The quants become f16 exactly.  A block is four m16n8k16 products (16 rows of W x 8 rows of x; two planes x two steps of 16 k, the smaller
 //     plane first) into sums of its own, which the block's f16 scale then takes to the tile's f32 sums: sum += d * block, rounded once.
 //   * A tile is 16 rows of W; `kw` warps, a slice each, share it, and 16 / kw such groups a CTA.  A warp streams its slices of its tiles through a
-//     private ring, one bulk copy of 2304 / 4352 bytes each.  The parts of a tile meet in shared memory, added in their order; the warps take
-//     turns at that.
+//     private ring, one bulk copy of 2304 / 4352 bytes each.  The parts of a tile meet in shared memory, added two by two in their order; the
+//     warps take turns at that.
 //   * K of more than 16 slices: sp CTAs take the same tiles and write raw sums to slabs; the last of them to finish (a ticket per group)
 //     adds them in their order and writes the outputs.  Nobody waits for anybody.
 //
@@ -210,13 +210,18 @@ __global__ void __launch_bounds__(GF_THREADS, 1)
             const bool my_turn = turn == kp;
             if (++turn == kw) turn = 0;
             if (!my_turn) continue;
-            sum = cells[0];
-            for (int p = 1; p < kw; p++) {
-                const float4 v = cells[p * 32];
-                sum.x += v.x;
-                sum.y += v.y;
-                sum.z += v.z;
-                sum.w += v.w;
+            // (two by two: half the roundings on the way.  N 14336, K 4096: error 1.16e-7 -> 1.06e-7, and 18.6 -> 18.2 us of Q4_0, 19.0 -> 18.4 of Q8_0
+            // with eight rows, since the loop needs no registers of its own)
+            sum = make_float4(0.f, 0.f, 0.f, 0.f);
+            int p = kw & 1;
+            if (p) sum = cells[0];
+#pragma unroll 2
+            for (; p < kw; p += 2) {
+                const float4 v = cells[p * 32], u = cells[p * 32 + 32];
+                sum.x += v.x + u.x;
+                sum.y += v.y + u.y;
+                sum.z += v.z + u.z;
+                sum.w += v.w + u.w;
             }
         }
         if (sp > 1)
@@ -258,15 +263,22 @@ __global__ void __launch_bounds__(GF_THREADS, 1)
     }
 }
 
-// CTAs that share K, and warps that share a tile: the fewest rounds of tiles, where meeting in slabs counts as three
+// CTAs that share K, and warps that share a tile, by 10 ns: a round of tiles takes longer the more warps convert at once; slabs cost a fixed part and
+// what the last CTA of a group does at the end, sixteen tiles at a time, sp parts of each.  (By rounds alone, slabs as three of them, K 5632 went to
+// eleven CTAs of two warps: Q4_0, N 16000 / 28672 / 49152 30.9 / 50.6 / 82.5 us, with three of eight 26.8 / 42.0 / 66.0; K 2304, N 49152 38.0 against
+// 31.6, K 4352, N 28672 37.5 against 35.6.)
 void gf_plan(const pg_ctx *ctx, const pg_gguf_weight *w, int *sp, int *kw)
 {
     const int64_t nslices = w->k / 256, tiles = (w->n + 15) / 16;
     int64_t best = 0;
     for (int64_t parts = (nslices + GF_WARPS - 1) / GF_WARPS; parts <= std::min<int64_t>(nslices, 16); parts++) {
-        const int64_t each = (nslices + parts - 1) / parts, slots = ctx->sm_count / parts * (GF_WARPS / each);
+        const int64_t each = (nslices + parts - 1) / parts, groups = GF_WARPS / each, slots = ctx->sm_count / parts * groups;
         if ((parts - 1) * each >= nslices) continue;
-        const int64_t cost = (tiles + slots - 1) / slots + (parts > 1 ? 3 : 0);
+        int64_t cost = (tiles + slots - 1) / slots * (80 + 7 * groups * each);
+        if (parts > 1) {
+            const int64_t units = std::min<int64_t>(ctx->sm_count / parts, (tiles + groups - 1) / groups), mine = (tiles + units - 1) / units;
+            cost += 250 + (mine + GF_WARPS - 1) / GF_WARPS * 14 * parts;
+        }
         if (best == 0 || cost < best) {
             best = cost;
             *sp = (int)parts;
