@@ -304,19 +304,29 @@ int32_t gf_launch(pg_ctx *ctx, const float *d_x, int M, const pg_gguf_weight *w,
 }  // namespace
 
 // Where the streaming form walks K in more than one chunk (it holds 16384 elements of x in all, rows rounded up to 1, 2, 4 or 8), and with four
-// rows on narrow layers.  Two rows only up to 2^25 elements of W: a second chunk costs them less there than the conversions do here.  us, streaming
-// form or tensor cores with TMEM (whichever was taken) / this:
+// rows on narrow layers.  One and two rows only up to 2^25 elements of W: a second chunk costs them less there than the conversions do here.
+// With few chunks the streaming form catches up on very wide layers, where its starts weigh least: the line lies between the 49152 columns
+// at which they are level or this is ahead, and 65536.  us, streaming form or tensor cores with TMEM (whichever was taken) / this (2 to 3 % more than
+// since the parts of a tile are added two by two):
 //   Q4_0     K 4096, N 14336: 4 rows 15.6 / 17.6, 5 18.8 / 18.0, 8 21.4 / 18.5   N 28672: 5 rows 29.9 / 29.9, 8 32.1 / 30.1
+//            N 43008: 5 rows 44.0 / 40.7, 8 46.8 / 41.6   N 65536: 5 rows 55.0 / 57.9, 8 57.6 / 58.3   N 128256: 5 rows 97.9 / 105.0, 8 100.8 / 107.9
 //            K 4096, N 4096: 3 rows 7.4 / 7.4, 4 8.2 / 7.7, 5 11.1 / 7.9, 8 12.1 / 8.4   N 1024: 4 rows 6.2 / 4.9, 8 9.8 / 5.7
+//            K 6144, N 32768: 3 rows 45.7 / 46.5, 8 53.8 / 48.1   N 65536: 3 rows 74.2 / 84.5, 8 85.3 / 86.5
+//            K 8192, N 28672: 3 rows 54.2 / 53.9, 8 66.3 / 55.4   N 65536: 3 rows 94.9 / 110.1, 8 112.1 / 111.1 (four chunks)
 //            K 14336, N 4096: 2 rows 17.9 / 19.7, 3 24.2 / 19.7, 8 25.5 / 20.7   K 9984, N 2490: 2 rows 13.6 / 11.0, 8 16.8 / 12.0
+//            K 16640: N 1024, 1 row 12.3 / 8.7, N 4096, 1 row 17.1 / 21.2   K 32768: N 1024, 1 row 17.9 / 13.4, N 4096, 1 row 26.4 / 35.1
 //            K 2048, N 12288: 4 rows 9.6 / 9.6, 8 10.3 / 10.4   N 128256: 8 rows 50.6 / 57.7   K 8192, N 8192: 2 rows 13.3 / 20.2, 3 20.9 / 20.4
-//   Q8_0     K 4096, N 14336: 4 rows 16.6 / 18.2, 5 19.5 / 18.2, 8 21.0 / 19.0   K 14336, N 4096: 2 rows 19.0 / 19.5, 8 26.2 / 20.7
+//   Q8_0     K 4096, N 14336: 4 rows 16.6 / 18.2, 5 19.5 / 18.2, 8 21.0 / 19.0   N 65536: 5 rows 56.8 / 54.8   N 128256: 5 rows 102.2 / 99.3
+//            K 8192, N 65536: 3 rows 96.1 / 103.6, 8 113.9 / 105.0   K 14336, N 4096: 2 rows 19.0 / 19.5, 8 26.2 / 20.7
+// (Below the line some shapes of Q4_0 are up to 1.1 times as slow here, three rows at K 4352, N 28672 most, 31.0 / 33.8; their error is a third of
+// the streaming form's, a tenth where channels stand out.)
 bool pgk_matmul_gguf_few_supports(const pg_ctx *ctx, const pg_gguf_weight *w, int64_t m)
 {
     if (!(w->tiled && m >= 1 && m <= 8 && w->k <= 256 * GF_WARPS * 16)) return false;
-    const int64_t rows = m > 4 ? 8 : m > 2 ? 4 : m;
-    if (w->k * rows > 16384) return m > 2 || w->n * w->k <= 1ll << 25;
-    return m == 4 && w->n <= 32ll * ctx->sm_count;
+    const int64_t rows = m > 4 ? 8 : m > 2 ? 4 : m, chunks = (w->k * rows + 16383) / 16384;
+    if (chunks < 2) return m == 4 && w->n <= 32ll * ctx->sm_count;
+    if (m <= 2) return w->n * w->k <= 1ll << 25;
+    return w->n <= 57344 || chunks >= (rows == 8 ? 4 : 3) || (rows == 8 && w->type == PG_GGUF_Q8_0);
 }
 
 // *taken = false: no workspace for the parts of K to be had (while a graph is recorded, or out of memory); nothing has been launched

@@ -253,6 +253,25 @@ def test_matmul_gguf_few_rows(pg, gpu, oracle_mt, kind, m, n, k):
     w.free()
 
 
+@pytest.mark.parametrize("kind", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("m,n,k", [(8, 57344, 2304), (8, 57361, 2304), (5, 57361, 4096), (3, 57344, 4352), (3, 57361, 4352), (4, 16001, 5632), (7, 9000, 7168),
+                                   (6, 4097, 6400), (3, 30000, 12544)])
+def test_matmul_gguf_few_rows_of_wide_layers(pg, gpu, oracle_mt, kind, m, n, k):
+    """On both sides of the number of columns from which the streaming form takes few chunks of K, and the ways of dividing K below it: several CTAs
+    with one and with several groups of warps, idle warps, many tiles to a group.  The matrix repeats 239 columns; the bound of the digits of the
+    streaming form, which is the wider one (above)."""
+    g = rng(n + k + m)
+    raw = oracle_mt.encode(kind, normal(g, (239, k), 0.02))
+    few = oracle_mt.dequant(kind, raw, 239 * k).reshape(239, k).astype(np.float64)
+    w = pg.gguf.GgufWeight(kind, raw.reshape(239, -1)[np.arange(n) % 239], n, k, gpu)
+    x = normal(g, (m, k))
+    x64 = np.abs(x).astype(np.float64)
+    bound = x64 @ np.abs(few).T * (2.0 ** -22 + 4 * 2.0 ** -23 + (k // 32 + 18) * 2.0 ** -24) + x64.max(1, keepdims=True) * 2.0 ** -22 * np.abs(few).sum(1)
+    error = np.abs(w.matmul(x, m) - (x.astype(np.float64) @ few.T)[:, np.arange(n) % 239])
+    assert (error <= bound[:, np.arange(n) % 239]).all() and gpu.device_status() == 0
+    w.free()
+
+
 def test_matmul_gguf_many_rows_recorded_without_a_run_before(pg, oracle_mt):
     """The workspace cannot grow in a recording: the rows then go through what the upload has reserved, in portions, with the same
     results."""
