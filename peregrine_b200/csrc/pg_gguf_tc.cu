@@ -922,19 +922,18 @@ int32_t gt_run(pg_ctx *ctx, const pg_gguf_weight *w, const void *planes, const f
 
 }  // namespace
 
-// From nine rows on, and for fewer -- where csrc/pg_gguf_few.cu finds no workspace or K is beyond it -- where the streaming form walks K in several
-// chunks (it has room for 16384 elements of x in all),
-// each with its own start: from four chunks on, from three on narrow layers, and from two with seven and eight rows there.  Q4_0, us,
-// streaming / this: K 14336, N 4096 at 2 / 3 / 5 / 8 rows 18.5 / 28.4 / 40.7 / 48.7 against 25.7 / 26.2 / 26.7 / 27.7; K 8192, N 8192 at 4 / 5 / 8
-// rows 23.3 / 29.4 / 34.2 against 28.2 / 28.3 / 28.9; K 6144, at 5 rows: N 4096 17.3 / 15.1, N 12000 29.7 / 32.9; K 4096, at 8 rows: N 4096
-// 13.9 / 12.4, N 14336 21.9 / 25.3.
+// From nine rows on.  For fewer only what csrc/pg_gguf_few.cu leaves -- one and two rows of large layers, K beyond 65536, parts of K without a
+// workspace (a recording) -- and of that what the streaming form walks in four chunks of K and more (it has room for 16384 elements of x in
+// all), or three on narrow layers.  Q4_0, us, streaming / this: K 14336, N 4096 at 3 / 5 / 8 rows 28.1 / 41.0 / 48.8 against 24.2 / 24.7 / 25.5; K 6144,
+// N 4096 at 5 rows 17.3 / 15.1; K 8192, N 8192 at 5 / 8 rows 28.3 / 32.9 against 25.6 / 26.6, N 28672 62.0 / 66.3 against 81.5 / 82.6.  (One and two rows
+// of K 32768 and 65536, N 4096, are slower here: two rows 39.3 / 79.2 against 48.1 / 87.1; their error is a quarter where channels stand out.)
 bool pgk_matmul_gguf_tc_supports(const pg_ctx *ctx, const pg_gguf_weight *w, int64_t m)
 {
     if (!(w->tiled && m >= 1 && m < (1 << 24) && w->n >= 1 && w->n < (1ll << 30))) return false;
     if (m > 8) return true;
     const int64_t rows = m > 4 ? 8 : m > 2 ? 4 : m, chunks = (w->k * rows + 16383) / 16384;
     const bool narrow = w->n <= 32ll * ctx->sm_count;
-    return chunks >= 4 || (narrow && (chunks == 3 || (chunks == 2 && m > 6)));
+    return chunks >= 4 || (narrow && chunks == 3);
 }
 
 int32_t pgk_gguf_tc_reserve(pg_ctx *ctx, int64_t k)
