@@ -282,9 +282,11 @@ static int32_t gemm_dispatch(pg_ctx *ctx, const int8_t *d_a, const float *d_as, 
             return pgk_gemm_i8_wstream(ctx, d_a, d_as, m, k, w->d_data_i8_t, w->d_scales, n, d_y, d_acc);
         case PG_ALGO_AUTO:
             // Up to sixteen rows the streaming kernel, but from 20 MB of weights on the tensor-core kernel where the former does not
-            // fill the GPU.  Quantiser and product, us, streaming / tensor cores: K 4096, N 14336 at 8 rows 14.05 / 14.15, at 9 15.6 / 14.2,
-            // at 16 15.9 / 14.5; N 10000 at 1 row 12.4 / 11.4, at 16 14.8 / 11.9; K 14336, N 4096 at 16 18.5 / 16.5; K 12800, N 10000 at 16
-            // 65.7 / 28.7; K 4096, N 4096 (17 MB) at 16 7.6 / 8.2.
+            // fill the GPU.  Quantiser and product, us, streaming / tensor cores: K 4096, N 14336 at 9 rows 15.5 / 12.8, at 16 15.7 / 12.9;
+            // N 10000 at 1 row 12.4 / 11.1, at 16 14.4 / 11.5; K 14336, N 4096 at 16 18.3 / 14.9; K 12800, N 10000 at 16 64.2 / 27.0;
+            // K 4096, N 4096 (17 MB) at 1 6.2 / 7.2, at 16 7.8 / 8.4.  (The line was drawn when one thread asked for all copies of the
+            // latter kernel.  With two it is the faster one also on layers that the former fills, from some 50 MB on: K 4096, N 14336 at
+            // 1 / 8 rows 13.2 / 13.6 against 12.5 / 12.8, K 16384, N 16384 at 1 49.0 / 47.1; below, K 5120, N 8192 at 1 10.5 / 11.2.)
             if (aligned && m <= 16 && k * n >= 20000000 && !pgk_gemm_i8_wstream_fills(ctx, m, k, n) && pgk_gemm_i8_mid_supports(ctx, m, k, n))
                 return pgk_gemm_i8_mid(ctx, d_a, d_as, m, k, w, d_y, d_acc);
             if (aligned && pgk_gemm_i8_wstream_supports(m, k, n))

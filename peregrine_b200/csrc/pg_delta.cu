@@ -7,7 +7,8 @@
 //
 //   one token per sequence   delta_step_kernel: convolution, unit norms, gates, the state update and the gated output
 //                            norm of one (head, sequence) in one CTA; the state is read and written once
-//   longer portions          delta_prep_kernel (convolution, unit norms, gates; a CTA per four tokens), delta_scan_kernel
+//   longer portions          delta_prep_kernel (convolution, unit norms, gates; a CTA per four tokens, or several with a part of
+//                            the heads each), delta_scan_kernel
 //                            (the recurrence, four tokens at a time: their read-outs come from the state the first of them
 //                            finds, corrected by the pairs' products k_a . k_b and q_a . k_b, so that one round of
 //                            reductions serves four tokens; a warp holds eight columns of a head's state in registers),

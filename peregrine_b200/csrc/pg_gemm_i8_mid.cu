@@ -55,10 +55,10 @@ __device__ __forceinline__ void md_settle()
 
 // TWO: a copy costs the thread that asks for it 230 cycles, so in a long part of K x has a thread of its own.  It starts later than one thread
 // for both does, which a short part does not make up for; the line lies between the 16 and the 28 k-blocks measured.  us, one thread / two:
-//   32 k-blocks a part (K 4096, N 14336), 12 / 17 / 40 / 100 rows  14.4 / 14.7 / 16.0 / 19.6   13.4 / 13.5 / 14.7 / 19.1
-//   28 (K 14336, N 4096)                                           16.1 / 16.7 / 18.7 / 20.0   15.3 / 15.8 / 17.3 / 19.3
-//   16 (K 4096, N 6144)                                             8.9 /  9.3 /  9.8 / 12.2    9.4 /  9.6 /  9.9 / 12.1
-//    8 (K 4096, N 4096), 17 / 40 / 64 rows                                 7.8 /  8.4 /  9.0           8.3 /  8.8 /  9.3
+//   32 k-blocks a part (K 4096, N 14336), 12 / 17 / 40 rows   14.4 / 14.7 / 16.0          13.4 / 13.5 / 14.7
+//   28 (K 14336, N 4096), 12 / 17 / 40 / 100 rows             16.1 / 16.7 / 18.7 / 20.0   15.3 / 15.8 / 17.3 / 19.3
+//   16 (K 4096, N 6144), 12 / 17 / 40 / 100 rows               8.9 /  9.3 /  9.8 / 12.2    9.4 /  9.6 /  9.9 / 12.1
+//    8 (K 4096, N 4096), 17 / 40 / 64 rows                     7.8 /  8.4 /  9.0           8.3 /  8.8 /  9.3
 template <bool TWO>
 __global__ void __launch_bounds__(MD_THREADS, 1)
     gemm_i8_mid_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const float *__restrict__ a_scales,
@@ -273,8 +273,10 @@ int32_t md_clusters(pg_ctx *ctx, int parts, int *fit)
 
 bool pgk_gemm_i8_mid_supports(pg_ctx *ctx, int64_t m, int64_t k, int64_t n)
 {
-    // (where every tile keeps its whole K, the epilogue's way through shared memory costs more than the other kernel's from about 100
-    // rows: K 4096, N 14336, 96 / 128 rows 15.9 / 17.1 us against 16.3 / 16.5)
+    // (where every tile keeps its whole K, the epilogue's way through shared memory costs more than the other kernel's from some number of
+    // rows on.  With quantiser, this / the other, us: K 4096, N 14336, 96 / 112 / 128 rows 16.2 / 17.5 / 18.7 against 18.2 / 18.5 / 18.7; K 2048,
+    // N 16384 13.5 / 14.5 / 15.7 against 13.5 / 14.1 / 14.2.  The line is that of one thread for the copies on either side; on long K it would
+    // lie behind 128 rows now: K 8192, N 12288, 100 rows 26.2 / 39.1)
     const int64_t tiles = (n + MD_N - 1) / MD_N;
     return m >= 1 && m <= 128 && n >= 1 && k >= 16 && k % 16 == 0 && k < (1ll << 31) && tiles <= ctx->sm_count && (m <= 96 || 2 * tiles <= ctx->sm_count);
 }

@@ -585,9 +585,13 @@ int32_t pgk_gemm_i8_tcgen05(pg_ctx *ctx, const int8_t *d_a, const float *d_as, i
     int bn = 64;
     if (tiles_m * ((n + 127) / 128) >= ctx->sm_count) bn = 128;
     if (tiles_m * ((n + 255) / 256) >= ctx->sm_count) bn = 256;
-    // One row of tiles (M <= 128): the MMAs are not what bounds the kernel then.  Measured at M = 64, a k-block (128
-    // bytes per column) takes a CTA 280 / 325 / 480 / 680 ns at 32 / 64 / 128 / 256 columns, whatever K and N are:
-    // about 1.8 ns x (128 + columns).  Take the tile width with the smallest waves x time-per-k-block (N 14336: one
+    // One row of tiles (M <= 128): the MMAs are not what bounds the kernel then.  Measured at M = 64 when one thread asked
+    // for both copies, a k-block (128 bytes per column) took a CTA 280 / 325 / 480 / 680 ns at 32 / 64 / 128 / 256 columns,
+    // whatever K and N are: about 1.8 ns x (128 + columns), which the model still goes by.  (With a thread for each it takes
+    // 240 / 240 / 240 / 320; 17 and 128 rows 231 ... 271 up to 128 columns, 319 and 368 at 256.  What the model chooses is the
+    // best width at K 4096, N 14336 and 20480 and up to 64 rows everywhere; from 65 rows on 256 columns where 128 are faster:
+    // us, 100 rows, K 4096, N 28672 33.4 / 31.9, N 128256 103.4 / 96.5, K 2048, N 32768 23.7 / 20.6.)
+    // Take the tile width with the smallest waves x time-per-k-block (N 14336: one
     // wave of 128-column tiles, 18.5 us, against 23.8 us for two waves of 64-column tiles; N 4096: 32-column tiles;
     // N 6144: 64-column tiles), and the smallest A tile that holds M rows (a deeper ring: 102 -> 92 us at N 128256,
     // 22.7 -> 18.6 us at M 17, N 14336; no change at M 64, N 14336).

@@ -30,8 +30,11 @@
 // What bounds it: the epilogue's chain per block -- barrier, some 100 cycles to read 32 columns of TMEM, back to the products -- at two or
 // three accumulators in flight; at MT = 160 a block takes 685 cycles, 320 of them products.  Waits by the whole warp that end in one
 // vote (pg_mbar_wait_warp) took a third off it.  Q4_0, N 14336, K 4096, us, 9 / 16 / 33 / 64 / 128 / 300 / 512 rows: 25 / 26 / 37 / 37 / 47 / 100 / 160
-// (33 rows and more with the quants in shared memory and two warps per quarter: 39 / 42 / 53 / 126 / 194).  Error against 64 bits 2e-7 ... 3e-7 with 1 %
-// of the channels x 20 (1.2e-6).  At eight rows and K 4096 the streaming form is the faster one (21 against 25 us).
+// (33 rows and more with the quants in shared memory and two warps per quarter: 39 / 42 / 53 / 126 / 194).
+// Error against 64 bits (2-norm, of either type, plain inputs or 1 % of the channels x 20), which follows from the longest chain of rounded
+// sums, by rows 9 ... 32 / 33 ... 64 / 128 / 300: N 14336, K 4096 2.9e-7 / 1.6e-7 / 2.1e-7 / 2.1e-7; N 4096, K 14336 2.8e-7 / 1.6e-7 / 2.1e-7 /
+// 2.8e-7; N 4096, K 1024 0.9e-7 / 0.9e-7 / 1.0e-7 / 1.2e-7.  (Tiles of 64 rows with an accumulator to each plane and one chain of sums: 2.9e-7,
+// 2.8e-7, 0.9e-7.  N 4096, K 1024 with K in four and two parts, as the form before took it at 128 and 300 rows: 0.95e-7, 1.03e-7.)
 // Every mbarrier wait is bounded (pg_async.cuh).
 #include <algorithm>
 
