@@ -9,7 +9,7 @@
 //   * A tile is 16 rows of W; `kw` warps, a slice each, share it, and 16 / kw such groups a CTA.  A warp streams its slices of its tiles through a
 //     private ring, one bulk copy of 2304 / 4352 bytes each.  The parts of a tile meet in shared memory, added two by two in their order; the
 //     warps take turns at that.
-//   * K of more than 16 slices: sp CTAs take the same tiles and write raw sums to slabs; the last of them to finish (a ticket per group)
+//   * K of more than 16 slices, and of fewer where gf_plan has it so: sp CTAs take the same tiles and write raw sums to slabs; the last of them to finish (a ticket per group)
 //     adds them in their order and writes the outputs.  Nobody waits for anybody.
 //
 // Why beside the streaming form: that one takes three int8 products per block and joins their digits in integer arithmetic, and its digit
